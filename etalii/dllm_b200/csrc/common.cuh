@@ -8,6 +8,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #define DLLM_OK 0
 #define DLLM_BAD_ARGUMENT (-1)
 #define DLLM_UNSUPPORTED_SIZE (-2)
@@ -54,6 +56,18 @@ static inline int dllm_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   config.attrs = attribute;
   config.numAttrs = dllm_pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, KArgs(args)...) == cudaSuccess ? DLLM_OK : DLLM_LAUNCH_FAILED;
+}
+
+// Lets a kernel have `bytes` of dynamic shared memory, asked for once per device (`done`: one bit per device, the
+// caller's static; a device beyond the 64th asks every time).
+static inline bool dllm_allow_shared(const void* kernel, int bytes, std::atomic<unsigned long long>& done) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return false;
+  unsigned long long bit = device < 64 ? 1ull << device : 0;
+  if (done.load(std::memory_order_acquire) & bit) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  done.fetch_or(bit, std::memory_order_release);
+  return true;
 }
 
 __device__ __forceinline__ float to_float(float v) { return v; }

@@ -120,10 +120,15 @@ __global__ void __launch_bounds__(LTHREADS) gemm_f32_large_kernel(void* __restri
   }
 }
 
-// ---- and for a few rows (decode steps): 32 columns a block, the reduction streamed through three stages -------------
-// A thread owns one column and four rows; W and A tiles of 32 values of k arrive by cp.async. Again one chain of
-// fused multiply-adds per output over k ascending from zero: a token's bits are the ones it gets in a long prompt.
-constexpr int SN = 32, SK = 32, SM_ROWS = 16, STHREADS = 128, SSTAGES = 3, SLD = SK + 4;
+// ---- and for a few rows (decode steps): the reduction streamed through a ring of stages -----------------------------
+// One chain of fused multiply-adds per output over k ascending from zero, as above: a token's bits are the ones it gets
+// in a long prompt. So a product cannot be faster than its K dependent multiply-adds (four cycles each: 3.1 us for
+// K = 1536), and the split is made to come close to that: a block takes COLS columns, few enough that the columns
+// spread over the whole device, a thread PER rows of one column, and W and A arrive by cp.async STAGES - 1 stages of
+// DEPTH values ahead of the chain. W's first stages are asked for before the kernel in front has finished.
+// Eight rows, 576 columns: K = 576 12.0 -> 3.3 us, K = 1536 27.5 -> 6.1 us (before: 32 columns a block, three stages of
+// 32 values, which was 18 blocks for the device and a round trip to L2 every other stage); 49152 x 576 52 -> 28.5 us.
+constexpr int SM_ROWS = 16;
 
 __device__ __forceinline__ void cp_async_f4(float* smem, const float* gmem, bool ok) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -131,59 +136,122 @@ __device__ __forceinline__ void cp_async_f4(float* smem, const float* gmem, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(STHREADS) gemm_f32_small_kernel(void* __restrict__ c, const float* __restrict__ a,
-                                                                  const float* __restrict__ w, int M, int N, int K) {
-  __shared__ __align__(16) float w_s[SSTAGES][SN][SLD];
-  __shared__ __align__(16) float a_s[SSTAGES][SM_ROWS][SLD];
-  int tid = threadIdx.x, col = tid & 31, rows0 = (tid >> 5) * 4;
-  int n0 = blockIdx.x * SN;
-  int tiles = (K + SK - 1) / SK;
-  auto issue = [&](int t) {
-    if (t < tiles) {
-      int buf = t % SSTAGES, k0 = t * SK;
-      for (int i = tid; i < (SN + SM_ROWS) * (SK / 4); i += STHREADS) {
-        int r = i / (SK / 4), k = (i % (SK / 4)) * 4;
-        if (r < SN) {
-          bool ok = n0 + r < N && k0 + k < K;
-          cp_async_f4(&w_s[buf][r][k], ok ? w + (size_t)(n0 + r) * K + k0 + k : w, ok);
-        } else {
-          int m = r - SN;
-          bool ok = m < M && k0 + k < K;
-          cp_async_f4(&a_s[buf][m][k], ok ? a + (size_t)m * K + k0 + k : a, ok);
-        }
-      }
+template <int EPI, int COLS, int ROWS, int PER, int DEPTH, int STAGES>
+__global__ void __launch_bounds__(COLS * ROWS / PER) gemm_f32_small_kernel(void* __restrict__ c, const float* __restrict__ a,
+                                                                           const float* __restrict__ w, int M, int N,
+                                                                           int K) {
+  constexpr int T = COLS * ROWS / PER, LD = DEPTH + 4, PIECES = DEPTH / 4, STAGE = (COLS + ROWS) * LD;
+  static_assert(T % 32 == 0 && (COLS * PIECES) % T == 0 && (ROWS * PIECES) % T == 0 && COLS % 2 == 0, "whole warps and copies");
+  extern __shared__ __align__(16) float ring[];  // [STAGES][COLS of W, then ROWS of A][LD]
+  int tid = threadIdx.x, col = tid % COLS, row0 = tid / COLS;  // rows row0 + i * (ROWS / PER)
+  int n0 = blockIdx.x * COLS;
+  int tiles = (K + DEPTH - 1) / DEPTH;
+  pdl_launch_dependents();
+  auto ask_w = [&](int t) {
+    float* stage = ring + (t % STAGES) * STAGE;
+#pragma unroll
+    for (int i = 0; i < COLS * PIECES / T; ++i) {
+      int at = tid + i * T, r = at / PIECES, k = (at % PIECES) * 4;
+      bool ok = n0 + r < N && t * DEPTH + k < K;
+      cp_async_f4(stage + r * LD + k, ok ? w + (size_t)(n0 + r) * K + t * DEPTH + k : w, ok);
     }
-    asm volatile("cp.async.commit_group;\n" ::);
   };
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  issue(0);
-  issue(1);
+  auto ask_a = [&](int t) {
+    float* stage = ring + (t % STAGES) * STAGE + COLS * LD;
+#pragma unroll
+    for (int i = 0; i < ROWS * PIECES / T; ++i) {
+      int at = tid + i * T, r = at / PIECES, k = (at % PIECES) * 4;
+      bool ok = r < M && t * DEPTH + k < K;
+      cp_async_f4(stage + r * LD + k, ok ? a + (size_t)r * K + t * DEPTH + k : a, ok);
+    }
+  };
+  auto close = [] { asm volatile("cp.async.commit_group;\n" ::); };
+  for (int t = 0; t < min(tiles, STAGES - 1); ++t) ask_w(t);
+  pdl_wait();
+  for (int t = 0; t < STAGES - 1; ++t) {
+    if (t < tiles) ask_a(t);
+    close();
+  }
+  float acc[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
   for (int t = 0; t < tiles; ++t) {
-    issue(t + 2);
-    asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-    __syncthreads();
-    int buf = t % SSTAGES;
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // (this stage has arrived for everybody, and everybody is done with the one before it)
+    if (t + STAGES - 1 < tiles) {
+      ask_w(t + STAGES - 1);
+      ask_a(t + STAGES - 1);
+    }
+    close();
+    const float* stage = ring + (t % STAGES) * STAGE;
+    const float* mine = stage + col * LD;
+    const float* rows = stage + (COLS + row0) * LD;
+    // (the values of the next GROUP pieces are on their way from shared memory while these are multiplied; the chains of
+    // a thread go side by side, since a warp issues in order)
+    constexpr int GROUP = PER == 1 ? 4 : 2;
+    float4 wv[2][GROUP], av[2][GROUP][PER];
+    auto load = [&](int slot, int k) {
 #pragma unroll
-    for (int k = 0; k < SK; k += 4) {
-      float4 wv = *(const float4*)&w_s[buf][col][k];
+      for (int g = 0; g < GROUP; ++g) {
+        wv[slot][g] = *(const float4*)(mine + k + 4 * g);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float4 av = *(const float4*)&a_s[buf][rows0 + i][k];
-        acc[i] = fmaf(av.x, wv.x, acc[i]);
-        acc[i] = fmaf(av.y, wv.y, acc[i]);
-        acc[i] = fmaf(av.z, wv.z, acc[i]);
-        acc[i] = fmaf(av.w, wv.w, acc[i]);
+        for (int i = 0; i < PER; ++i) av[slot][g][i] = *(const float4*)(rows + i * (ROWS / PER) * LD + k + 4 * g);
+      }
+    };
+    load(0, 0);
+#pragma unroll
+    for (int k = 0; k < DEPTH; k += 4 * GROUP) {
+      int slot = (k / (4 * GROUP)) & 1;
+      if (k + 4 * GROUP < DEPTH) load(slot ^ 1, k + 4 * GROUP);
+#pragma unroll
+      for (int g = 0; g < GROUP; ++g) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] = fmaf(av[slot][g][i].x, wv[slot][g].x, acc[i]);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] = fmaf(av[slot][g][i].y, wv[slot][g].y, acc[i]);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] = fmaf(av[slot][g][i].z, wv[slot][g].z, acc[i]);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] = fmaf(av[slot][g][i].w, wv[slot][g].w, acc[i]);
       }
     }
-    __syncthreads();  // the stage is free for the copy after next
   }
   // pairs of columns are stored by the even lane (the SwiGLU epilogue needs gate and up together)
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < PER; ++i) {
     float other = __shfl_down_sync(0xffffffffu, acc[i], 1);
-    if (!(col & 1)) epilogue_pair<EPI, float>(c, rows0 + i, n0 + col, M, N, acc[i], other);
+    if (!(col & 1)) epilogue_pair<EPI, float>(c, row0 + i * (ROWS / PER), n0 + col, M, N, acc[i], other);
   }
+}
+
+template <int EPI, int COLS, int ROWS, int PER, int DEPTH, int STAGES>
+int launch_small(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_f32_small_kernel<EPI, COLS, ROWS, PER, DEPTH, STAGES>;
+  constexpr int smem = STAGES * (COLS + ROWS) * (DEPTH + 4) * (int)sizeof(float);
+  static std::atomic<unsigned long long> allowed{0};
+  if (!dllm_allow_shared((const void*)kernel, smem, allowed)) return DLLM_LAUNCH_FAILED;
+  return dllm_launch_pdl(kernel, dim3((N + COLS - 1) / COLS), dim3(COLS * ROWS / PER), smem, stream, c, a, w, M, N, K);
+}
+
+// How the columns are split, by what was fastest with eight rows (all of it bounded by latency, so by how the columns
+// spread and how many chains a thread keeps going, not by the bytes):
+//   up to 1,184 columns   8 a block: 148 blocks and more (576 x 1536: 6.1 us; four columns 6.5, sixteen 9.0 to 11.5);
+//   up to 4,736           16 a block, two rows a thread, ten short stages (3072 x 576: 5.8 us; 8 columns 8.3, 32 6.7);
+//   up to 18,944          16 a block, four rows a thread (8192 x 2048: 25 us; two rows 30 to 35, 32 columns 27 to 35);
+//   more                  64 a block, eight rows a thread, which reads shared memory least (49152 x 576: 28.5 us, 4.0 TB/s;
+//                         16 columns 40, 32 columns 32).
+template <int EPI, int ROWS>
+int launch_small_by_columns(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  if (N <= 8 * 148) return launch_small<EPI, 8, ROWS, ROWS / 8, 128, 6>(c, a, w, M, N, K, stream);
+  if (N <= 32 * 148) return launch_small<EPI, 16, ROWS, 2, 64, 10>(c, a, w, M, N, K, stream);
+  if (N <= 128 * 148) return launch_small<EPI, 16, ROWS, 4, 128, 4>(c, a, w, M, N, K, stream);
+  return launch_small<EPI, 64, ROWS, 8, 64, 3>(c, a, w, M, N, K, stream);
+}
+
+template <int EPI>
+int launch_small_by_rows(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  return M <= 8 ? launch_small_by_columns<EPI, 8>(c, a, w, M, N, K, stream)
+                : launch_small_by_columns<EPI, 16>(c, a, w, M, N, K, stream);
 }
 }  // namespace
 
@@ -203,8 +271,11 @@ DLLM_EXPORT int dllm_gemm_f32(void* c, const float* a, const float* w, int M, in
     default: KERNEL<EPI_SWIGLU><<<GRID, THREADS_, 0, stream>>>(c, a, w, M, N, K); break;               \
   }
   if (M <= SM_ROWS) {
-    dim3 grid((N + SN - 1) / SN);
-    DLLM_BY_EPILOGUE(gemm_f32_small_kernel, grid, STHREADS)
+    switch (epilogue) {
+      case EPI_STORE_F32: return launch_small_by_rows<EPI_STORE_F32>(c, a, w, M, N, K, stream);
+      case EPI_RESIDUAL: return launch_small_by_rows<EPI_RESIDUAL>(c, a, w, M, N, K, stream);
+      default: return launch_small_by_rows<EPI_SWIGLU>(c, a, w, M, N, K, stream);
+    }
   } else if (M <= 64) {
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     DLLM_BY_EPILOGUE(gemm_f32_kernel, grid, THREADS)

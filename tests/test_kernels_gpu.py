@@ -74,6 +74,21 @@ def test_gemm_f32(m, n, k, epilogue):
     assert rel_error(c.cpu(), ref.cpu()) <= 2e-6
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 6, 4), (8, 1184, 132), (9, 1186, 768), (16, 4738, 60), (7, 18946, 196), (16, 18946, 68)])
+@pytest.mark.parametrize("epilogue", [0, 2, 3])
+def test_gemm_f32_few_rows(m, n, k, epilogue):
+    """The kernel for a few rows around the lines between its column splits, with ragged last tiles in every direction:
+    the bits of the tile kernel (one chain of multiply-adds an output in both), so no tolerance."""
+    a, w = _randn((m, k), torch.float32, 3), _randn((n, k), torch.float32, 4, 0.2)
+    many = torch.cat([a, _randn((80 - m, k), torch.float32, 5)])
+    cols = n // 2 if epilogue == 3 else n
+    start = _randn((80, cols), torch.float32, 6)
+    c, whole = start[:m].clone(), start.clone()
+    ops().gemm(c, a, w, epilogue)
+    ops().gemm(whole, many, w, epilogue)
+    assert torch.equal(c, whole[:m])
+
+
 def test_gemm_f32_rows_do_not_depend_on_the_batch():
     a, w = _randn((150, 136), torch.float32, 6), _randn((200, 136), torch.float32, 7)
     whole = torch.empty((150, 200), dtype=torch.float32, device=DEV)
