@@ -4,70 +4,142 @@
 #include "gemm_common.cuh"
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, THREADS = 256;
-
-template <int EPI>
-__global__ void __launch_bounds__(THREADS) gemm_f32_kernel(void* __restrict__ c, const float* __restrict__ a,
-                                                           const float* __restrict__ w, int M, int N, int K) {
-  __shared__ float as[BK][BM + 4];
-  __shared__ float ws[BK][BN + 4];
-  int tid = threadIdx.x;
-  int tx = tid & 15, ty = tid >> 4;
-  int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  int lrow = tid >> 2, lk = (tid & 3) * 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vw = va;
-    if (m0 + lrow < M && k0 + lk < K) va = *(const float4*)(a + (size_t)(m0 + lrow) * K + k0 + lk);
-    if (n0 + lrow < N && k0 + lk < K) vw = *(const float4*)(w + (size_t)(n0 + lrow) * K + k0 + lk);
-    as[lk + 0][lrow] = va.x; as[lk + 1][lrow] = va.y; as[lk + 2][lrow] = va.z; as[lk + 3][lrow] = va.w;
-    ws[lk + 0][lrow] = vw.x; ws[lk + 1][lrow] = vw.y; ws[lk + 2][lrow] = vw.z; ws[lk + 3][lrow] = vw.w;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float4 ra = *(const float4*)&as[k][ty * 4];
-      float4 rw = *(const float4*)&ws[k][tx * 4];
-      float av[4] = {ra.x, ra.y, ra.z, ra.w}, wv[4] = {rw.x, rw.y, rw.z, rw.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int m = m0 + ty * 4 + i, n = n0 + tx * 4;
-    epilogue_pair<EPI, float>(c, m, n, M, N, acc[i][0], acc[i][1]);
-    epilogue_pair<EPI, float>(c, m, n + 2, M, N, acc[i][2], acc[i][3]);
-  }
+__device__ __forceinline__ void cp_async_f4(float* smem, const float* gmem, bool ok) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  int bytes = ok ? 16 : 0;  // (a copy of no bytes fills the 16 bytes with zeros)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 
-// ---- the same product for many rows: 128 x 128 tiles, 8 x 8 outputs a thread ---------------------------------------
-// Two stages of shared memory; the next k tile travels from global memory into registers while this one is
-// multiplied. A thread's 64 outputs are 2 x 2 groups of 4 x 4, so its shared-memory reads are four 16-byte loads per
-// k. Every output is still one chain of fused multiply-adds over k ascending from zero: the same bits as above.
-constexpr int LM = 128, LN = 128, LK = 16, LTHREADS = 256;
+// ---- tiles of 64 x 64 and 32 x 32 outputs, 4 x 4 of them a thread ----------------------------------------------------
+// For products that have too few tiles of 128 x 128 (below) for the device. Bound by reads of shared memory (a warp's
+// 16-byte read takes four cycles whoever shares it, which 4 x 4 outputs a thread hide half of the multiply-adds under:
+// about 37 TFLOP/s), so nothing else is put there: rows of A and W arrive as they lie (k innermost, by cp.async,
+// STAGES - 1 steps of 32 values ahead), a thread reads four k of a row at a time, and its rows and columns are TILE / 4
+// apart, which keeps the reads free of bank conflicts.
+// Microseconds before (128 x 128 tiles, or 64 x 64 with one step of 16 values ahead for up to 64 rows) and now:
+// 2048 x 576 x 576 71 -> 43, 2048 x 576 x 1536 171 -> 98, 512 x 576 x 1536 167 -> 40, 32 x 576 x 1536 104 -> 31.
+constexpr int DEPTH = 32, TLD = DEPTH + 4;
+
+template <int EPI, int TILE, int STAGES, int BLOCKS>
+__global__ void __launch_bounds__(TILE * TILE / 16, BLOCKS) gemm_f32_tile_kernel(
+    void* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w, int M, int N, int K) {
+  constexpr int PER = 4, T = TILE * TILE / (PER * PER), APART = TILE / PER, STAGE = 2 * TILE * TLD;
+  constexpr int COPIES = 2 * TILE * (DEPTH / 4) / T;
+  static_assert(TILE % (T / 8) == 0, "a copy is A's or W's for the whole block");
+  extern __shared__ __align__(16) float ring[];  // [STAGES][rows of A, then rows of W][TLD]
+  int tid = threadIdx.x, tx = tid % APART, ty = tid / APART;  // rows ty + i * APART, columns tx + j * APART
+  int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
+  int tiles = (K + DEPTH - 1) / DEPTH;
+  auto ask = [&](int t) {
+    float* stage = ring + (t % STAGES) * STAGE;
+    int k = t * DEPTH + (tid & 7) * 4;
+#pragma unroll
+    for (int i = 0; i < COPIES; ++i) {
+      int r = (tid >> 3) + i * (T / 8);
+      bool from_a = i * (T / 8) < TILE;
+      int row = from_a ? m0 + r : n0 + r - TILE;
+      bool ok = k < K && row < (from_a ? M : N);
+      const float* base = from_a ? a : w;
+      cp_async_f4(stage + r * TLD + (tid & 7) * 4, ok ? base + (size_t)row * K + k : base, ok);
+    }
+  };
+  auto close = [] { asm volatile("cp.async.commit_group;\n" ::); };
+  float acc[PER][PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+#pragma unroll
+    for (int j = 0; j < PER; ++j) acc[i][j] = 0.f;
+  for (int t = 0; t < STAGES - 1; ++t) {
+    if (t < tiles) ask(t);
+    close();
+  }
+  for (int t = 0; t < tiles; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // (this stage has arrived for everybody, and everybody is done with the one before it)
+    if (t + STAGES - 1 < tiles) ask(t + STAGES - 1);
+    close();
+    const float* rows = ring + (t % STAGES) * STAGE + ty * TLD;
+    const float* cols = ring + (t % STAGES) * STAGE + (TILE + tx) * TLD;
+#pragma unroll
+    for (int k = 0; k < DEPTH; k += 4) {
+      float4 wv[PER];
+#pragma unroll
+      for (int j = 0; j < PER; ++j) wv[j] = *(const float4*)(cols + j * APART * TLD + k);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        float4 av = *(const float4*)(rows + i * APART * TLD + k);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) acc[i][j] = fmaf(av.x, wv[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) acc[i][j] = fmaf(av.y, wv[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) acc[i][j] = fmaf(av.z, wv[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) acc[i][j] = fmaf(av.w, wv[j].w, acc[i][j]);
+      }
+    }
+  }
+  // (columns are stored by the lane that has the even one: neighbouring columns lie in neighbouring lanes)
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      float other = __shfl_down_sync(0xffffffffu, acc[i][j], 1);
+      if (!(tx & 1)) epilogue_pair<EPI, float>(c, m0 + ty + i * APART, n0 + tx + j * APART, M, N, acc[i][j], other);
+    }
+}
+
+template <int EPI, int TILE, int STAGES, int BLOCKS>
+int launch_tile(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_f32_tile_kernel<EPI, TILE, STAGES, BLOCKS>;
+  constexpr int smem = STAGES * 2 * TILE * TLD * (int)sizeof(float);
+  static std::atomic<unsigned long long> allowed{0};
+  if (!dllm_allow_shared((const void*)kernel, smem, allowed)) return DLLM_LAUNCH_FAILED;
+  dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
+  if (grid.y > 65535) return DLLM_UNSUPPORTED_SIZE;
+  kernel<<<grid, TILE * TILE / 16, smem, stream>>>(c, a, w, M, N, K);
+  return dllm_launch_status();
+}
+
+// ---- tiles of 128 x 128 outputs, 8 x 8 of them a thread ----------------------------------------------------------------
+// Two stages of shared memory; the next k tile travels from global memory into registers while this one is multiplied.
+// A thread's 64 outputs are 2 x 2 groups of 4 x 4, so its shared-memory reads are four 16-byte loads per k; two
+// neighbouring columns share a packed multiply-add (`fma.rn.f32x2`: two correctly rounded multiply-adds in one issue
+// slot, which leaves slots for the loads and stores). Every output is one chain over k ascending from zero here too: the
+// same bits. 2048 x 3072 x 576: 200 -> 174 us (42 TFLOP/s); 8 x 16 outputs a thread: 186; rows as they lie with cp.async,
+// as for the smaller tiles: 240.
+constexpr int WM = 128, WN = 128, WK = 16;
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 
 template <int EPI>
-__global__ void __launch_bounds__(LTHREADS) gemm_f32_large_kernel(void* __restrict__ c, const float* __restrict__ a,
-                                                                  const float* __restrict__ w, int M, int N, int K) {
-  __shared__ __align__(16) float as[2][LK][LM + 4];
-  __shared__ __align__(16) float ws[2][LK][LN + 4];
+__global__ void __launch_bounds__(256, 2) gemm_f32_wide_kernel(
+    void* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w, int M, int N, int K) {
+  __shared__ __align__(16) float as[2][WK][WM + 4];
+  __shared__ __align__(16) float ws[2][WK][WN + 4];
   int tid = threadIdx.x;
-  int tx = tid & 15, ty = tid >> 4;             // 16 x 16 threads; outputs rows ty*4 + {0..3, 64..67}, cols likewise
-  int m0 = blockIdx.y * LM, n0 = blockIdx.x * LN;
+  int tx = tid & 15, ty = tid >> 4;             // rows ty * 4 + {0..3, 64..67}, columns likewise
+  int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
   int lrow = tid >> 2, lk = (tid & 3) * 4;      // a thread fetches rows lrow and lrow + 64, k lk .. lk + 3
-  float acc[8][8];
+  unsigned long long acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   float4 va[2], vw[2];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -89,20 +161,22 @@ __global__ void __launch_bounds__(LTHREADS) gemm_f32_large_kernel(void* __restri
   fetch(0);
   stash(0);
   __syncthreads();
-  int tiles = (K + LK - 1) / LK;
+  int tiles = (K + WK - 1) / WK;
   for (int t = 0; t < tiles; ++t) {
     int buf = t & 1;
-    if (t + 1 < tiles) fetch((t + 1) * LK);
+    if (t + 1 < tiles) fetch((t + 1) * WK);
 #pragma unroll
-    for (int k = 0; k < LK; ++k) {
+    for (int k = 0; k < WK; ++k) {
       float4 a0 = *(const float4*)&as[buf][k][ty * 4], a1 = *(const float4*)&as[buf][k][64 + ty * 4];
-      float4 w0 = *(const float4*)&ws[buf][k][tx * 4], w1 = *(const float4*)&ws[buf][k][64 + tx * 4];
       float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+      ulonglong2 w0 = *(const ulonglong2*)&ws[buf][k][tx * 4], w1 = *(const ulonglong2*)&ws[buf][k][64 + tx * 4];
+      unsigned long long wv[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 8; ++i) {
+        unsigned long long both = pack2(av[i], av[i]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma2(both, wv[j], acc[i][j]);
+      }
     }
     if (t + 1 < tiles) {
       stash(buf ^ 1);  // (the other stage was last read before the barrier that ended the step before)
@@ -113,11 +187,38 @@ __global__ void __launch_bounds__(LTHREADS) gemm_f32_large_kernel(void* __restri
   for (int i = 0; i < 8; ++i) {
     int m = m0 + (i >> 2) * 64 + ty * 4 + (i & 3);
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      int n = n0 + (j >> 2) * 64 + tx * 4 + (j & 3);
-      epilogue_pair<EPI, float>(c, m, n, M, N, acc[i][j], acc[i][j + 1]);
+    for (int j = 0; j < 4; ++j) {
+      int n = n0 + (j >> 1) * 64 + tx * 4 + 2 * (j & 1);
+      float2 v = unpack2(acc[i][j]);
+      epilogue_pair<EPI, float>(c, m, n, M, N, v.x, v.y);
     }
   }
+}
+
+template <int EPI>
+int launch_wide(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  dim3 grid((N + WN - 1) / WN, (M + WM - 1) / WM);
+  if (grid.y > 65535) return DLLM_UNSUPPORTED_SIZE;
+  gemm_f32_wide_kernel<EPI><<<grid, 256, 0, stream>>>(c, a, w, M, N, K);
+  return dllm_launch_status();
+}
+
+// Which tile: the fewest microseconds by rounds of one tile per multiprocessor. A round of K = 576 was measured at about
+// 57 us for 128 x 128 (37 to 45 TFLOP/s with all multiprocessors busy), 20 for 64 x 64 and, while few rounds are needed,
+// 8 for 32 x 32, plus a few to begin; all grow alike with K. So full devices take the large tile, and a product too small
+// for it (2048 x 576: 80 tiles of 128 x 128 for 148 multiprocessors) one that spreads over all of them.
+// Launched without programmatic dependence: blocks of the next kernel that wait on a multiprocessor for this one make the
+// launch after it spread unevenly (2048 x 576 x 576 back to back: 110 us instead of 72).
+template <int EPI>
+int launch_tiles(void* c, const float* a, const float* w, int M, int N, int K, cudaStream_t stream) {
+  auto rounds = [&](int tile) {
+    long long tiles = (long long)((M + tile - 1) / tile) * ((N + tile - 1) / tile);
+    return (tiles + 147) / 148;
+  };
+  long long wide = 57 * rounds(128) + 4, middle = 20 * rounds(64) + 2, small = 8 * rounds(32) + 2;
+  if (wide <= middle && wide <= small) return launch_wide<EPI>(c, a, w, M, N, K, stream);
+  if (middle <= small) return launch_tile<EPI, 64, 4, 2>(c, a, w, M, N, K, stream);
+  return launch_tile<EPI, 32, 6, 4>(c, a, w, M, N, K, stream);
 }
 
 // ---- and for a few rows (decode steps): the reduction streamed through a ring of stages -----------------------------
@@ -129,12 +230,6 @@ __global__ void __launch_bounds__(LTHREADS) gemm_f32_large_kernel(void* __restri
 // Eight rows, 576 columns: K = 576 12.0 -> 3.3 us, K = 1536 27.5 -> 6.1 us (before: 32 columns a block, three stages of
 // 32 values, which was 18 blocks for the device and a round trip to L2 every other stage); 49152 x 576 52 -> 28.5 us.
 constexpr int SM_ROWS = 16;
-
-__device__ __forceinline__ void cp_async_f4(float* smem, const float* gmem, bool ok) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  int bytes = ok ? 16 : 0;  // (a copy of no bytes fills the 16 bytes with zeros)
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
-}
 
 template <int EPI, int COLS, int ROWS, int PER, int DEPTH, int STAGES>
 __global__ void __launch_bounds__(COLS * ROWS / PER) gemm_f32_small_kernel(void* __restrict__ c, const float* __restrict__ a,
@@ -256,34 +351,18 @@ int launch_small_by_rows(void* c, const float* a, const float* w, int M, int N, 
 }  // namespace
 
 // C = A[M,K] * W[N,K]^T in float32; K a multiple of 4 (16-byte rows); N even for the SwiGLU epilogue (column pairs).
-// Up to 16 rows take the kernel that streams the reduction, 17 to 64 the 64 x 64 tiles, more the 128 x 128 tiles;
-// the three give an output the same bits.
+// Up to 16 rows take the kernel that streams the reduction, more the tiles that `launch_tiles` chooses; all give an
+// output the same bits.
 DLLM_EXPORT int dllm_gemm_f32(void* c, const float* a, const float* w, int M, int N, int K, int epilogue,
                               cudaStream_t stream) {
   if (M <= 0 || N <= 0) return DLLM_OK;
   if (K <= 0 || (K & 3) || ((N & 1) && epilogue == EPI_SWIGLU)) return DLLM_UNSUPPORTED_SIZE;
   if (epilogue < 0 || epilogue > EPI_SWIGLU) return DLLM_BAD_ARGUMENT;
   if (epilogue == EPI_STORE_T) epilogue = EPI_STORE_F32;  // (the activation type is float32 here)
-#define DLLM_BY_EPILOGUE(KERNEL, GRID, THREADS_)                                                      \
-  switch (epilogue) {                                                                                 \
-    case EPI_STORE_F32: KERNEL<EPI_STORE_F32><<<GRID, THREADS_, 0, stream>>>(c, a, w, M, N, K); break; \
-    case EPI_RESIDUAL: KERNEL<EPI_RESIDUAL><<<GRID, THREADS_, 0, stream>>>(c, a, w, M, N, K); break;   \
-    default: KERNEL<EPI_SWIGLU><<<GRID, THREADS_, 0, stream>>>(c, a, w, M, N, K); break;               \
+  bool few = M <= SM_ROWS;
+  switch (epilogue) {
+    case EPI_STORE_F32: return (few ? launch_small_by_rows<EPI_STORE_F32> : launch_tiles<EPI_STORE_F32>)(c, a, w, M, N, K, stream);
+    case EPI_RESIDUAL: return (few ? launch_small_by_rows<EPI_RESIDUAL> : launch_tiles<EPI_RESIDUAL>)(c, a, w, M, N, K, stream);
+    default: return (few ? launch_small_by_rows<EPI_SWIGLU> : launch_tiles<EPI_SWIGLU>)(c, a, w, M, N, K, stream);
   }
-  if (M <= SM_ROWS) {
-    switch (epilogue) {
-      case EPI_STORE_F32: return launch_small_by_rows<EPI_STORE_F32>(c, a, w, M, N, K, stream);
-      case EPI_RESIDUAL: return launch_small_by_rows<EPI_RESIDUAL>(c, a, w, M, N, K, stream);
-      default: return launch_small_by_rows<EPI_SWIGLU>(c, a, w, M, N, K, stream);
-    }
-  } else if (M <= 64) {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    DLLM_BY_EPILOGUE(gemm_f32_kernel, grid, THREADS)
-  } else {
-    dim3 grid((N + LN - 1) / LN, (M + LM - 1) / LM);
-    if (grid.y > 65535) return DLLM_UNSUPPORTED_SIZE;
-    DLLM_BY_EPILOGUE(gemm_f32_large_kernel, grid, LTHREADS)
-  }
-#undef DLLM_BY_EPILOGUE
-  return dllm_launch_status();
 }

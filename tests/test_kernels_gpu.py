@@ -89,6 +89,23 @@ def test_gemm_f32_few_rows(m, n, k, epilogue):
     assert torch.equal(c, whole[:m])
 
 
+@pytest.mark.parametrize("m,n,k", [(17, 6, 4), (33, 70, 100), (200, 576, 64), (500, 962, 36), (700, 3074, 20), (2050, 574, 68)])
+def test_gemm_f32_tiles(m, n, k):
+    """Products of more than 16 rows that take each of the tile sizes, ragged in every direction: every row has the bits
+    that the kernel for a few rows gives it (one chain of multiply-adds an output in all), and every epilogue's columns."""
+    a, w = _randn((m, k), torch.float32, 3), _randn((n, k), torch.float32, 4, 0.2)
+    for epilogue in (0, 2, 3):
+        c = _randn((m, n // 2 if epilogue == 3 else n), torch.float32, 6)
+        few = c.clone()
+        ops().gemm(c, a, w, epilogue)
+        for row in range(0, m, 16):
+            ops().gemm(few[row:row + 16], a[row:row + 16].contiguous(), w, epilogue)
+        assert torch.equal(c, few)
+    ref = torch.empty((m, n), dtype=torch.float32, device=DEV)
+    ops().gemm(ref, a, w, 0)
+    assert rel_error(ref.cpu(), (a.double() @ w.double().T).float().cpu()) <= 2e-6
+
+
 def test_gemm_f32_rows_do_not_depend_on_the_batch():
     a, w = _randn((150, 136), torch.float32, 6), _randn((200, 136), torch.float32, 7)
     whole = torch.empty((150, 200), dtype=torch.float32, device=DEV)
