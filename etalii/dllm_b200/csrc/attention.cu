@@ -1,9 +1,16 @@
-// Attention over the paged cache, general form: one warp per (token, query head). The warp walks the visible keys
-// of the token's own sequence in tiles of 32 (one key per lane for the scores, one value dimension per lane for the
-// weighted sum) with a running maximum and sum in float32. It serves whole prompts and single decoded tokens alike
-// and any head size that is a multiple of 8 up to 256, any number of heads and groups, with or without a window.
-// A (token, head) result depends only on that token's query and the keys it may see, so it is the same bits
-// however the tokens were cut into steps or batched.
+// Attention over the paged cache, general form: any head size that is a multiple of 8 up to 256, any number of heads and
+// groups, with or without a window, float32 and bfloat16, whole prompts and single tokens.
+//
+// Every kernel here computes the same thing in the same order, so that a (token, head) result has the same bits whichever
+// kernel gives it, however the tokens were cut into steps or batched:
+//   * keys are taken in chunks of 64 positions, aligned at multiples of 64 (the pages); a chunk's result depends on nothing
+//     but the query and the visible keys in it: the largest score m, weights exp(s - m), their sum l, and o = sum of
+//     weight * value per dimension, one chain of multiply-adds over ascending keys;
+//   * a score is two chains of multiply-adds, over the even and the odd dimensions ascending, added and then scaled;
+//   * the 64 weights are summed by a fixed tree: key + key 32 further, then the butterfly over 32;
+//   * the chunks' results meet in ascending order (`merge`).
+// Since chunks are independent, decoding gives each to a warp of its own (attention_chunks_kernel) and a prompt's tiles of
+// queries take them one after another (attention_tile_kernel).
 #include "common.cuh"
 
 namespace {
@@ -14,39 +21,56 @@ template <typename T> struct Vec;  // 16-byte vectors of the element type
 template <> struct Vec<float> { static constexpr int N = 4; };
 template <> struct Vec<__nv_bfloat16> { static constexpr int N = 8; };
 
-__device__ __forceinline__ float dot_vec(const float* q, const float* k) {
-  float4 v = *(const float4*)k;
-  return fmaf(q[3], v.w, fmaf(q[2], v.z, fmaf(q[1], v.y, q[0] * v.x)));
+// Packed pairs of float32 (the even and the odd dimensions' chains of a score side by side).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
 }
-__device__ __forceinline__ float dot_vec(const float* q, const __nv_bfloat16* k) {
-  uint4 raw = *(const uint4*)k;
-  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 x = __bfloat1622float2(p[i]);
-    s = fmaf(q[2 * i], x.x, s);
-    s = fmaf(q[2 * i + 1], x.y, s);
-  }
-  return s;
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
 
-// The same sums from a vector that is already in registers (one load of a key for several queries).
-__device__ __forceinline__ float4 load_vec(const float* k) { return *(const float4*)k; }
-__device__ __forceinline__ uint4 load_vec(const __nv_bfloat16* k) { return *(const uint4*)k; }
-__device__ __forceinline__ float dot_loaded(const float* q, float4 v) {
-  return fmaf(q[3], v.w, fmaf(q[2], v.z, fmaf(q[1], v.y, q[0] * v.x)));
+// The next dimensions of a score, sixteen bytes of a key: (even, odd) in `acc`.
+__device__ __forceinline__ void score_piece(float2& acc, const float* q, float4 k) {
+  acc.x = fmaf(q[0], k.x, acc.x);
+  acc.y = fmaf(q[1], k.y, acc.y);
+  acc.x = fmaf(q[2], k.z, acc.x);
+  acc.y = fmaf(q[3], k.w, acc.y);
 }
-__device__ __forceinline__ float dot_loaded(const float* q, uint4 raw) {
+__device__ __forceinline__ void score_piece(float2& acc, const float* q, uint4 raw) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  float s = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float2 x = __bfloat1622float2(p[i]);
-    s = fmaf(q[2 * i], x.x, s);
-    s = fmaf(q[2 * i + 1], x.y, s);
+    float2 k = __bfloat1622float2(p[i]);
+    acc.x = fmaf(q[2 * i], k.x, acc.x);
+    acc.y = fmaf(q[2 * i + 1], k.y, acc.y);
   }
-  return s;
+}
+__device__ __forceinline__ float4 load_vec(const float* k) { return *(const float4*)k; }
+__device__ __forceinline__ uint4 load_vec(const __nv_bfloat16* k) { return *(const uint4*)k; }
+
+// What is subtracted in an exponent: a chunk (or a run of chunks) whose scores are all -inf has weights of 0, not NaN.
+__device__ __forceinline__ float finite_or_zero(float m) { return m == -INFINITY ? 0.f : m; }
+
+// A chunk's result joins those before it: factors for the old and the new, the sum of weights and the maximum updated.
+// The first chunk (m = -inf, l = 0, o = 0) joins like any other: 0 * its factor + the chunk's.
+__device__ __forceinline__ void merge(float& m, float& l, float chunk_m, float chunk_l, float& keep, float& take) {
+  float m_new = fmaxf(m, chunk_m), shift = finite_or_zero(m_new);
+  keep = expf(m - shift);
+  take = expf(chunk_m - shift);
+  l = fmaf(l, keep, __fmul_rn(chunk_l, take));
+  m = m_new;
+}
+__device__ __forceinline__ float merge_output(float o, float keep, float chunk_o, float take) {
+  return fmaf(o, keep, __fmul_rn(chunk_o, take));
 }
 
 template <typename T>
@@ -74,35 +98,49 @@ __global__ void __launch_bounds__(WARPS * 32) attention_warp_kernel(
   for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) acc[i] = 0.f;
   const T* base = (const T*)cache.base;
 
-  for (int j0 = first; j0 < end; j0 += 32) {
-    int j = j0 + lane;
-    bool valid = j < end;
-    int page = valid ? pages[j / ps] : 0;
-    float s = -INFINITY;
-    if (valid) {
-      const T* krow = base + kv_offset(cache, page, 0, g, j % ps);
-      float dot = 0.f;
-      for (int d = 0; d < hd; d += Vec<T>::N) dot += dot_vec(&q_s[warp][d], krow + d);
-      s = dot * scale;
-    }
-    float m_new = fmaxf(m_run, warp_max(s));
-    float p = valid ? expf(s - m_new) : 0.f;
-    float corr = expf(m_run - m_new);  // 0 on the first tile (m_run = -inf)
-    l_run = l_run * corr + warp_sum(p);
+  for (int c0 = first / 64 * 64; c0 < end; c0 += 64) {
+    float s[2], p[2];
+    int page[2];
 #pragma unroll
-    for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) acc[i] *= corr;
-    m_run = m_new;
-    int count = min(32, end - j0);
-    for (int jj = 0; jj < count; ++jj) {
-      float pj = __shfl_sync(0xffffffffu, p, jj);
-      int pg = __shfl_sync(0xffffffffu, page, jj);
-      const T* vrow = base + kv_offset(cache, pg, 1, g, (j0 + jj) % ps);
-#pragma unroll
-      for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) {
-        int d = lane + 32 * i;
-        if (d < hd) acc[i] = fmaf(pj, to_float(vrow[d]), acc[i]);
+    for (int u = 0; u < 2; ++u) {
+      int j = c0 + lane + 32 * u;
+      bool valid = j >= first && j < end;
+      page[u] = valid ? pages[j / ps] : 0;
+      s[u] = -INFINITY;
+      if (valid) {
+        const T* krow = base + kv_offset(cache, page[u], 0, g, j % ps);
+        float2 dot = make_float2(0.f, 0.f);
+        for (int d = 0; d < hd; d += Vec<T>::N) score_piece(dot, &q_s[warp][d], load_vec(krow + d));
+        s[u] = (dot.x + dot.y) * scale;
       }
     }
+    float m = warp_max(fmaxf(s[0], s[1])), shift = finite_or_zero(m);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      int j = c0 + lane + 32 * u;
+      p[u] = j >= first && j < end ? expf(s[u] - shift) : 0.f;
+    }
+    float l = warp_sum(p[0] + p[1]), o[MAX_HEAD_DIM / 32];
+#pragma unroll
+    for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) o[i] = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      int from = max(0, first - c0 - 32 * u), to = min(32, end - c0 - 32 * u);
+      for (int jj = from; jj < to; ++jj) {
+        float pj = __shfl_sync(0xffffffffu, p[u], jj);
+        int pg = __shfl_sync(0xffffffffu, page[u], jj);
+        const T* vrow = base + kv_offset(cache, pg, 1, g, (c0 + 32 * u + jj) % ps);
+#pragma unroll
+        for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) {
+          int d = lane + 32 * i;
+          if (d < hd) o[i] = fmaf(pj, to_float(vrow[d]), o[i]);
+        }
+      }
+    }
+    float keep, take;
+    merge(m_run, l_run, m, l, keep, take);
+#pragma unroll
+    for (int i = 0; i < MAX_HEAD_DIM / 32; ++i) acc[i] = merge_output(acc[i], keep, o[i], take);
   }
   float inv = 1.0f / l_run;
   T* orow = out + ((size_t)t * heads + h) * hd;
@@ -116,13 +154,10 @@ __global__ void __launch_bounds__(WARPS * 32) attention_warp_kernel(
 // ---- the same attention, blockwise ------------------------------------------------------------------------------
 // A block serves one kv head and a run of consecutive tokens of the step; its warps are the (token, query head)
 // pairs of that run, R tokens a warp. The block copies the keys and values of the kv head page by page (64
-// positions) into shared memory, with the next page on its way (cp.async) while the warps work on this one, and
-// every warp walks the page's two tiles of 32 keys exactly as the kernel above walks its tiles: one key a lane for
-// the scores, one value dimension a lane for the weighted sum, the same running maximum and sum in the same order.
-// Tiles start at multiples of 32 from position 0, so without a window a (token, head) result has the same bits as
-// the kernel above gives (with a window the first tile is cut differently: same formula, other rounding), and it
-// depends only on the token's own query and visible keys: not on its tile mates, the cut of the steps or the batch.
-// Tokens of several sequences in one block are served sequence by sequence.
+// positions, one chunk) into shared memory, with the next page on its way (cp.async) while the warps work on this one.
+// Two keys a lane for the scores, one value dimension a lane for the weighted sum. Tokens of several sequences in one
+// block are served sequence by sequence. This form takes what the float32 kernels below do not: bfloat16, prompts with
+// other head sizes, single tokens whose chunks' results do not fit into a cluster's shared memory.
 template <typename T> struct Pad { static constexpr int N = 16 / sizeof(T); };  // 16 bytes: rows in different banks
 
 template <typename T>
@@ -156,7 +191,7 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
   T* kv_s = reinterpret_cast<T*>(smem_raw);       // [stages][k|v][64][ld]
   float* q_all = reinterpret_cast<float*>(smem_raw + (size_t)stages * 2 * 64 * ld * sizeof(T));
   float* q_s = q_all + (size_t)warp * R * hd;                        // this warp's R queries
-  float* p_s = q_all + (size_t)warps * R * hd + (size_t)warp * R * 32;  // and their weights for the tile at hand
+  float* p_s = q_all + (size_t)warps * R * hd + (size_t)warp * R * 64;  // and their weights for the page at hand
   int g = blockIdx.y, group = heads / cache.kv_heads;
   // (the last tokens of a prompt see the most keys: their blocks go first, the short ones fill the gaps behind)
   int t0 = (int)(gridDim.x - 1 - blockIdx.x) * block_tokens, t_stop = min(tokens, t0 + block_tokens);
@@ -208,61 +243,70 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
           asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         }
         __syncthreads();
-        // The warp's R tokens walk the tile together: a key is loaded once for the R scores and a value once for the
+        // The warp's R tokens walk the page together: a key is loaded once for the R scores and a value once for the
         // R weighted sums (what a token computes, and in which order, is what it would compute alone).
-        for (int j0 = p * 64; j0 < p * 64 + 64; j0 += 32) {
-          bool active[R], any = false, whole = hd == CHUNKS * 32;
+        int j0 = p * 64;
+        bool active[R], any = false, whole = hd == CHUNKS * 32;
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            active[r] = j0 < end[r] && j0 + 32 > first[r];  // (warp-uniform) a visible key in this tile
-            any = any || active[r];
-            whole = whole && (!active[r] || (first[r] <= j0 && j0 + 32 <= end[r]));
-          }
-          if (!any) continue;
-          int j = j0 + lane;
-          const T* krow = k_s + (j - p * 64) * ld;
-          float dot[R];
+        for (int r = 0; r < R; ++r) {
+          active[r] = j0 < end[r] && j0 + 64 > first[r];  // (warp-uniform) a visible key in this page
+          any = any || active[r];
+          whole = whole && (!active[r] || (first[r] <= j0 && j0 + 64 <= end[r]));
+        }
+        if (any) {
+          float weight[R][2], chunk_m[R], chunk_l[R], o[R][CHUNKS];
 #pragma unroll
-          for (int r = 0; r < R; ++r) dot[r] = 0.f;
-          if (hd == CHUNKS * 32) {
+          for (int u = 0; u < 2; ++u) {
+            const T* krow = k_s + (lane + 32 * u) * ld;
+            float2 dot[R];
 #pragma unroll
-            for (int d = 0; d < CHUNKS * 32; d += Vec<T>::N) {
-              auto key = load_vec(krow + d);
+            for (int r = 0; r < R; ++r) dot[r] = make_float2(0.f, 0.f);
+            if (hd == CHUNKS * 32) {
+#pragma unroll 8
+              for (int d = 0; d < CHUNKS * 32; d += Vec<T>::N) {
+                auto key = load_vec(krow + d);
 #pragma unroll
-              for (int r = 0; r < R; ++r) dot[r] += dot_loaded(&q_s[r * hd + d], key);
+                for (int r = 0; r < R; ++r) score_piece(dot[r], &q_s[r * hd + d], key);
+              }
+            } else {
+              for (int d = 0; d < hd; d += Vec<T>::N) {
+                auto key = load_vec(krow + d);
+#pragma unroll
+                for (int r = 0; r < R; ++r) score_piece(dot[r], &q_s[r * hd + d], key);
+              }
             }
-          } else {
-            for (int d = 0; d < hd; d += Vec<T>::N) {
-              auto key = load_vec(krow + d);
 #pragma unroll
-              for (int r = 0; r < R; ++r) dot[r] += dot_loaded(&q_s[r * hd + d], key);
-            }
+            for (int r = 0; r < R; ++r) weight[r][u] = (dot[r].x + dot[r].y) * scale;
           }
           // (a single token a warp, as in decoding, hands its weights from lane to lane by shuffles; several go
           // through shared memory, four weights a load)
-          float weight[R];
-          if (R > 1) __syncwarp();  // (the weights of the tile before have been read by every lane)
+          if (R > 1) __syncwarp();  // (the weights of the page before have been read by every lane)
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            weight[r] = 0.f;
             if (!active[r]) continue;
-            bool valid = j >= first[r] && j < end[r];
-            float sc = valid ? dot[r] * scale : -INFINITY;
-            float m_new = fmaxf(m_run[r], warp_max(sc));
-            float pr = valid ? expf(sc - m_new) : 0.f;
-            float corr = expf(m_run[r] - m_new);  // 0 on the first tile (m_run = -inf)
-            l_run[r] = l_run[r] * corr + warp_sum(pr);
+            bool valid[2];
 #pragma unroll
-            for (int i = 0; i < CHUNKS; ++i) acc[r][i] *= corr;
-            m_run[r] = m_new;
-            weight[r] = pr;
-            if (R > 1) p_s[r * 32 + lane] = pr;
+            for (int u = 0; u < 2; ++u) {
+              int j = j0 + lane + 32 * u;
+              valid[u] = j >= first[r] && j < end[r];
+              if (!valid[u]) weight[r][u] = -INFINITY;
+            }
+            chunk_m[r] = warp_max(fmaxf(weight[r][0], weight[r][1]));
+            float shift = finite_or_zero(chunk_m[r]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              weight[r][u] = valid[u] ? expf(weight[r][u] - shift) : 0.f;
+              if (R > 1) p_s[r * 64 + 32 * u + lane] = weight[r][u];
+            }
+            chunk_l[r] = warp_sum(weight[r][0] + weight[r][1]);
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) o[r][i] = 0.f;
           }
           if (R > 1) __syncwarp();
-          const T* vtile = v_s + (j0 - p * 64) * ld + lane;
-          if (whole) {  // whole tiles of a whole head for every token that sees the tile: no bounds in the loop
+          const T* vtile = v_s + lane;
+          if (whole) {  // whole pages of a whole head for every token that sees the page: no bounds in the loop
 #pragma unroll 4
-            for (int jj = 0; jj < 32; jj += 4) {
+            for (int jj = 0; jj < 64; jj += 4) {
               float v[4][CHUNKS];
 #pragma unroll
               for (int u = 0; u < 4; ++u)
@@ -270,22 +314,23 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
                 for (int i = 0; i < CHUNKS; ++i) v[u][i] = to_float(vtile[(jj + u) * ld + 32 * i]);
 #pragma unroll
               for (int r = 0; r < R; ++r) {
-                if (!active[r]) continue;  // (a token that does not see the tile must not meet what lies there)
+                if (!active[r]) continue;  // (a token that does not see the page must not meet what lies there)
                 float4 pj;
                 if (R > 1) {
-                  pj = *reinterpret_cast<const float4*>(&p_s[r * 32 + jj]);
+                  pj = *reinterpret_cast<const float4*>(&p_s[r * 64 + jj]);
                 } else {
-                  pj.x = __shfl_sync(0xffffffffu, weight[r], jj);
-                  pj.y = __shfl_sync(0xffffffffu, weight[r], jj + 1);
-                  pj.z = __shfl_sync(0xffffffffu, weight[r], jj + 2);
-                  pj.w = __shfl_sync(0xffffffffu, weight[r], jj + 3);
+                  float mine = jj < 32 ? weight[r][0] : weight[r][1];
+                  pj.x = __shfl_sync(0xffffffffu, mine, jj & 31);
+                  pj.y = __shfl_sync(0xffffffffu, mine, (jj & 31) + 1);
+                  pj.z = __shfl_sync(0xffffffffu, mine, (jj & 31) + 2);
+                  pj.w = __shfl_sync(0xffffffffu, mine, (jj & 31) + 3);
                 }
 #pragma unroll
                 for (int i = 0; i < CHUNKS; ++i) {
-                  acc[r][i] = fmaf(pj.x, v[0][i], acc[r][i]);
-                  acc[r][i] = fmaf(pj.y, v[1][i], acc[r][i]);
-                  acc[r][i] = fmaf(pj.z, v[2][i], acc[r][i]);
-                  acc[r][i] = fmaf(pj.w, v[3][i], acc[r][i]);
+                  o[r][i] = fmaf(pj.x, v[0][i], o[r][i]);
+                  o[r][i] = fmaf(pj.y, v[1][i], o[r][i]);
+                  o[r][i] = fmaf(pj.z, v[2][i], o[r][i]);
+                  o[r][i] = fmaf(pj.w, v[3][i], o[r][i]);
                 }
               }
             }
@@ -293,14 +338,23 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
 #pragma unroll
             for (int r = 0; r < R; ++r) {
               if (!active[r]) continue;
-              int from = max(0, first[r] - j0), to = min(32, end[r] - j0);
+              int from = max(0, first[r] - j0), to = min(64, end[r] - j0);
               for (int jj = from; jj < to; ++jj) {
-                float pj = R > 1 ? p_s[r * 32 + jj] : __shfl_sync(0xffffffffu, weight[r], jj);
+                float pj = R > 1 ? p_s[r * 64 + jj]
+                                 : __shfl_sync(0xffffffffu, jj < 32 ? weight[r][0] : weight[r][1], jj & 31);
 #pragma unroll
                 for (int i = 0; i < CHUNKS; ++i)
-                  if (lane + 32 * i < hd) acc[r][i] = fmaf(pj, to_float(vtile[jj * ld + 32 * i]), acc[r][i]);
+                  if (lane + 32 * i < hd) o[r][i] = fmaf(pj, to_float(vtile[jj * ld + 32 * i]), o[r][i]);
               }
             }
+          }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            if (!active[r]) continue;
+            float keep, take;
+            merge(m_run[r], l_run[r], chunk_m[r], chunk_l[r], keep, take);
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) acc[r][i] = merge_output(acc[r][i], keep, o[r][i], take);
           }
         }
         if (stages != 2) {
@@ -337,7 +391,7 @@ int launch_blocks(void* out, const void* q, const KvLayout& cache, const int* to
   int warps = token_slots * heads_per_pass;
   int ld = cache.head_dim + Pad<T>::N;
   size_t stage_bytes = (size_t)2 * 64 * ld * sizeof(T);
-  size_t q_bytes = (size_t)warps * R * (cache.head_dim + 32) * sizeof(float);  // queries and a tile's weights
+  size_t q_bytes = (size_t)warps * R * (cache.head_dim + 64) * sizeof(float);  // queries and a page's weights
   int stages = 2 * stage_bytes + q_bytes <= 200 * 1024 ? 2 : 1;
   size_t smem = stages * stage_bytes + q_bytes;
   static size_t configured = 0;
@@ -353,6 +407,409 @@ int launch_blocks(void* out, const void* q, const KvLayout& cache, const int* to
                                                                   slots, tokens, heads, scale, window,
                                                                   heads_per_pass, stages);
   return dllm_launch_status();
+}
+// ---- float32 prompts with heads of 64 and 128: tiles of 32 queries of one head ------------------------------------------
+// Bound by multiply-adds and the shared-memory reads that feed them, so it is laid out like a product: a block takes 32
+// consecutive tokens and one query head, a thread four tokens (ty + 8 i) by four keys (tx + 16 j) of the scores and by
+// HD / 16 dimensions of the outputs; a key, value or weight read from shared memory serves four multiply-adds, the even and
+// odd dimensions of a score and neighbouring output dimensions share a packed one. The next page's keys are on their way
+// while values are multiplied, the next values while scores are. 32 queries rather than 64: a prompt of 2,048 with nine
+// heads is 576 blocks, which level out over the device although the last ones see 32 times the keys of the first ones
+// (those go first). Before, a warp walked the keys for four tokens, and read a value and a weight for every four
+// multiply-adds: 492 us a layer at 2,048 tokens (9 query, 3 kv heads of 64), now 214 (23 TFLOP/s).
+constexpr int TILE_Q = 32, TILE_THREADS = 128;
+
+template <int HD>
+struct TileShared {
+  float q[TILE_Q][HD + 4], k[64][HD + 4], v[64][HD + 4], p[TILE_Q][64 + 4];
+  int end[TILE_Q];
+};
+
+template <int HD>
+__global__ void __launch_bounds__(TILE_THREADS, HD == 64 ? 4 : 2) attention_tile_kernel(
+    float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_seq,
+    const int* __restrict__ tok_pos, const int* __restrict__ slots, int tokens, int heads, float scale, int window) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TileShared<HD>& sm = *reinterpret_cast<TileShared<HD>*>(smem_raw);
+  constexpr int GROUPS = HD / 64;  // groups of four output dimensions a thread owns, 64 apart
+  int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  int h = blockIdx.x % heads, g = h / (heads / cache.kv_heads);
+  int t0 = ((int)(gridDim.x / heads) - 1 - (int)(blockIdx.x / heads)) * TILE_Q, t_stop = min(tokens, t0 + TILE_Q);
+  for (int i = tid; i < TILE_Q * (HD / 4); i += TILE_THREADS) {
+    int r = i / (HD / 4), d = i % (HD / 4) * 4;
+    float4 value = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t0 + r < tokens) value = *(const float4*)(q + ((size_t)(t0 + r) * heads + h) * HD + d);
+    *(float4*)&sm.q[r][d] = value;
+  }
+  auto copy_page = [&](float (*to)[HD + 4], int page, int which) {
+    const float* from = (const float*)cache.base + kv_offset(cache, page, which, g, 0);
+#pragma unroll 4
+    for (int i = tid; i < 64 * (HD / 4); i += TILE_THREADS) {
+      int r = i / (HD / 4), d = i % (HD / 4) * 4;
+      unsigned at = (unsigned)__cvta_generic_to_shared(&to[r][d]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(from + (size_t)r * HD + d));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+
+  for (int run_begin = t0; run_begin < t_stop;) {
+    // a run: the block's tokens of one sequence (positions ascend inside it)
+    int seq = tok_seq[run_begin], run_end = run_begin + 1;
+    while (run_end < t_stop && tok_seq[run_end] == seq) ++run_end;
+    const int* pages = cache.page_table + (size_t)slots[seq] * cache.max_pages;
+    int run_last = tok_pos[run_end - 1] + 1;  // keys [run_first, run_last) are read by somebody of the run
+    int first_end = tok_pos[run_begin] + 1;
+    int run_first = (window > 0 && first_end > window) ? first_end - window : 0;
+    int page_first = run_first / 64, page_last = (run_last - 1) / 64;
+    __syncthreads();  // (everybody is done with the run before)
+    if (tid < TILE_Q) sm.end[tid] = t0 + tid >= run_begin && t0 + tid < run_end ? tok_pos[t0 + tid] + 1 : 0;
+    copy_page(sm.k, pages[page_first], 0);
+    copy_page(sm.v, pages[page_first], 1);
+    __syncthreads();
+    int end[4], first[4];
+    float m_run[4], l_run[4];
+    unsigned long long acc[4][2 * GROUPS];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      end[i] = sm.end[ty + 8 * i];
+      first[i] = (window > 0 && end[i] > window) ? end[i] - window : 0;
+      m_run[i] = -INFINITY;
+      l_run[i] = 0.f;
+#pragma unroll
+      for (int x = 0; x < 2 * GROUPS; ++x) acc[i][x] = 0;
+    }
+    for (int p = page_first; p <= page_last; ++p) {
+      int j0 = p * 64;
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the page's keys (its values may still be on their way)
+      __syncthreads();
+      float s[4][4];
+      {
+        unsigned long long dot[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dot[i][j] = 0;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 4) {
+          ulonglong2 key[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) key[j] = *(const ulonglong2*)&sm.k[tx + 16 * j][d];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            ulonglong2 query = *(const ulonglong2*)&sm.q[ty + 8 * i][d];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.x, key[j].x, dot[i][j]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.y, key[j].y, dot[i][j]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float2 halves = unpack2(dot[i][j]);
+            s[i][j] = (halves.x + halves.y) * scale;
+          }
+      }
+      bool whole = true;  // every token of this thread that sees the page sees all of it
+      float chunk_m[4], chunk_l[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        bool sees = j0 < end[i] && j0 + 64 > first[i];  // (what a token that does not is given here is dropped below)
+        whole = whole && (!sees || (first[i] <= j0 && j0 + 64 <= end[i]));
+        bool valid[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          int key = j0 + tx + 16 * j;
+          valid[j] = key >= first[i] && key < end[i];
+          if (!valid[j]) s[i][j] = -INFINITY;
+        }
+        float m = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+        float shift = finite_or_zero(m);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = valid[j] ? expf(s[i][j] - shift) : 0.f;
+          sm.p[ty + 8 * i][tx + 16 * j] = s[i][j];
+        }
+        float l = (s[i][0] + s[i][2]) + (s[i][1] + s[i][3]);
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+        chunk_m[i] = m;
+        chunk_l[i] = l;
+      }
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the page's values
+      __syncthreads();  // values and weights are there, everybody is done with the keys
+      if (p < page_last) copy_page(sm.k, pages[p + 1], 0);
+      unsigned long long o[4][2 * GROUPS];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = 0;
+      if (__all_sync(0xffffffffu, whole)) {
+#pragma unroll 2
+        for (int jj = 0; jj < 64; jj += 4) {
+          float4 weight[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) weight[i] = *(const float4*)&sm.p[ty + 8 * i][jj];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            unsigned long long value[2 * GROUPS];
+#pragma unroll
+            for (int x = 0; x < GROUPS; ++x) {
+              ulonglong2 two = *(const ulonglong2*)&sm.v[jj + u][64 * x + 4 * tx];
+              value[2 * x] = two.x;
+              value[2 * x + 1] = two.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float one = u == 0 ? weight[i].x : u == 1 ? weight[i].y : u == 2 ? weight[i].z : weight[i].w;
+              unsigned long long both = pack2(one, one);
+#pragma unroll
+              for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = fma2(both, value[x], o[i][x]);
+            }
+          }
+        }
+      } else {  // (a token must not meet what lies at positions that it does not see)
+        int from = 64, to = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (j0 < end[i] && j0 + 64 > first[i]) {
+            from = min(from, max(0, first[i] - j0));
+            to = max(to, min(64, end[i] - j0));
+          }
+        }
+        for (int jj = from; jj < to; ++jj) {
+          unsigned long long value[2 * GROUPS];
+#pragma unroll
+          for (int x = 0; x < GROUPS; ++x) {
+            ulonglong2 two = *(const ulonglong2*)&sm.v[jj][64 * x + 4 * tx];
+            value[2 * x] = two.x;
+            value[2 * x + 1] = two.y;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (j0 + jj < first[i] || j0 + jj >= end[i]) continue;
+            float one = sm.p[ty + 8 * i][jj];
+            unsigned long long both = pack2(one, one);
+#pragma unroll
+            for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = fma2(both, value[x], o[i][x]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (j0 >= end[i] || j0 + 64 <= first[i]) continue;  // (no visible key in this page: it does not take part)
+        float keep, take;
+        merge(m_run[i], l_run[i], chunk_m[i], chunk_l[i], keep, take);
+#pragma unroll
+        for (int x = 0; x < 2 * GROUPS; ++x) {
+          float2 before = unpack2(acc[i][x]), now = unpack2(o[i][x]);
+          acc[i][x] = pack2(merge_output(before.x, keep, now.x, take), merge_output(before.y, keep, now.y, take));
+        }
+      }
+      __syncthreads();  // everybody is done with the values and weights
+      if (p < page_last) copy_page(sm.v, pages[p + 1], 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (end[i] == 0) continue;
+      float inv = 1.0f / l_run[i];
+      float* row = out + ((size_t)(t0 + ty + 8 * i) * heads + h) * HD;
+#pragma unroll
+      for (int x = 0; x < GROUPS; ++x) {
+        float2 lo = unpack2(acc[i][2 * x]), hi = unpack2(acc[i][2 * x + 1]);
+        *(float4*)(row + 64 * x + 4 * tx) = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+      }
+    }
+    run_begin = run_end;
+  }
+}
+
+template <int HD>
+int launch_tiles(float* out, const float* q, const KvLayout& cache, const int* tok_seq, const int* tok_pos, const int* slots,
+                 int tokens, int heads, float scale, int window, cudaStream_t stream) {
+  static std::atomic<unsigned long long> allowed{0};
+  constexpr int smem = (int)sizeof(TileShared<HD>);
+  if (!dllm_allow_shared((const void*)attention_tile_kernel<HD>, smem, allowed)) return DLLM_LAUNCH_FAILED;
+  long long blocks = (long long)((tokens + TILE_Q - 1) / TILE_Q) * heads;
+  if (blocks > 0x7fffffffLL) return DLLM_UNSUPPORTED_SIZE;
+  attention_tile_kernel<HD><<<(unsigned)blocks, TILE_THREADS, smem, stream>>>(out, q, cache, tok_seq, tok_pos, slots, tokens,
+                                                                              heads, scale, window);
+  return dllm_launch_status();
+}
+
+// ---- float32 single tokens: chunks of keys side by side ------------------------------------------------------------------
+// Bound by latency: one token's heads over a few thousand keys are little work, so the chunks of 64 keys are dealt out to
+// the blocks of a cluster (chunk c to block c mod cluster size) and `per_round` of them at a time to the warps of a block,
+// a warp per (chunk, head). Every chunk's (m, l, o) stays in the shared memory of the block that made it; after one cluster
+// barrier each output dimension is merged over the chunks in ascending order by one thread of the cluster, reading them
+// through distributed shared memory. A second barrier keeps the blocks' memory alive until everybody has read.
+// Eight sequences of 50 to 700 tokens, 9 query and 3 kv heads of 64: 38.8 us a layer with a warp walking all keys of its
+// head, now 13.1 (both measured as launches of their own).
+constexpr int CHUNK_WARPS = 16;
+
+__global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
+    float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_seq,
+    const int* __restrict__ tok_pos, const int* __restrict__ slots, int heads, float scale, int window, int heads_per_block,
+    int per_round, int room) {
+  extern __shared__ __align__(16) float smem[];
+  int hd = cache.head_dim, ld = hd + 4, group = heads / cache.kv_heads, pieces = hd / 4;
+  int size = (int)gridDim.x, rank = (int)blockIdx.x;  // (a cluster is a row of the grid)
+  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = (int)blockDim.x;
+  int parts = (group + heads_per_block - 1) / heads_per_block;
+  int g = (int)blockIdx.y / parts, head0 = (int)blockIdx.y % parts * heads_per_block, t = (int)blockIdx.z;
+  int here = min(heads_per_block, group - head0);    // heads of this block: g * group + head0 + [0, here)
+  float* kv_s = smem;                                // [per_round][k|v][64][ld]
+  float* q_s = kv_s + (size_t)per_round * 2 * 64 * ld;          // [heads_per_block][hd]
+  float* result = q_s + (size_t)heads_per_block * hd;           // [room][heads_per_block][hd + 2]: o, m, l
+  pdl_launch_dependents();
+  pdl_wait();
+  int end = tok_pos[t] + 1, first = (window > 0 && end > window) ? end - window : 0;
+  const int* pages = cache.page_table + (size_t)slots[tok_seq[t]] * cache.max_pages;
+  int chunk0 = first / 64, chunks = min((end + 63) / 64 - chunk0, room * size);  // (`room` covers what the caller says)
+  for (int i = threadIdx.x; i < here * hd; i += threads)
+    q_s[i] = q[((size_t)t * heads + g * group + head0) * hd + i];
+  int mine = warp / heads_per_block, head = warp % heads_per_block;
+  for (int c0 = rank; c0 < chunks; c0 += size * per_round) {
+    // this round: chunks c0, c0 + size, ... (per_round of them at most)
+    __syncthreads();  // (everybody is done with the round before; the queries are there behind the next barrier)
+    for (int i = threadIdx.x; i < per_round * 128 * pieces; i += threads) {
+      int d = i % pieces * 4, row = i / pieces % 64, which = i / pieces / 64 & 1, n = i / pieces / 128;
+      int c = c0 + n * size;
+      if (c < chunks && (chunk0 + c) * 64 + row < end) {  // (nobody reads what lies behind the last key)
+        unsigned at = (unsigned)__cvta_generic_to_shared(kv_s + ((size_t)(n * 2 + which) * 64 + row) * ld + d);
+        const float* from = (const float*)cache.base + kv_offset(cache, pages[chunk0 + c], which, g, row) + d;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(from));
+      }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    int c = c0 + mine * size;
+    if (mine < per_round && head < here && c < chunks) {
+      const float* k_s = kv_s + (size_t)mine * 128 * ld;
+      const float* v_s = k_s + 64 * ld;
+      const float* query = q_s + head * hd;
+      int j0 = (chunk0 + c) * 64;
+      float2 dot[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 4
+      for (int d = 0; d < hd; d += 4) {
+        float4 piece = *(const float4*)(query + d);
+        float values[4] = {piece.x, piece.y, piece.z, piece.w};
+        score_piece(dot[0], values, load_vec(k_s + lane * ld + d));
+        score_piece(dot[1], values, load_vec(k_s + (lane + 32) * ld + d));
+      }
+      float p[2];
+      bool valid[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        int j = j0 + lane + 32 * u;
+        valid[u] = j >= first && j < end;
+        p[u] = valid[u] ? (dot[u].x + dot[u].y) * scale : -INFINITY;
+      }
+      float m = warp_max(fmaxf(p[0], p[1])), shift = finite_or_zero(m);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) p[u] = valid[u] ? expf(p[u] - shift) : 0.f;
+      float l = warp_sum(p[0] + p[1]);
+      int from = max(0, first - j0), to = min(64, end - j0);
+      float* slot = result + ((size_t)(c / size) * heads_per_block + head) * (hd + 2);
+      for (int d0 = 0; d0 < hd; d0 += 64) {  // two dimensions a lane
+        float o0 = 0.f, o1 = 0.f;
+        const float* column = v_s + d0 + lane;
+        bool has0 = d0 + lane < hd, has1 = d0 + lane + 32 < hd;
+        auto step = [&](int at) {
+          float w = __shfl_sync(0xffffffffu, at < 32 ? p[0] : p[1], at & 31);
+          if (has0) o0 = fmaf(w, column[at * ld], o0);
+          if (has1) o1 = fmaf(w, column[at * ld + 32], o1);
+        };
+        if (from == 0 && to == 64) {
+#pragma unroll 16
+          for (int at = 0; at < 64; ++at) step(at);
+        } else {
+          for (int at = from; at < to; ++at) step(at);
+        }
+        if (has0) slot[d0 + lane] = o0;
+        if (has1) slot[d0 + lane + 32] = o1;
+      }
+      if (lane == 0) {
+        slot[hd] = m;
+        slot[hd + 1] = l;
+      }
+    }
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+  unsigned local = (unsigned)__cvta_generic_to_shared(result);
+  for (int i = rank * threads + threadIdx.x; i < here * hd; i += size * threads) {
+    int head_at = i / hd, d = i % hd;
+    float m_run = -INFINITY, l_run = 0.f, acc = 0.f;
+    for (int base = 0; base < chunks; base += 8) {  // (eight chunks' values are asked for before the first is merged)
+      float o[8], m[8], l[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        int c = base + x;
+        if (c >= chunks) continue;
+        unsigned at = local + 4u * (unsigned)(((c / size) * heads_per_block + head_at) * (hd + 2)), far;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(c % size));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o[x]) : "r"(far + 4u * (unsigned)d));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m[x]) : "r"(far + 4u * (unsigned)hd));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[x]) : "r"(far + 4u * (unsigned)hd + 4u));
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        if (base + x >= chunks) continue;
+        float keep, take;
+        merge(m_run, l_run, m[x], l[x], keep, take);
+        acc = merge_output(acc, keep, o[x], take);
+      }
+    }
+    out[((size_t)t * heads + g * group + head0) * hd + i] = acc * (1.0f / l_run);
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+
+// Refuses (DLLM_UNSUPPORTED_SIZE) what does not fit; the caller then takes the serial form, which gives the same bits.
+// `reach`: the most keys a token may see.
+int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* tok_seq, const int* tok_pos, const int* slots,
+                  int tokens, int heads, float scale, int window, long long reach, cudaStream_t stream) {
+  int group = heads / cache.kv_heads, hd = cache.head_dim, ld = hd + 4;
+  // (a window of w keys may begin anywhere in its first chunk)
+  long long chunks = (reach + 63) / 64;
+  if (window > 0 && window < reach) chunks = ((long long)window + 126) / 64;
+  if (tokens > 65535) return DLLM_UNSUPPORTED_SIZE;
+  int heads_per_block = group < CHUNK_WARPS ? group : CHUNK_WARPS;
+  int parts = (group + heads_per_block - 1) / heads_per_block;
+  long long rows = (long long)cache.kv_heads * parts;
+  if (rows > 65535) return DLLM_UNSUPPORTED_SIZE;
+  // As many blocks a cluster as there are chunks, up to 8, while three a multiprocessor hold them all.
+  int size = 1;
+  while (size < 8 && size < chunks && rows * tokens * size * 2 <= 3 * 148) size *= 2;
+  // As many chunks a round as give a block at least eight warps' work, within what shared memory holds beside the results.
+  int room = (int)((chunks + size - 1) / size), per_round = 1;
+  auto bytes = [&](int n) {
+    return ((size_t)n * 128 * ld + (size_t)heads_per_block * hd + (size_t)room * heads_per_block * (hd + 2)) * sizeof(float);
+  };
+  if (bytes(1) > 200 * 1024) return DLLM_UNSUPPORTED_SIZE;
+  while ((per_round + 1) * heads_per_block <= 8 && per_round < room && bytes(per_round + 1) <= 110 * 1024) ++per_round;
+  static std::atomic<unsigned long long> allowed{0};
+  if (!dllm_allow_shared((const void*)attention_chunks_kernel, 200 * 1024, allowed)) return DLLM_LAUNCH_FAILED;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(size, (unsigned)rows, tokens);
+  config.blockDim = dim3(32 * heads_per_block * per_round);
+  config.dynamicSmemBytes = bytes(per_round);
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = size;
+  attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&config, attention_chunks_kernel, out, q, cache, tok_seq, tok_pos, slots, heads, scale, window,
+                            heads_per_block, per_round, room) == cudaSuccess
+             ? DLLM_OK
+             : DLLM_LAUNCH_FAILED;
 }
 }  // namespace
 
@@ -377,13 +834,16 @@ DLLM_EXPORT int dllm_attention_general(void* out, const void* q, void* cache_bas
   return dllm_launch_status();
 }
 
-// The same attention with the same arguments, blockwise (see attention_block_kernel). `max_new`: the most new
-// tokens a sequence brings in this step: with one each (decoding) a block serves one token's heads, else runs of
-// tokens with two tokens a warp. Pages of 64 positions, at most 65,535 kv heads.
+// The same attention with the same arguments, blockwise; the same bits. `max_new`: the most new tokens a sequence brings
+// in this step: with one each (decoding) a block serves one token's heads, else runs of tokens. `max_context`: the most
+// keys any token of the step may see. Pages of 64 positions, at most 65,535 kv heads.
+// float32 takes the kernels made for it: single tokens their chunks side by side, prompts with heads of 64 and 128 in
+// 16-byte aligned rows the tiles of queries.
 DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base, const int* page_table,
                                       int max_pages, int page_size, int heads, int kv_heads, int head_dim,
                                       const int* tok_seq, const int* tok_pos, const int* slots, int tokens,
-                                      int max_new, float scale, int window, int dtype, cudaStream_t stream) {
+                                      int max_new, int max_context, float scale, int window, int dtype,
+                                      cudaStream_t stream) {
   if (tokens <= 0) return DLLM_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads) return DLLM_BAD_ARGUMENT;
   if (head_dim <= 0 || head_dim > MAX_HEAD_DIM || (head_dim & 7) || page_size != 64 || kv_heads > 65535)
@@ -399,6 +859,17 @@ DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base
   else if (chunks <= 4) DLLM_GO(T, R, 4);     \
   else DLLM_GO(T, R, 8)
   if (dtype == DLLM_F32) {
+    const float* rows = (const float*)q;
+    bool aligned = (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
+    if (!runs) {
+      int status = launch_chunks((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window,
+                                 max_context > 0 ? max_context : (long long)max_pages * page_size, stream);
+      if (status != DLLM_UNSUPPORTED_SIZE) return status;
+    } else if (head_dim == 64 && aligned) {
+      return launch_tiles<64>((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window, stream);
+    } else if (head_dim == 128 && aligned) {
+      return launch_tiles<128>((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window, stream);
+    }
     if (runs) { DLLM_BY_WIDTH(float, 4); }
     DLLM_BY_WIDTH(float, 1);
   }

@@ -233,8 +233,8 @@ _prototypes = {
                                               c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int,
                                               c_void_p],
     ("attention", "dllm_attention_blocks"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                             c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_int,
-                                             c_void_p],
+                                             c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
+                                             c_int, c_void_p],
     ("attention_decode", "dllm_attention_decode"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                                     c_int, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int,
                                                     c_void_p, c_void_p, c_void_p],
@@ -2130,17 +2130,17 @@ def attention_blocks_supported(cache) -> bool:
 
 
 def attention_blocks(out: torch.Tensor, q: torch.Tensor, cache, heads: int, scale: float, window: int, batch) -> None:
-    """`attention_general` blockwise: the keys and values of a kv head go through shared memory page by page and
-    serve every (token, head) pair of a run of tokens at once. Without a window a pair's result has the same bits
-    as `attention_general` gives; with one the same formula is rounded in other places. The float32 path's attention,
-    for whole prompts and single tokens alike."""
+    """`attention_general` blockwise: the keys and values of a kv head go through shared memory page by page and serve
+    many (token, head) pairs; single tokens in float32 have their chunks of 64 keys worked on side by side. The bits are
+    `attention_general`'s, and those a token gets alone or in any other cut. The float32 path's attention, for whole
+    prompts and single tokens alike."""
     _cuda(out, q)
     assert q.dtype == cache.dtype and out.dtype == cache.dtype and attention_blocks_supported(cache)
     _check(_fn("attention", "dllm_attention_blocks")(
         out.data_ptr(), q.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(), cache.max_pages, cache.page_size,
         heads, cache.kv_heads, cache.head_dim, batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(),
-        batch.slots.data_ptr(), batch.n_tokens, int(batch.max_new), float(scale), int(window or 0),
-        _code(cache.dtype), _stream()), "attention_blocks",
+        batch.slots.data_ptr(), batch.n_tokens, int(batch.max_new), int(batch.max_context), float(scale),
+        int(window or 0), _code(cache.dtype), _stream()), "attention_blocks",
         lambda: f"head_dim={cache.head_dim} must be a multiple of 8, at most 256; pages of 64")
 
 

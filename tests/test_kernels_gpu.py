@@ -347,6 +347,25 @@ def test_attention_blocks(dtype, tol, heads, kv_heads, head_dim, window, decode)
         assert torch.equal(alone[0], out[token])
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,window,lengths,new", [
+    (3, 1, 64, None, [31, 64, 1, 65, 33], [31, 64, 1, 2, 33]), (2, 2, 128, None, [97, 130], [97, 66]),
+    (9, 3, 64, 100, [300, 260], [300, 40]), (4, 1, 128, 64, [191], [191]), (9, 3, 64, None, [2300, 700, 64], [1, 1, 1]),
+    (32, 32, 64, None, [513, 1], [1, 1]), (20, 1, 16, 65, [400, 64, 65], [1, 1, 1]), (40, 2, 128, None, [1024], [1])])
+def test_attention_float32_bits(heads, kv_heads, head_dim, window, lengths, new):
+    """The float32 kernels (tiles of queries for prompts, chunks side by side for single tokens) against the kernel of one
+    warp a (token, head): the same bits with and without a window, and no NaN from positions that a token does not see."""
+    cache, view, batch = _cache_and_batch(torch.float32, kv_heads, head_dim, lengths, new)  # (no page is given back)
+    table = view.page_table.cpu()
+    for slot, length in zip(batch.h_slots, lengths):  # behind the last key of a sequence: whatever was there
+        if length % 64:
+            view.storage[int(table[slot, (length - 1) // 64]), :, :, length % 64:] = float("nan")
+    q = _randn((batch.n_tokens, heads * head_dim), torch.float32, 9)
+    out, other = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    ops().attention_blocks(out, q, view, heads, 0.3, window or 0, batch)
+    ops().attention_general(other, q, view, heads, 0.3, window or 0, batch)
+    assert bool(torch.isfinite(out).all()) and torch.equal(out, other)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_finds_a_far_key(dtype):
     """One key among hundreds matches the query: the output must be that key's value, wherever its page lies."""
