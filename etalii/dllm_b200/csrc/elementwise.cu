@@ -204,43 +204,103 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
   *reinterpret_cast<uint2*>(dst) = packed;
 }
 
-// Narrow rows (hidden a multiple of 4, at most 4096 floats): one warp per row, the row kept in registers between
-// the sum and the scaling, 16-byte loads. Lane l holds floats 4*(l + 32*i) ..; the sum is a fixed tree.
-template <typename T>
-__global__ void __launch_bounds__(256) rmsnorm_warp_kernel(T* __restrict__ out, const float* __restrict__ x,
-                                                           const float* __restrict__ weight,
-                                                           const int* __restrict__ rows, int n_rows, int hidden,
-                                                           float eps) {
+// Narrow rows (hidden a multiple of 4, at most 4096 floats), for the RMS norm and, CENTRED, for the layer norm: the row
+// stays in registers between the sums and the scaling, 16-byte loads. A row's pieces of 32 x 4 floats are dealt out to
+// eight strands; a lane sums each strand's values of its own, then the eight strands in order, then a fixed tree adds
+// the lanes. WARPS is 1 (a warp holds all eight strands of its row, eight rows a block) or 8 (a warp of the row's block
+// holds one strand): the same sums in the same order, so the same bits, whichever is launched.
+// A few rows are bounded by latency: one warp's chain of up to 32 loads and 128 multiply-adds, then the weight's loads.
+// With a block a row the chains are an eighth as long, and the weight, which no kernel of a step writes, is asked for
+// before the kernel in front has finished. One row of 4,096: 3.4 -> 1.4 us as a link of a
+// chain; eight of 2,048: 3.0 -> 1.4; layer norm of eight of 2,048: 3.4 -> 1.6.
+template <typename T, int WARPS, bool CENTRED>
+__global__ void __launch_bounds__(256) norm_rows_kernel(T* __restrict__ out, const float* __restrict__ x,
+                                                        const float* __restrict__ weight, const int* __restrict__ rows,
+                                                        int n_rows, int hidden, float eps) {
+  constexpr int STRANDS = 8 / WARPS, PER = 4;  // strands a warp holds, pieces of a strand
+  __shared__ float strand_sums[2][WARPS == 8 ? 8 : 1][32];
+  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, vecs = hidden >> 2;
+  int r = WARPS == 8 ? (int)blockIdx.x : (int)blockIdx.x * 8 + warp;
   pdl_launch_dependents();
-  pdl_wait();
-  int lane = threadIdx.x & 31;
-  int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (r >= n_rows) return;
-  const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * hidden);
-  int vecs = hidden >> 2;
-  float4 v[32];
-  float sum = 0.f;
+  const float4* wv = reinterpret_cast<const float4*>(weight);
+  float4 early[WARPS == 8 ? PER : 1];
+  if (WARPS == 8) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    int idx = lane + 32 * i;
-    if (idx < vecs) {
-      v[i] = src[idx];
-      sum = fmaf(v[i].x, v[i].x, sum); sum = fmaf(v[i].y, v[i].y, sum);
-      sum = fmaf(v[i].z, v[i].z, sum); sum = fmaf(v[i].w, v[i].w, sum);
+    for (int j = 0; j < PER; ++j) {
+      int idx = lane + 32 * (8 * j + warp);
+      if (idx < vecs) early[WARPS == 8 ? j : 0] = wv[idx];
     }
   }
-  sum = warp_sum(sum);
-  float inv = 1.0f / sqrtf(sum / (float)hidden + eps);
-  const float4* wv = reinterpret_cast<const float4*>(weight);
+  pdl_wait();
+  if (r >= n_rows) return;  // (never in a block whose warps meet below)
+  const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * hidden);
+  float4 v[STRANDS][PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j)
+#pragma unroll
+    for (int s = 0; s < STRANDS; ++s) {
+      int idx = lane + 32 * (8 * j + (WARPS == 8 ? warp : s));
+      if (idx < vecs) v[s][j] = src[idx];
+    }
+  auto row_sum = [&](int which, auto add) {  // `add(sum, vector)` over every strand's pieces; the row's total, in every lane
+    float sums[STRANDS];
+#pragma unroll
+    for (int s = 0; s < STRANDS; ++s) {
+      sums[s] = 0.f;
+#pragma unroll
+      for (int j = 0; j < PER; ++j)
+        if (lane + 32 * (8 * j + (WARPS == 8 ? warp : s)) < vecs) add(sums[s], v[s][j]);
+    }
+    float total = 0.f;
+    if (WARPS == 8) {
+      strand_sums[which][WARPS == 8 ? warp : 0][lane] = sums[0];
+      __syncthreads();
+#pragma unroll
+      for (int s = 0; s < 8; ++s) total += strand_sums[which][WARPS == 8 ? s : 0][lane];
+    } else {
+#pragma unroll
+      for (int s = 0; s < STRANDS; ++s) total += sums[s];
+    }
+    return warp_sum(total);
+  };
+  if (CENTRED) {
+    float mean = row_sum(1, [](float& sum, const float4& u) { sum += (u.x + u.y) + (u.z + u.w); }) / (float)hidden;
+#pragma unroll
+    for (int s = 0; s < STRANDS; ++s)
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        v[s][j].x -= mean; v[s][j].y -= mean; v[s][j].z -= mean; v[s][j].w -= mean;
+      }
+  }
+  float squares = row_sum(0, [](float& sum, const float4& u) {
+    sum = fmaf(u.x, u.x, sum); sum = fmaf(u.y, u.y, sum);
+    sum = fmaf(u.z, u.z, sum); sum = fmaf(u.w, u.w, sum);
+  });
+  float inv = 1.0f / sqrtf(squares / (float)hidden + eps);
   T* dst = out + (size_t)r * hidden;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    int idx = lane + 32 * i;
-    if (idx < vecs) {
-      float4 w4 = wv[idx];
-      store4(dst + 4 * idx, v[i].x * inv * w4.x, v[i].y * inv * w4.y, v[i].z * inv * w4.z, v[i].w * inv * w4.w);
+  for (int j = 0; j < PER; ++j)
+#pragma unroll
+    for (int s = 0; s < STRANDS; ++s) {
+      int idx = lane + 32 * (8 * j + (WARPS == 8 ? warp : s));
+      if (idx < vecs) {
+        float4 w4 = WARPS == 8 ? early[WARPS == 8 ? j : 0] : wv[idx];
+        float4 u = v[s][j];
+        store4(dst + 4 * idx, u.x * inv * w4.x, u.y * inv * w4.y, u.z * inv * w4.z, u.w * inv * w4.w);
+      }
     }
-  }
+}
+
+// A block a row for up to four rows a multiprocessor of at least 512 values (beyond that the device is full with a warp a
+// row, and narrower rows do not fill eight warps).
+template <typename T, bool CENTRED>
+int launch_norm_rows(T* out, const float* x, const float* weight, const int* rows, int n_rows, int hidden, float eps,
+                     cudaStream_t stream) {
+  if (n_rows <= 4 * 148 && hidden >= 512)
+    return dllm_launch_pdl(norm_rows_kernel<T, 8, CENTRED>, dim3(n_rows), dim3(256), 0, stream, out, x, weight, rows, n_rows,
+                           hidden, eps);
+  return dllm_launch_pdl(norm_rows_kernel<T, 1, CENTRED>, dim3((n_rows + 7) / 8), dim3(256), 0, stream, out, x, weight, rows,
+                         n_rows, hidden, eps);
 }
 
 // One norm for several readers: h = x[r] / rms(x[r]) * w goes to `plain` (rows of `hidden` values), to `ones` (rows of
@@ -320,13 +380,9 @@ DLLM_EXPORT int dllm_rmsnorm(void* out, const float* x, const float* weight, con
   if (n_rows <= 0) return DLLM_OK;
   if (hidden <= 0) return DLLM_BAD_ARGUMENT;
   if ((hidden & 3) == 0 && hidden <= 4096) {  // whatever the number of rows, so a row has the same bits everywhere
-    int blocks = (n_rows + 7) / 8;
-    if (out_dtype == DLLM_F32)
-      return dllm_launch_pdl(rmsnorm_warp_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)out, x, weight, rows,
-                             n_rows, hidden, eps);
+    if (out_dtype == DLLM_F32) return launch_norm_rows<float, false>((float*)out, x, weight, rows, n_rows, hidden, eps, stream);
     if (out_dtype == DLLM_BF16)
-      return dllm_launch_pdl(rmsnorm_warp_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream,
-                             (__nv_bfloat16*)out, x, weight, rows, n_rows, hidden, eps);
+      return launch_norm_rows<__nv_bfloat16, false>((__nv_bfloat16*)out, x, weight, rows, n_rows, hidden, eps, stream);
     return DLLM_BAD_ARGUMENT;
   }
   int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
@@ -583,66 +639,14 @@ __global__ void layernorm_kernel(T* __restrict__ out, const float* __restrict__ 
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) dst[i] = from_float<T>((src[i] - mean) * inv * weight[i]);
 }
 
-// Narrow rows (hidden a multiple of 4, at most 4096 floats): one warp per row, the row kept in registers between the
-// mean, the squared deviations and the scaling (one pass over memory), 16-byte loads, sums in a fixed tree.
-template <typename T>
-__global__ void __launch_bounds__(256) layernorm_warp_kernel(T* __restrict__ out, const float* __restrict__ x,
-                                                             const float* __restrict__ weight,
-                                                             const int* __restrict__ rows, int n_rows, int hidden,
-                                                             float eps) {
-  pdl_launch_dependents();
-  pdl_wait();
-  int lane = threadIdx.x & 31;
-  int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (r >= n_rows) return;
-  const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * hidden);
-  int vecs = hidden >> 2;
-  float4 v[32];
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    int idx = lane + 32 * i;
-    if (idx < vecs) {
-      v[i] = src[idx];
-      sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-    }
-  }
-  float mean = warp_sum(sum) / (float)hidden;
-  float squares = 0.f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    int idx = lane + 32 * i;
-    if (idx < vecs) {
-      v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
-      squares = fmaf(v[i].x, v[i].x, squares); squares = fmaf(v[i].y, v[i].y, squares);
-      squares = fmaf(v[i].z, v[i].z, squares); squares = fmaf(v[i].w, v[i].w, squares);
-    }
-  }
-  float inv = 1.0f / sqrtf(warp_sum(squares) / (float)hidden + eps);
-  const float4* wv = reinterpret_cast<const float4*>(weight);
-  T* dst = out + (size_t)r * hidden;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    int idx = lane + 32 * i;
-    if (idx < vecs) {
-      float4 w4 = wv[idx];
-      store4(dst + 4 * idx, v[i].x * inv * w4.x, v[i].y * inv * w4.y, v[i].z * inv * w4.z, v[i].w * inv * w4.w);
-    }
-  }
-}
-
 DLLM_EXPORT int dllm_layernorm(void* out, const float* x, const float* weight, const int* rows, int n_rows, int hidden,
                                float eps, int out_dtype, cudaStream_t stream) {
   if (n_rows <= 0) return DLLM_OK;
   if (hidden <= 0) return DLLM_BAD_ARGUMENT;
   if ((hidden & 3) == 0 && hidden <= 4096) {  // whatever the number of rows, so a row has the same bits everywhere
-    int blocks = (n_rows + 7) / 8;
-    if (out_dtype == DLLM_F32)
-      return dllm_launch_pdl(layernorm_warp_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)out, x, weight,
-                             rows, n_rows, hidden, eps);
+    if (out_dtype == DLLM_F32) return launch_norm_rows<float, true>((float*)out, x, weight, rows, n_rows, hidden, eps, stream);
     if (out_dtype == DLLM_BF16)
-      return dllm_launch_pdl(layernorm_warp_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream,
-                             (__nv_bfloat16*)out, x, weight, rows, n_rows, hidden, eps);
+      return launch_norm_rows<__nv_bfloat16, true>((__nv_bfloat16*)out, x, weight, rows, n_rows, hidden, eps, stream);
     return DLLM_BAD_ARGUMENT;
   }
   int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
@@ -756,10 +760,87 @@ __global__ void norm_sum_residual_kernel(float* __restrict__ residual, const flo
     residual[base + i] += factor * (a[base + i] * inv_a * wa[i] + b[base + i] * inv_b * wb[i]);
 }
 
+// The same for rows of a multiple of 4 values, 4,096 at most, 16-byte aligned: a thread keeps its values of a, b and the
+// residual in registers (the row is read once), both sums meet at one barrier, and the weights are asked for before the
+// kernel in front has finished. Eight rows of 2,048: 3.5 -> 1.7 us; 8,192 rows: 89 -> 40 us.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) norm_sum_residual_vector_kernel(
+    float* __restrict__ residual, const float* __restrict__ a, const float* __restrict__ wa, const float* __restrict__ b,
+    const float* __restrict__ wb, int hidden, float eps, float factor) {
+  __shared__ float sums[2][THREADS / 32];
+  constexpr int PER = 4;
+  pdl_launch_dependents();
+  int vecs = hidden >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float4 va[PER], vb[PER], old[PER], ka[PER], kb[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    int idx = threadIdx.x + THREADS * i;
+    if (idx < vecs) {
+      ka[i] = reinterpret_cast<const float4*>(wa)[idx];
+      kb[i] = reinterpret_cast<const float4*>(wb)[idx];
+    }
+  }
+  pdl_wait();
+  size_t base = (size_t)blockIdx.x * hidden;
+  float4* res = reinterpret_cast<float4*>(residual + base);
+  float sa = 0.f, sb = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    int idx = threadIdx.x + THREADS * i;
+    if (idx < vecs) {
+      va[i] = reinterpret_cast<const float4*>(a + base)[idx];
+      vb[i] = reinterpret_cast<const float4*>(b + base)[idx];
+      old[i] = res[idx];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    if (threadIdx.x + THREADS * i < vecs) {
+      sa = fmaf(va[i].x, va[i].x, sa); sa = fmaf(va[i].y, va[i].y, sa);
+      sa = fmaf(va[i].z, va[i].z, sa); sa = fmaf(va[i].w, va[i].w, sa);
+      sb = fmaf(vb[i].x, vb[i].x, sb); sb = fmaf(vb[i].y, vb[i].y, sb);
+      sb = fmaf(vb[i].z, vb[i].z, sb); sb = fmaf(vb[i].w, vb[i].w, sb);
+    }
+  }
+  sa = warp_sum(sa);
+  sb = warp_sum(sb);
+  if (lane == 0) {
+    sums[0][warp] = sa;
+    sums[1][warp] = sb;
+  }
+  __syncthreads();
+  float ta = 0.f, tb = 0.f;
+#pragma unroll
+  for (int w = 0; w < THREADS / 32; ++w) {
+    ta += sums[0][w];
+    tb += sums[1][w];
+  }
+  float inv_a = 1.0f / sqrtf(ta / (float)hidden + eps), inv_b = 1.0f / sqrtf(tb / (float)hidden + eps);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    int idx = threadIdx.x + THREADS * i;
+    if (idx < vecs)
+      res[idx] = make_float4(old[i].x + factor * (va[i].x * inv_a * ka[i].x + vb[i].x * inv_b * kb[i].x),
+                             old[i].y + factor * (va[i].y * inv_a * ka[i].y + vb[i].y * inv_b * kb[i].y),
+                             old[i].z + factor * (va[i].z * inv_a * ka[i].z + vb[i].z * inv_b * kb[i].z),
+                             old[i].w + factor * (va[i].w * inv_a * ka[i].w + vb[i].w * inv_b * kb[i].w));
+  }
+}
+
 DLLM_EXPORT int dllm_norm_sum_residual(float* residual, const float* a, const float* wa, const float* b, const float* wb,
                                        int rows, int hidden, float eps, float factor, cudaStream_t stream) {
   if (rows <= 0) return DLLM_OK;
   if (hidden <= 0) return DLLM_BAD_ARGUMENT;
+  bool aligned = (((uintptr_t)residual | (uintptr_t)a | (uintptr_t)wa | (uintptr_t)b | (uintptr_t)wb) & 15) == 0;
+  if ((hidden & 3) == 0 && hidden <= 4096 && aligned) {  // (whatever the number of rows: a row has the same bits everywhere)
+    // as few threads as hold the row: 2,048 rows of 576 took 8.6 us with 256 threads, 6.9 in the kernel above
+    auto go = [&](auto kernel, int threads) {
+      return dllm_launch_pdl(kernel, dim3(rows), dim3(threads), 0, stream, residual, a, wa, b, wb, hidden, eps, factor);
+    };
+    if (hidden <= 1024) return go(norm_sum_residual_vector_kernel<64>, 64);
+    if (hidden <= 2048) return go(norm_sum_residual_vector_kernel<128>, 128);
+    return go(norm_sum_residual_vector_kernel<256>, 256);
+  }
   int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
   return dllm_launch_pdl(norm_sum_residual_kernel, dim3(rows), dim3(threads), 0, stream, residual, a, wa, b, wb, hidden,
                          eps, factor);

@@ -59,6 +59,35 @@ def test_rmsnorm(dtype, tol, hidden, eps):
     assert torch.equal(out3, out[rows.long()])  # a gathered row has the same bits as the row in place
 
 
+@pytest.mark.parametrize("hidden", [512, 576, 1028, 2052, 4096])
+@pytest.mark.parametrize("centred", [False, True])
+def test_norm_rows_have_the_same_bits_among_few_and_many(hidden, centred):
+    """A block a row (up to 592 rows) and a warp a row (more) give a row the same bits, in float32 and rounded, with rows
+    that do not fill all eight strands and rows that do; against float64: a sum of `hidden` squares in float32."""
+    norm = ops().layernorm if centred else ops().rmsnorm
+    x, w = _randn((593, hidden), torch.float32, 1, 3.0), _randn((hidden,), torch.float32, 2) + 1
+    for dtype in (torch.float32, torch.bfloat16):
+        many, few = (torch.empty((n, hidden), dtype=dtype, device=DEV) for n in (593, 592))
+        norm(many, x, w, 1e-5)
+        norm(few, x[:592].contiguous(), w, 1e-5)
+        assert torch.equal(few, many[:592])
+    norm(out := torch.empty_like(x), x, w, 1e-5)
+    y = x.double() - (x.double().mean(-1, keepdim=True) if centred else 0.0)
+    want = y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert rel_error(out.cpu(), want.float().cpu()) <= 1e-6
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 4), (3, 1028), (8, 2048), (600, 4096), (2, 4100), (5, 70)])
+def test_norm_sum_residual(rows, hidden):
+    """Rows that fit into a thread's registers and rows that do not (over 4,096, no multiple of 4), against float64."""
+    x, a, b = (_randn((rows, hidden), torch.float32, s, 2.0) for s in (1, 2, 3))
+    wa, wb = (_randn((hidden,), torch.float32, s) + 1 for s in (4, 5))
+    norm = lambda y: y.double() * torch.rsqrt((y.double() ** 2).mean(-1, keepdim=True) + 1e-6)  # noqa: E731
+    want = x.double() + 0.5 * (norm(a) * wa.double() + norm(b) * wb.double())
+    ops().norm_sum_residual(x, a, wa, b, wb, 1e-6, 0.5)
+    assert rel_error(x.cpu(), want.float().cpu()) <= 1e-6
+
+
 GEMM_SHAPES = [(1, 64, 64), (3, 130, 72), (16, 96, 144), (17, 200, 136), (40, 576, 1536), (64, 130, 72), (77, 384, 160), (130, 66, 1544), (300, 258, 576)]
 
 
