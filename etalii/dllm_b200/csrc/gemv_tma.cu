@@ -2,15 +2,23 @@
 // where reading W once from HBM is the whole cost, so what counts is how many bytes are on their way at any time.
 // Here they travel into shared memory, not into registers: a producer warp issues bulk copies (cp.async.bulk, 2 KB
 // of one row of W or X per copy, completion counted by an mbarrier) into a ring of stages that holds about 200 KB
-// per multiprocessor, and two consumer warps multiply out of shared memory on the tensor cores (mma.sync m16n8k16
+// per multiprocessor, and consumer warps multiply out of shared memory on the tensor cores (mma.sync m16n8k16
 // with W as the 16-row operand, ldmatrix from rows padded by 16 bytes so that no two rows share a bank).
-// Blocks are persistent: a block walks over its tiles of 16 or 32 rows of W and the ring runs on across tiles.
-//   ROWS = 32: each consumer warp owns 16 rows of W over the whole reduction (no exchange between warps);
-//   ROWS = 16: the two warps share the rows and take alternate 16-value steps; the second hands its sums to the
-//              first.
-// Epilogues as the tile kernels: store (float32 / bfloat16), residual add in float32, SwiGLU on interleaved rows.
-// K must be a multiple of 64. Every wait on an mbarrier is bounded; a role that gives up records a status word.
-#include "gemm_common.cuh"
+// Blocks are persistent: a block walks over its tiles of W and the ring runs on across tiles.
+//   ROWS = 32: a tile is `height` rows (an even number, at most 32: the height that leaves the busiest multiprocessor the
+//              fewest rows, e.g. 147 tiles of 28 for 4,096 rows, where 128 tiles of 32 left 20 multiprocessors idle);
+//   ROWS = 16: sixteen rows (the q/k/v projection, whose tiles are eight rotary pairs).
+// Sixteen rows are the work of four consumer warps, which take 16-value steps in turn and add their sums in order: a
+// step is a chain of ldmatrix and product, so one warp gets through one about every 35 cycles, and two warps for a tile
+// could not keep up with memory. One row, before all of this (two consumers, tiles of 32 or 16) and now: 28672 x 4096 41.5 ->
+// 36.6 us, 128256 x 4096 167.5 -> 146.9, 4096 x 14336 23.6 -> 23.0, 4096 x 4096 8.7 -> 7.7; eight rows of 28672 x 4096
+// 51.2 -> 41.8.
+// RESIDENT: the rows of X lie in shared memory for the whole kernel, copied once, and the ring carries nothing but W. (As
+// a part of every stage they cost a copy a row and stage: with eight rows a quarter of all copies.) Where they take more
+// than 72 KB they stay a part of the stages.
+// Epilogues as the tile kernels: store (float32 / bfloat16), residual add in float32, SwiGLU on interleaved rows; rotation
+// and cache write behind the q/k/v projection. K must be a multiple of 64. Every wait on an mbarrier is bounded; a role that gives up records a status word.
+#include "gemv_common.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -20,7 +28,7 @@ constexpr int KC = 1024;                   // values of k per stage: 2 KB of eve
                                            // issuer about as much whatever its size, so copies are long)
 constexpr int ROW_BYTES = KC * 2;
 constexpr int PITCH = ROW_BYTES + 16;      // rows in shared memory: 16 bytes of padding (ldmatrix without conflicts)
-constexpr int THREADS = 96;                // warp 0 copies, warps 1 and 2 multiply
+constexpr int K_PARTS = 4;                 // consumer warps that share 16 rows of W
 constexpr int RING_BYTES = 216 * 1024;
 
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
@@ -34,65 +42,91 @@ __device__ __forceinline__ void ldmatrix_x4(unsigned* r, unsigned addr) {
 __device__ __forceinline__ void ldmatrix_x2(unsigned* r, unsigned addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
-__device__ __forceinline__ void mma_bf16(float* c, const unsigned* a, unsigned b0, unsigned b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+using gemv::mma_bf16;
 
-template <int ROWS, int NT> struct Shape {
+constexpr int RESIDENT_BYTES = 72 * 1024;  // the most that resident rows of X may take
+constexpr int MAX_CHUNKS = 32;             // stages a row of resident X may span (their arrivals are counted one by one)
+
+template <int ROWS, int NT, bool RESIDENT> struct Shape {
   static constexpr int TOKENS = NT * 8;                          // token rows of a stage (those beyond M stay unused)
-  static constexpr int STAGE_BYTES = (ROWS + TOKENS) * PITCH;
-  static constexpr int STAGES = RING_BYTES / STAGE_BYTES;
-  static constexpr int SCRATCH_FLOATS = 2 * 16 * (TOKENS + 1);   // a 16 x TOKENS tile per consumer warp
-  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + SCRATCH_FLOATS * sizeof(float) + 128;
+  static constexpr int STAGE_BYTES = (ROWS + (RESIDENT ? 0 : TOKENS)) * PITCH;
+  static constexpr int MAX_STAGES = RING_BYTES / STAGE_BYTES;
+  static constexpr int CONSUMERS = ROWS / 16 * K_PARTS, THREADS = 32 * (1 + CONSUMERS);  // (warp 0 copies)
+  static constexpr int SCRATCH_FLOATS = CONSUMERS * 16 * (TOKENS + 1);  // a 16 x TOKENS tile per consumer warp
+  // (resident rows of X, then the ring in what is left)
+  static int x_bytes(int M, int K) { return RESIDENT ? M * (2 * K + 16) : 0; }
+  static int stages(int M, int K) { return (RING_BYTES - x_bytes(M, K)) / STAGE_BYTES; }
+  static size_t smem(int M, int K) {
+    return (size_t)x_bytes(M, K) + (size_t)stages(M, K) * STAGE_BYTES + SCRATCH_FLOATS * sizeof(float) + 128;
+  }
+  static constexpr int MAX_SMEM = RING_BYTES + SCRATCH_FLOATS * (int)sizeof(float) + 128;
 };
 
-template <int ROWS, int NT, int EPI>
-__global__ void __launch_bounds__(THREADS, 1) gemv_tma_kernel(void* __restrict__ c, const bf16* __restrict__ x,
+template <int ROWS, int NT, int EPI, bool RESIDENT>
+__global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tma_kernel(void* __restrict__ c, const bf16* __restrict__ x,
                                                               const bf16* __restrict__ w, int M, int N, int K,
-                                                              int tiles, int* __restrict__ status) {
-  typedef Shape<ROWS, NT> S;
+                                                              int tiles, int height, int stages, int* __restrict__ status,
+                                                              RopeArgs rope) {
+  typedef Shape<ROWS, NT, RESIDENT> S;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* ring = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-  float* scratch = reinterpret_cast<float*>(ring + (size_t)S::STAGES * S::STAGE_BYTES);
-  __shared__ uint64_t full_bar[S::STAGES], empty_bar[S::STAGES];
+  unsigned char* x_s = (unsigned char*)(((uintptr_t)smem_raw + 15) & ~(uintptr_t)15);
+  const int x_pitch = 2 * K + 16;  // (K is a multiple of 64: the rows begin in different banks)
+  unsigned char* ring = x_s + (RESIDENT ? (size_t)M * x_pitch : 0);
+  float* scratch = reinterpret_cast<float*>(ring + (size_t)stages * S::STAGE_BYTES);
+  __shared__ uint64_t full_bar[S::MAX_STAGES], empty_bar[S::MAX_STAGES], x_bar[RESIDENT ? MAX_CHUNKS : 1];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int chunks = K / KC + (K % KC ? 1 : 0);  // stages per tile; the last may be shorter (K is a multiple of 64)
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 2); }
+    for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], S::CONSUMERS); }
+    if (RESIDENT)
+      for (int ch = 0; ch < chunks; ++ch) mbar_init(&x_bar[RESIDENT ? ch : 0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (EPI == EPI_QKV_ROPE) gemv::prefetch_cache_pages(rope, M);
 
   if (warp == 0) {
     // ---- producer: lane r copies row r of the tile's W; lanes also copy the token rows of X. The weights are
     // nobody's output: the first trip round the ring asks for them before the wait on the kernel before, and adds
     // the rows of X (which that kernel may have written) after it.
     auto fill = [&](int it, int tile, int ch, bool weights, bool tokens) {
-      int s = it % S::STAGES;
-      int row0 = tile * ROWS, rows_valid = min(ROWS, N - row0), k0 = ch * KC;
+      int s = it % stages;
+      int row0 = tile * height, rows_valid = min(height, N - row0), k0 = ch * KC;
       unsigned bytes = (unsigned)min(KC, K - k0) * 2u;
       unsigned char* stage = ring + (size_t)s * S::STAGE_BYTES;
       if (weights) {
-        if (lane == 0) mbar_expect_tx(&full_bar[s], bytes * (unsigned)(rows_valid + M));
+        if (lane == 0) mbar_expect_tx(&full_bar[s], bytes * (unsigned)(rows_valid + (RESIDENT ? 0 : M)));
         __syncwarp();
-        for (int r = lane; r < rows_valid; r += 32)
-          bulk_copy(stage + r * PITCH, w + (size_t)(row0 + r) * K + k0, bytes, &full_bar[s]);
+        for (int r = lane; r < rows_valid; r += 32) {
+          int row = row0 + r;
+          if (EPI == EPI_QKV_ROPE) {
+            int head, dim0;
+            bool paired;
+            row = gemv::tile_row<EPI>(tile, r, N, rope, head, dim0, paired);
+          }
+          bulk_copy(stage + r * PITCH, w + (size_t)row * K + k0, bytes, &full_bar[s]);
+        }
       }
-      if (tokens)
+      if (tokens && !RESIDENT)
         for (int m = lane; m < M; m += 32)
           bulk_copy(stage + (ROWS + m) * PITCH, x + (size_t)m * K + k0, bytes, &full_bar[s]);
     };
     int it = 0, tile = blockIdx.x, ch = 0;
-    for (; it < S::STAGES && tile < tiles; ++it) {  // the first trip: weights only
+    for (; it < stages && tile < tiles; ++it) {  // the first trip: weights only
       fill(it, tile, ch, true, false);
       if (++ch == chunks) { ch = 0; tile += gridDim.x; }
     }
     pdl_wait();
-    {
+    if (RESIDENT) {
+      for (int k = 0; k < chunks; ++k) {
+        unsigned bytes = (unsigned)min(KC, K - k * KC) * 2u;
+        if (lane == 0) mbar_expect_tx(&x_bar[RESIDENT ? k : 0], bytes * (unsigned)M);
+        __syncwarp();
+        for (int m = lane; m < M; m += 32)
+          bulk_copy(x_s + (size_t)m * x_pitch + k * ROW_BYTES, x + (size_t)m * K + k * KC, bytes, &x_bar[RESIDENT ? k : 0]);
+      }
+    } else {
       int it2 = 0, tile2 = blockIdx.x, ch2 = 0;
       for (; it2 < it; ++it2) {  // their rows of X
         fill(it2, tile2, ch2, false, true);
@@ -100,8 +134,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_tma_kernel(void* __restrict__
       }
     }
     for (; tile < tiles; ++it) {
-      int s = it % S::STAGES;
-      if (!mbar_wait(&empty_bar[s], ((it / S::STAGES) - 1) & 1)) {
+      int s = it % stages;
+      if (!mbar_wait(&empty_bar[s], ((it / stages) - 1) & 1)) {
         if (lane == 0) *(volatile int*)status = 32;
         break;
       }
@@ -111,18 +145,46 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_tma_kernel(void* __restrict__
   } else {
     // ---- consumers
     pdl_wait();  // C (for the residual) may come from the kernel before
-    int cw = warp - 1;                       // 0 or 1
+    int cw = warp - 1, half = cw / K_PARTS, part = cw % K_PARTS;  // which 16 rows of the tile, which steps
     int g = lane >> 2, t = lane & 3;
-    int row_base = ROWS == 32 ? cw * 16 : 0;  // first of this warp's 16 rows within the tile
+    int row_base = half * 16;
     // ldmatrix addresses inside a stage: W rows (lane & 15), k offset 8 for the upper lanes; X rows (lane & 7),
-    // k offset 8 for lanes 8..15 (and the second eight tokens for lanes 16..31 when NT == 2)
+    // k offset 8 for lanes 8..15 (and the second eight tokens for lanes 16..31 when NT == 2). Rows of X beyond M are
+    // whatever lies there, or the last row again where X is resident: their results are not stored.
     unsigned a_off = (unsigned)((row_base + (lane & 15)) * PITCH + (lane >> 4) * 16);
-    unsigned b_off =
-        (unsigned)((ROWS + (lane & 7) + (NT == 2 ? (lane >> 4) * 8 : 0)) * PITCH + ((lane >> 3) & 1) * 16);
-    float* mine = scratch + cw * 16 * (S::TOKENS + 1);
-    int it = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+    int token = (lane & 7) + (NT == 2 ? (lane >> 4) * 8 : 0);
+    unsigned b_off = RESIDENT ? smem_u32(x_s) + (unsigned)(min(token, M - 1) * x_pitch + ((lane >> 3) & 1) * 16)
+                              : (unsigned)((ROWS + token) * PITCH + ((lane >> 3) & 1) * 16);
+    constexpr int TILE_FLOATS = 16 * (S::TOKENS + 1);
+    float* group = scratch + (size_t)half * K_PARTS * TILE_FLOATS;  // the tiles of the warps that share these rows
+    float* mine = group + part * TILE_FLOATS;
+    int it = 0, member = part * 32 + lane;  // this thread among the group's
+    auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(K_PARTS * 32) : "memory"); };
+    bool ok = true;  // (a warp that gave up still meets the others of its group, tile by tile, and stores nothing)
+    // (in the q/k/v projection a thread stores the same pair and token of every tile: the token's position and cache page
+    // are asked for before the first product, the tile's angle before the tile's)
+    static_assert(EPI != EPI_QKV_ROPE || (NT == 1 && ROWS == 16), "one pair and token a thread");
+    int pos = 0, page = 0;
+    if (EPI == EPI_QKV_ROPE && member < 64 && (member & 7) < M) {
+      pos = rope.tok_pos[member & 7];
+      if (rope.write_cache)
+        page = rope.cache.page_table[(size_t)rope.slots[rope.tok_seq[member & 7]] * rope.cache.max_pages +
+                                     pos / rope.cache.page_size];
+    }
+    // (EPI_ARGMAX: the largest value that this thread has seen over all tiles, and its feature; features ascend, so the
+    // first of equal ones stays)
+    static_assert(EPI != EPI_ARGMAX || NT == 1, "one pair and token a thread");
+    float best_value = -INFINITY;
+    int best_feature = 0x7fffffff;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      int head = 0, dim0 = 0;
+      bool paired = false;
+      float2 turn = make_float2(1.f, 0.f);
+      if (EPI == EPI_QKV_ROPE) {
+        gemv::tile_row<EPI>(tile, 0, N, rope, head, dim0, paired);
+        if (paired && member < 64 && (member & 7) < M)
+          turn = rope.table[(size_t)pos * (rope.rotary_dim / 2) + dim0 + (member >> 3)];
+      }
       float acc[2][NT][4];  // two sets on alternate steps: a step does not wait for the one before
 #pragma unroll
       for (int e = 0; e < 2; ++e)
@@ -130,37 +192,36 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_tma_kernel(void* __restrict__
         for (int n = 0; n < NT; ++n)
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[e][n][i] = 0.f;
-      for (int ch = 0; ch < chunks; ++ch, ++it) {
-        int s = it % S::STAGES;
-        if (!mbar_wait(&full_bar[s], (it / S::STAGES) & 1)) {
+      for (int ch = 0; ch < chunks && ok; ++ch, ++it) {
+        int s = it % stages;
+        if (!mbar_wait(&full_bar[s], (it / stages) & 1) || (RESIDENT && !mbar_wait(&x_bar[RESIDENT ? ch : 0], 0))) {
           if (lane == 0) *(volatile int*)status = 33;
           ok = false;
           break;
         }
         unsigned stage = smem_u32(ring + (size_t)s * S::STAGE_BYTES);
-        int ksteps = min(KC, K - ch * KC) / 16;
-        // ROWS == 32: every step; ROWS == 16: this warp's alternate steps
-        constexpr int STRIDE = ROWS == 32 ? 1 : 2;
-        int first = ROWS == 32 ? 0 : cw;
-        // (a stage holds a multiple of four steps, so a warp's steps come in pairs: one for each set of sums)
-#pragma unroll 2
-        for (int ks = first; ks < ksteps; ks += 2 * STRIDE) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            unsigned a[4], b[4];
-            unsigned at = (unsigned)(ks + e * STRIDE) * 32u;
-            ldmatrix_x4(a, stage + a_off + at);
-            if (NT == 2) ldmatrix_x4(b, stage + b_off + at);
-            else ldmatrix_x2(b, stage + b_off + at);
-            mma_bf16(acc[e][0], a, b[0], b[1]);
-            if (NT == 2) mma_bf16(acc[e][NT - 1], a, b[2], b[3]);
-          }
+        unsigned x_at = RESIDENT ? b_off + (unsigned)(ch * ROW_BYTES) : stage + b_off;
+        int steps = min(KC, K - ch * KC) / (16 * K_PARTS);  // (K is a multiple of 64: as many for every warp)
+        auto step = [&](float (*into)[4], int j) {
+          unsigned a[4], b[4];
+          unsigned at = (unsigned)(j * K_PARTS + part) * 32u;
+          ldmatrix_x4(a, stage + a_off + at);
+          if (NT == 2) ldmatrix_x4(b, x_at + at);
+          else ldmatrix_x2(b, x_at + at);
+          mma_bf16(into[0], a, b[0], b[1]);
+          if (NT == 2) mma_bf16(into[NT - 1], a, b[2], b[3]);
+        };
+        int j = 0;
+#pragma unroll 4
+        for (; j + 1 < steps; j += 2) {
+          step(acc[0], j);
+          step(acc[1], j + 1);
         }
+        if (j < steps) step(acc[0], j);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[s]);  // this warp is done with the stage
       }
-      if (!ok) break;
-      // the warp's 16 x TOKENS tile to shared memory, then one (pair of rows, token) per thread and turn
+      // the warp's 16 x TOKENS tile to shared memory, then one (pair of rows, token) per thread of the group and turn
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
         mine[g * (S::TOKENS + 1) + n * 8 + 2 * t] = acc[0][n][0] + acc[1][n][0];
@@ -168,56 +229,129 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_tma_kernel(void* __restrict__
         mine[(g + 8) * (S::TOKENS + 1) + n * 8 + 2 * t] = acc[0][n][2] + acc[1][n][2];
         mine[(g + 8) * (S::TOKENS + 1) + n * 8 + 2 * t + 1] = acc[0][n][3] + acc[1][n][3];
       }
-      if (ROWS == 16) asm volatile("bar.sync 1, 64;" ::: "memory");  // both halves of the reduction are there
-      else __syncwarp();
-      if (ROWS == 32 || cw == 0) {
-        const float* other = scratch + 16 * (S::TOKENS + 1);
-        int n0 = tile * ROWS + row_base;
-        for (int idx = lane; idx < 8 * S::TOKENS; idx += 32) {
-          int p = idx / S::TOKENS, m = idx % S::TOKENS;
-          if (m >= M) continue;
-          float v0 = mine[(2 * p) * (S::TOKENS + 1) + m], v1 = mine[(2 * p + 1) * (S::TOKENS + 1) + m];
-          if (ROWS == 16) {
-            v0 += other[(2 * p) * (S::TOKENS + 1) + m];
-            v1 += other[(2 * p + 1) * (S::TOKENS + 1) + m];
+      meet();
+      int n0 = tile * height + row_base;
+      for (int idx = member; idx < 8 * S::TOKENS && ok; idx += K_PARTS * 32) {
+        int p = idx / S::TOKENS, m = idx % S::TOKENS;
+        // (rows 2 p and 2 p + 1 of the sixteen, or p and p + 8 for rotary pairs)
+        int r0 = EPI == EPI_QKV_ROPE ? p : 2 * p, r1 = EPI == EPI_QKV_ROPE ? p + 8 : 2 * p + 1;
+        if (m >= M || (EPI != EPI_QKV_ROPE && row_base + r0 >= height)) continue;
+        float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+        for (int k = 0; k < K_PARTS; ++k) {
+          v0 += group[k * TILE_FLOATS + r0 * (S::TOKENS + 1) + m];
+          v1 += group[k * TILE_FLOATS + r1 * (S::TOKENS + 1) + m];
+        }
+        if (EPI == EPI_QKV_ROPE) {
+          int hd = rope.cache.head_dim, nkv = rope.cache.kv_heads;
+          int d0 = dim0 + p, d1 = d0 + (paired ? rope.rotary_dim / 2 : 8);
+          if (paired) {
+            float a = v0, b = v1;
+            v0 = fmaf(a, turn.x, -(b * turn.y));
+            v1 = fmaf(a, turn.y, b * turn.x);
           }
+          bf16* dst;
+          if (head < rope.heads) {
+            dst = rope.q_out + ((size_t)m * rope.heads + head) * hd;
+          } else {
+            if (!rope.write_cache) continue;
+            int which = head < rope.heads + nkv ? 0 : 1, kvh = head - rope.heads - which * nkv;
+            dst = (bf16*)rope.cache.base + kv_offset(rope.cache, page, which, kvh, pos % rope.cache.page_size);
+          }
+          dst[d0] = __float2bfloat16_rn(v0);
+          dst[d1] = __float2bfloat16_rn(v1);
+        } else if (EPI == EPI_ARGMAX) {  // (a value that is not a number is never larger: it is never chosen)
+          int n = n0 + 2 * p;
+          if (n < N && v0 > best_value) { best_value = v0; best_feature = n; }
+          if (n + 1 < N && v1 > best_value) { best_value = v1; best_feature = n + 1; }
+        } else {
           epilogue_pair<EPI, bf16>(c, m, n0 + 2 * p, M, N, v0, v1);
         }
       }
-      if (ROWS == 16) asm volatile("bar.sync 1, 64;" ::: "memory");  // the scratch is free for the next tile
-      else __syncwarp();
+      meet();  // the scratch is free for the next tile
+    }
+    if (EPI == EPI_ARGMAX) {
+      // Pairs 0..3 of a token lie in the group's first warp, 4..7 in its second; every group leaves one candidate a token.
+      auto better = [&](float value, int feature) {
+        if (value > best_value || (value == best_value && feature < best_feature)) {
+          best_value = value;
+          best_feature = feature;
+        }
+      };
+#pragma unroll
+      for (int o = 8; o <= 16; o <<= 1) {
+        float value = __shfl_xor_sync(0xffffffffu, best_value, o);
+        int feature = __shfl_xor_sync(0xffffffffu, best_feature, o);
+        better(value, feature);
+      }
+      if (part == 1 && lane < 8) {
+        group[2 * lane] = best_value;
+        group[2 * lane + 1] = __int_as_float(best_feature);
+      }
+      meet();
+      if (part == 0 && lane < M) {
+        better(group[2 * lane], __float_as_int(group[2 * lane + 1]));
+        float* out = (float*)c + ((size_t)lane * 2 * gridDim.x + 2 * blockIdx.x + half) * 2;
+        out[0] = best_value;
+        out[1] = __int_as_float(best_feature);
+      }
     }
   }
 }
 
-template <int ROWS, int NT, int EPI>
-int launch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int* status, cudaStream_t stream) {
-  typedef Shape<ROWS, NT> S;
+int multiprocessors() {
   static int sms = 0;
   if (sms == 0) {
     int device = 0;
-    if (cudaFuncSetAttribute(gemv_tma_kernel<ROWS, NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)S::SMEM) != cudaSuccess ||
-        cudaGetDevice(&device) != cudaSuccess ||
+    if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) {
       sms = 0;
-      return DLLM_LAUNCH_FAILED;
     }
   }
-  int tiles = (N + ROWS - 1) / ROWS;
-  int blocks = tiles < sms ? tiles : sms;
-  return dllm_launch_pdl(gemv_tma_kernel<ROWS, NT, EPI>, dim3(blocks), dim3(THREADS), S::SMEM, stream, c, x, w, M, N,
-                         K, tiles, status);
+  return sms;
 }
 
-template <int ROWS, int NT>
-int dispatch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int epilogue, int* status,
-             cudaStream_t stream) {
+template <int ROWS, int NT, int EPI, bool RESIDENT>
+int launch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int height, int* status, const RopeArgs& rope,
+           cudaStream_t stream) {
+  typedef Shape<ROWS, NT, RESIDENT> S;
+  static std::atomic<unsigned long long> allowed{0};
+  int sms = multiprocessors();
+  if (sms == 0 || !dllm_allow_shared((const void*)gemv_tma_kernel<ROWS, NT, EPI, RESIDENT>, S::MAX_SMEM, allowed))
+    return DLLM_LAUNCH_FAILED;
+  int tiles = (N + height - 1) / height;
+  int blocks = tiles < sms ? tiles : sms;
+  return dllm_launch_pdl(gemv_tma_kernel<ROWS, NT, EPI, RESIDENT>, dim3(blocks), dim3(S::THREADS), S::smem(M, K), stream, c, x,
+                         w, M, N, K, tiles, height, S::stages(M, K), status, rope);
+}
+
+bool resident(int M, int K) { return M <= 8 && M * (2 * K + 16) <= RESIDENT_BYTES && (K + KC - 1) / KC <= MAX_CHUNKS; }
+
+// The height that leaves the busiest multiprocessor the fewest rows, the larger one where several do.
+int tile_height(int N, int sms) {
+  int height = 32;
+  long long fewest = 0;
+  for (int h = 32; h >= 16; h -= 2) {
+    long long rows = ((long long)((N + h - 1) / h) + sms - 1) / sms * h;
+    if (h == 32 || rows < fewest) {
+      fewest = rows;
+      height = h;
+    }
+  }
+  return height;
+}
+
+template <int NT, bool RESIDENT>
+int dispatch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int epilogue, int* status, cudaStream_t stream) {
+  int sms = multiprocessors();
+  if (sms == 0) return DLLM_LAUNCH_FAILED;
+  int height = tile_height(N, sms);
+  RopeArgs none{};
   switch (epilogue) {
-    case EPI_STORE_F32: return launch<ROWS, NT, EPI_STORE_F32>(c, x, w, M, N, K, status, stream);
-    case EPI_STORE_T: return launch<ROWS, NT, EPI_STORE_T>(c, x, w, M, N, K, status, stream);
-    case EPI_RESIDUAL: return launch<ROWS, NT, EPI_RESIDUAL>(c, x, w, M, N, K, status, stream);
-    case EPI_SWIGLU: return launch<ROWS, NT, EPI_SWIGLU>(c, x, w, M, N, K, status, stream);
+    case EPI_STORE_F32: return launch<32, NT, EPI_STORE_F32, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
+    case EPI_STORE_T: return launch<32, NT, EPI_STORE_T, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
+    case EPI_RESIDUAL: return launch<32, NT, EPI_RESIDUAL, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
+    case EPI_SWIGLU: return launch<32, NT, EPI_SWIGLU, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
     default: return DLLM_BAD_ARGUMENT;
   }
 }
@@ -232,21 +366,44 @@ DLLM_EXPORT int dllm_gemv_tma(void* c, const void* x, const void* w, int M, int 
   if (M > 16 || K <= 0 || (K & 63) || ((N & 1) && epilogue == EPI_SWIGLU) || ((uintptr_t)x & 15) ||
       ((uintptr_t)w & 15) || status == nullptr)
     return DLLM_UNSUPPORTED_SIZE;
-  static int sms = 0;
-  if (sms == 0) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
-      return DLLM_LAUNCH_FAILED;
-  }
-  // the tile height that leaves the busiest multiprocessor the fewest rows
-  long long rows32 = (long long)((((N + 31) / 32) + sms - 1) / sms) * 32;
-  long long rows16 = (long long)((((N + 15) / 16) + sms - 1) / sms) * 16;
-  bool tall = rows32 <= rows16;
   const bf16* xp = (const bf16*)x;
   const bf16* wp = (const bf16*)w;
-  if (M <= 8) return tall ? dispatch<32, 1>(c, xp, wp, M, N, K, epilogue, status, stream)
-                          : dispatch<16, 1>(c, xp, wp, M, N, K, epilogue, status, stream);
-  return tall ? dispatch<32, 2>(c, xp, wp, M, N, K, epilogue, status, stream)
-              : dispatch<16, 2>(c, xp, wp, M, N, K, epilogue, status, stream);
+  if (resident(M, K)) return dispatch<1, true>(c, xp, wp, M, N, K, epilogue, status, stream);
+  if (M <= 8) return dispatch<1, false>(c, xp, wp, M, N, K, epilogue, status, stream);
+  return dispatch<2, false>(c, xp, wp, M, N, K, epilogue, status, stream);
+}
+
+// The first stage of the greedy head product on the same ring (see EPI_ARGMAX), for up to eight tokens whose rows are
+// resident: candidates [M][*count](value, feature), two a block and token, for dllm_argmax_candidates. *count is at most
+// ceil(N / 16) for N of 4,736 and more; fewer rows of W are refused.
+DLLM_EXPORT int dllm_gemv_tma_argmax(float* candidates, const void* x, const void* w, int M, int N, int K, int* count,
+                                     int* status, cudaStream_t stream) {
+  int sms = multiprocessors();
+  if (sms == 0) return DLLM_LAUNCH_FAILED;
+  if (M <= 0 || N < 32 * sms || K <= 0 || (K & 63) || !resident(M, K) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) ||
+      status == nullptr || count == nullptr)
+    return DLLM_UNSUPPORTED_SIZE;
+  int height = tile_height(N, sms), tiles = (N + height - 1) / height;
+  *count = 2 * (tiles < sms ? tiles : sms);
+  return launch<32, 1, EPI_ARGMAX, true>(candidates, (const bf16*)x, (const bf16*)w, M, N, K, height, status, RopeArgs{},
+                                         stream);
+}
+
+// The q/k/v projection of a decode step on the same ring, arguments as `dllm_gemv_qkv_rope` without a norm in front:
+// for up to eight tokens whose rows are resident. head_dim and rotary_dim multiples of 16.
+DLLM_EXPORT int dllm_gemv_tma_qkv_rope(const void* x, const void* w, int M, int K, void* q_out, void* cache_base,
+                                       const int* page_table, int max_pages, int page_size, int heads, int kv_heads,
+                                       int head_dim, const float* table, int rotary_dim, const int* tok_seq,
+                                       const int* tok_pos, const int* slots, int write_cache, int prefetch_window,
+                                       int* status, cudaStream_t stream) {
+  if (M <= 0) return DLLM_OK;
+  if (K <= 0 || (K & 63) || !resident(M, K) || heads <= 0 || kv_heads <= 0 || head_dim <= 0 || (head_dim & 15) ||
+      rotary_dim < 0 || rotary_dim > head_dim || (rotary_dim & 15) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) ||
+      status == nullptr)
+    return DLLM_UNSUPPORTED_SIZE;
+  RopeArgs rope{(bf16*)q_out, KvLayout{cache_base, page_table, max_pages, page_size, kv_heads, head_dim},
+                (const float2*)table, table ? rotary_dim : 0, heads, tok_seq, tok_pos, slots, write_cache,
+                prefetch_window};
+  int N = (heads + 2 * kv_heads) * head_dim;
+  return launch<16, 1, EPI_QKV_ROPE, true>(nullptr, (const bf16*)x, (const bf16*)w, M, N, K, 16, status, rope, stream);
 }

@@ -226,6 +226,10 @@ _prototypes = {
                                         c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p],
     ("gemv", "dllm_argmax_candidates"): [c_void_p, c_void_p, c_int, c_int, c_void_p],
     ("gemv_tma", "dllm_gemv_tma"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    ("gemv_tma", "dllm_gemv_tma_argmax"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
+    ("gemv_tma", "dllm_gemv_tma_qkv_rope"): [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                             c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
+                                             c_int, c_void_p, c_void_p],
     ("gemv", "dllm_gemv_qkv_rope"): [c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                      c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p,
                                      c_void_p, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p],
@@ -1713,6 +1717,30 @@ def streams(rows: int, outputs: int, inner: int | None = None) -> bool:
 TMA_STREAM_BYTES = 48 << 20
 
 
+def resident_activations(rows: int, inner: int) -> bool:
+    """Whether the ring kernel (csrc/gemv_tma.cu) keeps the rows of activations in shared memory beside its ring."""
+    return rows <= 8 and rows * (2 * inner + 16) <= 72 * 1024
+
+
+def streams_with_resident_rows(rows: int, outputs: int, inner: int) -> bool:
+    """Whether a decode-sized product takes the ring kernel with its rows of activations resident, before the rules below
+    are asked. Measured, one row and eight: 28672 x 4096 36.6 and 41.8 us (register kernel 45.6 and 47.7, W as the 128-row
+    operand 45.5 and 44.0), 6144 x 4096 10.4 and 12.05 (11.7 and 12.4); rows of 2,048 values are better off in the
+    register kernel (16384 x 2048: 12.0 and 12.7 against 11.2 and 11.7)."""
+    if inner % 64 or inner < 4096 or not resident_activations(rows, inner):
+        return False
+    size = 2 * outputs * inner
+    # (4096 x 4096, 32 MB: 7.7 against 8.75 with one row, 8.8 against 9.0 with four, 9.95 against 9.2 with eight; 2048 x
+    # 8192, where tiles of 16 rows leave multiprocessors idle: 9.6 against 8.6)
+    return size >= TMA_STREAM_BYTES or (rows <= 4 and size >= TMA_STREAM_BYTES * 2 // 3 and outputs >= 4096)
+
+
+def streams_qkv_through_shared_memory(rows: int, outputs: int, inner: int) -> bool:
+    """The same for the q/k/v projection with rotation and cache write behind it: 6144 x 4096 12.3 us against 14.0 with one
+    row, 12.4 against 14.9 with eight; 6144 x 2048 8.7 against 6.0."""
+    return 2 * outputs * inner >= TMA_STREAM_BYTES and streams_with_resident_rows(rows, outputs, inner)
+
+
 def streams_through_shared_memory(rows: int, outputs: int, inner: int) -> bool:
     """Whether a decode-sized product takes the kernel that streams W through a ring of shared-memory stages.
     Measured against the kernel that streams through registers: it wins (0.71 to 0.97 of the HBM rate against 0.65 to
@@ -1720,8 +1748,8 @@ def streams_through_shared_memory(rows: int, outputs: int, inner: int) -> bool:
     megabytes; with more rows the copies of the activations cost it the lead."""
     if inner % 64 or 2 * outputs * inner < TMA_STREAM_BYTES:
         return False
-    # (up to 4 rows its lead holds, 6144 x 4096: 11.3 µs against 12.2; up to 8 rows only for very long rows of W,
-    # 4096 x 14336: 24.2 against 28.8)
+    # (up to 4 rows its lead holds; up to 8 rows only for very long rows of W, 4096 x 14336: 24.4 against 29.4. Where the
+    # activations stay in shared memory it leads further: `streams_with_resident_rows`)
     return (rows <= 4 and inner >= 4096) or (rows <= 8 and inner >= 8192)
 
 
@@ -1840,6 +1868,7 @@ def gemm(c: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_
     elif w.dtype == torch.bfloat16:
         streaming = (kernel == 2 and m <= GEMV_MAX_ROWS) or (kernel == 0 and streams(m, n, k))
         split = reduction_split(m, n, k) if (kernel == 0 and epilogue == EPI_RESIDUAL and norm_weight is None) else 1
+        resident = kernel == 0 and norm_weight is None and epilogue <= EPI_SWIGLU and streams_with_resident_rows(m, n, k)
         if kernel == 7 or split > 1:
             # W as the 128-row operand, the reduction cut into stretches, the parts summed into c by a second kernel
             assert a.dtype == torch.bfloat16 and norm_weight is None and epilogue == EPI_RESIDUAL and m <= 64
@@ -1847,14 +1876,14 @@ def gemm(c: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_
             parts = gemm_parts(a, w, split)
             status = _fn("elementwise", "dllm_sum_parts_residual")(c.data_ptr(), parts.data_ptr(), split, m * n,
                                                                    _stream())
-        elif kernel == 5 or (kernel == 0 and norm_weight is None and takes_weights_as_rows(m, n, k)):
+        elif kernel == 5 or (kernel == 0 and norm_weight is None and not resident and takes_weights_as_rows(m, n, k)):
             # the product the other way round: W is the 128-row operand, the tokens are the tile's columns
             assert a.dtype == torch.bfloat16 and norm_weight is None and m <= 256
             width = 32 if m <= 32 else (64 if m <= 64 else (128 if m <= 128 else 256))
             status = _fn("gemm_tcgen05", "dllm_gemm_tcgen05")(
                 c.data_ptr(), w.data_ptr(), a.data_ptr(), n, m, k, epilogue + 5, width, _status_word().data_ptr(),
                 _stream())
-        elif kernel == 4 or (kernel == 0 and norm_weight is None and streams_through_shared_memory(m, n, k)):
+        elif kernel == 4 or resident or (kernel == 0 and norm_weight is None and streams_through_shared_memory(m, n, k)):
             assert a.dtype == torch.bfloat16 and norm_weight is None
             status = _fn("gemv_tma", "dllm_gemv_tma")(c.data_ptr(), a.data_ptr(), w.data_ptr(), m, n, k, epilogue,
                                                       _status_word().data_ptr(), _stream())
@@ -1957,6 +1986,15 @@ def head_argmax(out_tokens: torch.Tensor, a: torch.Tensor, w: torch.Tensor, scra
     assert head_argmax_supported(m, w) and w.shape[1] == k and out_tokens.dtype == torch.int32
     assert scratch.dtype == torch.float32 and scratch.numel() >= head_argmax_scratch(m, n)
     assert a.dtype == (torch.float32 if norm_weight is not None else torch.bfloat16)
+    if norm_weight is None and n >= 16384 and streams_with_resident_rows(m, n, k):
+        # (128256 x 4096 with one row: 147 us against 182 for the register kernel)
+        count = ctypes.c_int(0)
+        _check(_fn("gemv_tma", "dllm_gemv_tma_argmax")(
+            scratch.data_ptr(), a.data_ptr(), w.data_ptr(), m, n, k, ctypes.addressof(count), _status_word().data_ptr(),
+            _stream()), "head_argmax product", lambda: f"M={m} N={n} K={k}")
+        _check(_fn("gemv", "dllm_argmax_candidates")(out_tokens.data_ptr(), scratch.data_ptr(), m, count.value, _stream()),
+               "head_argmax choice")
+        return
     _check(_fn("gemv", "dllm_gemv_bf16")(
         scratch.data_ptr(), a.data_ptr(), norm_weight.data_ptr() if norm_weight is not None else None, float(eps),
         w.data_ptr(), m, n, k, EPI_ARGMAX, *_prefetch_of(w), _stream()), "head_argmax product",
@@ -2057,8 +2095,8 @@ def gemv_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, 
     """The q/k/v projection of at most 64 tokens in one kernel (bfloat16): optional RMSNorm of the float32 residual
     in front, rotation of q and k, q to q_out, k and v into the paged cache. With `prefetch_window` >= 0 the kernel
     also asks L2 for the cached keys and values of the tokens' sequences (0: all of them, w: the last w), which the
-    attention kernel behind it reads. `kernel`: 0 chooses, 2 forces a block per 16 rows of W, 6 the reduction split
-    over a cluster (`cluster` blocks, 0 chooses)."""
+    attention kernel behind it reads. `kernel`: 0 chooses, 2 forces a block per 16 rows of W, 4 streaming through shared
+    memory (no norm), 6 the reduction split over a cluster (`cluster` blocks, 0 chooses)."""
     _cuda(a, w, q_out, table, norm_weight)
     m, k = batch.n_tokens, a.shape[1]
     assert w.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and q_out.dtype == torch.bfloat16
@@ -2067,6 +2105,16 @@ def gemv_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, 
     if table is not None:
         assert table.dtype == torch.float32 and table.shape[0] > batch.max_position, "position beyond the table"
         assert table.shape[1] == rotary_dim // 2 and table.shape[2] == 2
+    if kernel == 4 or (kernel == 0 and norm_weight is None and streams_qkv_through_shared_memory(m, w.shape[0], k)):
+        assert norm_weight is None
+        _check(_fn("gemv_tma", "dllm_gemv_tma_qkv_rope")(
+            a.data_ptr(), w.data_ptr(), m, k, q_out.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(),
+            cache.max_pages, cache.page_size, heads, cache.kv_heads, cache.head_dim,
+            table.data_ptr() if table is not None else None, rotary_dim if table is not None else 0,
+            batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(), batch.slots.data_ptr(), 1 if write_cache else 0,
+            int(prefetch_window), _status_word().data_ptr(), _stream()), "gemv_tma_qkv_rope",
+            lambda: f"M={m} (at most 8, of 72 KB in all), K={k} (multiple of 64), head_dim and rotary_dim multiples of 16")
+        return
     if kernel == 6 or (kernel == 0 and splits_over_clusters(m, w.shape[0], k)):
         _check(_fn("gemv_cluster", "dllm_gemv_cluster_qkv_rope")(
             a.data_ptr(), norm_weight.data_ptr() if norm_weight is not None else None, float(eps), w.data_ptr(), m, k,

@@ -194,6 +194,8 @@ class Attention:
         names = {"gemv", "gemm_tcgen05", "elementwise"}
         if any(ops.splits_over_clusters(64, w.shape[0], w.shape[1]) for w in (self.w_qkv, self.w_o) if w is not None):
             names.add("gemv_cluster")  # (steps of 17 to 64 tokens with weights this small)
+        if any(ops.streams_with_resident_rows(1, w.shape[0], w.shape[1]) for w in (self.w_qkv, self.w_o) if w is not None):
+            names.add("gemv_tma")
         if self.w_o is None:  # (given away)
             names |= {"sink_attention_decode", "sink_attention_prefill"}
             return names | ({"sink_attention_tcgen05"} if hd in TCGEN05_ATTENTION_FROM else set())

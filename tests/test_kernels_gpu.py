@@ -680,8 +680,17 @@ def test_gemv_qkv_rope_long_rows_and_more_tiles_than_blocks(normed):
     _check_gemv_qkv_rope(40, 8, 128, 128, normed, 3, 2240)
 
 
-def _check_gemv_qkv_rope(heads, kv_heads, head_dim, rotary, normed, rows_extra, k, kernel=2, cluster=0):
-    lengths, new = [70, 5, 129, 64, 200, 33], [1, 1, 3, 2, rows_extra, 1]
+@pytest.mark.parametrize("heads,kv_heads,head_dim,rotary", [(4, 2, 16, 16), (6, 3, 48, 32), (9, 3, 64, 64), (3, 1, 128, 0),
+                                                           (40, 8, 128, 128)])
+@pytest.mark.parametrize("new,k", [([1], 64), ([1, 1, 2], 1088), ([1, 1, 3, 2, 1], 2240), ([1], 14400)])
+def test_gemv_tma_qkv_rope(heads, kv_heads, head_dim, rotary, new, k):
+    """The projection on the bulk-copy ring: one to eight tokens, fewer and more tiles than blocks, short last stages."""
+    _check_gemv_qkv_rope(heads, kv_heads, head_dim, rotary, False, 0, k, kernel=4, new=new)
+
+
+def _check_gemv_qkv_rope(heads, kv_heads, head_dim, rotary, normed, rows_extra, k, kernel=2, cluster=0, new=None):
+    lengths, new = [70, 5, 129, 64, 200, 33], new or [1, 1, 3, 2, rows_extra, 1]
+    lengths = lengths[:len(new)]
     cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, lengths, new)
     n = batch.n_tokens
     table = None
@@ -1077,6 +1086,30 @@ def test_head_argmax_chooses_what_the_logits_would(m, n, k, normed):
     assert got[0].item() == 0 and (m <= 2 or got[2].item() == 0)
     finite = [r for r in range(m) if r not in (0, 2)]
     assert got[finite].tolist() == logits[finite].argmax(dim=1).tolist()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 16385, 4096), (8, 16400, 4160), (3, 20001, 4096)])
+def test_head_argmax_on_the_ring(m, n, k):
+    """The greedy choice on the bulk-copy ring (long rows of W): tiles that end in half a fragment, odd vocabularies, ties
+    between features of different blocks, rows without any number, all logits equal; against float64 where one value leads
+    by more than the sums' rounding."""
+    x, w = _randn((m, k), torch.bfloat16, 1), _randn((n, k), torch.bfloat16, 2, 0.1)
+    w[n - 1], w[n // 2] = w[3] * 8, w[3] * 8  # equal in every row, and the largest wherever row 3's product is positive
+    x[0] = 0
+    if m > 2:
+        x[2, 0] = float("nan")
+    got = torch.full((m,), -1, dtype=torch.int32, device=DEV)
+    scratch = torch.full((ops().head_argmax_scratch(m, n),), float("nan"), dtype=torch.float32, device=DEV)
+    assert ops().streams_with_resident_rows(m, n, k)
+    ops().head_argmax(got, x, w, scratch)
+    ops().raise_if_failed()
+    assert got[0].item() == 0 and (m <= 2 or got[2].item() == 0)
+    exact = x.double() @ w.double().T
+    for row in [r for r in range(m) if r not in (0, 2)]:
+        best = exact[row].topk(3).values
+        assert exact[row, got[row].item()] >= best[0] - 2e-5 * best[0].abs()  # (k products of 16 bits summed in 32)
+        if exact[row].argmax().item() in (n - 1, n // 2):
+            assert got[row].item() == n // 2
 
 
 @pytest.mark.parametrize("m,hidden,inner,outputs", [
