@@ -1,24 +1,27 @@
 // Prefill attention over the paged cache (bfloat16, head_dim 64 or 128) on the 5th-generation tensor cores. A block
 // takes 128 consecutive new tokens of one sequence and one query head and walks the sequence's cache pages (64 keys
 // each):
-//   softmax warps (0-7): two groups of four warps that take alternate steps (group j % 2 takes step j, with the
-//            score, P and output buffers number j % 2), one thread per query: read its row of scores from tensor
+//   softmax warps: groups of four warps that take the steps in turn (group j % GROUPS takes step j, with the score, P and
+//            output buffers of that number), one thread per query: read its row of scores from tensor
 //            memory (tcgen05.ld 32x32b), mask, maximum and sum in float32 (no shuffles: the row is the thread's
 //            own; the maximum a row subtracts is renewed only when a score exceeds it by 2^8, so most steps read
-//            their scores once), write the probabilities as bfloat16 into the swizzled P tile, fetch the group's
-//            previous P V and fold it into the float32 output kept in registers: O = O * 2^(m_old - m_new) + P V.
-//            At the end the second group hands its maximum, sum and output to the first through shared memory.
+//            their scores once) and write the probabilities as bfloat16 into the swizzled P tile. The outputs of a
+//            group add up in tensor memory, O += P V, over all its steps; only when a row's maximum is renewed its
+//            warp reads them, scales them by 2^(m_old - m_new) and writes them back. (Fetched and folded into
+//            registers every step they were a third of a thread's instructions and half of its registers, which at
+//            head_dim 128 left room for one group only: 32 query and 8 kv heads, 2,048 tokens 100 -> 79.7 us a layer,
+//            431 TFLOP/s. At head_dim 64 a third group, 9 query and 3 kv heads: 25.3 -> 22.5 us; 32 heads, prompts of 512
+//            to 4,096: 283 -> 260; a fourth group changed nothing, nor did eight stages of keys and values.)
+//            At the end the groups hand their maxima, sums and outputs to the first through shared memory.
 //   next warp: one lane issues TMA loads: the query tile once, then a page of keys and a page of values per step
 //            into rings of shared-memory stages (128-byte swizzle), signalled by mbarriers;
 //   next warp: one lane issues tcgen05.mma for the scores: S_j = Q K_j^T (M = 128 queries, N = 64 keys, K =
-//            head_dim) into one of two score buffers in tensor memory, as soon as the buffer is free and the keys
+//            head_dim) into the group's score buffer in tensor memory, as soon as the buffer is free and the keys
 //            are there;
 //   last warp: one lane issues tcgen05.mma for the outputs: O_j = P_j V_j (P from shared memory, V read MN-major as
-//            it lies in the cache) into one of two output buffers (a lane of its own: issuing a product costs a
+//            it lies in the cache) onto the group's outputs (a lane of its own: issuing a product costs a
 //            single thread tens of cycles, and the scores of the next steps must not queue behind a wait for P).
-// head_dim 128: operands are two 64-column boxes side by side, the outputs take twice the columns of tensor memory
-// and 128 registers of a softmax thread, so there is one softmax group (which then takes every step and alternates
-// between the two sets of buffers itself) and the block has seven warps.
+// head_dim 128: operands are two 64-column boxes side by side, the outputs take twice the columns of tensor memory.
 // Every wait on an mbarrier is bounded; a role that gives up records a status word and leaves, the block still frees
 // its tensor memory and the host raises.
 //
@@ -31,27 +34,28 @@
 namespace {
 using namespace tc5;
 typedef __nv_bfloat16 bf16;
-constexpr int BQ = 128, BKV = 64, STAGES = 4;
+constexpr int BQ = 128, BKV = 64;
 constexpr int P_BYTES = BQ * BKV * 2;
 
 template <int HD> struct Shape {
-  static constexpr int GROUPS = HD <= 64 ? 2 : 1;             // softmax groups of four warps
+  static constexpr int GROUPS = HD <= 64 ? 3 : 2;             // softmax groups of four warps
+  static constexpr int K_STAGES = HD <= 64 ? 5 : 3, V_STAGES = HD <= 64 ? 7 : 5;  // (values wait for their P: more of them)
   static constexpr int SOFT_WARPS = 4 * GROUPS;
   static constexpr int THREADS = (SOFT_WARPS + 3) * 32;       // + the warps of the three single issuing lanes
   static constexpr int BOXES = HD / 64;                       // 64-column boxes per row of an operand
   static constexpr int Q_BOX = BQ * 128, KV_BOX = BKV * 128;  // bytes of a box: rows of 128 bytes
   static constexpr int Q_BYTES = BOXES * Q_BOX, KV_BYTES = BOXES * KV_BOX;
-  // P tiles: with two groups a group would write its next P while its previous product may still read the last
-  // one, so each group has two; a single group alternates between the two buffers anyway
+  // P tiles: a group would write its next P while its previous product may still read the last one, so each has two
   static constexpr int P_TILES = 2 * GROUPS;
-  static constexpr size_t SMEM = Q_BYTES + 2 * STAGES * KV_BYTES + P_TILES * P_BYTES + 1024;
-  static constexpr unsigned TMEM_COLS = 2 * BKV + 2 * HD <= 256 ? 256 : 512;  // scores 2 x 64, outputs 2 x HD
-  static constexpr int EX_LD = HD + 2;  // floats per row of the exchange between the two softmax groups
+  static constexpr size_t SMEM = Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES + P_TILES * P_BYTES + 1024;
+  static constexpr unsigned TMEM_COLS = GROUPS * (BKV + HD) <= 256 ? 256 : 512;  // scores GROUPS x 64, outputs GROUPS x HD
+  static_assert(GROUPS * (BKV + HD) <= 512 && SMEM <= 227 * 1024 - 512, "tensor memory, shared memory");
+  static constexpr int EX_LD = HD + 2;  // floats per row of the exchange between the softmax groups
 };
 
 struct Barriers {
-  uint64_t q_full, k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES];
-  uint64_t s_full[2], s_empty[2], p_full[2], o_full[2], o_empty[2];
+  uint64_t q_full, k_full[8], k_empty[8], v_full[8], v_empty[8];
+  uint64_t s_full[4], s_empty[4], p_full[4], o_full[4];
 };
 
 template <int HD, bool OPTIONS, bool CAPPED>
@@ -62,8 +66,9 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
     float scale_log2, int window, int* __restrict__ status, ScoreOptions options) {
   typedef Shape<HD> S;
   constexpr int GROUPS = S::GROUPS, SOFT_WARPS = S::SOFT_WARPS, Q_BYTES = S::Q_BYTES, KV_BYTES = S::KV_BYTES;
+  constexpr int K_STAGES = S::K_STAGES, V_STAGES = S::V_STAGES;
   constexpr unsigned TMEM_COLS = S::TMEM_COLS;
-  int tile = blockIdx.x, h = blockIdx.y;
+  int tile = (int)(gridDim.x - 1 - blockIdx.x), h = blockIdx.y;  // (a prompt's last tiles see the most keys: they go first)
   int q0 = tile_first[tile];
   if (q0 % BQ) return;  // the host lists tiles of 64 tokens; every second one starts a tile of 128
   pdl_launch_dependents();
@@ -71,8 +76,8 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzle atoms: 1 KB
   unsigned char* q_s = tiles;
   unsigned char* k_s = q_s + Q_BYTES;
-  unsigned char* v_s = k_s + STAGES * KV_BYTES;
-  unsigned char* p_s = v_s + STAGES * KV_BYTES;
+  unsigned char* v_s = k_s + K_STAGES * KV_BYTES;
+  unsigned char* p_s = v_s + V_STAGES * KV_BYTES;
   __shared__ Barriers bar;
   __shared__ unsigned tmem_base_s;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,14 +97,12 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
 
   if (threadIdx.x == 0) {
     mbar_init(&bar.q_full, 1);
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&bar.k_full[s], 1); mbar_init(&bar.k_empty[s], 1);
-      mbar_init(&bar.v_full[s], 1); mbar_init(&bar.v_empty[s], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
+    for (int s = 0; s < K_STAGES; ++s) { mbar_init(&bar.k_full[s], 1); mbar_init(&bar.k_empty[s], 1); }
+    for (int s = 0; s < V_STAGES; ++s) { mbar_init(&bar.v_full[s], 1); mbar_init(&bar.v_empty[s], 1); }
+    for (int i = 0; i < GROUPS; ++i) {
       mbar_init(&bar.s_full[i], 1); mbar_init(&bar.s_empty[i], 4);   // the 4 warps of softmax group i
       mbar_init(&bar.p_full[i], 4);
-      mbar_init(&bar.o_full[i], 1); mbar_init(&bar.o_empty[i], 4);
+      mbar_init(&bar.o_full[i], 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
   __syncthreads();
   fence_after_sync();
   unsigned tmem_base = tmem_base_s;
-  unsigned tmem_s = tmem_base, tmem_o = tmem_base + 2 * BKV;
+  unsigned tmem_s = tmem_base, tmem_o = tmem_base + GROUPS * BKV;
   pdl_wait();  // the queries and the newest keys and values come from the kernel before; so does `out`'s last reader
 
   if (warp == SOFT_WARPS) {
@@ -119,20 +122,19 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
 #pragma unroll
       for (int x = 0; x < S::BOXES; ++x) tma_load_2d(q_s + x * S::Q_BOX, &map_q, &bar.q_full, h * HD + x * 64, tok0);
       for (int j = 0; j < steps; ++j) {
-        int s = j % STAGES;
-        unsigned parity = ((j / STAGES) - 1) & 1;
+        int sk = j % K_STAGES, sv = j % V_STAGES;
         int page = pages[walk.tile(j)];
         int row_k = ((page * 2 + 0) * cache.kv_heads + g) * BKV, row_v = ((page * 2 + 1) * cache.kv_heads + g) * BKV;
-        if (j >= STAGES && !mbar_wait(&bar.k_empty[s], parity)) { *(volatile int*)status = 12; break; }
-        mbar_expect_tx(&bar.k_full[s], KV_BYTES);
+        if (j >= K_STAGES && !mbar_wait(&bar.k_empty[sk], (j / K_STAGES - 1) & 1)) { *(volatile int*)status = 12; break; }
+        mbar_expect_tx(&bar.k_full[sk], KV_BYTES);
 #pragma unroll
         for (int x = 0; x < S::BOXES; ++x)
-          tma_load_2d(k_s + s * KV_BYTES + x * S::KV_BOX, &map_kv, &bar.k_full[s], x * 64, row_k);
-        if (j >= STAGES && !mbar_wait(&bar.v_empty[s], parity)) { *(volatile int*)status = 13; break; }
-        mbar_expect_tx(&bar.v_full[s], KV_BYTES);
+          tma_load_2d(k_s + sk * KV_BYTES + x * S::KV_BOX, &map_kv, &bar.k_full[sk], x * 64, row_k);
+        if (j >= V_STAGES && !mbar_wait(&bar.v_empty[sv], (j / V_STAGES - 1) & 1)) { *(volatile int*)status = 13; break; }
+        mbar_expect_tx(&bar.v_full[sv], KV_BYTES);
 #pragma unroll
         for (int x = 0; x < S::BOXES; ++x)
-          tma_load_2d(v_s + s * KV_BYTES + x * S::KV_BOX, &map_kv, &bar.v_full[s], x * 64, row_v);
+          tma_load_2d(v_s + sv * KV_BYTES + x * S::KV_BOX, &map_kv, &bar.v_full[sv], x * 64, row_v);
       }
     }
   } else if (warp == SOFT_WARPS + 1) {
@@ -141,10 +143,10 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
       bool ok = mbar_wait(&bar.q_full, 0);
       if (!ok) *(volatile int*)status = 14;
       unsigned q_addr = smem_u32(q_s);
-      for (int i = 0; i < steps && ok; ++i) {  // S_i = Q K_i^T into the score buffer of group i % 2
-        int sb = i & 1, s = i % STAGES;
-        if (!mbar_wait(&bar.k_full[s], (i / STAGES) & 1)) { *(volatile int*)status = 18; break; }
-        if (i >= 2 && !mbar_wait(&bar.s_empty[sb], ((i >> 1) - 1) & 1)) { *(volatile int*)status = 19; break; }
+      for (int i = 0; i < steps && ok; ++i) {  // S_i = Q K_i^T into the score buffer of group i % GROUPS
+        int sb = i % GROUPS, s = i % K_STAGES;
+        if (!mbar_wait(&bar.k_full[s], (i / K_STAGES) & 1)) { *(volatile int*)status = 18; break; }
+        if (i >= GROUPS && !mbar_wait(&bar.s_empty[sb], (i / GROUPS - 1) & 1)) { *(volatile int*)status = 19; break; }
         fence_after_sync();
         unsigned k_addr = smem_u32(k_s + s * KV_BYTES);
 #pragma unroll
@@ -160,11 +162,10 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
   } else if (warp == SOFT_WARPS + 2) {
     if (lane == 0) {
       constexpr unsigned idesc_o = instr_desc(BQ, 64, true);  // 64 output columns per product: one box of V
-      for (int i = 0; i < steps; ++i) {  // O_i = P_i V_i into the output buffer of group i % 2
-        int pb = i & 1, s = i % STAGES;
-        if (!mbar_wait(&bar.p_full[pb], (i >> 1) & 1)) { *(volatile int*)status = 15; break; }
-        if (!mbar_wait(&bar.v_full[s], (i / STAGES) & 1)) { *(volatile int*)status = 16; break; }
-        if (i >= 2 && !mbar_wait(&bar.o_empty[pb], ((i >> 1) - 1) & 1)) { *(volatile int*)status = 17; break; }
+      for (int i = 0; i < steps; ++i) {  // O += P_i V_i in the output buffer of group i % GROUPS
+        int pb = i % GROUPS, s = i % V_STAGES;
+        if (!mbar_wait(&bar.p_full[pb], (i / GROUPS) & 1)) { *(volatile int*)status = 15; break; }
+        if (!mbar_wait(&bar.v_full[s], (i / V_STAGES) & 1)) { *(volatile int*)status = 16; break; }
         fence_after_sync();
         unsigned p_addr = smem_u32(p_s + (i % S::P_TILES) * P_BYTES), v_addr = smem_u32(v_s + s * KV_BYTES);
 #pragma unroll
@@ -172,55 +173,39 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
 #pragma unroll
           for (int x = 0; x < S::BOXES; ++x)
             umma(tmem_o + (unsigned)(pb * HD + x * 64), smem_desc(p_addr + k * 32),
-                 smem_desc(v_addr + x * S::KV_BOX + k * 2048), idesc_o, k > 0 ? 1u : 0u);
+                 smem_desc(v_addr + x * S::KV_BOX + k * 2048), idesc_o, (k > 0 || i >= GROUPS) ? 1u : 0u);
         tcgen05_commit(&bar.v_empty[s]);
         tcgen05_commit(&bar.o_full[pb]);
       }
     }
   } else if (warp < SOFT_WARPS) {
-    // Step j works in the buffers (scores, P, outputs) number j % 2, for the (j / 2)-th time. With two groups, group
-    // wg takes the steps j = wg, wg + 2, ... and so always the same buffers; a single group takes every step.
+    // Step j works in the buffers (scores, P, outputs) number j % GROUPS, for the (j / GROUPS)-th time: group wg takes the
+    // steps j = wg, wg + GROUPS, ... and so always the same buffers.
     int wg = warp >> 2;
     int r = (warp & 3) * 32 + lane;              // this thread's query: row r of the tile, tensor-memory lane r
     int qp = pos0 + r;
     const int row_first = first_visible(qp, chunk, window), tile_first_key = first_visible(pos0 + BQ - 1, chunk, window);
     unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
-    float o[HD];
-#pragma unroll
-    for (int d = 0; d < HD; ++d) o[d] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, corr_saved = 1.f;
+    const unsigned o_addr = tmem_o + lane_base + (unsigned)(wg * HD);
+    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     const ScoreCap score(scale_log2 / SCORE_LOG2E, CAPPED ? options.cap : 0.f);
-    // fold step i's output into the running one: O = O * corr + P V
-    auto consume = [&](int i, float corr) -> bool {
-      const int ob = i & 1;
-      unsigned o_addr = tmem_o + lane_base + (unsigned)(ob * HD);
-      if (!mbar_wait(&bar.o_full[ob], (i >> 1) & 1)) {
-        if (lane == 0) *(volatile int*)status = 20;
-        return false;
+    // waits until the product of step i has been added to the group's outputs (step by step: none is left out, so the
+    // barrier is never more than one phase ahead)
+    auto added = [&](int i) -> bool {
+      if (mbar_wait(&bar.o_full[wg], (i / GROUPS) & 1)) {
+        fence_after_sync();
+        return true;
       }
-      fence_after_sync();
-      unsigned v[2][16];
-      tmem_load16_nowait(o_addr, v[0]);
-#pragma unroll
-      for (int c = 0; c < HD; c += 16) {
-        const int cur = (c >> 4) & 1;
-        tmem_wait_ld();
-        if (c + 16 < HD) tmem_load16_nowait(o_addr + (unsigned)(c + 16), v[cur ^ 1]);
-#pragma unroll
-        for (int d = 0; d < 16; ++d) o[c + d] = fmaf(o[c + d], corr, __uint_as_float(v[cur][d]));
-      }
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.o_empty[ob]);
-      return true;
+      if (lane == 0) *(volatile int*)status = 20;
+      return false;
     };
     int taken = 0;  // how many steps this group has taken
     for (int j = wg; j < steps; j += GROUPS, ++taken) {
-      const int sb = j & 1;
+      const int sb = wg;
       unsigned s_addr = tmem_s + lane_base + (unsigned)(sb * BKV);
       unsigned char* p_tile = p_s + (j % S::P_TILES) * P_BYTES;
-      if (!mbar_wait(&bar.s_full[sb], (j >> 1) & 1)) {
+      if (!mbar_wait(&bar.s_full[sb], (j / GROUPS) & 1)) {
         if (lane == 0) *(volatile int*)status = 21;
         ok = false;
         break;
@@ -231,7 +216,7 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
       bool edge = key0 + BKV - 1 > pos0 || key0 < tile_first_key;
       int key_hi = qp - key0, key_lo = row_first - key0;  // columns key_lo .. key_hi count,
       const int key_kept = OPTIONS ? options.keep - key0 : 0;                      // and those before key_kept
-      // (the P tile of this step is free: the product that read it last, P_TILES steps ago, has been consumed)
+      // (the P tile of this step is free: the product that read it last, P_TILES steps ago, has been waited for)
       // One sweep over the scores gives the probabilities relative to the maximum the row has used so far, and the
       // tile's own maximum on the way. The used maximum need not be the true one: any constant cancels in the
       // quotient, and as long as no score lies more than 8 (in the log2 domain) above it the probabilities stay
@@ -315,60 +300,86 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.s_empty[sb]);  // the scores are not needed again: the buffer may be rewritten
       // the group's previous product: it had the time of the sweep to finish
-      if (taken >= 1 && !consume(j - GROUPS, corr_saved)) { ok = false; break; }
-      corr_saved = corr;
+      if (taken >= 1 && !added(j - GROUPS)) { ok = false; break; }
+      if (taken >= 1 && __any_sync(0xffffffffu, corr != 1.f)) {
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 16) {
+          unsigned v[16];
+          tmem_load16(o_addr + (unsigned)c, v);
+#pragma unroll
+          for (int d = 0; d < 16; ++d) v[d] = __float_as_uint(__uint_as_float(v[d]) * corr);
+          tmem_store16(o_addr + (unsigned)c, v);
+        }
+        tmem_wait_st();
+        fence_before_sync();
+      }
       l_run = l_run * corr + row_sum;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes, read by the tensor cores
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.p_full[sb]);
     }
-    if (ok && taken >= 1) ok = consume(wg + (taken - 1) * GROUPS, corr_saved);
-    if (GROUPS == 1) {
-      if (ok && r < rows) {
-        float inv = OPTIONS ? sink_factor(m_run, l_run, options, h) : 1.0f / l_run;
-        bf16* dst = out + (OPTIONS ? (size_t)(tok0 + r) * options.out_stride + h * HD : ((size_t)(tok0 + r) * heads + h) * HD);
+    if (ok && taken >= 1) ok = added(wg + (taken - 1) * GROUPS);
+    auto load_outputs = [&](int c, float* o) {  // sixteen of the row's outputs (a group without a step has none)
+      unsigned v[16];
+      if (taken >= 1) tmem_load16(o_addr + (unsigned)c, v);
 #pragma unroll
-        for (int c = 0; c < HD / 8; ++c) {
-          uint4 w;
-          __nv_bfloat162* pk = reinterpret_cast<__nv_bfloat162*>(&w);
+      for (int d = 0; d < 16; ++d) o[d] = taken >= 1 ? __uint_as_float(v[d]) : 0.f;
+    };
+    // every product has been added: the shared memory of the keys, values and P is free for the exchange
+    asm volatile("bar.sync 1, %0;" ::"n"(SOFT_WARPS * 32) : "memory");
+    float* ex = reinterpret_cast<float*>(k_s) + (size_t)r * S::EX_LD;  // the row's place in the first exchange tile
+    constexpr size_t EX_TILE = (size_t)BQ * S::EX_LD;
+    if (wg > 0) {
+      float* to = ex + (wg - 1) * EX_TILE;
+      for (int c = 0; c < HD; c += 16) {
+        float o[16];
+        load_outputs(c, o);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            pk[i] = __floats2bfloat162_rn(o[c * 8 + 2 * i] * inv, o[c * 8 + 2 * i + 1] * inv);
-          *reinterpret_cast<uint4*>(dst + c * 8) = w;
-        }
+        for (int d = 0; d < 16; d += 2) *reinterpret_cast<float2*>(to + c + d) = make_float2(o[d], o[d + 1]);
       }
-    } else {
-      // every product has been consumed: the shared memory of the key and value stages is free for the exchange
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      float* ex = reinterpret_cast<float*>(k_s) + (size_t)r * S::EX_LD;
-      if (wg == 1) {
+      to[HD] = m_run;
+      to[HD + 1] = l_run;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(SOFT_WARPS * 32) : "memory");
+    if (wg == 0 && ok) {  // (whole warps read tensor memory; rows that do not exist are not stored)
+      float m = m_run, share[GROUPS];
 #pragma unroll
-        for (int d = 0; d < HD; d += 2) *reinterpret_cast<float2*>(ex + d) = make_float2(o[d], o[d + 1]);
-        ex[HD] = m_run;
-        ex[HD + 1] = l_run;
+      for (int i = 1; i < GROUPS; ++i) m = fmaxf(m, ex[(i - 1) * EX_TILE + HD]);
+      float m_use = m == -INFINITY ? 0.f : m;
+      share[0] = fast_exp2(m_run - m_use);
+      float l = l_run * share[0];
+#pragma unroll
+      for (int i = 1; i < GROUPS; ++i) {
+        share[i] = fast_exp2(ex[(i - 1) * EX_TILE + HD] - m_use);
+        l += ex[(i - 1) * EX_TILE + HD + 1] * share[i];
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (wg == 0 && ok && r < rows) {
-        float m_other = ex[HD], l_other = ex[HD + 1];
-        float m = fmaxf(m_run, m_other);
-        float m_use = m == -INFINITY ? 0.f : m;
-        float mine = fast_exp2(m_run - m_use), theirs = fast_exp2(m_other - m_use);
-        float l = l_run * mine + l_other * theirs;
-        float inv = OPTIONS ? sink_factor(m_use, l, options, h) : 1.0f / l;
-        mine *= inv;
-        theirs *= inv;
-        bf16* dst = out + (OPTIONS ? (size_t)(tok0 + r) * options.out_stride + h * HD : ((size_t)(tok0 + r) * heads + h) * HD);
+      float inv = OPTIONS ? sink_factor(m_use, l, options, h) : 1.0f / l;
 #pragma unroll
-        for (int c = 0; c < HD / 8; ++c) {
-          uint4 w;
-          __nv_bfloat162* pk = reinterpret_cast<__nv_bfloat162*>(&w);
+      for (int i = 0; i < GROUPS; ++i) share[i] *= inv;
+      bf16* dst = out + (OPTIONS ? (size_t)(tok0 + r) * options.out_stride + h * HD : ((size_t)(tok0 + r) * heads + h) * HD);
+      for (int c = 0; c < HD; c += 16) {
+        float o[16];
+        load_outputs(c, o);
+        if (r >= rows) continue;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            int d = c * 8 + 2 * i;
-            float2 other = *reinterpret_cast<const float2*>(ex + d);
-            pk[i] = __floats2bfloat162_rn(o[d] * mine + other.x * theirs, o[d + 1] * mine + other.y * theirs);
+        for (int d = 0; d < 16; d += 2) {
+          float x = o[d] * share[0], y = o[d + 1] * share[0];
+#pragma unroll
+          for (int i = 1; i < GROUPS; ++i) {
+            float2 other = *reinterpret_cast<const float2*>(ex + (i - 1) * EX_TILE + c + d);
+            x += other.x * share[i];
+            y += other.y * share[i];
           }
-          *reinterpret_cast<uint4*>(dst + c * 8) = w;
+          o[d] = x;
+          o[d + 1] = y;
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint4 w;
+          __nv_bfloat162* pk = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) pk[i] = __floats2bfloat162_rn(o[half * 8 + 2 * i], o[half * 8 + 2 * i + 1]);
+          *reinterpret_cast<uint4*>(dst + c + half * 8) = w;
         }
       }
     }

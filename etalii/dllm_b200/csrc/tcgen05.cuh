@@ -96,6 +96,15 @@ __device__ __forceinline__ void tmem_load16(unsigned taddr, unsigned* v) {
   tmem_load16_nowait(taddr, v);
   tmem_wait_ld();
 }
+// The same back to tensor memory; `tmem_wait_st` before anyone is told.
+__device__ __forceinline__ void tmem_store16(unsigned taddr, const unsigned* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // One warp allocates `columns` (a power of two, at least 32) and writes the base address to shared memory.
 __device__ __forceinline__ void tmem_alloc(unsigned* base_in_smem, unsigned columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
