@@ -99,29 +99,35 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   int newest = end - 1;
   constexpr int ROUND = CLUSTER * WARPS;  // tiles that all warps together take at a time
 
-  auto copy_page = [&](int key0) {
-    int page = pages[key0 / TILE_KEYS];
-    const bf16* ksrc = (const bf16*)cache.base + keys_of(page, 0);
-    const bf16* vsrc = (const bf16*)cache.base + values_of(page, 0);
-    if (hd == HD && vd == HD) {
+  // A page's keys (which = 0) or values (1), a copy group of their own: the next page's keys are asked for as soon as this
+  // page's scores are there, so that they travel during its softmax and second product, and its values behind that. (As
+  // one group behind the second product a warp had nothing on its way while it computed. 64 sequences of 128 to 2,048, 9
+  // query and 3 kv heads of 64: 14.8 -> 12.6 us; 8 of them 4.8 -> 4.5; 8 of 512 to 4,096, 32 heads: 33.9 -> 30.1.)
+  auto copy_half = [&](int page, int which) {
+    const bf16* src = (const bf16*)cache.base + (which == 0 ? keys_of(page, 0) : values_of(page, 0));
+    bf16* to = which == 0 ? k_s : v_s;
+    const int width = which == 0 ? hd : vd;
+    if (width == HD) {
 #pragma unroll
       for (int i = 0; i < TILE_KEYS * (HD / 8) / 32; ++i) {
         int idx = lane + 32 * i;
-        int dst = (idx / (HD / 8)) * LD + (idx % (HD / 8)) * 8;
-        cp_async_16(k_s + dst, ksrc + idx * 8);
-        cp_async_16(v_s + dst, vsrc + idx * 8);
+        cp_async_16(to + (idx / (HD / 8)) * LD + (idx % (HD / 8)) * 8, src + idx * 8);
       }
     } else {
       for (int idx = lane; idx < TILE_KEYS * (HD / 8); idx += 32) {
         int r = idx / (HD / 8), cc = idx % (HD / 8);
-        if (cc < chunks16) cp_async_16(k_s + r * LD + cc * 8, ksrc + (size_t)r * hd + cc * 8);
-        else *reinterpret_cast<uint4*>(k_s + r * LD + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
-        if (cc < value_chunks) cp_async_16(v_s + r * LD + cc * 8, vsrc + (size_t)r * vd + cc * 8);
-        else *reinterpret_cast<uint4*>(v_s + r * LD + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
+        if (cc < (width >> 3)) cp_async_16(to + r * LD + cc * 8, src + (size_t)r * width + cc * 8);
+        else *reinterpret_cast<uint4*>(to + r * LD + cc * 8) = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::);
-    return page;
+  };
+  auto close_group = [] { asm volatile("cp.async.commit_group;\n" ::); };
+  auto copy_page = [&](int key0) {
+    int page = pages[key0 / TILE_KEYS];
+    copy_half(page, 0);
+    close_group();
+    copy_half(page, 1);
+    close_group();
   };
 
   // this warp's first page: keys of earlier steps do not change any more, so it is copied before the wait on the
@@ -169,12 +175,12 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
     if (h0 != 0 && my_first < tiles) copy_page(key_of(my_first));
     for (int it = my_first; it < tiles; it += ROUND) {
       const int key0 = key_of(it);
-      asm volatile("cp.async.wait_group 0;\n" ::);
+      const bool more = it + ROUND < tiles;
+      const int next_page = more ? pages[key_of(it + ROUND) / TILE_KEYS] : 0;
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the keys (the values may still be on their way)
       __syncwarp();
       if (key0 == newest_tile) {  // the row the projection kernel has just written (chunks16 <= 16 lanes hold it)
-        int r = newest - key0;
-        if (lane < chunks16) *reinterpret_cast<uint4*>(k_s + r * LD + lane * 8) = newest_k;
-        if (lane < value_chunks) *reinterpret_cast<uint4*>(v_s + r * LD + lane * 8) = newest_v;
+        if (lane < chunks16) *reinterpret_cast<uint4*>(k_s + (newest - key0) * LD + lane * 8) = newest_k;
         __syncwarp();
       }
       float s[TILE_KEYS / 8][4];
@@ -193,6 +199,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
           mma_bf16(s[2 * jp + 1], q_frag[ks], bfr[2], bfr[3]);
         }
       }
+      __syncwarp();  // every lane has read the keys: their space is free
+      if (more) copy_half(next_page, 0);
+      close_group();
       if (OPTIONS && capped) {  // from here on in units of log2 e
 #pragma unroll
         for (int j = 0; j < TILE_KEYS / 8; ++j)
@@ -241,6 +250,12 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
         o_acc[i][0] *= corr[0]; o_acc[i][1] *= corr[0];
         o_acc[i][2] *= corr[1]; o_acc[i][3] *= corr[1];
       }
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the values (the next keys may still be on their way)
+      __syncwarp();
+      if (key0 == newest_tile) {
+        if (lane < value_chunks) *reinterpret_cast<uint4*>(v_s + (newest - key0) * LD + lane * 8) = newest_v;
+        __syncwarp();
+      }
 #pragma unroll
       for (int kk = 0; kk < TILE_KEYS / 16; ++kk) {
 #pragma unroll
@@ -252,8 +267,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
           mma_bf16(o_acc[2 * np + 1], p_frag[kk], bfr[2], bfr[3]);
         }
       }
-      __syncwarp();  // the page's space is free for the next copy
-      if (it + ROUND < tiles) copy_page(key_of(it + ROUND));
+      __syncwarp();  // and the values' space
+      if (more) copy_half(next_page, 1);
+      close_group();
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -395,6 +411,9 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     long long places = (long long)sms * (long long)(per_sm > 8 ? 8 : per_sm);
     if (pairs * 8 <= sms) shape = 4;
     else for (shape = 0; shape < 3 && (pairs << shape) * 20 < places * 17; ++shape) {}
+    // (heads up to 64: from more than half as many pairs as places on one block a pair, 256 pairs of 512 to 4,096 keys
+    // 30.1 µs against 32.4; 192 pairs of 128 to 2,048 keys 14.2 against 12.6)
+    if (HD <= 64 && shape == 1 && pairs * 20 >= places * 11) shape = 0;
     // (heads above 64: a block is two warps, and two blocks a pair even out contexts of unequal length better than
     // one; measured with 32 query and 8 kv heads of 128, contexts 128 to 2,304: 64 sequences 62.5 µs against 69.0,
     // 128 sequences 129.3 against 134.0)
