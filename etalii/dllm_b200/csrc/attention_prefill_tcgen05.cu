@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
       bf16* dst = out + (OPTIONS ? (size_t)(tok0 + r) * options.out_stride + h * HD : ((size_t)(tok0 + r) * heads + h) * HD);
       for (int c = 0; c < HD; c += 16) {
         float o[16];
+        __syncwarp();  // (lanes without a query part ways below; tensor memory is read by whole warps)
         load_outputs(c, o);
         if (r >= rows) continue;
 #pragma unroll

@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
 #pragma unroll 1
         for (int seg = seg_begin; seg < seg_end; ++seg) {
           float lo[W], hi[W];
+          __syncwarp();  // (lanes without a row part ways below; tensor memory is read by whole warps)
 #pragma unroll
           for (int col = 0; col < W; col += 16) {
             unsigned v[16];
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
         for (int cc = 0; cc < HALF; cc += 16) {
           int col = c0 + cc;
           unsigned v[16];
+          __syncwarp();  // (as above)
           tmem_load16(acc + (unsigned)col, v);
           if (cc + 16 >= HALF) release_accumulator();
           float f[16];

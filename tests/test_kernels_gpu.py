@@ -831,6 +831,25 @@ def test_attention_prefill_tcgen05(heads, kv_heads, window, head_dim):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_attention_prefill_tcgen05_ragged_tiles(head_dim):
+    """A last tile with fewer queries than lanes, at the edges of warps and between them: its tokens get the bits that they
+    get in a whole tile (later keys are masked there: factors of 0 and 1), and no row behind them is written."""
+    from etalii.dllm_b200.engine.batch import BatchBuffers
+
+    heads, kv_heads, whole = 2, 1, 256
+    cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, [whole], [whole])
+    q = _randn((whole, heads * head_dim), torch.bfloat16, 9)
+    want = torch.empty_like(q)
+    ops().attention_prefill_tcgen05(want, q, view, heads, 0.3, 0, batch)
+    for rows in (1, 7, 31, 32, 33, 63, 65, 96, 127, 129, 155, 250):
+        part = BatchBuffers(DEV).fill(batch.h_slots, [[1] * rows], [0], [[]])
+        out = torch.full_like(q, float("nan"))
+        ops().attention_prefill_tcgen05(out, q[:rows].contiguous(), view, heads, 0.3, 0, part)
+        assert torch.equal(out[:rows], want[:rows]) and bool(out[rows:].isnan().all()), rows
+    ops().raise_if_failed()
+
+
 @pytest.mark.parametrize("window", [None, 1000])
 @pytest.mark.parametrize("head_dim", [64, 128])
 def test_attention_prefill_tcgen05_long(window, head_dim):
