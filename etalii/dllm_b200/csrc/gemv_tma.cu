@@ -45,7 +45,8 @@ __device__ __forceinline__ void ldmatrix_x2(unsigned* r, unsigned addr) {
 using gemv::mma_bf16;
 
 constexpr int RESIDENT_BYTES = 72 * 1024;  // the most that resident rows of X may take
-constexpr int MAX_CHUNKS = 32;             // stages a row of resident X may span (their arrivals are counted one by one)
+// Stages a row of resident X may span (their arrivals are counted one by one): as many as the longest single row that fits.
+constexpr int MAX_CHUNKS = (RESIDENT_BYTES / 2 + KC - 1) / KC;
 
 template <int ROWS, int NT, bool RESIDENT> struct Shape {
   static constexpr int TOKENS = NT * 8;                          // token rows of a stage (those beyond M stay unused)
@@ -325,7 +326,8 @@ int launch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int heigh
                          w, M, N, K, tiles, height, S::stages(M, K), status, rope);
 }
 
-bool resident(int M, int K) { return M <= 8 && M * (2 * K + 16) <= RESIDENT_BYTES && (K + KC - 1) / KC <= MAX_CHUNKS; }
+// (`resident_activations` of kernels/ops.py is the same rule: who asks it calls the entry points below that want it kept)
+bool resident(int M, int K) { return M <= 8 && (long long)M * (2ll * K + 16) <= RESIDENT_BYTES; }
 
 // The height that leaves the busiest multiprocessor the fewest rows, the larger one where several do.
 int tile_height(int N, int sms) {

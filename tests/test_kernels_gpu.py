@@ -688,6 +688,26 @@ def test_gemv_tma_qkv_rope(heads, kv_heads, head_dim, rotary, new, k):
     _check_gemv_qkv_rope(heads, kv_heads, head_dim, rotary, False, 0, k, kernel=4, new=new)
 
 
+@pytest.mark.parametrize("k", [32768, 32832, 36800])
+def test_ring_takes_the_longest_rows_the_rule_calls_resident(k):
+    """One row of activations up to the 72 KB that may lie in shared memory: the calls that go to the ring by that rule
+    (the q/k/v projection, the greedy head, a plain product) run there, at the last size and around 32 stages a row."""
+    assert ops().resident_activations(1, k) and not ops().resident_activations(1, 36864)
+    assert ops().streams_qkv_through_shared_memory(1, 768, k)
+    _check_gemv_qkv_rope(8, 2, 64, 64, False, 0, k, kernel=0, new=[1])
+    n = 16386
+    w = torch.randn((n, k), dtype=torch.bfloat16, device=DEV, generator=torch.Generator(DEV).manual_seed(1)) * 0.02
+    x = _randn((1, k), torch.bfloat16, 2)
+    got = torch.full((1,), -1, dtype=torch.int32, device=DEV)
+    ops().head_argmax(got, x, w, torch.empty(ops().head_argmax_scratch(1, n), dtype=torch.float32, device=DEV))
+    logits = torch.empty((1, n), dtype=torch.float32, device=DEV)
+    ops().gemm(logits, x, w, ops().EPI_STORE_F32)
+    ops().raise_if_failed()
+    exact = torch.cat([x.double() @ part.double().T for part in w.split(2048)], dim=1)
+    assert rel_error(logits.cpu(), exact.cpu()) <= 1e-5  # (k products of 16 bits summed in 32)
+    assert exact[0, got[0].item()] >= exact.max() - 1e-5 * exact.abs().max()
+
+
 def _check_gemv_qkv_rope(heads, kv_heads, head_dim, rotary, normed, rows_extra, k, kernel=2, cluster=0, new=None):
     lengths, new = [70, 5, 129, 64, 200, 33], new or [1, 1, 3, 2, rows_extra, 1]
     lengths = lengths[:len(new)]
