@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(Shape<HD>::THREADS, 1) prefill_tcgen05_kernel(
   constexpr int GROUPS = S::GROUPS, SOFT_WARPS = S::SOFT_WARPS, Q_BYTES = S::Q_BYTES, KV_BYTES = S::KV_BYTES;
   constexpr int K_STAGES = S::K_STAGES, V_STAGES = S::V_STAGES;
   constexpr unsigned TMEM_COLS = S::TMEM_COLS;
-  int tile = (int)(gridDim.x - 1 - blockIdx.x), h = blockIdx.y;  // (a prompt's last tiles see the most keys: they go first)
+  int tile = blockIdx.x, h = blockIdx.y;  // (the host lists the tiles that see the most keys first, see below)
   int q0 = tile_first[tile];
   if (q0 % BQ) return;  // the host lists tiles of 64 tokens; every second one starts a tile of 128
   pdl_launch_dependents();
