@@ -99,10 +99,15 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   int newest = end - 1;
   constexpr int ROUND = CLUSTER * WARPS;  // tiles that all warps together take at a time
 
-  // A page's keys (which = 0) or values (1), a copy group of their own: the next page's keys are asked for as soon as this
-  // page's scores are there, so that they travel during its softmax and second product, and its values behind that. (As
-  // one group behind the second product a warp had nothing on its way while it computed. 64 sequences of 128 to 2,048, 9
-  // query and 3 kv heads of 64: 14.8 -> 12.6 us; 8 of them 4.8 -> 4.5; 8 of 512 to 4,096, 32 heads: 33.9 -> 30.1.)
+  // A page's keys (which = 0) or values (1). AHEAD: each is a copy group of its own, the next page's keys are asked for as
+  // soon as this page's scores are there, so that they travel during its softmax and second product, and its values behind
+  // that. (As one group behind the second product a warp has nothing on its way while it computes. 64 sequences of 128 to
+  // 2,048, 9 query and 3 kv heads of 64: 14.8 -> 12.6 us; 8 of them 4.8 -> 4.5; 8 of 512 to 4,096, 32 heads: 33.9 -> 30.1.)
+  // Not where it costs more than it gives. With options its registers leave two blocks of HD = 64 on a multiprocessor
+  // instead of three (232 against 164 a thread; 64 sequences of 1,000, 9 query and 3 kv heads: 16.6 us against 11.2). Heads
+  // of 128 gain 3 % at 4,000 keys (6 where one sequence is far longer than the rest) and lose 5 % at 64 (32 query and 8 kv
+  // heads, 1 to 256 sequences).
+  constexpr bool AHEAD = HD <= 64 && !OPTIONS;
   auto copy_half = [&](int page, int which) {
     const bf16* src = (const bf16*)cache.base + (which == 0 ? keys_of(page, 0) : values_of(page, 0));
     bf16* to = which == 0 ? k_s : v_s;
@@ -125,7 +130,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   auto copy_page = [&](int key0) {
     int page = pages[key0 / TILE_KEYS];
     copy_half(page, 0);
-    close_group();
+    if (AHEAD) close_group();
     copy_half(page, 1);
     close_group();
   };
@@ -176,11 +181,13 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
     for (int it = my_first; it < tiles; it += ROUND) {
       const int key0 = key_of(it);
       const bool more = it + ROUND < tiles;
-      const int next_page = more ? pages[key_of(it + ROUND) / TILE_KEYS] : 0;
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the keys (the values may still be on their way)
+      const int next_page = AHEAD && more ? pages[key_of(it + ROUND) / TILE_KEYS] : 0;
+      // the page; AHEAD: its keys (its values may still be on their way)
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(AHEAD ? 1 : 0) : "memory");
       __syncwarp();
       if (key0 == newest_tile) {  // the row the projection kernel has just written (chunks16 <= 16 lanes hold it)
         if (lane < chunks16) *reinterpret_cast<uint4*>(k_s + (newest - key0) * LD + lane * 8) = newest_k;
+        if (!AHEAD && lane < value_chunks) *reinterpret_cast<uint4*>(v_s + (newest - key0) * LD + lane * 8) = newest_v;
         __syncwarp();
       }
       float s[TILE_KEYS / 8][4];
@@ -199,9 +206,11 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
           mma_bf16(s[2 * jp + 1], q_frag[ks], bfr[2], bfr[3]);
         }
       }
-      __syncwarp();  // every lane has read the keys: their space is free
-      if (more) copy_half(next_page, 0);
-      close_group();
+      if (AHEAD) {
+        __syncwarp();  // every lane has read the keys: their space is free
+        if (more) copy_half(next_page, 0);
+        close_group();
+      }
       if (OPTIONS && capped) {  // from here on in units of log2 e
 #pragma unroll
         for (int j = 0; j < TILE_KEYS / 8; ++j)
@@ -250,11 +259,13 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
         o_acc[i][0] *= corr[0]; o_acc[i][1] *= corr[0];
         o_acc[i][2] *= corr[1]; o_acc[i][3] *= corr[1];
       }
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the values (the next keys may still be on their way)
-      __syncwarp();
-      if (key0 == newest_tile) {
-        if (lane < value_chunks) *reinterpret_cast<uint4*>(v_s + (newest - key0) * LD + lane * 8) = newest_v;
+      if (AHEAD) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the values (the next keys may still be on their way)
         __syncwarp();
+        if (key0 == newest_tile) {
+          if (lane < value_chunks) *reinterpret_cast<uint4*>(v_s + (newest - key0) * LD + lane * 8) = newest_v;
+          __syncwarp();
+        }
       }
 #pragma unroll
       for (int kk = 0; kk < TILE_KEYS / 16; ++kk) {
@@ -267,9 +278,13 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
           mma_bf16(o_acc[2 * np + 1], p_frag[kk], bfr[2], bfr[3]);
         }
       }
-      __syncwarp();  // and the values' space
-      if (more) copy_half(next_page, 1);
-      close_group();
+      __syncwarp();  // the page's space is free (AHEAD: what is left of it)
+      if (AHEAD) {
+        if (more) copy_half(next_page, 1);
+        close_group();
+      } else if (more) {
+        copy_page(key_of(it + ROUND));
+      }
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -411,8 +426,10 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     long long places = (long long)sms * (long long)(per_sm > 8 ? 8 : per_sm);
     if (pairs * 8 <= sms) shape = 4;
     else for (shape = 0; shape < 3 && (pairs << shape) * 20 < places * 17; ++shape) {}
-    // (heads up to 64: from more than half as many pairs as places on one block a pair, 256 pairs of 512 to 4,096 keys
-    // 30.1 µs against 32.4; 192 pairs of 128 to 2,048 keys 14.2 against 12.6)
+    // (heads up to 64: from more than half as many pairs as places on one block a pair; 192 pairs of 128 to 2,048 keys are
+    // below that and better off with two, 12.6 µs against 14.2. Above it, 256 to 512 pairs with heads of 32, 48 and 64, one
+    // block takes 0.37 to 0.95 of the time that two took, at 64 to 4,000 keys, of one length and of lengths from 128 to
+    // 2,048. The exception is one sequence of 4,096 keys among 255 of 128 with heads of 48: 29.0 against 24.0)
     if (HD <= 64 && shape == 1 && pairs * 20 >= places * 11) shape = 0;
     // (heads above 64: a block is two warps, and two blocks a pair even out contexts of unequal length better than
     // one; measured with 32 query and 8 kv heads of 128, contexts 128 to 2,304: 64 sequences 62.5 µs against 69.0,
