@@ -215,9 +215,10 @@ int launch_tiles(void* c, const float* a, const float* w, int M, int N, int K, c
     long long tiles = (long long)((M + tile - 1) / tile) * ((N + tile - 1) / tile);
     return (tiles + 147) / 148;
   };
+  auto fits = [&](int tile) { return (M + tile - 1) / tile <= 65535; };  // (rows of tiles are the grid's second dimension)
   long long wide = 57 * rounds(128) + 4, middle = 20 * rounds(64) + 2, small = 8 * rounds(32) + 2;
-  if (wide <= middle && wide <= small) return launch_wide<EPI>(c, a, w, M, N, K, stream);
-  if (middle <= small) return launch_tile<EPI, 64, 4, 2>(c, a, w, M, N, K, stream);
+  if (!fits(64) || (wide <= middle && (wide <= small || !fits(32)))) return launch_wide<EPI>(c, a, w, M, N, K, stream);
+  if (!fits(32) || middle <= small) return launch_tile<EPI, 64, 4, 2>(c, a, w, M, N, K, stream);
   return launch_tile<EPI, 32, 6, 4>(c, a, w, M, N, K, stream);
 }
 

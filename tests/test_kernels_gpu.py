@@ -135,6 +135,21 @@ def test_gemm_f32_tiles(m, n, k):
     assert rel_error(ref.cpu(), (a.double() @ w.double().T).float().cpu()) <= 2e-6
 
 
+@pytest.mark.parametrize("m,n", [(65535 * 32 + 1, 6), (65535 * 64 + 1, 40)])
+def test_gemm_f32_more_row_tiles_than_a_grid_has(m, n):
+    """Millions of rows by a few columns: where the small tiles would need more than 65,535 rows of tiles a larger one runs."""
+    g = torch.Generator(DEV).manual_seed(3)
+    a = torch.randn((m, 4), dtype=torch.float32, device=DEV, generator=g)
+    w = _randn((n, 4), torch.float32, 4)
+    c = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
+    ops().gemm(c, a, w, 0)
+    few = torch.empty((16, n), dtype=torch.float32, device=DEV)
+    for row in (0, m // 2, m - 16):
+        ops().gemm(few, a[row:row + 16].contiguous(), w, 0)
+        assert torch.equal(c[row:row + 16], few)
+    assert not bool(c.isnan().any())
+
+
 def test_gemm_f32_rows_do_not_depend_on_the_batch():
     a, w = _randn((150, 136), torch.float32, 6), _randn((200, 136), torch.float32, 7)
     whole = torch.empty((150, 200), dtype=torch.float32, device=DEV)
