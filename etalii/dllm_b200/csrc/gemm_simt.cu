@@ -103,31 +103,17 @@ int launch_tile(void* c, const float* a, const float* w, int M, int N, int K, cu
 
 // ---- tiles of 128 x 128 outputs, 8 x 8 of them a thread ----------------------------------------------------------------
 // Two stages of shared memory; the next k tile travels from global memory into registers while this one is multiplied.
-// A thread's 64 outputs are 2 x 2 groups of 4 x 4, so its shared-memory reads are four 16-byte loads per k; two
-// neighbouring columns share a packed multiply-add (`fma.rn.f32x2`: two correctly rounded multiply-adds in one issue
-// slot, which leaves slots for the loads and stores). Every output is one chain over k ascending from zero here too: the
-// same bits. 2048 x 3072 x 576: 200 -> 174 us (42 TFLOP/s); 8 x 16 outputs a thread: 186; rows as they lie with cp.async,
-// as for the smaller tiles: 240.
+// A thread's 64 outputs are 2 x 2 groups of 4 x 4, so its shared-memory reads are four 16-byte loads per k. Every output is
+// one chain over k ascending from zero here too: the same bits. Bounds for one block a multiprocessor: with bounds for two, with
+// packed multiply-adds (two outputs an instruction), or both, a round of one tile each is slower. 512 x 4096 x
+// 4096 (128 tiles): 396 us (43 TFLOP/s); bounds for two 458, packed 483, both 497. 2048 x 3072 x 576 (384 tiles): 176; 187,
+// 198, 179. 4096 x 4096 x 2048 (1,024 tiles): 1,397; 1,468, 1,665, 1,407. Only very many tiles gain by both (49152 columns,
+// 6,144 tiles: 2,437 against 2,352). 8 x 16 outputs a thread: 186 at 2048 x 3072 x 576; rows as they lie with cp.async, as
+// for the smaller tiles: 240.
 constexpr int WM = 128, WN = 128, WK = 16;
 
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 template <int EPI>
-__global__ void __launch_bounds__(256, 2) gemm_f32_wide_kernel(
+__global__ void __launch_bounds__(256, 1) gemm_f32_wide_kernel(
     void* __restrict__ c, const float* __restrict__ a, const float* __restrict__ w, int M, int N, int K) {
   __shared__ __align__(16) float as[2][WK][WM + 4];
   __shared__ __align__(16) float ws[2][WK][WN + 4];
@@ -135,11 +121,11 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_wide_kernel(
   int tx = tid & 15, ty = tid >> 4;             // rows ty * 4 + {0..3, 64..67}, columns likewise
   int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
   int lrow = tid >> 2, lk = (tid & 3) * 4;      // a thread fetches rows lrow and lrow + 64, k lk .. lk + 3
-  unsigned long long acc[8][4];
+  float acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
   float4 va[2], vw[2];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -168,15 +154,13 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_wide_kernel(
 #pragma unroll
     for (int k = 0; k < WK; ++k) {
       float4 a0 = *(const float4*)&as[buf][k][ty * 4], a1 = *(const float4*)&as[buf][k][64 + ty * 4];
+      float4 w0 = *(const float4*)&ws[buf][k][tx * 4], w1 = *(const float4*)&ws[buf][k][64 + tx * 4];
       float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      ulonglong2 w0 = *(const ulonglong2*)&ws[buf][k][tx * 4], w1 = *(const ulonglong2*)&ws[buf][k][64 + tx * 4];
-      unsigned long long wv[4] = {w0.x, w0.y, w1.x, w1.y};
+      float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        unsigned long long both = pack2(av[i], av[i]);
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma2(both, wv[j], acc[i][j]);
-      }
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
     }
     if (t + 1 < tiles) {
       stash(buf ^ 1);  // (the other stage was last read before the barrier that ended the step before)
@@ -187,10 +171,9 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_wide_kernel(
   for (int i = 0; i < 8; ++i) {
     int m = m0 + (i >> 2) * 64 + ty * 4 + (i & 3);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int n = n0 + (j >> 1) * 64 + tx * 4 + 2 * (j & 1);
-      float2 v = unpack2(acc[i][j]);
-      epilogue_pair<EPI, float>(c, m, n, M, N, v.x, v.y);
+    for (int j = 0; j < 8; j += 2) {
+      int n = n0 + (j >> 2) * 64 + tx * 4 + (j & 3);
+      epilogue_pair<EPI, float>(c, m, n, M, N, acc[i][j], acc[i][j + 1]);
     }
   }
 }
@@ -203,9 +186,9 @@ int launch_wide(void* c, const float* a, const float* w, int M, int N, int K, cu
   return dllm_launch_status();
 }
 
-// Which tile: the fewest microseconds by rounds of one tile per multiprocessor. A round of K = 576 was measured at about
-// 57 us for 128 x 128 (37 to 45 TFLOP/s with all multiprocessors busy), 20 for 64 x 64 and, while few rounds are needed,
-// 8 for 32 x 32, plus a few to begin; all grow alike with K. So full devices take the large tile, and a product too small
+// Which tile: the fewest microseconds by rounds of one tile per multiprocessor. Whole launches of K = 576, last rounds that
+// are partly empty among them, are fitted by 57 us a round of 128 x 128, 20 of 64 x 64 and, while few rounds are needed,
+// 8 of 32 x 32, plus a few to begin; all grow alike with K. So full devices take the large tile, and a product too small
 // for it (2048 x 576: 80 tiles of 128 x 128 for 148 multiprocessors) one that spreads over all of them.
 // Launched without programmatic dependence: blocks of the next kernel that wait on a multiprocessor for this one make the
 // launch after it spread unevenly (2048 x 576 x 576 back to back: 110 us instead of 72).
