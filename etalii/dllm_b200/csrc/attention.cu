@@ -54,6 +54,8 @@ __device__ __forceinline__ void score_piece(float2& acc, const float* q, uint4 r
     acc.y = fmaf(q[2 * i + 1], k.y, acc.y);
   }
 }
+// The score: a product of its own, never the front half of a fused multiply-add with what is subtracted from it later.
+__device__ __forceinline__ float scaled(float2 dot, float scale) { return __fmul_rn(dot.x + dot.y, scale); }
 __device__ __forceinline__ float4 load_vec(const float* k) { return *(const float4*)k; }
 __device__ __forceinline__ uint4 load_vec(const __nv_bfloat16* k) { return *(const uint4*)k; }
 
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_warp_kernel(
         const T* krow = base + kv_offset(cache, page[u], 0, g, j % ps);
         float2 dot = make_float2(0.f, 0.f);
         for (int d = 0; d < hd; d += Vec<T>::N) score_piece(dot, &q_s[warp][d], load_vec(krow + d));
-        s[u] = (dot.x + dot.y) * scale;
+        s[u] = scaled(dot, scale);
       }
     }
     float m = warp_max(fmaxf(s[0], s[1])), shift = finite_or_zero(m);
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
               }
             }
 #pragma unroll
-            for (int r = 0; r < R; ++r) weight[r][u] = (dot[r].x + dot[r].y) * scale;
+            for (int r = 0; r < R; ++r) weight[r][u] = scaled(dot[r], scale);
           }
           // (a single token a warp, as in decoding, hands its weights from lane to lane by shuffles; several go
           // through shared memory, four weights a load)
@@ -507,8 +509,7 @@ __global__ void __launch_bounds__(TILE_THREADS, HD == 64 ? 4 : 2) attention_tile
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            float2 halves = unpack2(dot[i][j]);
-            s[i][j] = (halves.x + halves.y) * scale;
+            s[i][j] = scaled(unpack2(dot[i][j]), scale);
           }
       }
       bool whole = true;  // every token of this thread that sees the page sees all of it
@@ -706,7 +707,7 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
       for (int u = 0; u < 2; ++u) {
         int j = j0 + lane + 32 * u;
         valid[u] = j >= first && j < end;
-        p[u] = valid[u] ? (dot[u].x + dot[u].y) * scale : -INFINITY;
+        p[u] = valid[u] ? scaled(dot[u], scale) : -INFINITY;
       }
       float m = warp_max(fmaxf(p[0], p[1])), shift = finite_or_zero(m);
 #pragma unroll
