@@ -654,7 +654,7 @@ constexpr int CHUNK_WARPS = 16;
 __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
     float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_seq,
     const int* __restrict__ tok_pos, const int* __restrict__ slots, int heads, float scale, int window, int heads_per_block,
-    int per_round, int room) {
+    int per_round, int room, int* __restrict__ status) {
   extern __shared__ __align__(16) float smem[];
   int hd = cache.head_dim, ld = hd + 4, group = heads / cache.kv_heads, pieces = hd / 4;
   int size = (int)gridDim.x, rank = (int)blockIdx.x;  // (a cluster is a row of the grid)
@@ -669,7 +669,10 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
   pdl_wait();
   int end = tok_pos[t] + 1, first = (window > 0 && end > window) ? end - window : 0;
   const int* pages = cache.page_table + (size_t)slots[tok_seq[t]] * cache.max_pages;
-  int chunk0 = first / 64, chunks = min((end + 63) / 64 - chunk0, room * size);  // (`room` covers what the caller says)
+  int chunk0 = first / 64, chunks = min((end + 63) / 64 - chunk0, room * size);
+  // (`room` covers what the caller says; a token that sees more gets no number, and the host is told)
+  bool told = chunks == (end + 63) / 64 - chunk0;
+  if (!told && threadIdx.x == 0) *(volatile int*)status = 50;
   for (int i = threadIdx.x; i < here * hd; i += threads)
     q_s[i] = q[((size_t)t * heads + g * group + head0) * hd + i];
   int mine = warp / heads_per_block, head = warp % heads_per_block;
@@ -764,7 +767,7 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
         acc = merge_output(acc, keep, o[x], take);
       }
     }
-    out[((size_t)t * heads + g * group + head0) * hd + i] = acc * (1.0f / l_run);
+    out[((size_t)t * heads + g * group + head0) * hd + i] = told ? acc * (1.0f / l_run) : __int_as_float(0x7fffffff);
   }
   asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
@@ -772,12 +775,12 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
 // Refuses (DLLM_UNSUPPORTED_SIZE) what does not fit; the caller then takes the serial form, which gives the same bits.
 // `reach`: the most keys a token may see.
 int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* tok_seq, const int* tok_pos, const int* slots,
-                  int tokens, int heads, float scale, int window, long long reach, cudaStream_t stream) {
+                  int tokens, int heads, float scale, int window, long long reach, int* status, cudaStream_t stream) {
   int group = heads / cache.kv_heads, hd = cache.head_dim, ld = hd + 4;
   // (a window of w keys may begin anywhere in its first chunk)
   long long chunks = (reach + 63) / 64;
   if (window > 0 && window < reach) chunks = ((long long)window + 126) / 64;
-  if (tokens > 65535) return DLLM_UNSUPPORTED_SIZE;
+  if (tokens > 65535 || status == nullptr) return DLLM_UNSUPPORTED_SIZE;
   int heads_per_block = group < CHUNK_WARPS ? group : CHUNK_WARPS;
   int parts = (group + heads_per_block - 1) / heads_per_block;
   long long rows = (long long)cache.kv_heads * parts;
@@ -808,7 +811,7 @@ int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* 
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&config, attention_chunks_kernel, out, q, cache, tok_seq, tok_pos, slots, heads, scale, window,
-                            heads_per_block, per_round, room) == cudaSuccess
+                            heads_per_block, per_round, room, status) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
 }
@@ -837,13 +840,14 @@ DLLM_EXPORT int dllm_attention_general(void* out, const void* q, void* cache_bas
 
 // The same attention with the same arguments, blockwise; the same bits. `max_new`: the most new tokens a sequence brings
 // in this step: with one each (decoding) a block serves one token's heads, else runs of tokens. `max_context`: the most
-// keys any token of the step may see. Pages of 64 positions, at most 65,535 kv heads.
+// keys any token of the step may see; one that sees more gets no number (NaN) and `status`, a word that the device can write,
+// is set to 50. Pages of 64 positions, at most 65,535 kv heads.
 // float32 takes the kernels made for it: single tokens their chunks side by side, prompts with heads of 64 and 128 in
 // 16-byte aligned rows the tiles of queries.
 DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base, const int* page_table,
                                       int max_pages, int page_size, int heads, int kv_heads, int head_dim,
                                       const int* tok_seq, const int* tok_pos, const int* slots, int tokens,
-                                      int max_new, int max_context, float scale, int window, int dtype,
+                                      int max_new, int max_context, float scale, int window, int dtype, int* status,
                                       cudaStream_t stream) {
   if (tokens <= 0) return DLLM_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads) return DLLM_BAD_ARGUMENT;
@@ -863,9 +867,9 @@ DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base
     const float* rows = (const float*)q;
     bool aligned = (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
     if (!runs) {
-      int status = launch_chunks((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window,
-                                 max_context > 0 ? max_context : (long long)max_pages * page_size, stream);
-      if (status != DLLM_UNSUPPORTED_SIZE) return status;
+      int done = launch_chunks((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window,
+                                 max_context > 0 ? max_context : (long long)max_pages * page_size, status, stream);
+      if (done != DLLM_UNSUPPORTED_SIZE) return done;
     } else if (head_dim == 64 && aligned) {
       return launch_tiles<64>((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window, stream);
     } else if (head_dim == 128 && aligned) {

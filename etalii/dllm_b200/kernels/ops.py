@@ -238,7 +238,7 @@ _prototypes = {
                                               c_void_p],
     ("attention", "dllm_attention_blocks"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                              c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
-                                             c_int, c_void_p],
+                                             c_int, c_void_p, c_void_p],
     ("attention_decode", "dllm_attention_decode"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                                     c_int, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int,
                                                     c_void_p, c_void_p, c_void_p],
@@ -1661,7 +1661,7 @@ def _status_word() -> torch.Tensor:
 def raise_if_failed() -> None:
     """Raises if a kernel has set the status word since the last look: a bounded wait on an mbarrier ran out
     (codes 2-5 the tile product, 12-21 the tcgen05 attention, 32-33 the product that streams through shared memory, 42-45
-    the experts' tile products)
+    the experts' tile products), a token saw more keys than its step was prepared for (50),
     or the embedding met a token outside its table (64). Results computed since are not valid. The word lives in
     pinned host memory, so the look costs no synchronisation; it is meaningful after the host has waited for the
     kernels in question (a `.tolist()`, a copy to the host, a synchronize)."""
@@ -1670,6 +1670,8 @@ def raise_if_failed() -> None:
         _async_status[0] = 0
         if code == 64:
             raise KernelError("the embedding was given a token outside its table; the step's results are invalid")
+        if code == 50:
+            raise KernelError("a token sees more keys than the step's max_context; the step's results are invalid")
         raise KernelError(f"a kernel gave up waiting on an mbarrier (role code {code}); the step's results are invalid")
 
 
@@ -2188,7 +2190,7 @@ def attention_blocks(out: torch.Tensor, q: torch.Tensor, cache, heads: int, scal
         out.data_ptr(), q.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(), cache.max_pages, cache.page_size,
         heads, cache.kv_heads, cache.head_dim, batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(),
         batch.slots.data_ptr(), batch.n_tokens, int(batch.max_new), int(batch.max_context), float(scale),
-        int(window or 0), _code(cache.dtype), _stream()), "attention_blocks",
+        int(window or 0), _code(cache.dtype), _status_word().data_ptr(), _stream()), "attention_blocks",
         lambda: f"head_dim={cache.head_dim} must be a multiple of 8, at most 256; pages of 64")
 
 

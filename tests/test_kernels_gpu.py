@@ -407,6 +407,29 @@ def test_attention_float32_bits(heads, kv_heads, head_dim, window, lengths, new)
     assert bool(torch.isfinite(out).all()) and torch.equal(out, other)
 
 
+def test_attention_of_more_keys_than_the_step_says():
+    """A step whose max_context is too small for a sequence: the host is told and the sequence's tokens get no number; the
+    others get theirs, and with the true bound so does it."""
+    from etalii.dllm_b200.kernels.ops import KernelError
+
+    heads, kv_heads, hd = 9, 3, 64
+    cache, view, batch = _cache_and_batch(torch.float32, kv_heads, hd, [2300, 300], [1, 1])
+    q = _randn((2, heads * hd), torch.float32, 9)
+    want, out = torch.empty_like(q), torch.zeros_like(q)
+    ops().attention_general(want, q, view, heads, 0.3, 0, batch)
+    batch.max_context = 1024
+    ops().attention_blocks(out, q, view, heads, 0.3, 0, batch)
+    torch.cuda.synchronize()
+    with pytest.raises(KernelError, match="more keys"):
+        ops().raise_if_failed()
+    assert bool(out[0].isnan().all()) and torch.equal(out[1], want[1])
+    batch.max_context = 2300
+    ops().attention_blocks(out, q, view, heads, 0.3, 0, batch)
+    torch.cuda.synchronize()
+    ops().raise_if_failed()
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_finds_a_far_key(dtype):
     """One key among hundreds matches the query: the output must be that key's value, wherever its page lies."""
