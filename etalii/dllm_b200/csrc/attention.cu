@@ -410,39 +410,31 @@ int launch_blocks(void* out, const void* q, const KvLayout& cache, const int* to
                                                                   heads_per_pass, stages);
   return dllm_launch_status();
 }
-// ---- float32 prompts with heads of 64 and 128: tiles of 32 queries of one head ------------------------------------------
+// ---- float32 with heads of 64 and 128: tiles of 32 queries of one head -----------------------------------------------------
 // Bound by multiply-adds and the shared-memory reads that feed them, so it is laid out like a product: a block takes 32
-// consecutive tokens and one query head, a thread four tokens (ty + 8 i) by four keys (tx + 16 j) of the scores and by
-// HD / 16 dimensions of the outputs; a key, value or weight read from shared memory serves four multiply-adds, the even and
-// odd dimensions of a score and neighbouring output dimensions share a packed one. The next page's keys are on their way
-// while values are multiplied, the next values while scores are. 32 queries rather than 64: a prompt of 2,048 with nine
-// heads is 576 blocks, which level out over the device although the last ones see 32 times the keys of the first ones
+// consecutive new tokens of a sequence and one query head, a thread four tokens (ty + 8 i) by four keys (tx + 16 j) of the
+// scores and by HD / 16 dimensions of the outputs; a key, value or weight read from shared memory serves four multiply-adds,
+// the even and odd dimensions of a score and neighbouring output dimensions share a packed one. The next page's keys are on
+// their way while values are multiplied, the next values while scores are. 32 queries rather than 64: a prompt of 2,048 with
+// nine heads is 576 blocks, which level out over the device although the last ones see 32 times the keys of the first ones
 // (those go first). Before, a warp walked the keys for four tokens, and read a value and a weight for every four
 // multiply-adds: 492 us a layer at 2,048 tokens (9 query, 3 kv heads of 64), now 214 (23 TFLOP/s).
+// A tile never spans two sequences, and one of up to eight tokens is one row a thread: a step in which many sequences bring a
+// token or two beside a prompt is many small blocks side by side.
 constexpr int TILE_Q = 32, TILE_THREADS = 128;
 
 template <int HD>
 struct TileShared {
   float q[TILE_Q][HD + 4], k[64][HD + 4], v[64][HD + 4], p[TILE_Q][64 + 4];
-  int end[TILE_Q];
 };
 
-template <int HD>
-__global__ void __launch_bounds__(TILE_THREADS, HD == 64 ? 4 : 2) attention_tile_kernel(
-    float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_seq,
-    const int* __restrict__ tok_pos, const int* __restrict__ slots, int tokens, int heads, float scale, int window) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TileShared<HD>& sm = *reinterpret_cast<TileShared<HD>*>(smem_raw);
+// One tile: `count` tokens, at most 8 * NI, from position pos0 of the sequence on; q and out at the first one's row.
+template <int HD, int NI>
+__device__ __forceinline__ void attend_tile(TileShared<HD>& sm, float* __restrict__ out, const float* __restrict__ q,
+                                            const KvLayout& cache, const int* __restrict__ pages, int count, int pos0, int h,
+                                            int g, int heads, float scale, int window) {
   constexpr int GROUPS = HD / 64;  // groups of four output dimensions a thread owns, 64 apart
   int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int h = blockIdx.x % heads, g = h / (heads / cache.kv_heads);
-  int t0 = ((int)(gridDim.x / heads) - 1 - (int)(blockIdx.x / heads)) * TILE_Q, t_stop = min(tokens, t0 + TILE_Q);
-  for (int i = tid; i < TILE_Q * (HD / 4); i += TILE_THREADS) {
-    int r = i / (HD / 4), d = i % (HD / 4) * 4;
-    float4 value = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t0 + r < tokens) value = *(const float4*)(q + ((size_t)(t0 + r) * heads + h) * HD + d);
-    *(float4*)&sm.q[r][d] = value;
-  }
   auto copy_page = [&](float (*to)[HD + 4], int page, int which) {
     const float* from = (const float*)cache.base + kv_offset(cache, page, which, g, 0);
 #pragma unroll 4
@@ -453,191 +445,206 @@ __global__ void __launch_bounds__(TILE_THREADS, HD == 64 ? 4 : 2) attention_tile
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
-
-  for (int run_begin = t0; run_begin < t_stop;) {
-    // a run: the block's tokens of one sequence (positions ascend inside it)
-    int seq = tok_seq[run_begin], run_end = run_begin + 1;
-    while (run_end < t_stop && tok_seq[run_end] == seq) ++run_end;
-    const int* pages = cache.page_table + (size_t)slots[seq] * cache.max_pages;
-    int run_last = tok_pos[run_end - 1] + 1;  // keys [run_first, run_last) are read by somebody of the run
-    int first_end = tok_pos[run_begin] + 1;
-    int run_first = (window > 0 && first_end > window) ? first_end - window : 0;
-    int page_first = run_first / 64, page_last = (run_last - 1) / 64;
-    __syncthreads();  // (everybody is done with the run before)
-    if (tid < TILE_Q) sm.end[tid] = t0 + tid >= run_begin && t0 + tid < run_end ? tok_pos[t0 + tid] + 1 : 0;
-    copy_page(sm.k, pages[page_first], 0);
-    copy_page(sm.v, pages[page_first], 1);
+  int run_first = (window > 0 && pos0 + 1 > window) ? pos0 + 1 - window : 0;  // keys from here on are seen by somebody
+  int page_first = run_first / 64, page_last = (pos0 + count - 1) / 64;
+  copy_page(sm.k, pages[page_first], 0);
+  copy_page(sm.v, pages[page_first], 1);
+  for (int i = tid; i < 8 * NI * (HD / 4); i += TILE_THREADS) {
+    int r = i / (HD / 4), d = i % (HD / 4) * 4;
+    float4 value = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < count) value = *(const float4*)(q + ((size_t)r * heads + h) * HD + d);
+    *(float4*)&sm.q[r][d] = value;
+  }
+  int end[NI], first[NI];  // keys [first, end) are seen by row ty + 8 i
+  float m_run[NI], l_run[NI];
+  unsigned long long acc[NI][2 * GROUPS];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    end[i] = ty + 8 * i < count ? pos0 + ty + 8 * i + 1 : 0;
+    first[i] = (window > 0 && end[i] > window) ? end[i] - window : 0;
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.f;
+#pragma unroll
+    for (int x = 0; x < 2 * GROUPS; ++x) acc[i][x] = 0;
+  }
+  for (int p = page_first; p <= page_last; ++p) {
+    int j0 = p * 64;
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the page's keys (its values may still be on their way)
     __syncthreads();
-    int end[4], first[4];
-    float m_run[4], l_run[4];
-    unsigned long long acc[4][2 * GROUPS];
+    float s[NI][4];
+    {
+      unsigned long long dot[NI][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      end[i] = sm.end[ty + 8 * i];
-      first[i] = (window > 0 && end[i] > window) ? end[i] - window : 0;
-      m_run[i] = -INFINITY;
-      l_run[i] = 0.f;
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
-      for (int x = 0; x < 2 * GROUPS; ++x) acc[i][x] = 0;
-    }
-    for (int p = page_first; p <= page_last; ++p) {
-      int j0 = p * 64;
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the page's keys (its values may still be on their way)
-      __syncthreads();
-      float s[4][4];
-      {
-        unsigned long long dot[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dot[i][j] = 0;
+        for (int j = 0; j < 4; ++j) dot[i][j] = 0;
 #pragma unroll 4
-        for (int d = 0; d < HD; d += 4) {
-          ulonglong2 key[4];
+      for (int d = 0; d < HD; d += 4) {
+        ulonglong2 key[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) key[j] = *(const ulonglong2*)&sm.k[tx + 16 * j][d];
+        for (int j = 0; j < 4; ++j) key[j] = *(const ulonglong2*)&sm.k[tx + 16 * j][d];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            ulonglong2 query = *(const ulonglong2*)&sm.q[ty + 8 * i][d];
+        for (int i = 0; i < NI; ++i) {
+          ulonglong2 query = *(const ulonglong2*)&sm.q[ty + 8 * i][d];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.x, key[j].x, dot[i][j]);
+          for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.x, key[j].x, dot[i][j]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.y, key[j].y, dot[i][j]);
-          }
+          for (int j = 0; j < 4; ++j) dot[i][j] = fma2(query.y, key[j].y, dot[i][j]);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            s[i][j] = scaled(unpack2(dot[i][j]), scale);
-          }
       }
-      bool whole = true;  // every token of this thread that sees the page sees all of it
-      float chunk_m[4], chunk_l[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        bool sees = j0 < end[i] && j0 + 64 > first[i];  // (what a token that does not is given here is dropped below)
-        whole = whole && (!sees || (first[i] <= j0 && j0 + 64 <= end[i]));
-        bool valid[4];
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          int key = j0 + tx + 16 * j;
-          valid[j] = key >= first[i] && key < end[i];
-          if (!valid[j]) s[i][j] = -INFINITY;
+          s[i][j] = scaled(unpack2(dot[i][j]), scale);
         }
-        float m = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+    }
+    bool whole = true;  // every token of this thread that sees the page sees all of it
+    float chunk_m[NI], chunk_l[NI];
 #pragma unroll
-        for (int x = 8; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
-        float shift = finite_or_zero(m);
+    for (int i = 0; i < NI; ++i) {
+      bool sees = j0 < end[i] && j0 + 64 > first[i];  // (what a token that does not is given here is dropped below)
+      whole = whole && (!sees || (first[i] <= j0 && j0 + 64 <= end[i]));
+      bool valid[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s[i][j] = valid[j] ? expf(s[i][j] - shift) : 0.f;
-          sm.p[ty + 8 * i][tx + 16 * j] = s[i][j];
-        }
-        float l = (s[i][0] + s[i][2]) + (s[i][1] + s[i][3]);
-#pragma unroll
-        for (int x = 8; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
-        chunk_m[i] = m;
-        chunk_l[i] = l;
+      for (int j = 0; j < 4; ++j) {
+        int key = j0 + tx + 16 * j;
+        valid[j] = key >= first[i] && key < end[i];
+        if (!valid[j]) s[i][j] = -INFINITY;
       }
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the page's values
-      __syncthreads();  // values and weights are there, everybody is done with the keys
-      if (p < page_last) copy_page(sm.k, pages[p + 1], 0);
-      unsigned long long o[4][2 * GROUPS];
+      float m = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int x = 8; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+      float shift = finite_or_zero(m);
 #pragma unroll
-        for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = 0;
-      if (__all_sync(0xffffffffu, whole)) {
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = valid[j] ? expf(s[i][j] - shift) : 0.f;
+        sm.p[ty + 8 * i][tx + 16 * j] = s[i][j];
+      }
+      float l = (s[i][0] + s[i][2]) + (s[i][1] + s[i][3]);
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+      chunk_m[i] = m;
+      chunk_l[i] = l;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // the page's values
+    __syncthreads();  // values and weights are there, everybody is done with the keys
+    if (p < page_last) copy_page(sm.k, pages[p + 1], 0);
+    unsigned long long o[NI][2 * GROUPS];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = 0;
+    if (__all_sync(0xffffffffu, whole)) {
 #pragma unroll 2
-        for (int jj = 0; jj < 64; jj += 4) {
-          float4 weight[4];
+      for (int jj = 0; jj < 64; jj += 4) {
+        float4 weight[NI];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) weight[i] = *(const float4*)&sm.p[ty + 8 * i][jj];
+        for (int i = 0; i < NI; ++i) weight[i] = *(const float4*)&sm.p[ty + 8 * i][jj];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            unsigned long long value[2 * GROUPS];
-#pragma unroll
-            for (int x = 0; x < GROUPS; ++x) {
-              ulonglong2 two = *(const ulonglong2*)&sm.v[jj + u][64 * x + 4 * tx];
-              value[2 * x] = two.x;
-              value[2 * x + 1] = two.y;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float one = u == 0 ? weight[i].x : u == 1 ? weight[i].y : u == 2 ? weight[i].z : weight[i].w;
-              unsigned long long both = pack2(one, one);
-#pragma unroll
-              for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = fma2(both, value[x], o[i][x]);
-            }
-          }
-        }
-      } else {  // (a token must not meet what lies at positions that it does not see)
-        int from = 64, to = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (j0 < end[i] && j0 + 64 > first[i]) {
-            from = min(from, max(0, first[i] - j0));
-            to = max(to, min(64, end[i] - j0));
-          }
-        }
-        for (int jj = from; jj < to; ++jj) {
+        for (int u = 0; u < 4; ++u) {
           unsigned long long value[2 * GROUPS];
 #pragma unroll
           for (int x = 0; x < GROUPS; ++x) {
-            ulonglong2 two = *(const ulonglong2*)&sm.v[jj][64 * x + 4 * tx];
+            ulonglong2 two = *(const ulonglong2*)&sm.v[jj + u][64 * x + 4 * tx];
             value[2 * x] = two.x;
             value[2 * x + 1] = two.y;
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (j0 + jj < first[i] || j0 + jj >= end[i]) continue;
-            float one = sm.p[ty + 8 * i][jj];
+          for (int i = 0; i < NI; ++i) {
+            float one = u == 0 ? weight[i].x : u == 1 ? weight[i].y : u == 2 ? weight[i].z : weight[i].w;
             unsigned long long both = pack2(one, one);
 #pragma unroll
             for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = fma2(both, value[x], o[i][x]);
           }
         }
       }
+    } else {  // (a token must not meet what lies at positions that it does not see)
+      int from = 64, to = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (j0 >= end[i] || j0 + 64 <= first[i]) continue;  // (no visible key in this page: it does not take part)
-        float keep, take;
-        merge(m_run[i], l_run[i], chunk_m[i], chunk_l[i], keep, take);
-#pragma unroll
-        for (int x = 0; x < 2 * GROUPS; ++x) {
-          float2 before = unpack2(acc[i][x]), now = unpack2(o[i][x]);
-          acc[i][x] = pack2(merge_output(before.x, keep, now.x, take), merge_output(before.y, keep, now.y, take));
+      for (int i = 0; i < NI; ++i) {
+        if (j0 < end[i] && j0 + 64 > first[i]) {
+          from = min(from, max(0, first[i] - j0));
+          to = max(to, min(64, end[i] - j0));
         }
       }
-      __syncthreads();  // everybody is done with the values and weights
-      if (p < page_last) copy_page(sm.v, pages[p + 1], 1);
-    }
+      for (int jj = from; jj < to; ++jj) {
+        unsigned long long value[2 * GROUPS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (end[i] == 0) continue;
-      float inv = 1.0f / l_run[i];
-      float* row = out + ((size_t)(t0 + ty + 8 * i) * heads + h) * HD;
+        for (int x = 0; x < GROUPS; ++x) {
+          ulonglong2 two = *(const ulonglong2*)&sm.v[jj][64 * x + 4 * tx];
+          value[2 * x] = two.x;
+          value[2 * x + 1] = two.y;
+        }
 #pragma unroll
-      for (int x = 0; x < GROUPS; ++x) {
-        float2 lo = unpack2(acc[i][2 * x]), hi = unpack2(acc[i][2 * x + 1]);
-        *(float4*)(row + 64 * x + 4 * tx) = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+        for (int i = 0; i < NI; ++i) {
+          if (j0 + jj < first[i] || j0 + jj >= end[i]) continue;
+          float one = sm.p[ty + 8 * i][jj];
+          unsigned long long both = pack2(one, one);
+#pragma unroll
+          for (int x = 0; x < 2 * GROUPS; ++x) o[i][x] = fma2(both, value[x], o[i][x]);
+        }
       }
     }
-    run_begin = run_end;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      if (j0 >= end[i] || j0 + 64 <= first[i]) continue;  // (no visible key in this page: it does not take part)
+      float keep, take;
+      merge(m_run[i], l_run[i], chunk_m[i], chunk_l[i], keep, take);
+#pragma unroll
+      for (int x = 0; x < 2 * GROUPS; ++x) {
+        float2 before = unpack2(acc[i][x]), now = unpack2(o[i][x]);
+        acc[i][x] = pack2(merge_output(before.x, keep, now.x, take), merge_output(before.y, keep, now.y, take));
+      }
+    }
+    __syncthreads();  // everybody is done with the values and weights
+    if (p < page_last) copy_page(sm.v, pages[p + 1], 1);
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    if (end[i] == 0) continue;
+    float inv = 1.0f / l_run[i];
+    float* row = out + ((size_t)(ty + 8 * i) * heads + h) * HD;
+#pragma unroll
+    for (int x = 0; x < GROUPS; ++x) {
+      float2 lo = unpack2(acc[i][2 * x]), hi = unpack2(acc[i][2 * x + 1]);
+      *(float4*)(row + 64 * x + 4 * tx) = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+    }
   }
 }
 
+// `tile_seq` / `tile_first`: the sequence of each stretch of up to 64 new tokens and its first token among that sequence's, the
+// longest contexts first. A stretch is two tiles, the later one first.
 template <int HD>
-int launch_tiles(float* out, const float* q, const KvLayout& cache, const int* tok_seq, const int* tok_pos, const int* slots,
-                 int tokens, int heads, float scale, int window, cudaStream_t stream) {
+__global__ void __launch_bounds__(TILE_THREADS, HD == 64 ? 4 : 2) attention_tile_kernel(
+    float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
+    const int* __restrict__ slots, const int* __restrict__ tile_seq, const int* __restrict__ tile_first,
+    const int* __restrict__ cu_seqlens, int heads, float scale, int window) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TileShared<HD>& sm = *reinterpret_cast<TileShared<HD>*>(smem_raw);
+  int h = blockIdx.x % heads, item = blockIdx.x / heads, seq = tile_seq[item >> 1];
+  int t0 = cu_seqlens[seq] + tile_first[item >> 1] + (item & 1 ? 0 : TILE_Q);
+  int count = min(TILE_Q, cu_seqlens[seq + 1] - t0);
+  if (count <= 0) return;
+  const int* pages = cache.page_table + (size_t)slots[seq] * cache.max_pages;
+  const float* rows = q + (size_t)t0 * heads * HD;
+  float* to = out + (size_t)t0 * heads * HD;
+  int g = h / (heads / cache.kv_heads), pos0 = tok_pos[t0];  // (a sequence's new tokens have ascending positions)
+  if (count <= 8) attend_tile<HD, 1>(sm, to, rows, cache, pages, count, pos0, h, g, heads, scale, window);
+  else attend_tile<HD, 4>(sm, to, rows, cache, pages, count, pos0, h, g, heads, scale, window);
+}
+
+template <int HD>
+int launch_tiles(float* out, const float* q, const KvLayout& cache, const int* tok_pos, const int* slots, const int* tile_seq,
+                 const int* tile_first, const int* cu_seqlens, int tiles, int heads, float scale, int window,
+                 cudaStream_t stream) {
   static std::atomic<unsigned long long> allowed{0};
   constexpr int smem = (int)sizeof(TileShared<HD>);
   if (!dllm_allow_shared((const void*)attention_tile_kernel<HD>, smem, allowed)) return DLLM_LAUNCH_FAILED;
-  long long blocks = (long long)((tokens + TILE_Q - 1) / TILE_Q) * heads;
+  long long blocks = 2ll * tiles * heads;
   if (blocks > 0x7fffffffLL) return DLLM_UNSUPPORTED_SIZE;
-  attention_tile_kernel<HD><<<(unsigned)blocks, TILE_THREADS, smem, stream>>>(out, q, cache, tok_seq, tok_pos, slots, tokens,
-                                                                              heads, scale, window);
+  attention_tile_kernel<HD><<<(unsigned)blocks, TILE_THREADS, smem, stream>>>(
+      out, q, cache, tok_pos, slots, tile_seq, tile_first, cu_seqlens, heads, scale, window);
   return dllm_launch_status();
 }
 
@@ -841,13 +848,16 @@ DLLM_EXPORT int dllm_attention_general(void* out, const void* q, void* cache_bas
 // The same attention with the same arguments, blockwise; the same bits. `max_new`: the most new tokens a sequence brings
 // in this step: with one each (decoding) a block serves one token's heads, else runs of tokens. `max_context`: the most
 // keys any token of the step may see; one that sees more gets no number (NaN) and `status`, a word that the device can write,
-// is set to 50. Pages of 64 positions, at most 65,535 kv heads.
+// is set to 50. tile_seq / tile_first / cu_seqlens: for each of `tiles` stretches of up to 64 new tokens its sequence and its
+// first token among that sequence's, and where the sequences' new tokens begin (may be absent, tiles = 0). Pages of 64
+// positions, at most 65,535 kv heads.
 // float32 takes the kernels made for it: single tokens their chunks side by side, prompts with heads of 64 and 128 in
 // 16-byte aligned rows the tiles of queries.
 DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base, const int* page_table,
                                       int max_pages, int page_size, int heads, int kv_heads, int head_dim,
                                       const int* tok_seq, const int* tok_pos, const int* slots, int tokens,
-                                      int max_new, int max_context, float scale, int window, int dtype, int* status,
+                                      int max_new, int max_context, const int* tile_seq, const int* tile_first,
+                                      const int* cu_seqlens, int tiles, float scale, int window, int dtype, int* status,
                                       cudaStream_t stream) {
   if (tokens <= 0) return DLLM_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads) return DLLM_BAD_ARGUMENT;
@@ -865,15 +875,22 @@ DLLM_EXPORT int dllm_attention_blocks(void* out, const void* q, void* cache_base
   else DLLM_GO(T, R, 8)
   if (dtype == DLLM_F32) {
     const float* rows = (const float*)q;
-    bool aligned = (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
+    float* to = (float*)out;
+    bool tiled = (head_dim == 64 || head_dim == 128) && (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
     if (!runs) {
-      int done = launch_chunks((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window,
-                                 max_context > 0 ? max_context : (long long)max_pages * page_size, status, stream);
+      int done = launch_chunks(to, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window,
+                               max_context > 0 ? max_context : (long long)max_pages * page_size, status, stream);
       if (done != DLLM_UNSUPPORTED_SIZE) return done;
-    } else if (head_dim == 64 && aligned) {
-      return launch_tiles<64>((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window, stream);
-    } else if (head_dim == 128 && aligned) {
-      return launch_tiles<128>((float*)out, rows, cache, tok_seq, tok_pos, slots, tokens, heads, scale, window, stream);
+    } else if (tiled && tiles > 0) {
+      // A tile is one query head's, the serial form's block all heads' of a kv head: with many sequences of a token or two
+      // and several heads a kv head, that is less work once tiles fill the device. 200 tokens of 300 keys and one prompt of
+      // two, us here and there: 32 query and 8 kv heads of 128 702 and 570, 40 and 2 of 64 375 and 246, 9 and 3 of 64 96 and
+      // 485; 32 tokens of 500 and a prompt of 100: 196 and 875, 108 and 386, 48 and 749.
+      bool crowd = heads / kv_heads >= 4 && tokens < 4ll * tiles && (long long)tiles * heads * (head_dim / 64) >= 5000;
+      if (!crowd)
+        return (head_dim == 64 ? launch_tiles<64> : launch_tiles<128>)(to, rows, cache, tok_pos, slots, tile_seq,
+                                                                       tile_first, cu_seqlens, tiles, heads, scale, window,
+                                                                       stream);
     }
     if (runs) { DLLM_BY_WIDTH(float, 4); }
     DLLM_BY_WIDTH(float, 1);

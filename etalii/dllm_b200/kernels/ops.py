@@ -237,8 +237,8 @@ _prototypes = {
                                               c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int,
                                               c_void_p],
     ("attention", "dllm_attention_blocks"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                             c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
-                                             c_int, c_void_p, c_void_p],
+                                             c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                                             c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p, c_void_p],
     ("attention_decode", "dllm_attention_decode"): [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                                     c_int, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int,
                                                     c_void_p, c_void_p, c_void_p],
@@ -2189,8 +2189,9 @@ def attention_blocks(out: torch.Tensor, q: torch.Tensor, cache, heads: int, scal
     _check(_fn("attention", "dllm_attention_blocks")(
         out.data_ptr(), q.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(), cache.max_pages, cache.page_size,
         heads, cache.kv_heads, cache.head_dim, batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(),
-        batch.slots.data_ptr(), batch.n_tokens, int(batch.max_new), int(batch.max_context), float(scale),
-        int(window or 0), _code(cache.dtype), _status_word().data_ptr(), _stream()), "attention_blocks",
+        batch.slots.data_ptr(), batch.n_tokens, int(batch.max_new), int(batch.max_context), batch.tile_seq.data_ptr(),
+        batch.tile_first.data_ptr(), batch.cu_seqlens.data_ptr(), batch.n_tiles, float(scale), int(window or 0),
+        _code(cache.dtype), _status_word().data_ptr(), _stream()), "attention_blocks",
         lambda: f"head_dim={cache.head_dim} must be a multiple of 8, at most 256; pages of 64")
 
 

@@ -391,7 +391,11 @@ def test_attention_blocks(dtype, tol, heads, kv_heads, head_dim, window, decode)
 @pytest.mark.parametrize("heads,kv_heads,head_dim,window,lengths,new", [
     (3, 1, 64, None, [31, 64, 1, 65, 33], [31, 64, 1, 2, 33]), (2, 2, 128, None, [97, 130], [97, 66]),
     (9, 3, 64, 100, [300, 260], [300, 40]), (4, 1, 128, 64, [191], [191]), (9, 3, 64, None, [2300, 700, 64], [1, 1, 1]),
-    (32, 32, 64, None, [513, 1], [1, 1]), (20, 1, 16, 65, [400, 64, 65], [1, 1, 1]), (40, 2, 128, None, [1024], [1])])
+    (32, 32, 64, None, [513, 1], [1, 1]), (20, 1, 16, 65, [400, 64, 65], [1, 1, 1]), (40, 2, 128, None, [1024], [1]),
+    # single tokens beside a prompt: tiles of one to eight rows, of more, and a second tile of a stretch with one row
+    (9, 3, 64, None, [100, 65, 200] + [70] * 20, [33, 8, 9] + [1] * 20), (8, 8, 128, 90, [300, 64, 129, 1], [64, 1, 7, 1]),
+    # the same with so many sequences that a block takes all heads of a kv head instead
+    (32, 8, 64, None, [70] * 156 + [40], [1] * 156 + [40]), (16, 1, 128, 33, [65] * 157, [2] + [1] * 156)])
 def test_attention_float32_bits(heads, kv_heads, head_dim, window, lengths, new):
     """The float32 kernels (tiles of queries for prompts, chunks side by side for single tokens) against the kernel of one
     warp a (token, head): the same bits with and without a window, and no NaN from positions that a token does not see."""
