@@ -185,6 +185,10 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
     const int* __restrict__ tok_pos, const int* __restrict__ slots, int tokens, int heads, float scale, int window,
     int heads_per_pass, int stages) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  // Values are multiplied without bounds over spans of keys that every token sees all of: the page, or for rows of 32 values
+  // its halves (a page with an edge in it then keeps one: 8 heads of 32, prompt of 2,048 under a window of 100, 92 -> 50 us.
+  // Longer rows have no registers for that beside short prompts' needs: 4 heads of 256, seven tokens each, 68.6 -> 76.4).
+  constexpr int SPANS = R > 1 && CHUNKS == 1 ? 2 : 1, SPAN = 64 / SPANS;
   int hd = cache.head_dim, ld = hd + Pad<T>::N;
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   int token_slots = warps / heads_per_pass;       // warps = token_slots * heads_per_pass
@@ -248,17 +252,30 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
         // The warp's R tokens walk the page together: a key is loaded once for the R scores and a value once for the
         // R weighted sums (what a token computes, and in which order, is what it would compute alone).
         int j0 = p * 64;
-        bool active[R], any = false, whole = hd == CHUNKS * 32;
+        bool active[R], any = false, lower = false, upper = false, whole = hd == CHUNKS * 32;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           active[r] = j0 < end[r] && j0 + 64 > first[r];  // (warp-uniform) a visible key in this page
           any = any || active[r];
+          lower = lower || (active[r] && first[r] < j0 + 32);
+          upper = upper || (active[r] && j0 + 32 < end[r]);
           whole = whole && (!active[r] || (first[r] <= j0 && j0 + 64 <= end[r]));
         }
         if (any) {
-          float weight[R][2], chunk_m[R], chunk_l[R], o[R][CHUNKS];
+          float weight[R][2], chunk_m[R], chunk_l[R];
+          auto join = [&](int r, const float* o) {  // the page's result joins those before it
+            float keep, take;
+            merge(m_run[r], l_run[r], chunk_m[r], chunk_l[r], keep, take);
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) acc[r][i] = merge_output(acc[r][i], keep, o[i], take);
+          };
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
+            if (!(u == 0 ? lower : upper)) {  // 32 keys that nobody sees: masked below, as any such key
+#pragma unroll
+              for (int r = 0; r < R; ++r) weight[r][u] = 0.f;
+              continue;
+            }
             const T* krow = k_s + (lane + 32 * u) * ld;
             float2 dot[R];
 #pragma unroll
@@ -301,62 +318,89 @@ __global__ void __launch_bounds__(512) attention_block_kernel(
               if (R > 1) p_s[r * 64 + 32 * u + lane] = weight[r][u];
             }
             chunk_l[r] = warp_sum(weight[r][0] + weight[r][1]);
-#pragma unroll
-            for (int i = 0; i < CHUNKS; ++i) o[r][i] = 0.f;
           }
           if (R > 1) __syncwarp();
           const T* vtile = v_s + lane;
-          if (whole) {  // whole pages of a whole head for every token that sees the page: no bounds in the loop
-#pragma unroll 4
-            for (int jj = 0; jj < 64; jj += 4) {
-              float v[4][CHUNKS];
+          auto weight_of = [&](int r, int jj) {
+            return R > 1 ? p_s[r * 64 + jj] : __shfl_sync(0xffffffffu, jj < 32 ? weight[r][0] : weight[r][1], jj & 31);
+          };
+          if (hd == CHUNKS * 32 && (SPANS > 1 || whole)) {
+            float o[R][CHUNKS];
 #pragma unroll
-              for (int u = 0; u < 4; ++u)
+            for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int i = 0; i < CHUNKS; ++i) v[u][i] = to_float(vtile[(jj + u) * ld + 32 * i]);
+              for (int i = 0; i < CHUNKS; ++i) o[r][i] = 0.f;
+#pragma unroll
+            for (int span = 0; span < SPANS; ++span) {
+              const int k0 = span * SPAN;
+              bool sees[R], all = true;
 #pragma unroll
               for (int r = 0; r < R; ++r) {
-                if (!active[r]) continue;  // (a token that does not see the page must not meet what lies there)
-                float4 pj;
-                if (R > 1) {
-                  pj = *reinterpret_cast<const float4*>(&p_s[r * 64 + jj]);
-                } else {
-                  float mine = jj < 32 ? weight[r][0] : weight[r][1];
-                  pj.x = __shfl_sync(0xffffffffu, mine, jj & 31);
-                  pj.y = __shfl_sync(0xffffffffu, mine, (jj & 31) + 1);
-                  pj.z = __shfl_sync(0xffffffffu, mine, (jj & 31) + 2);
-                  pj.w = __shfl_sync(0xffffffffu, mine, (jj & 31) + 3);
-                }
+                sees[r] = SPANS > 1 ? active[r] && j0 + k0 < end[r] && j0 + k0 + SPAN > first[r] : active[r];
+                if (SPANS > 1) all = all && (!sees[r] || (first[r] <= j0 + k0 && j0 + k0 + SPAN <= end[r]));
+              }
+              if (all) {  // every token that sees the span sees all of it: no bounds in the loop
+#pragma unroll 4
+                for (int jj = k0; jj < k0 + SPAN; jj += 4) {
+                  float v[4][CHUNKS];
 #pragma unroll
-                for (int i = 0; i < CHUNKS; ++i) {
-                  o[r][i] = fmaf(pj.x, v[0][i], o[r][i]);
-                  o[r][i] = fmaf(pj.y, v[1][i], o[r][i]);
-                  o[r][i] = fmaf(pj.z, v[2][i], o[r][i]);
-                  o[r][i] = fmaf(pj.w, v[3][i], o[r][i]);
+                  for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int i = 0; i < CHUNKS; ++i) v[u][i] = to_float(vtile[(jj + u) * ld + 32 * i]);
+#pragma unroll
+                  for (int r = 0; r < R; ++r) {
+                    if (!sees[r]) continue;  // (a token that does not see the keys must not meet what lies there)
+                    float4 pj;
+                    if (R > 1) {
+                      pj = *reinterpret_cast<const float4*>(&p_s[r * 64 + jj]);
+                    } else {
+                      float mine = jj < 32 ? weight[r][0] : weight[r][1];
+                      pj.x = __shfl_sync(0xffffffffu, mine, jj & 31);
+                      pj.y = __shfl_sync(0xffffffffu, mine, (jj & 31) + 1);
+                      pj.z = __shfl_sync(0xffffffffu, mine, (jj & 31) + 2);
+                      pj.w = __shfl_sync(0xffffffffu, mine, (jj & 31) + 3);
+                    }
+#pragma unroll
+                    for (int i = 0; i < CHUNKS; ++i) {
+                      o[r][i] = fmaf(pj.x, v[0][i], o[r][i]);
+                      o[r][i] = fmaf(pj.y, v[1][i], o[r][i]);
+                      o[r][i] = fmaf(pj.z, v[2][i], o[r][i]);
+                      o[r][i] = fmaf(pj.w, v[3][i], o[r][i]);
+                    }
+                  }
+                }
+              } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  if (!sees[r]) continue;
+                  int from = max(k0, first[r] - j0), to = min(k0 + SPAN, end[r] - j0);
+                  for (int jj = from; jj < to; ++jj) {
+                    float pj = weight_of(r, jj);
+#pragma unroll
+                    for (int i = 0; i < CHUNKS; ++i) o[r][i] = fmaf(pj, to_float(vtile[jj * ld + 32 * i]), o[r][i]);
+                  }
                 }
               }
             }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (active[r]) join(r, o[r]);
           } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
               if (!active[r]) continue;
+              float o[CHUNKS];
+#pragma unroll
+              for (int i = 0; i < CHUNKS; ++i) o[i] = 0.f;
               int from = max(0, first[r] - j0), to = min(64, end[r] - j0);
               for (int jj = from; jj < to; ++jj) {
-                float pj = R > 1 ? p_s[r * 64 + jj]
-                                 : __shfl_sync(0xffffffffu, jj < 32 ? weight[r][0] : weight[r][1], jj & 31);
+                float pj = weight_of(r, jj);
 #pragma unroll
                 for (int i = 0; i < CHUNKS; ++i)
-                  if (lane + 32 * i < hd) o[r][i] = fmaf(pj, to_float(vtile[jj * ld + 32 * i]), o[r][i]);
+                  if (lane + 32 * i < hd) o[i] = fmaf(pj, to_float(vtile[jj * ld + 32 * i]), o[i]);
               }
+              join(r, o);
             }
-          }
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if (!active[r]) continue;
-            float keep, take;
-            merge(m_run[r], l_run[r], chunk_m[r], chunk_l[r], keep, take);
-#pragma unroll
-            for (int i = 0; i < CHUNKS; ++i) acc[r][i] = merge_output(acc[r][i], keep, o[r][i], take);
           }
         }
         if (stages != 2) {
@@ -779,8 +823,13 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
   asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
 }
 
-// Refuses (DLLM_UNSUPPORTED_SIZE) what does not fit; the caller then takes the serial form, which gives the same bits.
-// `reach`: the most keys a token may see.
+// Refuses (DLLM_UNSUPPORTED_SIZE) what does not fit and what the serial form (attention_block_kernel, the same bits) is faster
+// at; the caller then takes that. `reach`: the most keys a token may see.
+// A chunk costs more here than there, and there is a cluster barrier to pay, so it has to be worth it: enough chunks in a row
+// that walking them one after another takes longer, and few enough (token, kv head) pairs that the device has room beside
+// them. Microseconds here against there, 9 query and 3 kv heads of 64: one token of 30 keys 7.9 and 5.4, of 100 8.6 and 8.7,
+// of 500 9.1 and 26.5, of 2,000 20.6 and 101; 2,000 keys and 32 tokens 58 and 103, 64 tokens 133 and 119, 128 tokens 243 and
+// 138. Rows of 256 values, 4 query and 2 kv heads: 500 keys and 8 tokens 56 and 70, 16 tokens 84 and 70.
 int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* tok_seq, const int* tok_pos, const int* slots,
                   int tokens, int heads, float scale, int window, long long reach, int* status, cudaStream_t stream) {
   int group = heads / cache.kv_heads, hd = cache.head_dim, ld = hd + 4;
@@ -792,6 +841,10 @@ int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* 
   int parts = (group + heads_per_block - 1) / heads_per_block;
   long long rows = (long long)cache.kv_heads * parts;
   if (rows > 65535) return DLLM_UNSUPPORTED_SIZE;
+  // (two or three chunks: only where the serial form has many heads a block, or short rows and little else to do)
+  long long values = rows * tokens * hd;
+  bool few = chunks >= 2 && values <= 4096 && (group > 8 || hd <= 24);
+  if (!(chunks >= 4 || few) || values > (hd <= 128 ? 8192 : 4096)) return DLLM_UNSUPPORTED_SIZE;
   // As many blocks a cluster as there are chunks, up to 8, while three a multiprocessor hold them all.
   int size = 1;
   while (size < 8 && size < chunks && rows * tokens * size * 2 <= 3 * 148) size *= 2;
@@ -800,8 +853,11 @@ int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* 
   auto bytes = [&](int n) {
     return ((size_t)n * 128 * ld + (size_t)heads_per_block * hd + (size_t)room * heads_per_block * (hd + 2)) * sizeof(float);
   };
-  if (bytes(1) > 200 * 1024) return DLLM_UNSUPPORTED_SIZE;
+  if (bytes(1) > 200 * 1024 || room > 256) return DLLM_UNSUPPORTED_SIZE;
   while ((per_round + 1) * heads_per_block <= 8 && per_round < room && bytes(per_round + 1) <= 110 * 1024) ++per_round;
+  // (more than one and a half rounds of blocks: 8 query heads of 128 to each of 8 kv heads, 8 tokens of 8,000: 597 and 500)
+  long long resident = 148ll * (227 * 1024 / ((long long)bytes(per_round) + 2048));
+  if (2 * rows * tokens * size > 3 * resident) return DLLM_UNSUPPORTED_SIZE;
   static std::atomic<unsigned long long> allowed{0};
   if (!dllm_allow_shared((const void*)attention_chunks_kernel, 200 * 1024, allowed)) return DLLM_LAUNCH_FAILED;
   cudaLaunchConfig_t config = {};

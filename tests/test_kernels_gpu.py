@@ -392,6 +392,11 @@ def test_attention_blocks(dtype, tol, heads, kv_heads, head_dim, window, decode)
     (3, 1, 64, None, [31, 64, 1, 65, 33], [31, 64, 1, 2, 33]), (2, 2, 128, None, [97, 130], [97, 66]),
     (9, 3, 64, 100, [300, 260], [300, 40]), (4, 1, 128, 64, [191], [191]), (9, 3, 64, None, [2300, 700, 64], [1, 1, 1]),
     (32, 32, 64, None, [513, 1], [1, 1]), (20, 1, 16, 65, [400, 64, 65], [1, 1, 1]), (40, 2, 128, None, [1024], [1]),
+    # single tokens too many or of too few keys for a cluster: the serial form; three chunks and four, two where they pay
+    (9, 3, 64, None, [257] * 43, [1] * 43), (9, 3, 64, None, [257] * 42, [1] * 42), (4, 1, 64, None, [192], [1]),
+    (4, 1, 64, None, [193], [1]), (18, 2, 24, None, [65, 64], [1, 1]), (2, 1, 256, None, [300] * 17, [1] * 17),
+    # rows of 32 values: halves of a page that a window's edge leaves whole
+    (4, 4, 32, 40, [200, 100], [130, 1]), (4, 2, 32, None, [33, 64, 31], [33, 2, 31]),
     # single tokens beside a prompt: tiles of one to eight rows, of more, and a second tile of a stretch with one row
     (9, 3, 64, None, [100, 65, 200] + [70] * 20, [33, 8, 9] + [1] * 20), (8, 8, 128, 90, [300, 64, 129, 1], [64, 1, 7, 1]),
     # the same with so many sequences that a block takes all heads of a kv head instead
