@@ -1,23 +1,27 @@
 // Weight-streaming products for decode on large matrices (at most 16 rows of activations, bfloat16): C = X * W^T
 // where reading W once from HBM is the whole cost, so what counts is how many bytes are on their way at any time.
 // Here they travel into shared memory, not into registers: a producer warp issues bulk copies (cp.async.bulk, 2 KB
-// of one row of W or X per copy, completion counted by an mbarrier) into a ring of stages that holds about 200 KB
-// per multiprocessor, and consumer warps multiply out of shared memory on the tensor cores (mma.sync m16n8k16
+// of one row of W or X per copy, completion counted by an mbarrier) into a ring of stages that holds up to 216 KB
+// per multiprocessor (less what resident rows of X take, below), and consumer warps multiply out of shared memory on the tensor cores (mma.sync m16n8k16
 // with W as the 16-row operand, ldmatrix from rows padded by 16 bytes so that no two rows share a bank).
 // Blocks are persistent: a block walks over its tiles of W and the ring runs on across tiles.
-//   ROWS = 32: a tile is `height` rows (an even number, at most 32: the height that leaves the busiest multiprocessor the
-//              fewest rows, e.g. 147 tiles of 28 for 4,096 rows, where 128 tiles of 32 left 20 multiprocessors idle);
-//   ROWS = 16: sixteen rows (the q/k/v projection, whose tiles are eight rotary pairs).
+//   a tile is `height` rows (an even number from 16 to 32: the height that leaves the busiest multiprocessor the fewest
+//   rows, e.g. 147 tiles of 28 for 4,096 rows, where 128 tiles of 32 left 20 multiprocessors idle). A stage of the ring
+//   holds `height` rows, so that low tiles do not mean fewer bytes on their way;
+//   ROWS = 32: tiles of 18 rows and more; ROWS = 16: of sixteen (few rows of W, and the q/k/v projection, whose tiles are
+//   eight rotary pairs). With stages of 32 rows whatever the height, one row took 32.4 us for 1024 x 28672 instead of 22.1
+//   and 20.2 for 2048 x 16384 instead of 14.3.
 // Sixteen rows are the work of four consumer warps, which take 16-value steps in turn and add their sums in order: a
 // step is a chain of ldmatrix and product, so one warp gets through one about every 35 cycles, and two warps for a tile
-// could not keep up with memory. One row, before all of this (two consumers, tiles of 32 or 16) and now: 28672 x 4096 41.5 ->
-// 36.6 us, 128256 x 4096 167.5 -> 146.9, 4096 x 14336 23.6 -> 23.0, 4096 x 4096 8.7 -> 7.7; eight rows of 28672 x 4096
-// 51.2 -> 41.8.
+// could not keep up with memory. One row, W out of L2, before all of this (two consumers, tiles of 32 or 16) and now: 28672 x
+// 4096 40.0 -> 34.1 us, 128256 x 4096 167 -> 144, 4096 x 14336 23.1 -> 19.6, 4096 x 4096 8.8 -> 7.9; eight rows of 28672 x
+// 4096 50.1 -> 38.7, of 4096 x 14336 24.3 -> 23.0.
 // RESIDENT: the rows of X lie in shared memory for the whole kernel, copied once, and the ring carries nothing but W. (As
 // a part of every stage they cost a copy a row and stage: with eight rows a quarter of all copies.) Where they take more
-// than 72 KB they stay a part of the stages.
+// than 72 KB they stay a part of the stages. The ring is 144 to 213 KB beside them.
 // Epilogues as the tile kernels: store (float32 / bfloat16), residual add in float32, SwiGLU on interleaved rows; rotation
-// and cache write behind the q/k/v projection. K must be a multiple of 64. Every wait on an mbarrier is bounded; a role that gives up records a status word.
+// and cache write behind the q/k/v projection; the greedy choice behind the head. K must be a multiple of 64. Every wait on
+// an mbarrier is bounded; a role that gives up records a status word.
 #include "gemv_common.cuh"
 #include "tcgen05.cuh"
 
@@ -50,15 +54,15 @@ constexpr int MAX_CHUNKS = (RESIDENT_BYTES / 2 + KC - 1) / KC;
 
 template <int ROWS, int NT, bool RESIDENT> struct Shape {
   static constexpr int TOKENS = NT * 8;                          // token rows of a stage (those beyond M stay unused)
-  static constexpr int STAGE_BYTES = (ROWS + (RESIDENT ? 0 : TOKENS)) * PITCH;
-  static constexpr int MAX_STAGES = RING_BYTES / STAGE_BYTES;
+  static __host__ __device__ constexpr int stage_bytes(int height) { return (height + (RESIDENT ? 0 : TOKENS)) * PITCH; }
+  static constexpr int MAX_STAGES = RING_BYTES / ((16 + (RESIDENT ? 0 : TOKENS)) * PITCH);  // (no tile is lower)
   static constexpr int CONSUMERS = ROWS / 16 * K_PARTS, THREADS = 32 * (1 + CONSUMERS);  // (warp 0 copies)
   static constexpr int SCRATCH_FLOATS = CONSUMERS * 16 * (TOKENS + 1);  // a 16 x TOKENS tile per consumer warp
   // (resident rows of X, then the ring in what is left)
   static int x_bytes(int M, int K) { return RESIDENT ? M * (2 * K + 16) : 0; }
-  static int stages(int M, int K) { return (RING_BYTES - x_bytes(M, K)) / STAGE_BYTES; }
-  static size_t smem(int M, int K) {
-    return (size_t)x_bytes(M, K) + (size_t)stages(M, K) * STAGE_BYTES + SCRATCH_FLOATS * sizeof(float) + 128;
+  static int stages(int M, int K, int height) { return (RING_BYTES - x_bytes(M, K)) / stage_bytes(height); }
+  static size_t smem(int M, int K, int height) {
+    return (size_t)x_bytes(M, K) + (size_t)stages(M, K, height) * stage_bytes(height) + SCRATCH_FLOATS * sizeof(float) + 128;
   }
   static constexpr int MAX_SMEM = RING_BYTES + SCRATCH_FLOATS * (int)sizeof(float) + 128;
 };
@@ -73,7 +77,8 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
   unsigned char* x_s = (unsigned char*)(((uintptr_t)smem_raw + 15) & ~(uintptr_t)15);
   const int x_pitch = 2 * K + 16;  // (K is a multiple of 64: the rows begin in different banks)
   unsigned char* ring = x_s + (RESIDENT ? (size_t)M * x_pitch : 0);
-  float* scratch = reinterpret_cast<float*>(ring + (size_t)stages * S::STAGE_BYTES);
+  const int stage_bytes = S::stage_bytes(ROWS == 16 ? 16 : height);
+  float* scratch = reinterpret_cast<float*>(ring + (size_t)stages * stage_bytes);
   __shared__ uint64_t full_bar[S::MAX_STAGES], empty_bar[S::MAX_STAGES], x_bar[RESIDENT ? MAX_CHUNKS : 1];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int chunks = K / KC + (K % KC ? 1 : 0);  // stages per tile; the last may be shorter (K is a multiple of 64)
@@ -91,11 +96,10 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
     // ---- producer: lane r copies row r of the tile's W; lanes also copy the token rows of X. The weights are
     // nobody's output: the first trip round the ring asks for them before the wait on the kernel before, and adds
     // the rows of X (which that kernel may have written) after it.
-    auto fill = [&](int it, int tile, int ch, bool weights, bool tokens) {
-      int s = it % stages;
+    auto fill = [&](int s, int tile, int ch, bool weights, bool tokens) {
       int row0 = tile * height, rows_valid = min(height, N - row0), k0 = ch * KC;
       unsigned bytes = (unsigned)min(KC, K - k0) * 2u;
-      unsigned char* stage = ring + (size_t)s * S::STAGE_BYTES;
+      unsigned char* stage = ring + (size_t)s * stage_bytes;
       if (weights) {
         if (lane == 0) mbar_expect_tx(&full_bar[s], bytes * (unsigned)(rows_valid + (RESIDENT ? 0 : M)));
         __syncwarp();
@@ -111,37 +115,41 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
       }
       if (tokens && !RESIDENT)
         for (int m = lane; m < M; m += 32)
-          bulk_copy(stage + (ROWS + m) * PITCH, x + (size_t)m * K + k0, bytes, &full_bar[s]);
+          bulk_copy(stage + (height + m) * PITCH, x + (size_t)m * K + k0, bytes, &full_bar[s]);
     };
-    int it = 0, tile = blockIdx.x, ch = 0;
-    for (; it < stages && tile < tiles; ++it) {  // the first trip: weights only
-      fill(it, tile, ch, true, false);
+    int filled = 0, tile = blockIdx.x, ch = 0;
+    for (; filled < stages && tile < tiles; ++filled) {  // the first trip: weights only
+      fill(filled, tile, ch, true, false);
       if (++ch == chunks) { ch = 0; tile += gridDim.x; }
     }
     pdl_wait();
     if (RESIDENT) {
-      for (int k = 0; k < chunks; ++k) {
-        unsigned bytes = (unsigned)min(KC, K - k * KC) * 2u;
-        if (lane == 0) mbar_expect_tx(&x_bar[RESIDENT ? k : 0], bytes * (unsigned)M);
-        __syncwarp();
-        for (int m = lane; m < M; m += 32)
-          bulk_copy(x_s + (size_t)m * x_pitch + k * ROW_BYTES, x + (size_t)m * K + k * KC, bytes, &x_bar[RESIDENT ? k : 0]);
+      // (a lane a stage for what is expected, then a lane a copy: a row of 36 stages is two turns, not 36)
+      auto stage_row = [&](int k) { return (unsigned)min(KC, K - k * KC) * 2u; };
+      for (int k = lane; k < chunks; k += 32) mbar_expect_tx(&x_bar[RESIDENT ? k : 0], stage_row(k) * (unsigned)M);
+      __syncwarp();
+      for (int i = lane; i < chunks * M; i += 32) {
+        int k = i / M, m = i % M;
+        bulk_copy(x_s + (size_t)m * x_pitch + k * ROW_BYTES, x + (size_t)m * K + k * KC, stage_row(k), &x_bar[RESIDENT ? k : 0]);
       }
     } else {
-      int it2 = 0, tile2 = blockIdx.x, ch2 = 0;
-      for (; it2 < it; ++it2) {  // their rows of X
-        fill(it2, tile2, ch2, false, true);
+      int tile2 = blockIdx.x, ch2 = 0;
+      for (int s = 0; s < filled; ++s) {  // their rows of X
+        fill(s, tile2, ch2, false, true);
         if (++ch2 == chunks) { ch2 = 0; tile2 += gridDim.x; }
       }
     }
-    for (; tile < tiles; ++it) {
-      int s = it % stages;
-      if (!mbar_wait(&empty_bar[s], ((it / stages) - 1) & 1)) {
+    // (laps are counted along: divided by a number of stages that the compiler does not know, they cost 0.1 us a stage)
+    int s = 0;
+    unsigned lap = 0;
+    while (tile < tiles) {
+      if (!mbar_wait(&empty_bar[s], lap)) {
         if (lane == 0) *(volatile int*)status = 32;
         break;
       }
-      fill(it, tile, ch, true, true);
+      fill(s, tile, ch, true, true);
       if (++ch == chunks) { ch = 0; tile += gridDim.x; }
+      if (++s == stages) { s = 0; lap ^= 1; }
     }
   } else {
     // ---- consumers
@@ -150,16 +158,19 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
     int g = lane >> 2, t = lane & 3;
     int row_base = half * 16;
     // ldmatrix addresses inside a stage: W rows (lane & 15), k offset 8 for the upper lanes; X rows (lane & 7),
-    // k offset 8 for lanes 8..15 (and the second eight tokens for lanes 16..31 when NT == 2). Rows of X beyond M are
-    // whatever lies there, or the last row again where X is resident: their results are not stored.
-    unsigned a_off = (unsigned)((row_base + (lane & 15)) * PITCH + (lane >> 4) * 16);
+    // k offset 8 for lanes 8..15 (and the second eight tokens for lanes 16..31 when NT == 2). Rows of W beyond the tile's
+    // height are its last row again, rows of X beyond M whatever lies there, or the last row again where X is resident:
+    // their results are not stored.
+    unsigned a_off = (unsigned)(min(row_base + (lane & 15), height - 1) * PITCH + (lane >> 4) * 16);
     int token = (lane & 7) + (NT == 2 ? (lane >> 4) * 8 : 0);
     unsigned b_off = RESIDENT ? smem_u32(x_s) + (unsigned)(min(token, M - 1) * x_pitch + ((lane >> 3) & 1) * 16)
-                              : (unsigned)((ROWS + token) * PITCH + ((lane >> 3) & 1) * 16);
+                              : (unsigned)((height + token) * PITCH + ((lane >> 3) & 1) * 16);
     constexpr int TILE_FLOATS = 16 * (S::TOKENS + 1);
     float* group = scratch + (size_t)half * K_PARTS * TILE_FLOATS;  // the tiles of the warps that share these rows
     float* mine = group + part * TILE_FLOATS;
-    int it = 0, member = part * 32 + lane;  // this thread among the group's
+    int member = part * 32 + lane;  // this thread among the group's
+    int s = 0;  // the ring's next stage and lap
+    unsigned lap = 0;
     auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + half), "n"(K_PARTS * 32) : "memory"); };
     bool ok = true;  // (a warp that gave up still meets the others of its group, tile by tile, and stores nothing)
     // (in the q/k/v projection a thread stores the same pair and token of every tile: the token's position and cache page
@@ -193,14 +204,13 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
         for (int n = 0; n < NT; ++n)
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[e][n][i] = 0.f;
-      for (int ch = 0; ch < chunks && ok; ++ch, ++it) {
-        int s = it % stages;
-        if (!mbar_wait(&full_bar[s], (it / stages) & 1) || (RESIDENT && !mbar_wait(&x_bar[RESIDENT ? ch : 0], 0))) {
+      for (int ch = 0; ch < chunks && ok; ++ch) {
+        if (!mbar_wait(&full_bar[s], lap) || (RESIDENT && !mbar_wait(&x_bar[RESIDENT ? ch : 0], 0))) {
           if (lane == 0) *(volatile int*)status = 33;
           ok = false;
           break;
         }
-        unsigned stage = smem_u32(ring + (size_t)s * S::STAGE_BYTES);
+        unsigned stage = smem_u32(ring + (size_t)s * stage_bytes);
         unsigned x_at = RESIDENT ? b_off + (unsigned)(ch * ROW_BYTES) : stage + b_off;
         int steps = min(KC, K - ch * KC) / (16 * K_PARTS);  // (K is a multiple of 64: as many for every warp)
         auto step = [&](float (*into)[4], int j) {
@@ -221,6 +231,7 @@ __global__ void __launch_bounds__(Shape<ROWS, NT, RESIDENT>::THREADS, 1) gemv_tm
         if (j < steps) step(acc[0], j);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[s]);  // this warp is done with the stage
+        if (++s == stages) { s = 0; lap ^= 1; }
       }
       // the warp's 16 x TOKENS tile to shared memory, then one (pair of rows, token) per thread of the group and turn
 #pragma unroll
@@ -322,8 +333,8 @@ int launch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int heigh
     return DLLM_LAUNCH_FAILED;
   int tiles = (N + height - 1) / height;
   int blocks = tiles < sms ? tiles : sms;
-  return dllm_launch_pdl(gemv_tma_kernel<ROWS, NT, EPI, RESIDENT>, dim3(blocks), dim3(S::THREADS), S::smem(M, K), stream, c, x,
-                         w, M, N, K, tiles, height, S::stages(M, K), status, rope);
+  return dllm_launch_pdl(gemv_tma_kernel<ROWS, NT, EPI, RESIDENT>, dim3(blocks), dim3(S::THREADS), S::smem(M, K, height),
+                         stream, c, x, w, M, N, K, tiles, height, S::stages(M, K, height), status, rope);
 }
 
 // (`resident_activations` of kernels/ops.py is the same rule: who asks it calls the entry points below that want it kept)
@@ -348,12 +359,14 @@ int dispatch(void* c, const bf16* x, const bf16* w, int M, int N, int K, int epi
   int sms = multiprocessors();
   if (sms == 0) return DLLM_LAUNCH_FAILED;
   int height = tile_height(N, sms);
-  RopeArgs none{};
+  auto go = [&](auto low, auto high) {
+    return (height == 16 ? low : high)(c, x, w, M, N, K, height, status, RopeArgs{}, stream);
+  };
   switch (epilogue) {
-    case EPI_STORE_F32: return launch<32, NT, EPI_STORE_F32, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
-    case EPI_STORE_T: return launch<32, NT, EPI_STORE_T, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
-    case EPI_RESIDUAL: return launch<32, NT, EPI_RESIDUAL, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
-    case EPI_SWIGLU: return launch<32, NT, EPI_SWIGLU, RESIDENT>(c, x, w, M, N, K, height, status, none, stream);
+    case EPI_STORE_F32: return go(launch<16, NT, EPI_STORE_F32, RESIDENT>, launch<32, NT, EPI_STORE_F32, RESIDENT>);
+    case EPI_STORE_T: return go(launch<16, NT, EPI_STORE_T, RESIDENT>, launch<32, NT, EPI_STORE_T, RESIDENT>);
+    case EPI_RESIDUAL: return go(launch<16, NT, EPI_RESIDUAL, RESIDENT>, launch<32, NT, EPI_RESIDUAL, RESIDENT>);
+    case EPI_SWIGLU: return go(launch<16, NT, EPI_SWIGLU, RESIDENT>, launch<32, NT, EPI_SWIGLU, RESIDENT>);
     default: return DLLM_BAD_ARGUMENT;
   }
 }

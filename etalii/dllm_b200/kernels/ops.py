@@ -1726,21 +1726,27 @@ def resident_activations(rows: int, inner: int) -> bool:
 
 def streams_with_resident_rows(rows: int, outputs: int, inner: int) -> bool:
     """Whether a decode-sized product takes the ring kernel with its rows of activations resident, before the rules below
-    are asked. Measured, one row and eight: 28672 x 4096 36.6 and 41.8 us (register kernel 45.6 and 47.7, W as the 128-row
-    operand 45.5 and 44.0), 6144 x 4096 10.4 and 12.05 (11.7 and 12.4); rows of 2,048 values are better off in the
-    register kernel (16384 x 2048: 12.0 and 12.7 against 11.2 and 11.7)."""
+    are asked. Measured with W out of L2, one row and eight: 28672 x 4096 34.1 and 38.7 us (register kernel 44.1 and 46.7, W
+    as the 128-row operand 45.5 and 41.1), 7168 x 4096 12.2 and 17.0 (17.1 and 17.8); rows of 2,048 values are better off in
+    the register kernel (16384 x 2048: 12.0 and 12.7 against 11.2 and 11.7)."""
     if inner % 64 or inner < 4096 or not resident_activations(rows, inner):
         return False
     size = 2 * outputs * inner
-    # (4096 x 4096, 32 MB: 7.7 against 8.75 with one row, 8.8 against 9.0 with four, 9.95 against 9.2 with eight; 2048 x
-    # 8192, where tiles of 16 rows leave multiprocessors idle: 9.6 against 8.6)
-    return size >= TMA_STREAM_BYTES or (rows <= 4 and size >= TMA_STREAM_BYTES * 2 // 3 and outputs >= 4096)
+    # (4096 x 4096, 32 MB: 7.9 against 8.6 with one row, 8.3 against 8.85 with three, 9.9 against 9.05 with eight; 4608 x 5376,
+    # 47 MB: 10.0 against 12.05 and 11.0 against 12.5; 2048 x 8192, where tiles of 16 rows leave multiprocessors idle: 9.6
+    # against 8.6)
+    if size < TMA_STREAM_BYTES:
+        return rows <= 4 and size >= TMA_STREAM_BYTES * 2 // 3 and outputs >= 4096
+    # (six rows and more of up to 5,120 values leave a ring of two or three stages: 6144 x 4096 with eight 13.9 against 13.2,
+    # 6400 x 4096 14.1 against 13.3, but 6656 x 4096 13.2 against 13.4, and 5120 x 5120 with seven 14.4 against 17.9)
+    return rows <= 5 or inner >= 5120 or size >= TMA_STREAM_BYTES + (4 << 20)
 
 
 def streams_qkv_through_shared_memory(rows: int, outputs: int, inner: int) -> bool:
-    """The same for the q/k/v projection with rotation and cache write behind it: 6144 x 4096 12.3 us against 14.0 with one
-    row, 12.4 against 14.9 with eight; 6144 x 2048 8.7 against 6.0."""
-    return 2 * outputs * inner >= TMA_STREAM_BYTES and streams_with_resident_rows(rows, outputs, inner)
+    """The same for the q/k/v projection with rotation and cache write behind it: 6144 x 4096 11.6 us against 13.8 with one
+    row, 11.6 against 14.8 with eight; 6144 x 2048 8.7 against 6.0."""
+    return 2 * outputs * inner >= TMA_STREAM_BYTES and inner % 64 == 0 and inner >= 4096 and \
+        resident_activations(rows, inner)
 
 
 def streams_through_shared_memory(rows: int, outputs: int, inner: int) -> bool:
@@ -1989,7 +1995,7 @@ def head_argmax(out_tokens: torch.Tensor, a: torch.Tensor, w: torch.Tensor, scra
     assert scratch.dtype == torch.float32 and scratch.numel() >= head_argmax_scratch(m, n)
     assert a.dtype == (torch.float32 if norm_weight is not None else torch.bfloat16)
     if norm_weight is None and n >= 16384 and streams_with_resident_rows(m, n, k):
-        # (128256 x 4096 with one row: 147 us against 182 for the register kernel)
+        # (128256 x 4096 with one row: 145 us against 188 for the register kernel, with eight 162 against 211)
         count = ctypes.c_int(0)
         _check(_fn("gemv_tma", "dllm_gemv_tma_argmax")(
             scratch.data_ptr(), a.data_ptr(), w.data_ptr(), m, n, k, ctypes.addressof(count), _status_word().data_ptr(),

@@ -149,6 +149,11 @@ def test_kernel_choice_rules_for_products():
     assert ops.streams_through_shared_memory(1, 28672, 4096) and not ops.streams_through_shared_memory(8, 28672, 4096)
     assert ops.streams_through_shared_memory(8, 4096, 14336) and not ops.streams_through_shared_memory(9, 4096, 14336)
     assert not ops.streams_through_shared_memory(1, 16384, 2048)      # short rows of W
+    assert ops.streams_with_resident_rows(5, 6144, 4096) and not ops.streams_with_resident_rows(6, 6144, 4096)
+    assert ops.streams_with_resident_rows(8, 6656, 4096) and ops.streams_with_resident_rows(7, 5120, 5120)
+    assert ops.streams_with_resident_rows(4, 4096, 4096) and not ops.streams_with_resident_rows(5, 4096, 4096)
+    assert ops.resident_activations(8, 4544) and not ops.resident_activations(8, 4608)
+    assert ops.streams_qkv_through_shared_memory(8, 6144, 4096) and not ops.streams_qkv_through_shared_memory(1, 6144, 2048)
     assert not ops.streams_through_shared_memory(1, 4096, 4096 + 8)   # a reduction that is no multiple of 64
     # a narrow W with a long reduction and 33 to 64 rows: the reduction is cut so that every multiprocessor reads
     assert ops.reduction_split(64, 4096, 14336) == 8 and ops.reduction_split(64, 2048, 8192) == 8

@@ -226,6 +226,26 @@ def test_gemm_streaming_through_shared_memory(m, n, k, epilogue):
     assert torch.equal(again, c)
 
 
+@pytest.mark.parametrize("m,n,k", [(3, 50, 14400), (8, 33, 14400), (8, 70, 4544), (8, 70, 4608), (1, 40, 36800), (1, 40, 36864),
+                                   (2, 2601, 4160), (6, 2601, 6208), (5, 4729, 1088), (8, 4097, 2112), (16, 2601, 1088)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
+def test_ring_with_activations_beside_it_and_in_its_stages(m, n, k, epilogue):
+    """Activations on both sides of the 72 KB that lie beside the ring (those above travel in its stages), one to sixteen
+    rows, in tiles of 16, 18, 28 and 32 rows of W with a ragged last one."""
+    n += n % 2 if epilogue == 3 else 0
+    a, w = _randn((m, k), torch.bfloat16, 3), _randn((n, k), torch.bfloat16, 4, 0.05)
+    cols = n // 2 if epilogue == 3 else n
+    start = _randn((m, cols), torch.float32 if epilogue in (0, 2) else torch.bfloat16, 5)
+    c, again, ref = start.clone(), start.clone(), start.clone()
+    ops().gemm(c, a, w, epilogue, kernel=4)
+    ops().gemm(again, a, w, epilogue, kernel=4)
+    torch.cuda.synchronize()
+    ops().raise_if_failed()
+    PK.gemm(ref, a, w, epilogue)
+    assert rel_error(c.float().cpu(), ref.float().cpu()) <= (2e-5 if epilogue in (0, 2) else 8e-3)
+    assert torch.equal(again, c)
+
+
 @pytest.mark.parametrize("m", [1, 17, 33, 64, 100, 256])
 @pytest.mark.parametrize("n,k", [(128, 64), (130, 576), (1001, 1088), (4100, 512), (300, 2240), (19000, 128)])
 @pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
