@@ -1198,21 +1198,38 @@ def test_head_argmax_on_the_ring(m, n, k):
     by more than the sums' rounding."""
     x, w = _randn((m, k), torch.bfloat16, 1), _randn((n, k), torch.bfloat16, 2, 0.1)
     w[n - 1], w[n // 2] = w[3] * 8, w[3] * 8  # equal in every row, and the largest wherever row 3's product is positive
-    x[0] = 0
-    if m > 2:
-        x[2, 0] = float("nan")
+    special = (0, 2) if m > 2 else ()
+    if special:
+        x[0], x[2, 0] = 0, float("nan")
     got = torch.full((m,), -1, dtype=torch.int32, device=DEV)
     scratch = torch.full((ops().head_argmax_scratch(m, n),), float("nan"), dtype=torch.float32, device=DEV)
     assert ops().streams_with_resident_rows(m, n, k)
     ops().head_argmax(got, x, w, scratch)
     ops().raise_if_failed()
-    assert got[0].item() == 0 and (m <= 2 or got[2].item() == 0)
+    assert all(got[row].item() == 0 for row in special)
     exact = x.double() @ w.double().T
-    for row in [r for r in range(m) if r not in (0, 2)]:
+    for row in [r for r in range(m) if r not in special]:
         best = exact[row].topk(3).values
         assert exact[row, got[row].item()] >= best[0] - 2e-5 * best[0].abs()  # (k products of 16 bits summed in 32)
         if exact[row].argmax().item() in (n - 1, n // 2):
             assert got[row].item() == n // 2
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 16385, 4096), (8, 16401, 4160)])
+def test_head_argmax_on_the_ring_finds_the_largest_wherever_it_is(m, n, k):
+    """One feature's logit stands far above the rest (|x| summed): the first, the last of an odd vocabulary, both halves of
+    a tile, the ends of a tile and of a block's walk."""
+    x, w = _randn((m, k), torch.bfloat16, 1), _randn((n, k), torch.bfloat16, 2, 0.1)
+    got = torch.full((m,), -1, dtype=torch.int32, device=DEV)
+    scratch = torch.full((ops().head_argmax_scratch(m, n),), float("nan"), dtype=torch.float32, device=DEV)
+    for i, feature in enumerate((0, 1, 15, 16, 17, 18, 27, 28, 31, 32, n // 2, n - 18, n - 2, n - 1)):
+        row = i % m
+        saved = w[feature].clone()
+        w[feature] = x[row].sign()
+        ops().head_argmax(got, x, w, scratch)
+        ops().raise_if_failed()
+        assert got[row].item() == feature
+        w[feature] = saved
 
 
 @pytest.mark.parametrize("m,hidden,inner,outputs", [
