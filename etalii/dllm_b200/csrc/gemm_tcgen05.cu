@@ -22,6 +22,7 @@ namespace {
 using namespace tc5;
 typedef __nv_bfloat16 bf16;
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
+constexpr long long L2_SHARE = 64ll << 20, PANEL_BYTES = 16ll << 20;  // (see launch_shape)
 
 // DEEP: a ring of nine or ten stages (about 215 KB) for a block that has its multiprocessor to itself: a product
 // with no more tiles than the device has multiprocessors and a short reduction then brings a tile's whole operand
@@ -29,15 +30,16 @@ constexpr int BM = 128, BK = 64, UMMA_K = 16;
 template <int BN, bool DEEP = false, int EPI_STAGE = 0> struct Shape {
   static constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
   static constexpr int ACC_COLS = BN < 32 ? 32 : BN;   // columns of one accumulator
-  static constexpr int TMEM_COLS = 2 * ACC_COLS;       // two accumulators: a power of two, at least 32
+  static constexpr int ACC_STRIDE = BN == 192 ? 256 : ACC_COLS;
+  static constexpr int TMEM_COLS = 2 * ACC_STRIDE;     // two accumulators: a power of two, at least 32
   // about 96 KB a block where that is enough (two blocks share an SM, 2 x TMEM_COLS <= 512 columns); the 256-wide
-  // tile takes four 48 KB stages and all of the tensor memory, so one block owns the SM
+  // tile takes four 48 KB stages and all of the tensor memory, so one block owns the SM; the 192-wide one five of 40 KB
   // (a 64-wide tile that stages its epilogue gives one of its four stages for it, so that two blocks still fit)
   static constexpr int STAGES = DEEP ? (220 * 1024) / (A_BYTES + B_BYTES)
-                                     : (BN >= 256 ? 4 : (BN >= 128 ? 3 : (EPI_STAGE > 0 ? 3 : 4)));
+                                     : (BN == 192 ? 5 : (BN >= 256 ? 4 : (BN >= 128 ? 3 : (EPI_STAGE > 0 ? 3 : 4))));
   // (EPI_STAGE: bytes behind the ring through which an epilogue makes its global stores whole lines)
   static constexpr size_t SMEM = (size_t)STAGES * (A_BYTES + B_BYTES) + 1024 + EPI_STAGE;
-  static constexpr int BLOCKS_PER_SM = (DEEP || BN >= 256) ? 1 : 2;
+  static constexpr int BLOCKS_PER_SM = (DEEP || BN >= 192) ? 1 : 2;
   // Epilogue warps: one per quarter of the tensor memory's lanes, or two that take half the columns each. A row's
   // epilogue is a chain of loads and special functions, so wide tiles gain from twice the warps (2048 x 2048 x 8192
   // with the residual: 128-wide 70 against 114 µs, 256-wide 61 against 64); narrow tiles of short products lose
@@ -58,7 +60,7 @@ template <int BN, bool DEEP = false, int EPI_STAGE = 0> struct Shape {
 template <int BN, int EPI, bool DEEP> struct EpilogueStage {
   static constexpr int BYTES = (EPI == EPI_SWIGLU && BN == 256 && !DEEP) ? 8 * 4096
                                : ((EPI == EPI_RESIDUAL && BN == 64 && !DEEP) ? 4 * 32 * 36 * 4
-                               : ((EPI == EPI_RESIDUAL && BN == 256 && !DEEP) ? 8 * 32 * 20 * 4 : 0));  // (see below)
+                               : ((EPI == EPI_RESIDUAL && BN >= 192 && !DEEP) ? 8 * 32 * 20 * 4 : 0));  // (see below)
 };
 
 // Item `item` of a block's list: a tile and, where the reduction is cut (k_split > 1), one stretch of its k tiles.
@@ -69,12 +71,23 @@ __device__ __forceinline__ WorkItem work_item(int item, int total, int k_tiles, 
   return WorkItem{item - split * total, split, split * k_tiles / k_split, (split + 1) * k_tiles / k_split};
 }
 
+// Where a tile lies. Tiles go down the rows of A first, in panels of `m_group` tiles of rows: a panel and then the next
+// column of W's tiles, until the panel has met all of W; the next panel follows. The host makes a panel as many rows as
+// stay in L2 (`launch`), so that A comes from HBM once however many columns of tiles read it.
+struct TilePlace { int m, n; };
+__device__ __forceinline__ TilePlace tile_place(int tile, int m_tiles, int n_tiles, int m_group) {
+  if (m_group >= m_tiles) return TilePlace{tile % m_tiles, tile / m_tiles};
+  int panel = tile / (m_group * n_tiles), at = tile - panel * m_group * n_tiles;
+  int high = min(m_group, m_tiles - panel * m_group);
+  return TilePlace{panel * m_group + at % high, at / high};
+}
+
 template <int BN, int EPI, bool DEEP, int HD>
 __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLOCKS_PER_SM) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                const __grid_constant__ CUtensorMap map_w,
                                                                void* __restrict__ c, int M, int N, int K,
                                                                int* __restrict__ status, RopeArgs rope, int m_tiles,
-                                                               int n_tiles, int k_split, NormArgs norm) {
+                                                               int n_tiles, int k_split, NormArgs norm, int m_group) {
   typedef Shape<BN, DEEP, EpilogueStage<BN, EPI, DEEP>::BYTES> S;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzle atoms: 1 KB
@@ -112,7 +125,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
       bool ok = true;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
         WorkItem w = work_item(item, total, k_tiles, k_split);
-        int m0 = (w.tile % m_tiles) * BM, n0 = (w.tile / m_tiles) * BN;
+        TilePlace place = tile_place(w.tile, m_tiles, n_tiles, m_group);
+        int m0 = place.m * BM, n0 = place.n * BN;
         for (int kt = w.kt_begin; kt < w.kt_end; ++kt, ++it) {
           int s = it % S::STAGES;
           if (it >= S::STAGES && !mbar_wait(&empty_bar[s], ((it / S::STAGES) - 1) & 1)) {
@@ -136,7 +150,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
         int buf = lt & 1;
         if (lt >= 2 && !mbar_wait(&acc_empty[buf], ((lt >> 1) - 1) & 1)) { *(volatile int*)status = 5; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        unsigned acc = tmem_base + (unsigned)(buf * S::ACC_COLS);
+        unsigned acc = tmem_base + (unsigned)(buf * S::ACC_STRIDE);
         WorkItem w = work_item(item, total, k_tiles, k_split);
         for (int kt = w.kt_begin; kt < w.kt_end; ++kt, ++it) {
           int s = it % S::STAGES;
@@ -165,8 +179,8 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
     for (int item = blockIdx.x; item < items; item += gridDim.x, ++lt) {
       int buf = lt & 1;
       WorkItem w = work_item(item, total, k_tiles, k_split);
-      int t = w.tile;
-      int m0 = (t % m_tiles) * BM, n_tile = t / m_tiles, n0 = n_tile * BN;
+      TilePlace place = tile_place(w.tile, m_tiles, n_tiles, m_group);
+      int m0 = place.m * BM, n_tile = place.n, n0 = n_tile * BN;
       void* c_part = EPI == EPI_T_STORE_F32 ? (void*)((float*)c + (size_t)w.split * M * N) : c;
       int m = m0 + quarter * 32 + lane;
       // (narrow tiles: the row's old residual values are all asked for before the accumulator is read, so their
@@ -219,7 +233,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      unsigned acc = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * S::ACC_COLS);
+      unsigned acc = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * S::ACC_STRIDE);
       auto release_accumulator = [&]() {  // this warp's last values are in registers: the accumulator may be reused
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -319,9 +333,9 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
           if (mr < M && nc < N) *reinterpret_cast<uint4*>((bf16*)c + (size_t)mr * (N / 2) + (nc >> 1)) = o;
         }
         __syncwarp();  // (the block's next tile overwrites the staged rows)
-      } else if (EPI == EPI_RESIDUAL && BN == 256 && !DEEP && (N & 3) == 0) {
-        // The residual epilogue of the 256-wide tile, through shared memory as well: 16 columns at a time (there is
-        // room for 32 rows x 20 floats per warp behind four stages of 48 KB), four lanes a row, eight rows an
+      } else if (EPI == EPI_RESIDUAL && BN >= 192 && !DEEP && (N & 3) == 0) {
+        // The residual epilogue of the 192- and 256-wide tiles, through shared memory as well: 16 columns at a time (there is
+        // room for 32 rows x 20 floats per warp behind the stages), four lanes a row, eight rows an
         // instruction; the old values of the next 32 columns are asked for before these are summed. Measured as links
         // of a chain, with the copy and the sums of squares: 2048 x 2048 x 2048 27.0 µs (a plain bfloat16 store of
         // the same product: 15.2) -> 20.7 µs, 2048 x 4096 x 4096 74.8 µs (53.5) -> 66.5 µs.
@@ -511,8 +525,25 @@ int launch_shape(void* c, const CUtensorMap& map_a, const CUtensorMap& map_w, in
   long long total = (long long)m_tiles * n_tiles * k_split;
   int blocks = sms * S::BLOCKS_PER_SM;
   if (blocks > total) blocks = (int)total;
+  // Panels pay where A outgrows L2 and W does not (rows of A down one column of W's tiles after the other read A from HBM
+  // once a column or so; panels read W once a panel). Microseconds down the columns / in panels of 16 MB: 69602 x 576 x 1536
+  // (A 214 MB, 192-wide tiles) 400 / 254, 18432 x 2048 x 8192 (302 MB) 602 / 540, 18432 x 2048 x 2048 (75 MB) 212 / 197;
+  // panels of 32 and 48 MB come to 256 and 267, 553 and 609, 199 and 202. With W as large as A, or A within L2, nothing is
+  // gained: 4096 x 4096 x 14336 430 / 443, 8192 x 28672 x 4096 1,498 / 1,595, 2048 x 4096 x 14336 198 / 204.
+  long long m_group = m_tiles;
+  if ((long long)M * K * 2 > L2_SHARE && (long long)N * K * 2 <= L2_SHARE) m_group = PANEL_BYTES / ((long long)BM * K * 2);
+  m_group = m_group < 1 ? 1 : (m_group > m_tiles ? m_tiles : m_group);
   return dllm_launch_pdl(gemm_tcgen05_kernel<BN, EPI, DEEP, HD>, dim3(blocks), dim3(S::THREADS), S::SMEM, stream, map_a, map_w,
-                         c, M, N, K, status, rope, m_tiles, n_tiles, k_split, norm);
+                         c, M, N, K, status, rope, m_tiles, n_tiles, k_split, norm, (int)m_group);
+}
+
+int multiprocessors() {
+  static int sms = 0;
+  int device = 0, found = 0;
+  if (sms == 0 && cudaGetDevice(&device) == cudaSuccess &&
+      cudaDeviceGetAttribute(&found, cudaDevAttrMultiProcessorCount, device) == cudaSuccess)
+    sms = found;
+  return sms;
 }
 
 template <int BN, int EPI, int HD = 0>
@@ -523,13 +554,8 @@ int launch(void* c, const void* a, const void* w, int M, int N, int K, int* stat
   int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
   long long total = (long long)m_tiles * n_tiles;
   if (total * k_split > 0x7fffffff) return DLLM_UNSUPPORTED_SIZE;
-  static int sms = 0;
-  if (sms == 0) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
-      return DLLM_LAUNCH_FAILED;
-  }
+  int sms = multiprocessors();
+  if (sms <= 0) return DLLM_LAUNCH_FAILED;
   constexpr bool CAN_DEEP = BN == 64 && EPI <= EPI_QKV_ROPE;  // (the shapes where it was measured to pay)
   if (CAN_DEEP && total <= sms && K > 4 * BK)
     return launch_shape<BN, EPI, CAN_DEEP, HD>(c, map_a, map_w, M, N, K, status, stream, rope, m_tiles, n_tiles, sms,
@@ -557,7 +583,8 @@ int dispatch(void* c, const void* a, const void* w, int M, int N, int K, int epi
 }  // namespace
 
 // C = A[M,K] * W[N,K]^T (bfloat16, float32 accumulation in tensor memory). K must be a multiple of 8 (16-byte row
-// pitch for TMA), N even for the SwiGLU epilogue, and A and W 16-byte aligned. `tile_n`: 32, 64 or 128 columns of C per block (0 chooses).
+// pitch for TMA), N even for the SwiGLU epilogue, and A and W 16-byte aligned. `tile_n`: 32, 64, 128, 256 or, with the residual
+// epilogue, 192 columns of C per block (0 chooses).
 // `status` is a word the device can write (device or pinned host memory); the kernel sets it non-zero if one of its
 // bounded waits ran out (2: producer, 3: product issuer, 4: epilogue).
 // Epilogues 5..8 are 0..3 for a product taken the other way round: the caller passes W as A (M = output features)
@@ -583,6 +610,16 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
     // (32-wide tiles for a narrow output, 2048 x 576, are 0.2 to 0.5 µs faster alone and slower in a step: twice
     // the parts of the rows' sums of squares for the next product to read)
     else tile_n = 64;
+    // A residual sum into a multiple of 192 columns: 192-wide tiles read A a third as often and use the tensor cores at
+    // their full rate, which 64-wide ones cannot. A round of either (192-wide one block a multiprocessor, 64-wide two) takes
+    // about as long, so the fewer rounds decide. 576 columns, K = 576 and 1536, microseconds 64-wide / 192-wide: 4,096 rows
+    // (one round, one) 11.0 / 12.5, 16.1 / 17.7; 6,144 (two, one) 17.2 / 12.7, 25.5 / 17.8; 8,704 (three, two) 21.2 / 19.1,
+    // 33.4 / 27.2; 17,408 (five, three) 38.0 / 29.8, 63.0 / 43.3; 69,602 164 / 118, 375 / 153. (Heads of 64 behind the
+    // q/k/v product, three a tile, lose instead: its epilogue is the longer part. 2,048 rows: 1,948 -> 2,258 a prompt.)
+    if (tile_n == 64 && epilogue == EPI_RESIDUAL && N % 192 == 0) {
+      long long sms = multiprocessors(), wide = m_tiles * (N / 192), narrow = 3 * wide;
+      if (sms > 0 && (wide + sms - 1) / sms < (narrow + 2 * sms - 1) / (2 * sms)) tile_n = 192;
+    }
   }
   if (n_tiles_out != nullptr)  // (a part per epilogue warp's share of a tile: see the epilogue)
     *n_tiles_out = (tile_n >= 128 ? 2 : 1) * ((N + tile_n - 1) / tile_n);
@@ -590,6 +627,9 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
     case 32: return dispatch<32>(c, a, w, M, N, K, epilogue, status, stream, norm, k_split);
     case 64: return dispatch<64>(c, a, w, M, N, K, epilogue, status, stream, norm, k_split);
     case 128: return dispatch<128>(c, a, w, M, N, K, epilogue, status, stream, norm, k_split);
+    case 192:
+      if (epilogue == EPI_RESIDUAL) return launch<192, EPI_RESIDUAL>(c, a, w, M, N, K, status, stream, RopeArgs{}, norm);
+      return DLLM_BAD_ARGUMENT;
     case 256: return dispatch<256>(c, a, w, M, N, K, epilogue, status, stream, norm, k_split);
     default: return DLLM_BAD_ARGUMENT;
   }

@@ -1275,3 +1275,27 @@ def test_tile_products_with_the_norm_folded_around_them(m, hidden, inner, output
     ops().gemm_normed(again, copy1, folded, ops().EPI_STORE_F32, ssq1, 1, eps)
     assert rel_error(again.cpu(), got.cpu()) <= 1e-5
     ops().raise_if_failed()
+
+
+@pytest.mark.parametrize("m,hidden,inner", [
+    (4225, 576, 136),    # one round of 192-wide tiles, the last one a single row
+    (12400, 192, 64),    # the width of one tile, one stage of the ring
+    (4100, 640, 320),    # no multiple of 192: more 64-wide tiles than blocks, the rows staged behind the ring
+    (66001, 384, 520),   # A outgrows its share of L2: panels of rows, the last one shorter; blocks with several tiles
+    (33000, 256, 1032),  # the same with 256-wide tiles
+])
+def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner):
+    """The product that writes the residual, its copy and its sums of squares against float64 (float32 sums of `inner`
+    products of values around 0.05)."""
+    x0, a = _randn((m, hidden), torch.float32, 1, 2.0), _randn((m, inner), torch.bfloat16, 2)
+    w = _randn((hidden, inner), torch.bfloat16, 3, 0.05)
+    x, plain = x0.clone(), x0.clone()
+    copy = torch.full((m, hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ssq = torch.full((m * (-(-hidden // 16)),), float("nan"), dtype=torch.float32, device=DEV)
+    parts = ops().gemm_residual_norm(x, copy, ssq, a, w)
+    ops().gemm(plain, a, w, ops().EPI_RESIDUAL, kernel=3)
+    ops().raise_if_failed()
+    want = x0.double() + a.double() @ w.double().T
+    assert rel_error(x.cpu(), want.cpu()) <= 2e-5 and torch.equal(plain, x)
+    assert torch.equal(copy, x.to(torch.bfloat16))
+    assert rel_error(ssq[: m * parts].view(parts, m).sum(dim=0).cpu(), (x.double() ** 2).sum(dim=1).cpu()) <= 1e-5
