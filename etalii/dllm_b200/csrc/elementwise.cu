@@ -471,6 +471,67 @@ __global__ void rope_cache_kernel(const float* __restrict__ qkv, T* __restrict__
   }
 }
 
+// The same for heads whose length and rotated length are multiples of eight, 16-byte aligned: a thread moves eight values,
+// four pairs of the rotated ones (two 16-byte loads half a rotation apart) or eight neighbours of the others, and threads run
+// over tokens, heads and pieces without gaps. Bound by its bytes; the form above, a thread a value in blocks of one head,
+// loads both partners of every pair twice and page numbers once a value: 9 query and 3 kv heads of 64, 2,048 tokens 32.0 ->
+// 4.0 us (15.7 MB in float32), 2,997 tokens 46.6 -> 4.9; 32 and 8 heads of 128 101 -> 16.6. For a few tokens, where its
+// divisions are what counts, the form above stays: eight tokens 1.76 us there, 2.06 here.
+template <typename T> __device__ __forceinline__ void store4(T* dst, float4 v);
+template <> __device__ __forceinline__ void store4<float>(float* dst, float4 v) { *reinterpret_cast<float4*>(dst) = v; }
+template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* dst, float4 v) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<unsigned*>(&lo), *reinterpret_cast<unsigned*>(&hi));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) rope_cache_vector_kernel(const float* __restrict__ qkv, T* __restrict__ q_out,
+                                                                KvLayout cache, const float2* __restrict__ table,
+                                                                int rotary_dim, int heads, const int* __restrict__ tok_seq,
+                                                                const int* __restrict__ tok_pos,
+                                                                const int* __restrict__ slots, int written_heads, int parts,
+                                                                size_t part_stride, size_t pieces) {
+  pdl_launch_dependents();
+  pdl_wait();
+  size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (at >= pieces) return;
+  unsigned hd = cache.head_dim, nkv = cache.kv_heads, per_head = hd / 8, per_token = per_head * written_heads;
+  int t = (int)(at / per_token);
+  unsigned in_token = (unsigned)(at - (size_t)t * per_token), h = in_token / per_head, u = in_token - h * per_head;
+  int pos = tok_pos[t];
+  T* dst;
+  if (h < (unsigned)heads) {
+    dst = q_out + ((size_t)t * heads + h) * hd;
+  } else {
+    int which = h < heads + nkv ? 0 : 1;
+    int page = cache.page_table[(size_t)slots[tok_seq[t]] * cache.max_pages + pos / cache.page_size];
+    dst = (T*)cache.base + kv_offset(cache, page, which, h - heads - which * nkv, pos % cache.page_size);
+  }
+  const float* src = qkv + ((size_t)t * (heads + 2 * nkv) + h) * hd;
+  auto value = [&](unsigned i) {
+    float4 sum = *reinterpret_cast<const float4*>(src + i);
+    for (int p = 1; p < parts; ++p) {
+      float4 v = *reinterpret_cast<const float4*>(src + (size_t)p * part_stride + i);
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    return sum;
+  };
+  unsigned half = rotary_dim / 2;
+  if (table != nullptr && h < heads + nkv && 4 * u < half) {
+    float4 a = value(4 * u), b = value(half + 4 * u);
+    const float4* cs = reinterpret_cast<const float4*>(table + (size_t)pos * half + 4 * u);
+    float4 c0 = cs[0], c1 = cs[1];  // (cos, sin) of two pairs each
+    store4(dst + 4 * u, make_float4(fmaf(a.x, c0.x, -(b.x * c0.y)), fmaf(a.y, c0.z, -(b.y * c0.w)),
+                                    fmaf(a.z, c1.x, -(b.z * c1.y)), fmaf(a.w, c1.z, -(b.w * c1.w))));
+    store4(dst + half + 4 * u, make_float4(fmaf(a.x, c0.y, b.x * c0.x), fmaf(a.y, c0.w, b.y * c0.z),
+                                           fmaf(a.z, c1.y, b.z * c1.x), fmaf(a.w, c1.w, b.w * c1.z)));
+  } else {  // (behind half / 4 pieces of the rotated values, or all of the head)
+    float4 a = value(8 * u), b = value(8 * u + 4);
+    store4(dst + 8 * u, a);
+    store4(dst + 8 * u + 4, b);
+  }
+}
+
 DLLM_EXPORT int dllm_rope_cache_write(const float* qkv, void* q_out, void* cache_base, const int* page_table,
                                       int max_pages, int page_size, int heads, int kv_heads, int head_dim,
                                       const float* table, int rotary_dim, const int* tok_seq, const int* tok_pos,
@@ -481,6 +542,22 @@ DLLM_EXPORT int dllm_rope_cache_write(const float* qkv, void* q_out, void* cache
       parts < 1 || part_stride < 0)
     return DLLM_BAD_ARGUMENT;
   KvLayout cache{cache_base, page_table, max_pages, page_size, kv_heads, head_dim};
+  const bool vector = tokens > 64 && head_dim % 8 == 0 && (table == nullptr || rotary_dim % 8 == 0) && (part_stride & 3) == 0 &&
+                      !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)cache_base | (uintptr_t)table) & 15);
+  if (vector && (dtype == DLLM_F32 || dtype == DLLM_BF16)) {
+    int written_heads = write_cache ? heads + 2 * kv_heads : heads;
+    size_t pieces = (size_t)tokens * written_heads * (head_dim / 8), blocks = (pieces + 127) / 128;
+    if (blocks <= 0x7fffffff) {
+      int rotated = table == nullptr ? 0 : rotary_dim;
+      if (dtype == DLLM_F32)
+        return dllm_launch_pdl(rope_cache_vector_kernel<float>, dim3((unsigned)blocks), dim3(128), 0, stream, qkv,
+                               (float*)q_out, cache, (const float2*)table, rotated, heads, tok_seq, tok_pos, slots,
+                               written_heads, parts, (size_t)part_stride, pieces);
+      return dllm_launch_pdl(rope_cache_vector_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(128), 0, stream, qkv,
+                             (__nv_bfloat16*)q_out, cache, (const float2*)table, rotated, heads, tok_seq, tok_pos, slots,
+                             written_heads, parts, (size_t)part_stride, pieces);
+    }
+  }
   dim3 grid(tokens, heads + 2 * kv_heads);
   int threads = head_dim >= 128 ? 128 : (head_dim > 32 ? 64 : 32);
   if (dtype == DLLM_F32)

@@ -1299,3 +1299,11 @@ def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner):
     assert rel_error(x.cpu(), want.cpu()) <= 2e-5 and torch.equal(plain, x)
     assert torch.equal(copy, x.to(torch.bfloat16))
     assert rel_error(ssq[: m * parts].view(parts, m).sum(dim=0).cpu(), (x.double() ** 2).sum(dim=1).cpu()) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-6), (torch.bfloat16, 8e-3)])
+@pytest.mark.parametrize("heads,kv_heads,head_dim,rotary", [
+    (9, 3, 64, 64), (3, 1, 128, 0), (5, 5, 40, 24), (1, 1, 8, 8),  # eight values a thread: blocks that end inside a head
+    (4, 2, 24, 12), (2, 1, 64, 20)])                               # rotations that are no multiples of eight
+def test_rope_cache_write_in_pieces_of_eight(dtype, tol, heads, kv_heads, head_dim, rotary):
+    test_rope_cache_write(dtype, tol, heads, kv_heads, head_dim, rotary)
