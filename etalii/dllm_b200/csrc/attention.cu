@@ -699,15 +699,24 @@ int launch_tiles(float* out, const float* q, const KvLayout& cache, const int* t
 // barrier each output dimension is merged over the chunks in ascending order by one thread of the cluster, reading them
 // through distributed shared memory. A second barrier keeps the blocks' memory alive until everybody has read.
 // Eight sequences of 50 to 700 tokens, 9 query and 3 kv heads of 64: 38.8 us a layer with a warp walking all keys of its
-// head, now 13.1 (both measured as launches of their own).
+// head.
+// Keys and values of earlier steps are nobody's output in this one, nor are positions, slots and page numbers: the first
+// round's rows travel before the wait on the kernel in front, but for the newest, which that kernel writes. HD: the head
+// size where it is known to the compiler (64 and 128: the copies' places are shifts then, and the loops over the dimensions
+// are flat), 0 for all others. With that, page numbers read once a chunk instead of once a piece, the outputs dealt out to
+// all blocks and sixteen chunks asked for at a time in the merge, us before and now: 9 query and 3 kv heads of 64, eight
+// sequences of 50 to 700 13.4 -> 8.1, of 2,000 28.5 -> 19.0, sixteen of 260 13.0 -> 7.7; 32 and 8 heads of 128, four of 500
+// 16.3 -> 10.8; 4 and 2 of 256, two of 500 27.4 -> 11.5.
 constexpr int CHUNK_WARPS = 16;
 
+template <int HD>
 __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
     float* __restrict__ out, const float* __restrict__ q, KvLayout cache, const int* __restrict__ tok_seq,
     const int* __restrict__ tok_pos, const int* __restrict__ slots, int heads, float scale, int window, int heads_per_block,
     int per_round, int room, int* __restrict__ status) {
   extern __shared__ __align__(16) float smem[];
-  int hd = cache.head_dim, ld = hd + 4, group = heads / cache.kv_heads, pieces = hd / 4;
+  const int hd = HD ? HD : cache.head_dim, ld = hd + 4, pieces = hd / 4;
+  int group = heads / cache.kv_heads;
   int size = (int)gridDim.x, rank = (int)blockIdx.x;  // (a cluster is a row of the grid)
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = (int)blockDim.x;
   int parts = (group + heads_per_block - 1) / heads_per_block;
@@ -717,27 +726,44 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
   float* q_s = kv_s + (size_t)per_round * 2 * 64 * ld;          // [heads_per_block][hd]
   float* result = q_s + (size_t)heads_per_block * hd;           // [room][heads_per_block][hd + 2]: o, m, l
   pdl_launch_dependents();
-  pdl_wait();
   int end = tok_pos[t] + 1, first = (window > 0 && end > window) ? end - window : 0;
   const int* pages = cache.page_table + (size_t)slots[tok_seq[t]] * cache.max_pages;
   int chunk0 = first / 64, chunks = min((end + 63) / 64 - chunk0, room * size);
   // (`room` covers what the caller says; a token that sees more gets no number, and the host is told)
   bool told = chunks == (end + 63) / 64 - chunk0;
+  int mine = warp / heads_per_block, head = warp % heads_per_block;
+  auto copy_rows = [&](int n, int c, int from, int to) {  // rows [from, to) of chunk c's keys and values, to place n
+    const float* base = (const float*)cache.base;
+    size_t keys = kv_offset(cache, pages[chunk0 + c], 0, g, 0), values = kv_offset(cache, pages[chunk0 + c], 1, g, 0);
+    int count = (to - from) * pieces;
+    for (int i = threadIdx.x; i < 2 * count; i += threads) {
+      int which = i >= count, j = i - which * count;
+      int row = from + j / pieces, d = j % pieces * 4;
+      unsigned at = (unsigned)__cvta_generic_to_shared(kv_s + ((size_t)(n * 2 + which) * 64 + row) * ld + d);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(at),
+                   "l"(base + (which ? values : keys) + (size_t)row * hd + d));
+    }
+  };
+  // Chunks c0, c0 + size, ... (per_round of them at most); nobody reads what lies behind the last key. `before`: the rows
+  // that were there before this step; `newest`: the one that was not.
+  auto ask = [&](int c0, bool before, bool newest) {
+    for (int n = 0; n < per_round && c0 + n * size < chunks; ++n) {
+      int c = c0 + n * size, last = min(64, end - (chunk0 + c) * 64);  // (rows of it that exist)
+      bool has_newest = (chunk0 + c) * 64 + last == end;
+      if (before) copy_rows(n, c, 0, has_newest ? last - 1 : last);
+      if (newest && has_newest) copy_rows(n, c, last - 1, last);
+    }
+  };
+  ask(rank, true, false);
+  pdl_wait();
   if (!told && threadIdx.x == 0) *(volatile int*)status = 50;
+  ask(rank, false, true);
   for (int i = threadIdx.x; i < here * hd; i += threads)
     q_s[i] = q[((size_t)t * heads + g * group + head0) * hd + i];
-  int mine = warp / heads_per_block, head = warp % heads_per_block;
   for (int c0 = rank; c0 < chunks; c0 += size * per_round) {
-    // this round: chunks c0, c0 + size, ... (per_round of them at most)
-    __syncthreads();  // (everybody is done with the round before; the queries are there behind the next barrier)
-    for (int i = threadIdx.x; i < per_round * 128 * pieces; i += threads) {
-      int d = i % pieces * 4, row = i / pieces % 64, which = i / pieces / 64 & 1, n = i / pieces / 128;
-      int c = c0 + n * size;
-      if (c < chunks && (chunk0 + c) * 64 + row < end) {  // (nobody reads what lies behind the last key)
-        unsigned at = (unsigned)__cvta_generic_to_shared(kv_s + ((size_t)(n * 2 + which) * 64 + row) * ld + d);
-        const float* from = (const float*)cache.base + kv_offset(cache, pages[chunk0 + c], which, g, row) + d;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(from));
-      }
+    if (c0 != rank) {
+      __syncthreads();  // (everybody is done with the round before)
+      ask(c0, true, true);
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
@@ -748,7 +774,7 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
       const float* query = q_s + head * hd;
       int j0 = (chunk0 + c) * 64;
       float2 dot[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll 4
+#pragma unroll (HD ? 8 : 4)
       for (int d = 0; d < hd; d += 4) {
         float4 piece = *(const float4*)(query + d);
         float values[4] = {piece.x, piece.y, piece.z, piece.w};
@@ -795,23 +821,26 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
   }
   asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
   unsigned local = (unsigned)__cvta_generic_to_shared(result);
-  for (int i = rank * threads + threadIdx.x; i < here * hd; i += size * threads) {
+  // (the outputs are dealt out evenly: every block of the cluster has some)
+  int total = here * hd, per = (total + size - 1) / size;
+  for (int i = rank * per + (int)threadIdx.x; i < min(total, (rank + 1) * per); i += threads) {
     int head_at = i / hd, d = i % hd;
     float m_run = -INFINITY, l_run = 0.f, acc = 0.f;
-    for (int base = 0; base < chunks; base += 8) {  // (eight chunks' values are asked for before the first is merged)
-      float o[8], m[8], l[8];
+    for (int base = 0; base < chunks; base += 16) {  // (sixteen chunks' values are asked for before the first is merged)
+      float o[16], m[16], l[16];
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
+      for (int x = 0; x < 16; ++x) {
         int c = base + x;
         if (c >= chunks) continue;
-        unsigned at = local + 4u * (unsigned)(((c / size) * heads_per_block + head_at) * (hd + 2)), far;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(c % size));
+        int place = c / size;
+        unsigned at = local + 4u * (unsigned)((place * heads_per_block + head_at) * (hd + 2)), far;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at), "r"(c - place * size));
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o[x]) : "r"(far + 4u * (unsigned)d));
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m[x]) : "r"(far + 4u * (unsigned)hd));
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[x]) : "r"(far + 4u * (unsigned)hd + 4u));
       }
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
+      for (int x = 0; x < 16; ++x) {
         if (base + x >= chunks) continue;
         float keep, take;
         merge(m_run, l_run, m[x], l[x], keep, take);
@@ -858,8 +887,9 @@ int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* 
   // (more than one and a half rounds of blocks: 8 query heads of 128 to each of 8 kv heads, 8 tokens of 8,000: 597 and 500)
   long long resident = 148ll * (227 * 1024 / ((long long)bytes(per_round) + 2048));
   if (2 * rows * tokens * size > 3 * resident) return DLLM_UNSUPPORTED_SIZE;
-  static std::atomic<unsigned long long> allowed{0};
-  if (!dllm_allow_shared((const void*)attention_chunks_kernel, 200 * 1024, allowed)) return DLLM_LAUNCH_FAILED;
+  auto kernel = hd == 64 ? attention_chunks_kernel<64> : (hd == 128 ? attention_chunks_kernel<128> : attention_chunks_kernel<0>);
+  static std::atomic<unsigned long long> allowed[3];
+  if (!dllm_allow_shared((const void*)kernel, 200 * 1024, allowed[hd == 64 ? 0 : (hd == 128 ? 1 : 2)])) return DLLM_LAUNCH_FAILED;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(size, (unsigned)rows, tokens);
   config.blockDim = dim3(32 * heads_per_block * per_round);
@@ -873,7 +903,7 @@ int launch_chunks(float* out, const float* q, const KvLayout& cache, const int* 
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&config, attention_chunks_kernel, out, q, cache, tok_seq, tok_pos, slots, heads, scale, window,
+  return cudaLaunchKernelEx(&config, kernel, out, q, cache, tok_seq, tok_pos, slots, heads, scale, window,
                             heads_per_block, per_round, room, status) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
