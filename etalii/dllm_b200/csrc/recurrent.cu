@@ -8,7 +8,7 @@
 //                            same sum with v = 1 as one more column of S (the normaliser n_t), read out as n_t . q_t
 //   state-space duality:     (whose prompts may run in segments side by side) the same without a normaliser, heads sharing k and q, and o_t = S^T q_t + skip v_t
 //
-// One kernel serves prompts and single tokens: a block owns 16 columns of one head's S for one sequence and walks
+// One kernel serves prompts and single tokens: a block owns 16 columns (or twice as many, two a lane) of one head's S for one sequence and walks
 // that sequence's new tokens in order, from the state the cache holds to the state it leaves there. A column's
 // recurrence does not involve the other columns, so columns are the parallel dimension besides heads and sequences.
 // Inside a warp a lane holds `RPL` rows of one column in pieces of four (8 or 16 lanes a column; piece i of lane r starts
@@ -18,6 +18,8 @@
 // 16 tokens and hidden behind the arithmetic of the stage before. Everything is float32: inputs, state, sums.
 //
 // State layout: [slot][head][column][row], a column's rows contiguous (a lane's rows are one or more 16-byte loads).
+#include <type_traits>
+
 #include "common.cuh"
 
 #define SCAN_COLS 16  // columns of S a block owns
@@ -91,26 +93,26 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 // whose read-out gets a share of v; MODE 5: the same without a read-out (what a segment leaves of a zero state). TOKENS: tokens a stage. LPC lanes share a column (8 or
 // 16), each with RPL rows of it: the block has 16 * LPC threads. Few lanes a column mean few shuffles and few
 // instructions a token; many lanes mean more warps to hide latency behind, which is what a step with few sequences
-// and heads needs (one warp per scheduler issues a dependent instruction every four cycles and no faster).
-template <int RPL, int LPC, int MODE, int TOKENS, int STAGES>
+// and heads needs (one warp per scheduler issues a dependent instruction every four cycles and no faster). CPL: columns a lane holds its rows of.
+template <int RPL, int LPC, int MODE, int TOKENS, int STAGES, int CPL>
 __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
   constexpr int DIMP = RPL * LPC;  // rows a stage holds per token (the head's dim rounded up)
   constexpr int CPW = 32 / LPC;    // columns a warp owns
-  constexpr int SCAN_THREADS = SCAN_COLS * LPC;
+  constexpr int SCAN_THREADS = SCAN_COLS * LPC, COLS = SCAN_COLS * CPL;
   constexpr int VECTORS = MODE == 3 ? 3 : MODE == 5 ? 1 : 2;
   constexpr int V_AT = VECTORS * DIMP;  // where the values start in a stage row
-  constexpr int PER_TOKEN = V_AT + SCAN_COLS + 4;
+  constexpr int PER_TOKEN = V_AT + COLS + 4;
   constexpr int PIECES = PER_TOKEN / 4;  // 16-byte pieces of a token's stage row
-  extern __shared__ __align__(16) float stage[];  // [STAGES][TOKENS][PER_TOKEN]: k | q | (decays) | v (16 columns) | g, beta, k.q, -
+  extern __shared__ __align__(16) float stage[];  // [STAGES][TOKENS][PER_TOKEN]: k | q | (decays) | v (COLS columns) | g, beta, k.q, -
   pdl_launch_dependents();
   constexpr bool SEGMENTS = MODE >= 4;
   const bool segmented = SEGMENTS && a.segment > 0;
-  const int head = blockIdx.y, col0 = blockIdx.x * SCAN_COLS;
+  const int head = blockIdx.y, col0 = blockIdx.x * COLS;
   const int seq = segmented ? blockIdx.z / a.segments : blockIdx.z, part = segmented ? blockIdx.z % a.segments : 0;
   const int qk_head = head / (a.heads / a.qk_heads);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rg = lane / CPW, cc = lane % CPW;
-  const int col = col0 + warp * CPW + cc;
+  const int place = (warp * CPW + cc) * CPL, col = col0 + place;  // the lane's first column, in the block and in S
   const float decay = MODE == 0 ? a.decay[head] : 0.f, skip = MODE == 4 ? a.skip[head] : 0.f;
   const int state_cols = a.vdim + (MODE == 2 ? 1 : 0);
   pdl_wait();
@@ -130,13 +132,15 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
     count = min(a.segment, count - part * a.segment);
   }
 
-  float S[RPL];  // (dim is a multiple of 4 and so is a lane's first row: a piece of 4 rows is inside the head or not)
+  float S[CPL][RPL];  // (dim is a multiple of 4 and so is a lane's first row: a piece of 4 rows is inside the head or not)
 #pragma unroll
-  for (int j = 0; j < RPL; j += 4) {
-    float4 s4 = (MODE != 5 && col < state_cols && j * LPC + rg * 4 < a.dim)
-                    ? *reinterpret_cast<const float4*>(start + j * LPC) : make_float4(0.f, 0.f, 0.f, 0.f);
-    S[j] = s4.x; S[j + 1] = s4.y; S[j + 2] = s4.z; S[j + 3] = s4.w;
-  }
+  for (int e = 0; e < CPL; ++e)
+#pragma unroll
+    for (int j = 0; j < RPL; j += 4) {
+      float4 s4 = (MODE != 5 && col + e < state_cols && j * LPC + rg * 4 < a.dim)
+                      ? *reinterpret_cast<const float4*>(start + (size_t)e * a.dim + j * LPC) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[e][j] = s4.x; S[e][j + 1] = s4.y; S[e][j + 2] = s4.z; S[e][j + 3] = s4.w;
+    }
 
   auto fill = [&](int chunk, int buffer) {
     float* dst = stage + (size_t)buffer * TOKENS * PER_TOKEN;
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
           if (e - DIMP < a.dim) src = q0 + row + (e - DIMP);
         } else if (MODE == 3 && e < 3 * DIMP) {
           if (e - 2 * DIMP < a.dim) src = d0 + t * a.decay_stride + (e - 2 * DIMP);
-        } else if (e < V_AT + SCAN_COLS) {
+        } else if (e < V_AT + COLS) {
           if (col0 + e - V_AT < a.vdim) src = v0 + row + (e - V_AT);
         } else if (MODE >= 1) {
           const float* aux = a.aux + (size_t)(first + t0 + t) * a.aux_stride;
@@ -182,11 +186,11 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
           if (e - DIMP < a.dim) src = a.q + token * a.stride + qk_head * a.dim + (e - DIMP);
         } else if (MODE == 3 && e < 3 * DIMP) {
           if (e - 2 * DIMP < a.dim) src = a.decays + token * a.decay_stride + head * a.dim + (e - 2 * DIMP);
-        } else if (e < V_AT + SCAN_COLS) {
+        } else if (e < V_AT + COLS) {
           int c = col0 + e - V_AT;
           if (c < a.vdim) src = a.v + token * a.stride + head * a.vdim + c;
         } else if (MODE >= 1) {
-          int which = e - V_AT - SCAN_COLS;
+          int which = e - V_AT - COLS;
           if (which == 0) src = a.aux + token * a.aux_stride + head;
           else if (which == 1) src = a.aux + token * a.aux_stride + a.heads + head;
           else if (which == 2 && MODE < 4) src = a.aux + token * a.aux_stride + 2 * a.heads + qk_head;
@@ -199,30 +203,53 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
   };
 
   float product = 1.f;  // MODE 5: the product of the tokens' factors
-  // one token of the decayed sum: the state moves on, the lane's part of S^T q comes back. Two rows an instruction
-  // (the packed float32 multiply-add of sm_100: the same roundings as two single ones, half the issue slots).
-  auto decayed = [&](const float* row) -> float {
-    float v = row[V_AT + warp * CPW + cc];
-    float keep = decay;
-    if (MODE == 2 || MODE >= 4) {  // this token's own factors; the column behind the values is written with v = 1
-      keep = row[V_AT + SCAN_COLS];
-      v = (MODE == 2 && col == a.vdim ? 1.0f : v) * row[V_AT + SCAN_COLS + 1];
-    }
-    if (MODE == 5) product *= keep;
-    const float2 vv = make_float2(v, v), dd = make_float2(keep, keep);
-    float2 p = make_float2(0.f, 0.f);
+  // Some tokens of the decayed sum: their rows are asked of shared memory first (the loads do not depend on the state, and
+  // serve all of the lane's columns), then the state walks through them, the lane's part of S^T q being left in `to`. Two rows
+  // an instruction (the packed float32 multiply-add of sm_100: the same roundings as two single ones, half the issue slots).
+  auto decayed = [&](const float* rows, auto tokens, float* to) {
+    constexpr int GROUP = decltype(tokens)::value;
+    constexpr int PADL = LPC + 4;
+    float4 kq[GROUP][RPL / 2];
+    float v[GROUP][CPL], keep[GROUP];
 #pragma unroll
-    for (int j = 0; j < RPL; j += 4) {
-      float4 k4 = *reinterpret_cast<const float4*>(row + j * LPC + rg * 4);
-      float2 s01 = __ffma2_rn(dd, make_float2(S[j], S[j + 1]), __fmul2_rn(make_float2(k4.x, k4.y), vv));
-      float2 s23 = __ffma2_rn(dd, make_float2(S[j + 2], S[j + 3]), __fmul2_rn(make_float2(k4.z, k4.w), vv));
-      S[j] = s01.x; S[j + 1] = s01.y; S[j + 2] = s23.x; S[j + 3] = s23.y;
-      if (MODE == 5) continue;
-      float4 q4 = *reinterpret_cast<const float4*>(row + DIMP + j * LPC + rg * 4);
-      p = __ffma2_rn(s01, make_float2(q4.x, q4.y), p);
-      p = __ffma2_rn(s23, make_float2(q4.z, q4.w), p);
+    for (int w = 0; w < GROUP; ++w) {
+      const float* row = rows + w * PER_TOKEN;
+      keep[w] = decay;
+      if (MODE == 2 || MODE >= 4) keep[w] = row[V_AT + COLS];  // this token's own factors
+      if (MODE == 5) product *= keep[w];
+#pragma unroll
+      for (int e = 0; e < CPL; ++e) {
+        v[w][e] = row[V_AT + place + e];
+        if (MODE == 2 || MODE >= 4)  // (the column behind the values is written with v = 1)
+          v[w][e] = (MODE == 2 && col + e == a.vdim ? 1.0f : v[w][e]) * row[V_AT + COLS + 1];
+      }
+#pragma unroll
+      for (int j = 0; j < RPL; j += 4) {
+        kq[w][j / 2] = *reinterpret_cast<const float4*>(row + j * LPC + rg * 4);
+        if (MODE != 5) kq[w][j / 2 + 1] = *reinterpret_cast<const float4*>(row + DIMP + j * LPC + rg * 4);
+      }
     }
-    return p.x + p.y;
+#pragma unroll
+    for (int w = 0; w < GROUP; ++w) {
+      const float2 dd = make_float2(keep[w], keep[w]);
+#pragma unroll
+      for (int e = 0; e < CPL; ++e) {
+        const float2 vv = make_float2(v[w][e], v[w][e]);
+        float2 p = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < RPL; j += 4) {
+          float4 k4 = kq[w][j / 2];
+          float2 s01 = __ffma2_rn(dd, make_float2(S[e][j], S[e][j + 1]), __fmul2_rn(make_float2(k4.x, k4.y), vv));
+          float2 s23 = __ffma2_rn(dd, make_float2(S[e][j + 2], S[e][j + 3]), __fmul2_rn(make_float2(k4.z, k4.w), vv));
+          S[e][j] = s01.x; S[e][j + 1] = s01.y; S[e][j + 2] = s23.x; S[e][j + 3] = s23.y;
+          if (MODE == 5) continue;
+          float4 q4 = kq[w][j / 2 + 1];
+          p = __ffma2_rn(s01, make_float2(q4.x, q4.y), p);
+          p = __ffma2_rn(s23, make_float2(q4.z, q4.w), p);
+        }
+        if (MODE != 5) to[(w * COLS + place + e) * PADL + rg] = p.x + p.y;
+      }
+    }
   };
 
   const int chunks = (count + TOKENS - 1) / TOKENS;
@@ -243,55 +270,15 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
     const int here = min(TOKENS, count - chunk * TOKENS);
     // Every lane leaves its part of a token's read-out in shared memory; after the chunk the block adds the parts up, a
     // thread per token and column, and writes whole pieces of rows.
-    float* parts = stage + (size_t)STAGES * TOKENS * PER_TOKEN;  // [TOKENS][16 columns][LPC + 4]
+    float* parts = stage + (size_t)STAGES * TOKENS * PER_TOKEN;  // [TOKENS][COLS][LPC + 4]
     constexpr int PADL = LPC + 4;
     if (MODE == 0 || MODE == 2 || MODE >= 4) {
       // The decayed sum's read-out does not feed the state: nothing but the state's own multiply-add links two tokens.
-      // a group of tokens at a time: all their rows are asked of shared memory first (the loads do not depend on the
-      // state), then the state walks through them
       constexpr int GROUP = RPL <= 8 ? 4 : 2;
       int u = 0;
-      for (; u + GROUP <= here; u += GROUP) {
-        float4 kq[GROUP][RPL / 2];
-        float v[GROUP], keep[GROUP];
-#pragma unroll
-        for (int w = 0; w < GROUP; ++w) {
-          const float* row = base + (u + w) * PER_TOKEN;
-          v[w] = row[V_AT + warp * CPW + cc];
-          keep[w] = decay;
-          if (MODE == 2 || MODE >= 4) {
-            keep[w] = row[V_AT + SCAN_COLS];
-            v[w] = (MODE == 2 && col == a.vdim ? 1.0f : v[w]) * row[V_AT + SCAN_COLS + 1];
-          }
-          if (MODE == 5) product *= keep[w];
-#pragma unroll
-          for (int j = 0; j < RPL; j += 4) {
-            kq[w][j / 2] = *reinterpret_cast<const float4*>(row + j * LPC + rg * 4);
-            if (MODE != 5) kq[w][j / 2 + 1] = *reinterpret_cast<const float4*>(row + DIMP + j * LPC + rg * 4);
-          }
-        }
-#pragma unroll
-        for (int w = 0; w < GROUP; ++w) {
-          const float2 vv = make_float2(v[w], v[w]), dd = make_float2(keep[w], keep[w]);
-          float2 p = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int j = 0; j < RPL; j += 4) {
-            float4 k4 = kq[w][j / 2];
-            float2 s01 = __ffma2_rn(dd, make_float2(S[j], S[j + 1]), __fmul2_rn(make_float2(k4.x, k4.y), vv));
-            float2 s23 = __ffma2_rn(dd, make_float2(S[j + 2], S[j + 3]), __fmul2_rn(make_float2(k4.z, k4.w), vv));
-            S[j] = s01.x; S[j + 1] = s01.y; S[j + 2] = s23.x; S[j + 3] = s23.y;
-            if (MODE == 5) continue;
-            float4 q4 = kq[w][j / 2 + 1];
-            p = __ffma2_rn(s01, make_float2(q4.x, q4.y), p);
-            p = __ffma2_rn(s23, make_float2(q4.z, q4.w), p);
-          }
-          if (MODE != 5) parts[((u + w) * SCAN_COLS + warp * CPW + cc) * PADL + rg] = p.x + p.y;
-        }
-      }
-      for (; u < here; ++u) {
-        const float p = decayed(base + u * PER_TOKEN);
-        if (MODE != 5) parts[(u * SCAN_COLS + warp * CPW + cc) * PADL + rg] = p;
-      }
+      for (; u + GROUP <= here; u += GROUP)
+        decayed(base + u * PER_TOKEN, std::integral_constant<int, GROUP>{}, parts + (size_t)u * COLS * PADL);
+      for (; u < here; ++u) decayed(base + u * PER_TOKEN, std::integral_constant<int, 1>{}, parts + (size_t)u * COLS * PADL);
     } else {
       // The delta rule: what the state answers to k feeds the write, so the sum S^T k is finished token by token (the
       // shuffles are most of the time from one token to the next); S^T q waits for the end of the chunk. A token's rows
@@ -299,7 +286,7 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
       constexpr bool AHEAD = RPL <= 16;  // (with 32 rows a lane there are no registers for a second token)
       constexpr int V4 = RPL / 4;
       float4 k4[V4], q4[V4], g4[MODE == 3 ? V4 : 1];
-      float v, beta, kq, g = 1.f;
+      float v[CPL], beta, kq, g = 1.f;
       auto fetch = [&](int t) {
         const float* row = base + t * PER_TOKEN;
 #pragma unroll
@@ -308,53 +295,67 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
           k4[j] = *reinterpret_cast<const float4*>(row + 4 * (j * LPC + rg));
           q4[j] = *reinterpret_cast<const float4*>(row + DIMP + 4 * (j * LPC + rg));
         }
-        v = row[V_AT + warp * CPW + cc];
-        if (MODE == 1) g = row[V_AT + SCAN_COLS];
-        beta = row[V_AT + SCAN_COLS + 1];
-        kq = row[V_AT + SCAN_COLS + 2];
+#pragma unroll
+        for (int e = 0; e < CPL; ++e) v[e] = row[V_AT + place + e];
+        if (MODE == 1) g = row[V_AT + COLS];
+        beta = row[V_AT + COLS + 1];
+        kq = row[V_AT + COLS + 2];
       };
       fetch(0);
 #pragma unroll 2
       for (int t = 0; t < here; ++t) {
         if (!AHEAD && t > 0) fetch(t);
-        float2 sk[2] = {}, sq[2] = {};  // S^T k and S^T q before this token's write, in two chains each
+        float2 sk[CPL][2] = {}, sq[CPL][2] = {};  // S^T k and S^T q before this token's write, in two chains each
         float2 kk[RPL / 2];
 #pragma unroll
         for (int j = 0; j < V4; ++j) {
-          float2 s01 = make_float2(S[4 * j], S[4 * j + 1]), s23 = make_float2(S[4 * j + 2], S[4 * j + 3]);
-          if (MODE == 3) {  // the rows shrink first: what follows reads and moves on the shrunk state
-            s01 = __fmul2_rn(s01, make_float2(g4[j].x, g4[j].y));
-            s23 = __fmul2_rn(s23, make_float2(g4[j].z, g4[j].w));
-            S[4 * j] = s01.x; S[4 * j + 1] = s01.y; S[4 * j + 2] = s23.x; S[4 * j + 3] = s23.y;
-          }
           kk[2 * j] = make_float2(k4[j].x, k4[j].y);
           kk[2 * j + 1] = make_float2(k4[j].z, k4[j].w);
-          sk[0] = __ffma2_rn(s01, kk[2 * j], sk[0]);
-          sk[1] = __ffma2_rn(s23, kk[2 * j + 1], sk[1]);
-          sq[0] = __ffma2_rn(s01, make_float2(q4[j].x, q4[j].y), sq[0]);
-          sq[1] = __ffma2_rn(s23, make_float2(q4[j].z, q4[j].w), sq[1]);
+#pragma unroll
+          for (int e = 0; e < CPL; ++e) {
+            float2 s01 = make_float2(S[e][4 * j], S[e][4 * j + 1]), s23 = make_float2(S[e][4 * j + 2], S[e][4 * j + 3]);
+            if (MODE == 3) {  // the rows shrink first: what follows reads and moves on the shrunk state
+              s01 = __fmul2_rn(s01, make_float2(g4[j].x, g4[j].y));
+              s23 = __fmul2_rn(s23, make_float2(g4[j].z, g4[j].w));
+              S[e][4 * j] = s01.x; S[e][4 * j + 1] = s01.y; S[e][4 * j + 2] = s23.x; S[e][4 * j + 3] = s23.y;
+            }
+            sk[e][0] = __ffma2_rn(s01, kk[2 * j], sk[e][0]);
+            sk[e][1] = __ffma2_rn(s23, kk[2 * j + 1], sk[e][1]);
+            sq[e][0] = __ffma2_rn(s01, make_float2(q4[j].x, q4[j].y), sq[e][0]);
+            sq[e][1] = __ffma2_rn(s23, make_float2(q4[j].z, q4[j].w), sq[e][1]);
+          }
         }
-        const float v_now = v, beta_now = beta, kq_now = kq, g_now = g;
+        float v_now[CPL];
+#pragma unroll
+        for (int e = 0; e < CPL; ++e) v_now[e] = v[e];
+        const float beta_now = beta, kq_now = kq, g_now = g;
         if (AHEAD) fetch(min(t + 1, here - 1));
-        float answer = (sk[0].x + sk[0].y) + (sk[1].x + sk[1].y);
+        float answer[CPL];
 #pragma unroll
-        for (int o = CPW; o <= 16; o <<= 1) answer += __shfl_xor_sync(0xffffffffu, answer, o);
-        const float u = beta_now * (v_now - g_now * answer);
-        const float2 uu = make_float2(u, u), gg = make_float2(g_now, g_now);
+        for (int e = 0; e < CPL; ++e) answer[e] = (sk[e][0].x + sk[e][0].y) + (sk[e][1].x + sk[e][1].y);
 #pragma unroll
-        for (int j = 0; j < RPL; j += 2) {
-          float2 now = make_float2(S[j], S[j + 1]);
-          float2 next = __ffma2_rn(kk[j / 2], uu, MODE == 3 ? now : __fmul2_rn(gg, now));
-          S[j] = next.x; S[j + 1] = next.y;
+        for (int o = CPW; o <= 16; o <<= 1)
+#pragma unroll
+          for (int e = 0; e < CPL; ++e) answer[e] += __shfl_xor_sync(0xffffffffu, answer[e], o);
+#pragma unroll
+        for (int e = 0; e < CPL; ++e) {
+          const float u = beta_now * (v_now[e] - g_now * answer[e]);
+          const float2 uu = make_float2(u, u), gg = make_float2(g_now, g_now);
+#pragma unroll
+          for (int j = 0; j < RPL; j += 2) {
+            float2 now = make_float2(S[e][j], S[e][j + 1]);
+            float2 next = __ffma2_rn(kk[j / 2], uu, MODE == 3 ? now : __fmul2_rn(gg, now));
+            S[e][j] = next.x; S[e][j + 1] = next.y;
+          }
+          // (g S + k u^T)^T q = g S^T q + u (k . q): the read-out of the state after the write, without a second sum
+          float read = g_now * ((sq[e][0].x + sq[e][0].y) + (sq[e][1].x + sq[e][1].y));
+          parts[(t * COLS + place + e) * PADL + rg] = rg == 0 ? fmaf(u, kq_now, read) : read;
         }
-        // (g S + k u^T)^T q = g S^T q + u (k . q): the read-out of the state after the write, without a second sum
-        float read = g_now * ((sq[0].x + sq[0].y) + (sq[1].x + sq[1].y));
-        parts[(t * SCAN_COLS + warp * CPW + cc) * PADL + rg] = rg == 0 ? fmaf(u, kq_now, read) : read;
       }
     }
     __syncthreads();
-    for (int i = tid; MODE != 5 && i < here * SCAN_COLS; i += SCAN_THREADS) {
-      int u = i / SCAN_COLS, c = i % SCAN_COLS;
+    for (int i = tid; MODE != 5 && i < here * COLS; i += SCAN_THREADS) {
+      int u = i / COLS, c = i % COLS;
       const float4* mine = reinterpret_cast<const float4*>(parts + i * PADL);
       float sum = 0.f;
 #pragma unroll
@@ -371,24 +372,28 @@ __global__ void __launch_bounds__(SCAN_COLS * LPC) scan_kernel(ScanArgs a) {
     __syncthreads();  // the stage is filled again in the next round
   }
 #pragma unroll
-  for (int j = 0; j < RPL; j += 4)
-    if (leaves && col < state_cols && j * LPC + rg * 4 < a.dim)
-      *reinterpret_cast<float4*>(my_state + j * LPC) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
+  for (int e = 0; e < CPL; ++e)
+#pragma unroll
+    for (int j = 0; j < RPL; j += 4)
+      if (leaves && col + e < state_cols && j * LPC + rg * 4 < a.dim)
+        *reinterpret_cast<float4*>(my_state + (size_t)e * a.dim + j * LPC) =
+            make_float4(S[e][j], S[e][j + 1], S[e][j + 2], S[e][j + 3]);
   if (MODE == 5 && col0 == 0 && tid == 0) a.segment_decay[(size_t)blockIdx.z * a.heads + head] = product;
 }
 
-template <int RPL, int LPC, int MODE, int TOKENS, int STAGES>
+template <int RPL, int LPC, int MODE, int TOKENS, int STAGES, int CPL = 1>
 static int launch_scan_case(const ScanArgs& a, dim3 grid, cudaStream_t stream) {
-  size_t bytes = (size_t)STAGES * TOKENS * ((MODE == 3 ? 3 : MODE == 5 ? 1 : 2) * RPL * LPC + SCAN_COLS + 4) * sizeof(float);
-  if (MODE != 5) bytes += (size_t)TOKENS * SCAN_COLS * (LPC + 4) * sizeof(float);  // the parts of the read-out
+  constexpr int COLS = SCAN_COLS * CPL;
+  size_t bytes = (size_t)STAGES * TOKENS * ((MODE == 3 ? 3 : MODE == 5 ? 1 : 2) * RPL * LPC + COLS + 4) * sizeof(float);
+  if (MODE != 5) bytes += (size_t)TOKENS * COLS * (LPC + 4) * sizeof(float);  // the parts of the read-out
   static bool allowed = false;  // (more than 48 KB of dynamic shared memory has to be asked for once)
   if (bytes > 48 * 1024 && !allowed) {
-    if (cudaFuncSetAttribute(scan_kernel<RPL, LPC, MODE, TOKENS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(scan_kernel<RPL, LPC, MODE, TOKENS, STAGES, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)bytes) != cudaSuccess)
       return DLLM_LAUNCH_FAILED;
     allowed = true;
   }
-  return dllm_launch_pdl(scan_kernel<RPL, LPC, MODE, TOKENS, STAGES>, grid, dim3(SCAN_COLS * LPC), bytes, stream, a);
+  return dllm_launch_pdl(scan_kernel<RPL, LPC, MODE, TOKENS, STAGES, CPL>, grid, dim3(SCAN_COLS * LPC), bytes, stream, a);
 }
 
 // `longest`: the most new tokens a sequence of the step has (the host knows; the kernel reads the real counts).
@@ -404,6 +409,19 @@ static int launch_scan(const ScanArgs& a, int sequences, int longest, cudaStream
   // (the delta rules too, whose tokens are linked by a sum over a column's lanes: with 16 heads of 64 and a prompt of
   // 2,048 tokens 454 us against 527 with 8 lanes, with heads of 128 694 against 746)
   bool deep = longest > 32;  // several stages for prompts, two for steps of single tokens and short portions
+  // Many sequences and heads of 65 to 128 rows: two columns a lane. What bounds them is shared memory: a lane reads 16 bytes of
+  // k and of q for four rows of one column, four cycles of the multiprocessor's each for four multiply-adds a lane, and four
+  // stages of sixteen tokens leave room for two blocks of four warps. A second column a lane needs no second read, and short
+  // stages leave room for more warps. 16 heads of 128 x 128, us before and now: eight prompts of 128 to 2,048 tokens decay
+  // 1,054 -> 650, delta 1,490 -> 1,004; eight of 1,088 983 -> 481, 1,357 -> 813; of 100 97 -> 48, 128 -> 79; sixteen of 64 109 ->
+  // 52, 149 -> 82. (Four columns a lane: 725 and 1,194, 441 and 750; one column in two stages of sixteen: 751 and 1,075.)
+  if constexpr (MODE <= 1) {
+    if (deep && dimp == 128 && lanes == 8 && a.vdim % (2 * SCAN_COLS) == 0) {
+      dim3 half(a.vdim / (2 * SCAN_COLS), grid.y, grid.z);
+      if constexpr (MODE == 0) return launch_scan_case<8, 16, MODE, 8, 3, 2>(a, half, stream);
+      else return launch_scan_case<16, 8, MODE, 16, 2, 2>(a, half, stream);
+    }
+  }
 #define SCAN_CASE(RPL, LPC, TOKENS)                                                                 \
   if (dimp == RPL * LPC && lanes == LPC)                                                            \
     return deep ? launch_scan_case<RPL, LPC, MODE, TOKENS, MODE == 3 ? 3 : 4>(a, grid, stream)      \
