@@ -9,6 +9,7 @@
 //   warps 2.. read the accumulator (tcgen05.ld 32x32b, a lane per row; four warps for tiles up to 64 columns, eight
 //            for wider ones: two per 32 rows, with half the columns each) and apply the epilogue: store float32 or
 //            bfloat16, add into the float32 residual, or SwiGLU on interleaved gate/up columns.
+// Up to 512 rows with a long reduction take the clusters of gemm_split.cuh instead (`split_stretches`).
 // A product of few tokens can run the other way round (W as the 128-row operand, the tile is C^T), and then also with
 // its reduction cut into stretches: a block's work items are (tile, stretch) pairs and every stretch stores its own
 // partial result, which a second kernel sums in order (for a W with fewer tiles than the device has multiprocessors).
@@ -582,6 +583,8 @@ int dispatch(void* c, const void* a, const void* w, int M, int N, int K, int epi
 }
 }  // namespace
 
+#include "gemm_split.cuh"
+
 // C = A[M,K] * W[N,K]^T (bfloat16, float32 accumulation in tensor memory). K must be a multiple of 8 (16-byte row
 // pitch for TMA), N even for the SwiGLU epilogue, and A and W 16-byte aligned. `tile_n`: 32, 64, 128, 256 or, with the residual
 // epilogue, 192 columns of C per block (0 chooses).
@@ -598,6 +601,18 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
   if (K <= 0 || (K & 7) || ((N & 1) && epilogue == EPI_SWIGLU) || ((M & 1) && epilogue == EPI_T_SWIGLU) ||
       ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || status == nullptr)
     return DLLM_UNSUPPORTED_SIZE;
+  const bool own_choice = tile_n == 0 && epilogue <= EPI_SWIGLU && ((uintptr_t)c & 15) == 0 && N <= 65535 * SplitShape::BN;
+  if (int split = own_choice ? split_stretches(M, N, K) : 0) {
+    if (n_tiles_out != nullptr) *n_tiles_out = (N + SplitShape::BN - 1) / SplitShape::BN;
+    switch (epilogue) {
+#define DLLM_SPLIT(EPI) case EPI: return launch_split<EPI>(c, a, w, M, N, K, split, status, stream, RopeArgs{}, norm)
+      DLLM_SPLIT(EPI_STORE_F32);
+      DLLM_SPLIT(EPI_STORE_T);
+      DLLM_SPLIT(EPI_RESIDUAL);
+      DLLM_SPLIT(EPI_SWIGLU);
+#undef DLLM_SPLIT
+    }
+  }
   if (tile_n == 0) {
     long long m_tiles = (M + BM - 1) / BM;
     long long tiles256 = m_tiles * ((N + 255) / 256);
@@ -700,6 +715,11 @@ static int qkv_rope_entry(const void* a, const void* w, int M, int K, void* q_ou
   int N = (heads + 2 * kv_heads) * head_dim;
   // a tile is one head, or four heads of 64 / two of 128 where the product is large enough to fill the device with
   // the wide tiles (which reuse A four times as often: 1.0 to 1.2 PFLOP/s against 0.6)
+  const bool even = head_dim >= 64 && N <= 65535 * SplitShape::BN && ((uintptr_t)q_out & 7) == 0 && ((uintptr_t)cache_base & 7) == 0;
+  if (int split = even ? split_stretches(M, N, K) : 0)
+    return head_dim == 64
+               ? launch_split<EPI_QKV_ROPE, 64>(nullptr, a, w, M, N, K, split, status, stream, rope, norm)
+               : launch_split<EPI_QKV_ROPE, 128>(nullptr, a, w, M, N, K, split, status, stream, rope, norm);
   bool wide = M >= 1024 && K >= 1024 && (long long)((M + BM - 1) / BM) * ((N + 255) / 256) >= 64;
   switch (head_dim) {
     case 32: return launch<32, EPI_QKV_ROPE, 32>(nullptr, a, w, M, N, K, status, stream, rope, norm);

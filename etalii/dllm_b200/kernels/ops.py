@@ -2075,9 +2075,11 @@ def table_by_pair(table: torch.Tensor) -> torch.Tensor:
 
 
 def gemm_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, table: torch.Tensor | None,
-                  rotary_dim: int, heads: int, batch, write_cache: bool = True) -> None:
+                  rotary_dim: int, heads: int, batch, write_cache: bool = True,
+                  ssq: torch.Tensor | None = None, parts: int = 1, eps: float = 0.0) -> None:
     """The q/k/v projection of a prefill-sized step in the tcgen05 tile kernel, ending in the rotation of q and k and
-    the write of k and v into the paged cache (no float32 q/k/v in memory, no separate rotation kernel)."""
+    the write of k and v into the paged cache (no float32 q/k/v in memory, no separate rotation kernel). With `ssq`
+    [parts, tokens] the rows of `a` are un-normed and every row of the product is scaled as in `gemm_normed`."""
     _cuda(a, w, q_out, table)
     m, k = batch.n_tokens, a.shape[1]
     assert gemm_qkv_rope_supported(cache, rotary_dim, table is not None)
@@ -2087,13 +2089,15 @@ def gemm_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, 
         assert table.dtype == torch.float32 and table.shape[0] > batch.max_position, "position beyond the table"
         assert table.shape[1] == rotary_dim // 2 and table.shape[2] == 2
     by_pair = table_by_pair(table) if table is not None else None  # (the layout this kernel reads)
-    _check(_fn("gemm_tcgen05", "dllm_gemm_tcgen05_qkv_rope")(
+    name = "dllm_gemm_tcgen05_qkv_rope" + ("" if ssq is None else "_normed")
+    norm = () if ssq is None else (ssq.data_ptr(), int(parts), float(eps))
+    _check(_fn("gemm_tcgen05", name)(
         a.data_ptr(), w.data_ptr(), m, k, q_out.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(),
         cache.max_pages, cache.page_size, heads, cache.kv_heads, cache.head_dim,
         by_pair.data_ptr() if by_pair is not None else None, rotary_dim if table is not None else 0,
         table.shape[0] if table is not None else 0,
         batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(), batch.slots.data_ptr(), 1 if write_cache else 0,
-        _status_word().data_ptr(), _stream()), "gemm_qkv_rope", lambda: f"M={m} K={k} head_dim={cache.head_dim}")
+        *norm, _status_word().data_ptr(), _stream()), "gemm_qkv_rope", lambda: f"M={m} K={k} head_dim={cache.head_dim}")
 
 
 def gemv_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, table: torch.Tensor | None,

@@ -1307,3 +1307,99 @@ def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner):
     (4, 2, 24, 12), (2, 1, 64, 20)])                               # rotations that are no multiples of eight
 def test_rope_cache_write_in_pieces_of_eight(dtype, tol, heads, kv_heads, head_dim, rotary):
     test_rope_cache_write(dtype, tol, heads, kv_heads, head_dim, rotary)
+
+
+@pytest.mark.parametrize("dim,vdim,heads,lengths", [
+    (128, 128, 16, [33, 1, 70, 40, 5]),               # a block's columns: two a lane, short last stages
+    (68, 32, 16, [1 + 9 * i % 50 for i in range(20)]),  # rows that end inside a lane's pieces, one block of columns
+    (100, 160, 12, [35, 2, 64, 17, 16, 8]),
+])
+def test_scans_with_two_columns_a_lane(dim, vdim, heads, lengths):
+    """Decayed outer products and the gated delta rule where there are blocks enough for two columns a lane, from a state
+    and to one, against float64 token by token (float32 sums of `dim` products and of the tokens behind one another)."""
+    cache, view, batch = _cache_and_batch(torch.float32, 1, 64, lengths, lengths)
+    assert batch.max_new > 32 and -(-vdim // 16) * heads * len(lengths) * 4 >= 148 * 16
+    n, slots = batch.n_tokens, batch.h_slots
+    keys = torch.nn.functional.normalize(_randn((n, 2 * heads, dim), torch.float32, 1), dim=-1).view(n, -1)
+    rows = torch.cat([keys, _randn((n, heads * vdim), torch.float32, 2)], dim=1).contiguous()
+    decay = 1.0 - 2.0 ** -(3.0 + torch.arange(heads, device=DEV) % 5)
+    q, k = (rows[:, i * heads * dim:(i + 1) * heads * dim].view(n, heads, dim).double() for i in range(2))
+    v = rows[:, 2 * heads * dim:].view(n, heads, vdim).double()
+    gates = _randn((n, 2 * heads), torch.float32, 3).sigmoid()
+    aux = torch.cat([gates, (q * k).sum(-1).float()], dim=1).contiguous()
+    for delta in (False, True):
+        state = _randn((max(slots) + 1, heads, vdim, dim), torch.float32, 4)
+        want_state, want = state.double(), torch.empty((n, heads, vdim), dtype=torch.float64, device=DEV)
+        out = torch.full((n, heads * vdim), float("nan"), dtype=torch.float32, device=DEV)
+        if delta:
+            ops().delta_scan(out, rows, aux, heads, heads, dim, vdim, state, batch)
+        else:
+            ops().decay_scan(out, rows, 0, heads * dim, 2 * heads * dim, heads, dim, vdim, decay, False, 0.5, state, batch)
+        at = 0
+        for slot, count in zip(slots, lengths):
+            s = want_state[slot]
+            for t in range(at, at + count):
+                if delta:
+                    s = s * gates[t, :heads].double()[:, None, None]
+                    u = gates[t, heads:].double()[:, None] * (v[t] - torch.einsum("hvd,hd->hv", s, k[t]))
+                else:
+                    s, u = s * decay.double()[:, None, None], v[t]
+                s = s + u[:, :, None] * k[t][:, None, :]
+                want[t] = torch.einsum("hvd,hd->hv", s, q[t]) * (1.0 if delta else 0.5)
+            want_state[slot] = s
+            at += count
+        assert rel_error(out.cpu(), want.reshape(n, -1).cpu()) <= 2e-6, delta
+        assert rel_error(state.cpu(), want_state.cpu()) <= 2e-6, delta
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (65, 4100, 1032),    # a last tile of four columns, a last k tile of eight values
+    (128, 2048, 2048), (129, 2064, 2056), (256, 1024, 4104),  # one and two tiles of rows, clusters of up to eight
+    (200, 20480, 1032),  # as many tiles as the device takes at once: nothing is cut
+])
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
+def test_products_of_a_few_hundred_rows_cut_over_a_cluster(m, n, k, epilogue):
+    test_gemm_tcgen05(m, n, k, epilogue, 0)
+
+
+@pytest.mark.parametrize("m,hidden,inner,outputs", [
+    (100, 2048, 2056, 4096), (256, 1040, 4104, 4108),
+    (512, 576, 1536, 256), (300, 1088, 1032, 6404),  # up to four tiles of rows
+])
+def test_cut_products_with_the_norm_folded_around_them(m, hidden, inner, outputs):
+    test_tile_products_with_the_norm_folded_around_them(m, hidden, inner, outputs)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,rotary,k,new", [
+    (21, 6, 64, 64, 2056, [60, 70, 1, 9]), (29, 3, 64, 0, 2056, [200, 56]), (13, 2, 128, 128, 2056, [64, 1]),
+    (9, 3, 64, 64, 1032, [1] * 70), (5, 1, 128, 128, 1096, [500, 9])])
+def test_cut_qkv_rope(heads, kv_heads, head_dim, rotary, k, new):
+    """The q/k/v product cut over a cluster with a norm's factor of one: its rotation and cache rows."""
+    lengths = [c + 30 * i for i, c in enumerate(new)]
+    cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, lengths, new)
+    n = batch.n_tokens
+    table = None
+    if rotary:
+        angles = torch.arange(2560, dtype=torch.float64)[:, None] * torch.rand(rotary // 2, dtype=torch.float64)[None]
+        table = torch.stack([angles.cos(), angles.sin()], -1).float().to(DEV)
+    w = _randn(((heads + 2 * kv_heads) * head_dim, k), torch.bfloat16, 4, 0.05)
+    x = _randn((n, k), torch.bfloat16, 6)
+    q = torch.zeros((n, heads * head_dim), dtype=torch.bfloat16, device=DEV)
+    before = view.storage.clone()
+    ssq = torch.full((n,), float(k), dtype=torch.float32, device=DEV)
+    for write in (True, False):
+        target = torch.zeros_like(q)
+        ops().gemm_qkv_rope(x, w, target, view, table, rotary, heads, batch, write, ssq=ssq, parts=1, eps=0.0)
+        ops().raise_if_failed()
+        if write:
+            q, written = target, view.storage.clone()
+    assert torch.equal(target, q) and torch.equal(view.storage, written)
+    qkv = (x.double() @ w.double().T).float().cpu()
+    ref_view = type(view)(before.cpu().clone(), view.page_table.cpu(), view.page_size, kv_heads, head_dim, None)
+    ref_q = torch.zeros((n, heads * head_dim), dtype=torch.bfloat16)
+    cpu_batch = type("B", (), {"n_tokens": n, "tok_pos": batch.tok_pos.cpu(), "tok_seq": batch.tok_seq.cpu(),
+                               "slots": batch.slots.cpu()})
+    PK.rope_cache_write(qkv, ref_q, ref_view, table.cpu() if rotary else None, rotary, heads, cpu_batch, True)
+    assert rel_error(q.float().cpu(), ref_q.float()) <= 8e-3
+    assert rel_error(written.float().cpu(), ref_view.storage.float()) <= 8e-3
+    assert (written != before).any(dim=-1).sum().item() <= n * kv_heads * 2
