@@ -49,6 +49,7 @@ struct Shared {
   int reduce_i[32];
   unsigned warp_ties[THREADS / 32];
   unsigned few_n, few_key[FEW], few_sorted[FEW];  // the last candidates of a search (see find_prefix)
+  int few_id[FEW];
 };
 
 // ---- the cluster: barrier and reads of the same variable in another block's shared memory
@@ -377,6 +378,47 @@ __device__ void cluster_argmax(float& v, int& idx, Shared& sh, Turn& turn) {
   }
 }
 
+// One warp chooses among the at most 32 candidates that the blocks of the cluster have left in their lists (few_n, few_key,
+// few_id: all that min-p keeps): what the searches of `sample_kernel` would choose, by the same whole-number masses. Lane i
+// takes the i-th entry, finds its place in the order (p descending, id ascending) and the mass up to and with it; the first
+// whose running mass exceeds the target is the choice.
+template <int CL>
+__device__ __forceinline__ int choose_among_few(Shared& sh, int lane, int count, double u) {
+  unsigned key = 0, slot = (unsigned)lane;
+  int id = 0x7fffffff;
+  bool mine = false;
+#pragma unroll
+  for (unsigned r = 0; r < CL; ++r) {
+    unsigned here = remote_u32(&sh.few_n, r);
+    if (!mine && slot < here) {
+      key = remote_u32(&sh.few_key[slot], r);
+      id = (int)remote_u32(&sh.few_id[slot], r);
+      mine = true;
+    }
+    if (!mine) slot -= here;
+  }
+  const unsigned long long mass = mine ? to_fx(__uint_as_float(key)) : 0ull;
+  unsigned long long through = 0, total = 0;
+  int before = 0;
+  for (int i = 0; i < count; ++i) {
+    unsigned other = __shfl_sync(0xffffffffu, key, i);
+    int other_id = __shfl_sync(0xffffffffu, id, i);
+    unsigned long long other_mass = __shfl_sync(0xffffffffu, mass, i);
+    bool first = other > key || (other == key && other_id < id);
+    before += first ? 1 : 0;
+    through += first || other_id == id ? other_mass : 0ull;
+    total += other_mass;
+  }
+  unsigned long long target = (unsigned long long)(u * (double)total);
+  if (total > 0 && target >= total) target = total - 1;
+  // the first place at which the running mass exceeds the target, else the last one
+  int place = mine && through > target ? before : count - 1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) place = min(place, __shfl_xor_sync(0xffffffffu, place, o));
+  unsigned holder = __ballot_sync(0xffffffffu, mine && before == place);
+  return __shfl_sync(0xffffffffu, id, __ffs(holder) - 1);
+}
+
 template <int CL>
 __global__ void __launch_bounds__(THREADS, 1) sample_kernel(
     int* __restrict__ out_tokens, const float* __restrict__ logits, long long row_stride, int vocab,
@@ -492,11 +534,42 @@ __global__ void __launch_bounds__(THREADS, 1) sample_kernel(
   }
   if (min_p > 0.0) {
     cluster_sync();  // the largest probability may have been written by another block of the cluster
+    if (tid == 0) sh.few_n = 0;  // (a search of top-p's may have read the lists until that barrier)
+    __syncthreads();
     double floor_p = min_p * (double)__ldcg(p + best_i);
     unsigned long long local = 0;
-    for (int i = first; i < vocab; i += stride) local += ((double)p[i] >= floor_p) ? 1ull : 0ull;
+    for (int i = first; i < vocab; i += stride) {
+      float v = p[i];
+      if ((double)v >= floor_p) {
+        ++local;
+        if (*(volatile unsigned*)&sh.few_n > (unsigned)FEW) continue;  // (too many already: nobody queues for a place)
+        unsigned place = atomicAdd(&sh.few_n, 1u);
+        if (place < (unsigned)FEW) {
+          sh.few_key[place] = __float_as_uint(v);
+          sh.few_id[place] = i;
+        }
+      }
+    }
     unsigned long long n = cluster_sum_u64<CL>(local, sh, turn);
     if (n >= 1 && n < keep) keep = n;
+    // Few enough, and nothing else cuts them: they are the kept prefix, and the two searches, each several passes over the
+    // row, are not needed. (The lists are read behind the barrier of the sum. A row with one clear choice,
+    // vocabulary 49,152: 64 rows 72.2 -> 29.7 us, 8 rows 36.6 -> 14.9.)
+    if (n >= 1 && n == keep && n <= (unsigned long long)FEW) {
+      if (rank == 0 && tid < 32) {
+        double u = 0.0;
+        if (tid == 0) {
+          unsigned long long* state = rng + (size_t)rng_rows[row] * 4;
+          unsigned long long s[4] = {state[0], state[1], state[2], state[3]};
+          u = next_double(s);
+          state[0] = s[0]; state[1] = s[1]; state[2] = s[2]; state[3] = s[3];
+        }
+        int chosen = choose_among_few<CL>(sh, tid, (int)n, __shfl_sync(0xffffffffu, u, 0));
+        if (tid == 0) out_tokens[row] = chosen;
+      }
+      cluster_sync();  // nobody leaves while its list may still be read
+      return;
+    }
   }
   unsigned long long total;
   if (keep >= (unsigned long long)vocab) {  // everything is kept: the total is a plain sum, no search needed

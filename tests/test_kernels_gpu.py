@@ -1403,3 +1403,22 @@ def test_cut_qkv_rope(heads, kv_heads, head_dim, rotary, k, new):
     assert rel_error(q.float().cpu(), ref_q.float()) <= 8e-3
     assert rel_error(written.float().cpu(), ref_view.storage.float()) <= 8e-3
     assert (written != before).any(dim=-1).sum().item() <= n * kv_heads * 2
+
+
+@pytest.mark.parametrize("rows", [4, 20, 40, 80])  # eight blocks a row, four, two, one
+@pytest.mark.parametrize("ties", [False, True])
+def test_sample_where_min_p_keeps_a_few_candidates(rows, ties):
+    """One to 32 kept candidates are chosen from without a search, 33 by one; equal probabilities among them go by id. With
+    top-k and top-p that cut them further, and that do not."""
+    g = torch.Generator().manual_seed(rows + ties)
+    vocab = 3001
+    logits = torch.randn((rows, vocab), generator=g) - 30
+    for r in range(rows):
+        kept = (1, 2, 5, 31, 32, 33, 40)[r % 7]
+        ids = torch.randperm(vocab, generator=g)[:kept]
+        logits[r, ids] = torch.randint(0, 3, (kept,), generator=g).float() if ties else torch.rand(kept, generator=g) * 2.5
+    seeds = [5 * r + 2 for r in range(rows)]
+    for options in ({"temperature": 1.0, "min_p": 0.05}, {"temperature": 1.0, "min_p": 0.05, "top_k": 31},
+                    {"temperature": 0.9, "min_p": 0.04, "top_p": 0.9}):
+        got, want = _sample_both(logits, options, seeds)
+        assert got == want, options
