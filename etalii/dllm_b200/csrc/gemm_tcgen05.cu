@@ -602,7 +602,7 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
       ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || status == nullptr)
     return DLLM_UNSUPPORTED_SIZE;
   const bool own_choice = tile_n == 0 && epilogue <= EPI_SWIGLU && ((uintptr_t)c & 15) == 0 && N <= 65535 * SplitShape::BN;
-  if (int split = own_choice ? split_stretches(M, N, K) : 0) {
+  if (int split = own_choice ? split_stretches<EPI_STORE_T>(M, N, K) : 0) {
     if (n_tiles_out != nullptr) *n_tiles_out = (N + SplitShape::BN - 1) / SplitShape::BN;
     switch (epilogue) {
 #define DLLM_SPLIT(EPI) case EPI: return launch_split<EPI>(c, a, w, M, N, K, split, status, stream, RopeArgs{}, norm)
@@ -616,7 +616,8 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
   if (tile_n == 0) {
     long long m_tiles = (M + BM - 1) / BM;
     long long tiles256 = m_tiles * ((N + 255) / 256);
-    if (M <= 256) tile_n = 32;  // few rows: many narrow tiles
+    // few rows: many narrow tiles (a tile of rows more, and 28672 x 4096 has enough wide ones: 143.5 against 61.8 µs)
+    if (M <= 128 || (M <= 256 && !(N % 256 == 0 && tiles256 >= 128))) tile_n = 32;
     // enough 256-wide tiles to give every multiprocessor one: the widest tile reuses A most (measured: 1.0 to 1.4
     // PFLOP/s from K = 2048 up, against 0.6 to 1.2 for the 128-wide tile; at K = 576, 2048 x 3072 with SwiGLU:
     // 11.5 µs against 12.7 and 13.5 for 128 and 64)
@@ -716,7 +717,7 @@ static int qkv_rope_entry(const void* a, const void* w, int M, int K, void* q_ou
   // a tile is one head, or four heads of 64 / two of 128 where the product is large enough to fill the device with
   // the wide tiles (which reuse A four times as often: 1.0 to 1.2 PFLOP/s against 0.6)
   const bool even = head_dim >= 64 && N <= 65535 * SplitShape::BN && ((uintptr_t)q_out & 7) == 0 && ((uintptr_t)cache_base & 7) == 0;
-  if (int split = even ? split_stretches(M, N, K) : 0)
+  if (int split = even ? split_stretches<EPI_QKV_ROPE>(M, N, K) : 0)
     return head_dim == 64
                ? launch_split<EPI_QKV_ROPE, 64>(nullptr, a, w, M, N, K, split, status, stream, rope, norm)
                : launch_split<EPI_QKV_ROPE, 128>(nullptr, a, w, M, N, K, split, status, stream, rope, norm);
