@@ -56,9 +56,9 @@ __device__ __forceinline__ float remote_float(const float* local, unsigned rank)
 // CLUSTER blocks of WARPS warps serve one (sequence, kv head). Few (sequence, kv head) pairs: many blocks per pair
 // to fill the device and shorten every chain of pages; many pairs: one block per pair, no exchange between blocks.
 template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
-__global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
-    bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
-    const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
+__device__ __forceinline__ void decode_attention(
+    bf16* __restrict__ out, const bf16* __restrict__ q, const KvLayout& cache, const int* __restrict__ tok_pos,
+    const int* __restrict__ slots, int heads, float scale_log2, int window, const ScoreOptions& options) {
   constexpr int LD = HD + 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* kv_s = reinterpret_cast<bf16*>(smem_raw);        // per warp: K [64][LD], V [64][LD]
@@ -78,7 +78,13 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   auto values_of = [&](int page, int row) {
     return OPTIONS ? value_at(wide, page, g, row) : kv_offset(cache, page, 1, g, row);
   };
-  pdl_launch_dependents();
+  // When the next kernels may start. Started with this one they ask for their weights and wait, on the same multiprocessors
+  // and the same HBM, which costs this kernel more than it gives them; behind the keys they still start under its exchange.
+  // Whole calls, ms, at the start / here: 135M shape batch 1 27.5 / 26.9, 8 69.5 / 68.0, 64 115.5 / 113.0; 1.7B shape batch 8 with
+  // the same rule in the products (gemv.cu) 132.2 / 125.8. Not with heads of 128, where one sequence's attention leaves HBM to
+  // the next weights: 8B shape 93.8 / 94.4.
+  constexpr bool LATE = HD <= 64;
+  if (!LATE) pdl_launch_dependents();
   int end = tok_pos[b] + 1;    // positions and slots are written only by the step's last kernel
   const int chunk = OPTIONS ? options.chunk : 0;
   int first = first_visible(end - 1, chunk, window);
@@ -87,13 +93,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   const KeyWalk walk(end - 1, end - 1, window, OPTIONS ? options.keep : 0, TILE_KEYS, chunk);
   auto key_of = [&](int it) { return OPTIONS ? walk.tile(it) * TILE_KEYS : base + it * TILE_KEYS; };
   const int tiles = OPTIONS ? walk.count : (end - base + TILE_KEYS - 1) / TILE_KEYS;
-  // All of the sequence's tiles are the first block's: the others leave, and there is nobody to meet: no cluster barriers, no
-  // reads of the other blocks' memory. (They are the same for every block of the cluster: positions are not written while
-  // this kernel may run.) us before and now: 9 query and 3 kv heads of 64, one sequence of 80 keys 3.4 -> 2.7, of 200 3.5 ->
-  // 2.7, 64 of 200 6.0 -> 5.1; 32 and 8 heads of 128, one of 120 4.6 -> 3.7; 32 and 32 of 64, 100, 100, 100 and 4,000 keys 17.4 ->
-  // 12.3.
-  const bool alone = CLUSTER == 1 || tiles <= WARPS;
-  if (alone && rank != 0) return;
   const ScoreCap score(scale_log2 / SCORE_LOG2E, OPTIONS ? options.cap : 0.f);
   const bool capped = OPTIONS && options.cap > 0.f;
   const float unit = capped ? 1.0f : scale_log2;  // what a score still has to be multiplied by
@@ -299,6 +298,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
       l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
     }
     __syncthreads();  // every warp is done with its keys and values: the space becomes the exchange buffer
+    if (LATE && h0 == 0) pdl_launch_dependents();
     if (tq == 0) {
       sm_ml[warp][gq][0] = m_run[0]; sm_ml[warp][gq][1] = l_run[0];
       sm_ml[warp][gq + 8][0] = m_run[1]; sm_ml[warp][gq + 8][1] = l_run[1];
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
       if (d == 0) { cta_ml[h][0] = m; cta_ml[h][1] = l; }
     }
     const int out_row = OPTIONS ? options.out_stride : heads * hd;
-    if (alone) {
+    if (CLUSTER == 1) {
       __syncthreads();
       for (int idx = threadIdx.x; idx < nh * vd; idx += WARPS * 32) {
         int h = idx / vd, d = idx % vd, head = g * group + h0 + h;
@@ -365,9 +365,33 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
             __float2bfloat16_rn(OPTIONS ? o * sink_factor(m, l, options, head) : o / l);
       }
     }
-    if (!alone) cluster_sync();  // nobody leaves (or reuses the space) while others still read its partial result
+    if (CLUSTER > 1) cluster_sync();  // nobody leaves (or reuses the space) while others still read its partial result
     else __syncthreads();
   }
+}
+
+// A cluster whose sequence has no more tiles than one block has warps is that block: the others leave, and there is nobody
+// to meet: no cluster barriers, no reads of the other blocks' memory. (The tiles are the same for every block of the cluster:
+// positions are not written while this kernel may run.) us before and now: 9 query and 3 kv heads of 64, one sequence of 80
+// keys 3.4 -> 2.7, of 200 3.5 -> 2.7, 64 of 200 6.0 -> 5.1; 32 and 8 heads of 128, one of 120 4.6 -> 3.7; 32 and 32 of 64, 100,
+// 100, 100 and 4,000 keys 17.4 -> 12.3. The two are compiled apart: with one body and a flag the long sequences' took 0.1 us
+// longer.
+template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
+__global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
+    bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
+    const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
+  if (CLUSTER > 1) {
+    int newest = tok_pos[blockIdx.z];
+    const int chunk = OPTIONS ? options.chunk : 0;
+    int tiles = OPTIONS ? KeyWalk(newest, newest, window, options.keep, TILE_KEYS, chunk).count
+                        : newest / TILE_KEYS - first_visible(newest, chunk, window) / TILE_KEYS + 1;
+    if (tiles <= WARPS) {
+      if (blockIdx.x == 0)
+        decode_attention<HD, 1, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, scale_log2, window, options);
+      return;
+    }
+  }
+  decode_attention<HD, CLUSTER, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, scale_log2, window, options);
 }
 
 template <int HD, int WARPS>
