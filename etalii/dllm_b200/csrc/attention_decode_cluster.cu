@@ -374,13 +374,14 @@ __device__ __forceinline__ void decode_attention(
 // to meet: no cluster barriers, no reads of the other blocks' memory. (The tiles are the same for every block of the cluster:
 // positions are not written while this kernel may run.) us before and now: 9 query and 3 kv heads of 64, one sequence of 80
 // keys 3.4 -> 2.7, of 200 3.5 -> 2.7, 64 of 200 6.0 -> 5.1; 32 and 8 heads of 128, one of 120 4.6 -> 3.7; 32 and 32 of 64, 100,
-// 100, 100 and 4,000 keys 17.4 -> 12.3. The two are compiled apart: with one body and a flag the long sequences' took 0.1 us
-// longer.
-template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
+// 100, 100 and 4,000 keys 17.4 -> 12.3. Only for up to four sequences (SOLO): in a batch of short and long ones the two bodies
+// side by side cost more than they give (135M shape, batch 8 of 128 to 2,048 67.4 ms a call without, 68.1 with, batch 64 112.0 and
+// 112.9; batch 1 28.6 and 27.6).
+template <int HD, int CLUSTER, int WARPS, bool OPTIONS, bool SOLO>
 __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
     bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
     const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
-  if (CLUSTER > 1) {
+  if (SOLO && CLUSTER > 1) {
     int newest = tok_pos[blockIdx.z];
     const int chunk = OPTIONS ? options.chunk : 0;
     int tiles = OPTIONS ? KeyWalk(newest, newest, window, options.keep, TILE_KEYS, chunk).count
@@ -401,13 +402,13 @@ constexpr size_t block_smem() {
   return kv_bytes > red_bytes ? kv_bytes : red_bytes;
 }
 
-template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
+template <int HD, int CLUSTER, int WARPS, bool OPTIONS, bool SOLO>
 int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, const int* slots, int heads,
            int sequences, float scale, int window, const ScoreOptions& options, cudaStream_t stream) {
   constexpr size_t smem = block_smem<HD, WARPS>();
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS>,
+    if (cudaFuncSetAttribute(decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS, SOLO>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return DLLM_LAUNCH_FAILED;
     configured = true;
@@ -426,7 +427,7 @@ int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, 
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&config, decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS>, (bf16*)out, (const bf16*)q,
+  return cudaLaunchKernelEx(&config, decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS, SOLO>, (bf16*)out, (const bf16*)q,
                             cache, tok_pos, slots, heads, scale * SCORE_LOG2E, window, options) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
@@ -468,7 +469,8 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     if (HD > 64 && shape == 0 && pairs <= 4 * places) shape = 1;
   }
 #define DLLM_GO(CL, WARPS) \
-  return launch<HD, CL, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
+  return (sequences <= 4 && CL > 1 ? launch<HD, CL, WARPS, OPTIONS, (CL > 1)> : launch<HD, CL, WARPS, OPTIONS, false>)( \
+      out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
   switch (shape) {
     case 0: DLLM_GO(1, NW);
     case 1: DLLM_GO(2, NW);

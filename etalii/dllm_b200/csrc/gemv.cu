@@ -44,7 +44,7 @@ struct Early {
   }
 };
 
-constexpr long long LATE_FROM = 16ll << 20;  // bytes of W (see the kernel)
+constexpr long long LATE_FROM = 4ll << 20;  // bytes of W (see the kernel)
 
 template <int WARPS, int NT, int EPI, bool NORM, bool PIPE>
 __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, const void* __restrict__ a,
@@ -84,8 +84,10 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   Early<EPI, NT> early;
   // A large W keeps HBM busy by itself: the next kernels, which would ask for theirs at once and wait, start when this
-  // block's share has been multiplied (1.7B shape, batch 8, with the same in the attention 132.2 -> 125.8 ms a call; two
-  // layers of linear attention and two of softmax, 2,048 wide, 31.4 -> 30.5). From 16 MB on: at 32 and 64 MB 132.7 and 132.2.
+  // block's share has been multiplied (1.7B shape, batch 8, with the same in the attention 132.2 -> 125.8 ms a call). From
+  // 4 MB on: with 32 and 64 MB 132.7 and 132.2; with 16 and 4 four layers of linear attention and softmax, 2,048 wide, take
+  // 30.5 and 29.9; without a limit the small products of the 135M shape, batch 8, lose what the early start gives them,
+  // 68.1 against 81.6.
   const bool late = 2ll * N * K >= LATE_FROM;
   if (!late) pdl_launch_dependents();
   // A stretch is MAX_STEPS k steps. Every load of a stretch is issued before its first product. For long rows
