@@ -725,7 +725,6 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
   float* kv_s = smem;                                // [per_round][k|v][64][ld]
   float* q_s = kv_s + (size_t)per_round * 2 * 64 * ld;          // [heads_per_block][hd]
   float* result = q_s + (size_t)heads_per_block * hd;           // [room][heads_per_block][hd + 2]: o, m, l
-  pdl_launch_dependents();
   int end = tok_pos[t] + 1, first = (window > 0 && end > window) ? end - window : 0;
   const int* pages = cache.page_table + (size_t)slots[tok_seq[t]] * cache.max_pages;
   int chunk0 = first / 64, chunks = min((end + 63) / 64 - chunk0, room * size);
@@ -820,6 +819,7 @@ __global__ void __launch_bounds__(CHUNK_WARPS * 32) attention_chunks_kernel(
     }
   }
   asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+  pdl_launch_dependents();  // (behind the chunks: see the products of few rows in gemm_simt.cu)
   unsigned local = (unsigned)__cvta_generic_to_shared(result);
   // (the outputs are dealt out evenly: every block of the cluster has some)
   int total = here * hd, per = (total + size - 1) / size;

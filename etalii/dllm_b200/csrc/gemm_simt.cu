@@ -225,7 +225,6 @@ __global__ void __launch_bounds__(COLS * ROWS / PER) gemm_f32_small_kernel(void*
   int tid = threadIdx.x, col = tid % COLS, row0 = tid / COLS;  // rows row0 + i * (ROWS / PER)
   int n0 = blockIdx.x * COLS;
   int tiles = (K + DEPTH - 1) / DEPTH;
-  pdl_launch_dependents();
   auto ask_w = [&](int t) {
     float* stage = ring + (t % STAGES) * STAGE;
 #pragma unroll
@@ -247,6 +246,9 @@ __global__ void __launch_bounds__(COLS * ROWS / PER) gemm_f32_small_kernel(void*
   auto close = [] { asm volatile("cp.async.commit_group;\n" ::); };
   for (int t = 0; t < min(tiles, STAGES - 1); ++t) ask_w(t);
   pdl_wait();
+  // (the next kernel starts here and not with this one: those behind it would all ask for their weights and wait beside it.
+  // Eight sequences of the 135M shape in float32, with the same in the attention of single tokens, 63.8 -> 56.1 ms a call)
+  pdl_launch_dependents();
   for (int t = 0; t < STAGES - 1; ++t) {
     if (t < tiles) ask_a(t);
     close();
