@@ -1,4 +1,4 @@
-// The tile product for a few hundred rows of activations and a long reduction (a short prompt): tiles of 128 x 128 whose
+// The tile product for hundreds of rows of activations and a long reduction (a short prompt): tiles of 128 x 128 whose
 // reduction is shared by the 1, 2, 4 or 8 blocks of a thread-block cluster. Part of gemm_tcgen05.cu.
 //
 // What bounds such a product is W, read once from HBM, as long as every multiprocessor takes part and the activations are
@@ -234,6 +234,8 @@ __global__ void __launch_bounds__(SplitShape::THREADS, SplitShape::BLOCKS_PER_SM
 //   576 x 1536             10.2 / 5.7        10.8 / 6.5        10.9 / 7.2        11.3 / 7.9         10.7 / 8.9
 //   28672 x 4096 SwiGLU    87.6 / 47.5       88.4 / 49.1      144.2 / 81.0      145.2 / 87.4       108.5 / 166.0
 //   16384 x 2048 SwiGLU    24.3 / 16.9       24.5 / 18.4       43.7 / 21.4       44.1 / 22.2        31.6 / 41.5
+// With 768, 1,145 and 1,536 rows: 2048 x 2048 27.1 / 15.7, 28.6 / 16.5, 31.3 / 23.0; 2048 x 8192 66.2 / 37.1, 67.8 / 39.6, 73.1 /
+// 65.0; 576 x 1536 10.8 / 9.9, 10.9 / 10.1, 11.1 / 10.6, but with 2,048 12.2 / 14.2.
 // Two and more tiles of rows come here while 256-wide tiles of gemm_tcgen05_kernel would leave multiprocessors without one
 // (it takes those from 128 on: 28672 x 4096 with 129 and 256 rows 61.8 / 64.7, 16384 x 2048 18.8 / 19.3). A reduction of 576
 // values has nothing to share: 576 x 576 5.7 / 5.7, 6.2 / 6.8, 6.5 / 7.0; 3072 x 576 5.2 / 5.9, 5.2 / 6.9, 5.5 / 7.5. The q/k/v
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(SplitShape::THREADS, SplitShape::BLOCKS_PER_SM
 // 500 39.0 / 52.7; 6144 x 2048 (heads of 64) 13.9 / 12.9, 15.3 / 17.9, 15.2 / 19.6, 27.8 / 30.0.
 template <int EPI> int split_stretches(int M, int N, int K) {
   const int k_tiles = (K + BK - 1) / BK, m_tiles = (M + BM - 1) / BM;
-  if (M <= 64 || M > 512 || (N & 3) || k_tiles < 16) return 0;
+  if (M <= 64 || M > 1536 || (N & 3) || k_tiles < 16) return 0;
   if (EPI == EPI_QKV_ROPE && m_tiles > (K >= 4096 ? 3 : 1)) return 0;
   if (m_tiles > 1 && N % 256 == 0 && (long long)m_tiles * (N / 256) >= 128) return 0;
   const long long tiles = (long long)m_tiles * ((N + SplitShape::BN - 1) / SplitShape::BN);

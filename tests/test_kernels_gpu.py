@@ -1364,7 +1364,7 @@ def test_products_of_a_few_hundred_rows_cut_over_a_cluster(m, n, k, epilogue):
 
 @pytest.mark.parametrize("m,hidden,inner,outputs", [
     (100, 2048, 2056, 4096), (256, 1040, 4104, 4108),
-    (512, 576, 1536, 256), (300, 1088, 1032, 6404),  # up to four tiles of rows
+    (512, 576, 1536, 256), (300, 1088, 1032, 6404), (1536, 320, 1096, 256),  # up to twelve tiles of rows
 ])
 def test_cut_products_with_the_norm_folded_around_them(m, hidden, inner, outputs):
     test_tile_products_with_the_norm_folded_around_them(m, hidden, inner, outputs)
