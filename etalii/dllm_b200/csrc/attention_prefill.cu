@@ -75,13 +75,6 @@ __global__ void __launch_bounds__(THREADS, HD <= 64 ? 2 : 1) prefill_kernel(
   const WideKv wide{cache.base, cache.page_table, cache.max_pages, cache.page_size, cache.kv_heads, hd, vd};
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(WARPS * 32) : "memory"); };
 
-  // queries -> shared memory (rows beyond the tile and dims beyond head_dim are zero)
-  for (int idx = threadIdx.x; idx < BM * (HD / 8); idx += THREADS) {
-    int r = idx / (HD / 8), c = idx % (HD / 8);
-    bool ok = r < rows && c < chunks;
-    const bf16* src = ok ? q + ((size_t)(tok0 + r) * heads + h) * hd + c * 8 : q;
-    cp_async_16(q_s + r * LD + c * 8, src, ok);
-  }
   int last_pos = pos0 + rows - 1;                                   // last query's position
   // the key tiles the block's queries see between them, by their number in the walk
   const int chunk = OPTIONS ? options.chunk : 0;
@@ -90,6 +83,18 @@ __global__ void __launch_bounds__(THREADS, HD <= 64 ? 2 : 1) prefill_kernel(
   // the pages of the key tiles this block will read, fetched once (not one dependent load per tile)
   __shared__ int page_s[MAX_TILES];
   for (int i = threadIdx.x; i < walk.count && i < MAX_TILES; i += THREADS) page_s[i] = pages[walk.tile(i)];
+  // What the step's metadata says has been read while the kernel in front ended; queries and the newest keys and values are
+  // its output. (Launched only behind that kernel's end, sixteen texts of up to 143 tokens through the 135M shape took 1,518 us
+  // a call, now 1,440.)
+  pdl_wait();
+  pdl_launch_dependents();
+  // queries -> shared memory (rows beyond the tile and dims beyond head_dim are zero)
+  for (int idx = threadIdx.x; idx < BM * (HD / 8); idx += THREADS) {
+    int r = idx / (HD / 8), c = idx % (HD / 8);
+    bool ok = r < rows && c < chunks;
+    const bf16* src = ok ? q + ((size_t)(tok0 + r) * heads + h) * hd + c * 8 : q;
+    cp_async_16(q_s + r * LD + c * 8, src, ok);
+  }
   __syncthreads();
 
   const int flat_dst = (tid / (HD / 8)) * LD + (tid % (HD / 8)) * 8, flat_src = tid * 8;
@@ -316,10 +321,8 @@ int launch(void* out, const void* q, const KvLayout& cache, const int* tile_seq,
     configured = true;
   }
   dim3 grid(tiles, heads);
-  prefill_kernel<HD, OPTIONS><<<grid, THREADS, smem, stream>>>((bf16*)out, (const bf16*)q, cache, tile_seq, tile_first,
-                                                      cu_seqlens, start, slots, heads,
-                                                      scale * SCORE_LOG2E, window, options);
-  return dllm_launch_status();
+  return dllm_launch_pdl(prefill_kernel<HD, OPTIONS>, grid, dim3(THREADS), smem, stream, (bf16*)out, (const bf16*)q, cache,
+                         tile_seq, tile_first, cu_seqlens, start, slots, heads, scale * SCORE_LOG2E, window, options);
 }
 }  // namespace
 
