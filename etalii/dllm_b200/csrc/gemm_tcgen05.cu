@@ -76,14 +76,16 @@ __device__ __forceinline__ WorkItem work_item(int item, int total, int k_tiles, 
 // column of W's tiles, until the panel has met all of W; the next panel follows. The host makes a panel as many rows as
 // stay in L2 (`launch`), so that A comes from HBM once however many columns of tiles read it.
 struct TilePlace { int m, n; };
+// (Kernels of their own: the choice at run time cost every product 0.2 us, 122 of them a 2,048-token prompt.)
+template <bool PANELS>
 __device__ __forceinline__ TilePlace tile_place(int tile, int m_tiles, int n_tiles, int m_group) {
-  if (m_group >= m_tiles) return TilePlace{tile % m_tiles, tile / m_tiles};
+  if (!PANELS) return TilePlace{tile % m_tiles, tile / m_tiles};
   int panel = tile / (m_group * n_tiles), at = tile - panel * m_group * n_tiles;
   int high = min(m_group, m_tiles - panel * m_group);
   return TilePlace{panel * m_group + at % high, at / high};
 }
 
-template <int BN, int EPI, bool DEEP, int HD>
+template <int BN, int EPI, bool DEEP, int HD, bool PANELS>
 __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLOCKS_PER_SM) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                const __grid_constant__ CUtensorMap map_w,
                                                                void* __restrict__ c, int M, int N, int K,
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
       bool ok = true;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
         WorkItem w = work_item(item, total, k_tiles, k_split);
-        TilePlace place = tile_place(w.tile, m_tiles, n_tiles, m_group);
+        TilePlace place = tile_place<PANELS>(w.tile, m_tiles, n_tiles, m_group);
         int m0 = place.m * BM, n0 = place.n * BN;
         for (int kt = w.kt_begin; kt < w.kt_end; ++kt, ++it) {
           int s = it % S::STAGES;
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(Shape<BN, DEEP>::THREADS, Shape<BN, DEEP>::BLO
     for (int item = blockIdx.x; item < items; item += gridDim.x, ++lt) {
       int buf = lt & 1;
       WorkItem w = work_item(item, total, k_tiles, k_split);
-      TilePlace place = tile_place(w.tile, m_tiles, n_tiles, m_group);
+      TilePlace place = tile_place<PANELS>(w.tile, m_tiles, n_tiles, m_group);
       int m0 = place.m * BM, n_tile = place.n, n0 = n_tile * BN;
       void* c_part = EPI == EPI_T_STORE_F32 ? (void*)((float*)c + (size_t)w.split * M * N) : c;
       int m = m0 + quarter * 32 + lane;
@@ -516,13 +518,6 @@ int launch_shape(void* c, const CUtensorMap& map_a, const CUtensorMap& map_w, in
                  cudaStream_t stream, const RopeArgs& rope, int m_tiles, int n_tiles, int sms, const NormArgs& norm,
                  int k_split = 1) {
   typedef Shape<BN, DEEP, EpilogueStage<BN, EPI, DEEP>::BYTES> S;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, EPI, DEEP, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)S::SMEM) != cudaSuccess)
-      return DLLM_LAUNCH_FAILED;
-    configured = true;
-  }
   long long total = (long long)m_tiles * n_tiles * k_split;
   int blocks = sms * S::BLOCKS_PER_SM;
   if (blocks > total) blocks = (int)total;
@@ -534,8 +529,15 @@ int launch_shape(void* c, const CUtensorMap& map_a, const CUtensorMap& map_w, in
   long long m_group = m_tiles;
   if ((long long)M * K * 2 > L2_SHARE && (long long)N * K * 2 <= L2_SHARE) m_group = PANEL_BYTES / ((long long)BM * K * 2);
   m_group = m_group < 1 ? 1 : (m_group > m_tiles ? m_tiles : m_group);
-  return dllm_launch_pdl(gemm_tcgen05_kernel<BN, EPI, DEEP, HD>, dim3(blocks), dim3(S::THREADS), S::SMEM, stream, map_a, map_w,
-                         c, M, N, K, status, rope, m_tiles, n_tiles, k_split, norm, (int)m_group);
+  constexpr bool MAY_PANEL = !DEEP && EPI <= EPI_QKV_ROPE;  // (a deep ring has a tile a block, transposed products few columns)
+  auto go = [&](auto kernel, std::atomic<unsigned long long>& allowed) -> int {
+    if (!dllm_allow_shared((const void*)kernel, (int)S::SMEM, allowed)) return DLLM_LAUNCH_FAILED;
+    return dllm_launch_pdl(kernel, dim3(blocks), dim3(S::THREADS), S::SMEM, stream, map_a, map_w, c, M, N, K, status, rope,
+                           m_tiles, n_tiles, k_split, norm, (int)m_group);
+  };
+  static std::atomic<unsigned long long> allowed[2];
+  if (MAY_PANEL && m_group < m_tiles) return go(gemm_tcgen05_kernel<BN, EPI, DEEP, HD, MAY_PANEL>, allowed[1]);
+  return go(gemm_tcgen05_kernel<BN, EPI, DEEP, HD, false>, allowed[0]);
 }
 
 int multiprocessors() {
