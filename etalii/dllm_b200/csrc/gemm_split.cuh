@@ -33,7 +33,6 @@ __global__ void __launch_bounds__(SplitShape::THREADS, SplitShape::BLOCKS_PER_SM
   const int split = (int)gridDim.x, rank = (int)blockIdx.x, n_tile = (int)blockIdx.y;
   const int m0 = (int)blockIdx.z * BM, n0 = n_tile * S::BN;
   const int k_tiles = (K + BK - 1) / BK, kt_begin = rank * k_tiles / split, kt_end = (rank + 1) * k_tiles / split;
-  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(&acc_full, 1);
@@ -44,6 +43,9 @@ __global__ void __launch_bounds__(SplitShape::THREADS, SplitShape::BLOCKS_PER_SM
   __syncthreads();
   fence_after_sync();
   const unsigned tmem_base = tmem_base_s;
+  // (only now: a block of the next kernel that came first to this multiprocessor's tensor memory would hold it until this
+  // grid has ended)
+  pdl_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
