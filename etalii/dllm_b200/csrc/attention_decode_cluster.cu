@@ -374,9 +374,10 @@ __device__ __forceinline__ void decode_attention(
 // to meet: no cluster barriers, no reads of the other blocks' memory. (The tiles are the same for every block of the cluster:
 // positions are not written while this kernel may run.) us before and now: 9 query and 3 kv heads of 64, one sequence of 80
 // keys 3.4 -> 2.7, of 200 3.5 -> 2.7, 64 of 200 6.0 -> 5.1; 32 and 8 heads of 128, one of 120 4.6 -> 3.7; 32 and 32 of 64, 100,
-// 100, 100 and 4,000 keys 17.4 -> 12.3. Only for up to four sequences (SOLO): in a batch of short and long ones the two bodies
+// 100, 100 and 4,000 keys 17.4 -> 12.3. Only for up to four sequences, one with heads above 64 (SOLO): in a batch of short and long ones the two bodies
 // side by side cost more than they give (135M shape, batch 8 of 128 to 2,048 67.4 ms a call without, 68.1 with, batch 64 112.0 and
-// 112.9; batch 1 28.6 and 27.6).
+// 112.9; batch 1 28.6 and 27.6; four prompts of 30 to 200, 20 tokens each, 11.3 with and 11.5 without; 8B shape, three of 20 to
+// 250, 10 tokens each, 41.4 with and 40.1 without).
 template <int HD, int CLUSTER, int WARPS, bool OPTIONS, bool SOLO>
 __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
     bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
@@ -469,7 +470,7 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     if (HD > 64 && shape == 0 && pairs <= 4 * places) shape = 1;
   }
 #define DLLM_GO(CL, WARPS) \
-  return (sequences <= 4 && CL > 1 ? launch<HD, CL, WARPS, OPTIONS, (CL > 1)> : launch<HD, CL, WARPS, OPTIONS, false>)( \
+  return (sequences <= (HD <= 64 ? 4 : 1) && CL > 1 ? launch<HD, CL, WARPS, OPTIONS, (CL > 1)> : launch<HD, CL, WARPS, OPTIONS, false>)( \
       out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
   switch (shape) {
     case 0: DLLM_GO(1, NW);
