@@ -56,9 +56,9 @@ __device__ __forceinline__ float remote_float(const float* local, unsigned rank)
 // CLUSTER blocks of WARPS warps serve one (sequence, kv head). Few (sequence, kv head) pairs: many blocks per pair
 // to fill the device and shorten every chain of pages; many pairs: one block per pair, no exchange between blocks.
 template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
-__device__ __forceinline__ void decode_attention(
-    bf16* __restrict__ out, const bf16* __restrict__ q, const KvLayout& cache, const int* __restrict__ tok_pos,
-    const int* __restrict__ slots, int heads, float scale_log2, int window, const ScoreOptions& options) {
+__global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
+    bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
+    const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
   constexpr int LD = HD + 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* kv_s = reinterpret_cast<bf16*>(smem_raw);        // per warp: K [64][LD], V [64][LD]
@@ -93,6 +93,14 @@ __device__ __forceinline__ void decode_attention(
   const KeyWalk walk(end - 1, end - 1, window, OPTIONS ? options.keep : 0, TILE_KEYS, chunk);
   auto key_of = [&](int it) { return OPTIONS ? walk.tile(it) * TILE_KEYS : base + it * TILE_KEYS; };
   const int tiles = OPTIONS ? walk.count : (end - base + TILE_KEYS - 1) / TILE_KEYS;
+  // A cluster whose sequence has no more tiles than one block has warps is that block: the others leave, and there is nobody
+  // to meet, so no cluster barriers and no reads of the other blocks' memory. (The tiles are the same for every block of the
+  // cluster: positions are not written while this kernel may run.) One body serves both, so that every batch has the choice and
+  // long contexts pay nothing for it. A decode step, us, without and with: 135M shape, 1 sequence of 100 keys 367 and 354, 4 417
+  // and 369, 16 686 and 540, 16 of 128 to 2,060 764 and 677, 8 of them 467 and 465. (As a second body beside this one it
+  // cost long contexts 3 to 5 %: 8B shape, one sequence of 500, 1,900 and 4,000 keys 2,825, 2,837 and 2,985, here 2,740, 2,760 and 2,854.)
+  const bool alone = CLUSTER > 1 && tiles <= WARPS;
+  if (alone && rank > 0) return;
   const ScoreCap score(scale_log2 / SCORE_LOG2E, OPTIONS ? options.cap : 0.f);
   const bool capped = OPTIONS && options.cap > 0.f;
   const float unit = capped ? 1.0f : scale_log2;  // what a score still has to be multiplied by
@@ -327,7 +335,7 @@ __device__ __forceinline__ void decode_attention(
       if (d == 0) { cta_ml[h][0] = m; cta_ml[h][1] = l; }
     }
     const int out_row = OPTIONS ? options.out_stride : heads * hd;
-    if (CLUSTER == 1) {
+    if (CLUSTER == 1 || alone) {
       __syncthreads();
       for (int idx = threadIdx.x; idx < nh * vd; idx += WARPS * 32) {
         int h = idx / vd, d = idx % vd, head = g * group + h0 + h;
@@ -365,35 +373,9 @@ __device__ __forceinline__ void decode_attention(
             __float2bfloat16_rn(OPTIONS ? o * sink_factor(m, l, options, head) : o / l);
       }
     }
-    if (CLUSTER > 1) cluster_sync();  // nobody leaves (or reuses the space) while others still read its partial result
+    if (CLUSTER > 1 && !alone) cluster_sync();  // nobody leaves (or reuses the space) while others still read its partial result
     else __syncthreads();
   }
-}
-
-// A cluster whose sequence has no more tiles than one block has warps is that block: the others leave, and there is nobody
-// to meet: no cluster barriers, no reads of the other blocks' memory. (The tiles are the same for every block of the cluster:
-// positions are not written while this kernel may run.) us before and now: 9 query and 3 kv heads of 64, one sequence of 80
-// keys 3.4 -> 2.7, of 200 3.5 -> 2.7, 64 of 200 6.0 -> 5.1; 32 and 8 heads of 128, one of 120 4.6 -> 3.7; 32 and 32 of 64, 100,
-// 100, 100 and 4,000 keys 17.4 -> 12.3. Only for up to four sequences, one with heads above 64 (SOLO): in a batch of short and long ones the two bodies
-// side by side cost more than they give (135M shape, batch 8 of 128 to 2,048 67.4 ms a call without, 68.1 with, batch 64 112.0 and
-// 112.9; batch 1 28.6 and 27.6; four prompts of 30 to 200, 20 tokens each, 11.3 with and 11.5 without; 8B shape, three of 20 to
-// 250, 10 tokens each, 41.4 with and 40.1 without).
-template <int HD, int CLUSTER, int WARPS, bool OPTIONS, bool SOLO>
-__global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
-    bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
-    const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
-  if (SOLO && CLUSTER > 1) {
-    int newest = tok_pos[blockIdx.z];
-    const int chunk = OPTIONS ? options.chunk : 0;
-    int tiles = OPTIONS ? KeyWalk(newest, newest, window, options.keep, TILE_KEYS, chunk).count
-                        : newest / TILE_KEYS - first_visible(newest, chunk, window) / TILE_KEYS + 1;
-    if (tiles <= WARPS) {
-      if (blockIdx.x == 0)
-        decode_attention<HD, 1, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, scale_log2, window, options);
-      return;
-    }
-  }
-  decode_attention<HD, CLUSTER, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, scale_log2, window, options);
 }
 
 template <int HD, int WARPS>
@@ -403,13 +385,13 @@ constexpr size_t block_smem() {
   return kv_bytes > red_bytes ? kv_bytes : red_bytes;
 }
 
-template <int HD, int CLUSTER, int WARPS, bool OPTIONS, bool SOLO>
+template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
 int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, const int* slots, int heads,
            int sequences, float scale, int window, const ScoreOptions& options, cudaStream_t stream) {
   constexpr size_t smem = block_smem<HD, WARPS>();
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS, SOLO>,
+    if (cudaFuncSetAttribute(decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return DLLM_LAUNCH_FAILED;
     configured = true;
@@ -428,7 +410,7 @@ int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, 
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&config, decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS, SOLO>, (bf16*)out, (const bf16*)q,
+  return cudaLaunchKernelEx(&config, decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS>, (bf16*)out, (const bf16*)q,
                             cache, tok_pos, slots, heads, scale * SCORE_LOG2E, window, options) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
@@ -470,8 +452,7 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     if (HD > 64 && shape == 0 && pairs <= 4 * places) shape = 1;
   }
 #define DLLM_GO(CL, WARPS) \
-  return (sequences <= (HD <= 64 ? 4 : 1) && CL > 1 ? launch<HD, CL, WARPS, OPTIONS, (CL > 1)> : launch<HD, CL, WARPS, OPTIONS, false>)( \
-      out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
+  return launch<HD, CL, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
   switch (shape) {
     case 0: DLLM_GO(1, NW);
     case 1: DLLM_GO(2, NW);

@@ -1077,6 +1077,40 @@ def test_attention_decode_cluster(heads, kv_heads, head_dim, window, lengths):
         assert torch.equal(again, out), shape
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,window", [(9, 3, 64, None), (4, 2, 32, None), (34, 2, 48, 150),
+                                                           (8, 1, 128, None), (6, 2, 80, 100)])
+@pytest.mark.parametrize("lengths", [[1], [64], [65], [128], [129], [256], [257], [1, 65, 129, 257], [100, 100, 100, 1900],
+                                     [1000, 30, 1 + 256, 2060, 128, 256, 700, 5]], ids=str)
+def test_attention_decode_cluster_where_some_sequences_are_one_blocks(heads, kv_heads, head_dim, window, lengths):
+    """Contexts of as many pages as a block has warps (two, or four) are one block's, which the others of the cluster leave to
+    it; a page more, and the cluster shares them. Both beside one another in a launch."""
+    cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, lengths, [1] * len(lengths), window)
+    q = _randn((len(lengths), heads * head_dim), torch.bfloat16, 9)
+    want = torch.zeros_like(q)
+    ops().attention_general(want, q, view, heads, 0.3, window or 0, batch)  # itself checked against the plain one
+    for shape in range(-1, ops().DECODE_CLUSTER_SHAPES):
+        out = torch.full_like(q, float("nan"))
+        ops().attention_decode_cluster(out, q, view, heads, 0.3, window or 0, batch, shape)
+        worst = (out.float() - want.float()).abs().max(dim=1).values
+        assert (worst <= 8e-3 * want.float().abs().max()).all(), (shape, worst.tolist())
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(6, 2, 64), (4, 1, 24), (8, 2, 128)])
+@pytest.mark.parametrize("window,keep,chunk", [(0, 0, 0), (70, 66, 0), (0, 0, 96)])
+@pytest.mark.parametrize("lengths", [[40], [129], [60, 130, 257, 900]], ids=str)
+def test_sink_attention_decode_where_some_sequences_are_one_blocks(heads, kv_heads, head_dim, window, keep, chunk, lengths):
+    """The same with capped scores, a sink, kept positions or chunks, against the general kernel (a warp a token and head)."""
+    cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, lengths, [1] * len(lengths))
+    q, sinks = _randn((len(lengths), heads * head_dim), torch.bfloat16, 9), _randn((heads,), torch.float32, 4)
+    want = torch.zeros_like(q)
+    ops().sink_attention(want, q, view, heads, 0.3, 9.0, sinks, window, keep, batch, chunk=chunk)
+    for shape in range(-1, ops().DECODE_CLUSTER_SHAPES):
+        out = torch.full_like(q, float("nan"))
+        ops().sink_attention_decode(out, q, view, heads, 0.3, 9.0, sinks, window, keep, batch, shape, chunk=chunk)
+        worst = (out.float() - want.float()).abs().max(dim=1).values
+        assert (worst <= 8e-3 * want.float().abs().max()).all(), (shape, worst.tolist())
+
+
 def test_attention_decode_cluster_finds_a_far_key():
     heads, kv_heads, hd = 4, 2, 32
     cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, hd, [700], [1])
