@@ -15,6 +15,7 @@
 namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int TILE_KEYS = 64;
+enum Start { START_AT_ONCE, START_BEHIND_WAIT, START_BEHIND_KEYS };  // when the next kernel may start (see launch_shape)
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -58,7 +59,7 @@ __device__ __forceinline__ float remote_float(const float* local, unsigned rank)
 template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
 __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
     bf16* __restrict__ out, const bf16* __restrict__ q, KvLayout cache, const int* __restrict__ tok_pos,
-    const int* __restrict__ slots, int heads, float scale_log2, int window, ScoreOptions options) {
+    const int* __restrict__ slots, int heads, float scale_log2, int window, Start when, ScoreOptions options) {
   constexpr int LD = HD + 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* kv_s = reinterpret_cast<bf16*>(smem_raw);        // per warp: K [64][LD], V [64][LD]
@@ -78,13 +79,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   auto values_of = [&](int page, int row) {
     return OPTIONS ? value_at(wide, page, g, row) : kv_offset(cache, page, 1, g, row);
   };
-  // When the next kernels may start. Started with this one they ask for their weights and wait, on the same multiprocessors
-  // and the same HBM, which costs this kernel more than it gives them; behind the keys they still start under its exchange.
-  // Whole calls, ms, at the start / here: 135M shape batch 1 27.5 / 26.9, 8 69.5 / 68.0, 64 115.5 / 113.0; 1.7B shape batch 8 with
-  // the same rule in the products (gemv.cu) 132.2 / 125.8. Not with heads of 128, where one sequence's attention leaves HBM to
-  // the next weights: 8B shape 93.8 / 94.4.
-  constexpr bool LATE = HD <= 64;
-  if (!LATE) pdl_launch_dependents();
+  if (when == START_AT_ONCE) pdl_launch_dependents();
   int end = tok_pos[b] + 1;    // positions and slots are written only by the step's last kernel
   const int chunk = OPTIONS ? options.chunk : 0;
   int first = first_visible(end - 1, chunk, window);
@@ -159,7 +154,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   int newest_tile = (newest / TILE_KEYS) * TILE_KEYS;
   bool owns_newest = tiles - 1 >= my_first && (tiles - 1 - my_first) % ROUND == 0;  // (it is in the walk's last tile)
   uint4 newest_k = make_uint4(0u, 0u, 0u, 0u), newest_v = newest_k;
+  if (when == START_BEHIND_WAIT && tiles > ROUND) pdl_launch_dependents();
   pdl_wait();
+  if (when == START_BEHIND_WAIT) pdl_launch_dependents();
   if (owns_newest) {
     int page = pages[newest / TILE_KEYS];
     int r = newest - newest_tile;
@@ -306,7 +303,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
       l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
     }
     __syncthreads();  // every warp is done with its keys and values: the space becomes the exchange buffer
-    if (LATE && h0 == 0) pdl_launch_dependents();
+    if (when == START_BEHIND_KEYS && h0 == 0) pdl_launch_dependents();
     if (tq == 0) {
       sm_ml[warp][gq][0] = m_run[0]; sm_ml[warp][gq][1] = l_run[0];
       sm_ml[warp][gq + 8][0] = m_run[1]; sm_ml[warp][gq + 8][1] = l_run[1];
@@ -387,7 +384,7 @@ constexpr size_t block_smem() {
 
 template <int HD, int CLUSTER, int WARPS, bool OPTIONS>
 int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, const int* slots, int heads,
-           int sequences, float scale, int window, const ScoreOptions& options, cudaStream_t stream) {
+           int sequences, float scale, int window, const ScoreOptions& options, Start when, cudaStream_t stream) {
   constexpr size_t smem = block_smem<HD, WARPS>();
   static bool configured = false;
   if (!configured) {
@@ -411,7 +408,7 @@ int launch(void* out, const void* q, const KvLayout& cache, const int* tok_pos, 
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&config, decode_attention_cluster_kernel<HD, CLUSTER, WARPS, OPTIONS>, (bf16*)out, (const bf16*)q,
-                            cache, tok_pos, slots, heads, scale * SCORE_LOG2E, window, options) == cudaSuccess
+                            cache, tok_pos, slots, heads, scale * SCORE_LOG2E, window, when, options) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
 }
@@ -451,8 +448,20 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     // 128 sequences 129.3 against 134.0)
     if (HD > 64 && shape == 0 && pairs <= 4 * places) shape = 1;
   }
+  // When the next kernel may start. Started with this one, it and those behind it ask for their weights and take places on the
+  // multiprocessors that read the keys; started behind the keys, its beginning is added to the step. In between lies its start
+  // behind this one's wait (or at once where one cluster's pages are several rounds): one kernel ahead, no more. Decode steps, us,
+  // at once / behind the wait / behind the keys: 135M shape (3 kv heads), one sequence of 1,900 keys 392 / 370 / 392, two 410 /
+  // 385 / 413, four 437 / 423 / 425, of 500 keys 416 / 420 / 410; eight of 500 437 / 437 / 417, of 1,900 454 / 443 / 437, of 128 to
+  // 2,060 473 / 464 / 465; sixteen of them 674 / 677 / 688; 33 957 / 960 / 944; 64 of 1,900 1,325 / 1,302 / 1,273. 1.7B shape (32 kv
+  // heads), one of 100 907 / 875 / 925, two of 128 to 2,100 1,099 / 1,088 / 1,098, four 1,214 / 1,197 / 1,163. So: behind the keys
+  // where pairs fill the device, and for five to eight sequences, whose small products (gemv.cu) start at once and would all
+  // come into the keys' way. Heads of 128: at once (8B shape: none of the three differs by 1 %).
+  Start when = START_BEHIND_WAIT;
+  if (HD > 64) when = START_AT_ONCE;
+  else if ((long long)sequences * cache.kv_heads >= 96 || (sequences > 4 && sequences <= 8)) when = START_BEHIND_KEYS;
 #define DLLM_GO(CL, WARPS) \
-  return launch<HD, CL, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, stream)
+  return launch<HD, CL, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, when, stream)
   switch (shape) {
     case 0: DLLM_GO(1, NW);
     case 1: DLLM_GO(2, NW);
