@@ -44,13 +44,15 @@ struct Early {
   }
 };
 
-constexpr long long LATE_FROM = 4ll << 20;  // bytes of W (see the kernel)
+// Bytes of W from which the next kernels do not start with a product (see the kernel). With 16 MB four layers of linear attention
+// and softmax, 2,048 wide, batch 8, take 30.5 ms a call, with 4 MB 29.9; 1.7B shape, batch 8, 132.7 with 32 MB, 132.2 with 64.
+constexpr long long LATE_FROM = 4ll << 20;
 
 template <int WARPS, int NT, int EPI, bool NORM, bool PIPE>
 __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, const void* __restrict__ a,
                                                           const float* __restrict__ norm_w, float eps,
                                                           const bf16* __restrict__ w, int M, int N, int K,
-                                                          RopeArgs rope, Prefetch pf, int items) {
+                                                          RopeArgs rope, Prefetch pf, int tiles) {
   // 32-value k steps whose loads a warp issues before the first product (fewer when more tokens need registers)
   constexpr int MAX_STEPS = NORM ? (NT == 1 ? 6 : (NT == 2 ? 3 : 1)) : (NT == 1 ? 8 : (NT == 2 ? 4 : 2));
   // exchange space of the warps: [WARPS][TILE][NT * 8 + 1] partial tiles, then [WARPS][NT * 8] sums of squares
@@ -83,13 +85,18 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
   }
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   Early<EPI, NT> early;
-  // A large W keeps HBM busy by itself: the next kernels, which would ask for theirs at once and wait, start when this
-  // block's share has been multiplied (1.7B shape, batch 8, with the same in the attention 132.2 -> 125.8 ms a call). From
-  // 4 MB on: with 32 and 64 MB 132.7 and 132.2; with 16 and 4 four layers of linear attention and softmax, 2,048 wide, take
-  // 30.5 and 29.9; without a limit the small products of the 135M shape, batch 8, lose what the early start gives them,
-  // 68.1 against 81.6.
-  const bool late = 2ll * N * K >= LATE_FROM;
-  if (!late) pdl_launch_dependents();
+  // When the next kernels may start: with this one, so that three or four of them wait with their first weights in registers
+  // (135M shape, 8 sequences of 500 keys, 420 us a decode step; 461 with the start behind the wait), but not where W is large and
+  // keeps HBM and the multiprocessors busy by itself. Up to eight rows it is then behind the wait: one kernel ahead. Behind the
+  // products, as with more rows, the next kernel's beginning is added to each of a layer's four products. Us a step, at once /
+  // behind the wait / behind the products: 1.7B shape, 1 sequence of 1,900 keys 1,056 / 1,013 / 1,082; 2 of 500 1,260 / 1,261 /
+  // 1,497, of 1,900 1,288 / 1,315 / 1,583; 4 of 1,900 1,352 / 1,268 / 1,327; 8 of 1,900 1,494 / 1,472 / 1,480; four layers of linear
+  // attention and softmax, 2,048 wide, 8 of 500 295 / 269 / 285. More rows: 8B shape, 16 of 100 4,720 / 4,722 / 3,980.
+  // `tiles`: the number of them, negative where that is so: a comparison of sizes in front of the start at once costs the small
+  // products 1 % of a step.
+  const bool large = NT == 1 ? tiles < 0 : 2ll * N * K >= LATE_FROM, late = NT > 1 && large;
+  const int items = NT == 1 ? abs(tiles) : tiles;
+  if (!large) pdl_launch_dependents();
   // A stretch is MAX_STEPS k steps. Every load of a stretch is issued before its first product. For long rows
   // (PIPE: a warp has more than one stretch) the weights of the NEXT stretch are requested before this stretch's
   // products start, so that the row streams without pauses.
@@ -113,6 +120,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
         if (!PIPE || !waited) {
           prefetch_share(pf);
           pdl_wait();  // the weights above are nobody's output; everything below may be the previous kernel's
+          if (NT == 1 && large) pdl_launch_dependents();
           waited = true;
         }
         early.load(c, tid, M, N, item, rope, paired, dim0);
@@ -344,7 +352,7 @@ int launch_one(int items, void* c, const void* a, const float* norm_w, float eps
   // costs more than the overlap brings)
   int blocks = (PIPE && items > resident) ? resident : items;
   return dllm_launch_pdl(gemv_kernel<WARPS, NT, EPI, NORM, PIPE>, dim3(blocks), dim3(WARPS * 32), smem, stream, c, a,
-                         norm_w, eps, w, M, N, K, rope, pf, items);
+                         norm_w, eps, w, M, N, K, rope, pf, NT == 1 && 2ll * N * K >= LATE_FROM ? -items : items);
 }
 
 template <int EPI, bool NORM>
