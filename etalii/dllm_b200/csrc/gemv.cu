@@ -96,7 +96,11 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
   // products 1 % of a step.
   const bool large = NT == 1 ? tiles < 0 : 2ll * N * K >= LATE_FROM, late = NT > 1 && large;
   const int items = NT == 1 ? abs(tiles) : tiles;
-  if (!large) pdl_launch_dependents();
+  // Nine to sixteen rows' small residual products stand between cluster products that start the next kernels at once
+  // (gemv_cluster.cu) and do that behind their wait themselves: 135M shape, us a step, at once / behind it: 12 sequences of 500
+  // keys 617 / 597, of 1,900 657 / 616, of 20 to 600 605 / 565; 16 of 500 749 / 696.
+  constexpr bool AHEAD = NT == 2 && EPI == EPI_RESIDUAL && !PIPE;
+  if (!large && !AHEAD) pdl_launch_dependents();
   // A stretch is MAX_STEPS k steps. Every load of a stretch is issued before its first product. For long rows
   // (PIPE: a warp has more than one stretch) the weights of the NEXT stretch are requested before this stretch's
   // products start, so that the row streams without pauses.
@@ -120,7 +124,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
         if (!PIPE || !waited) {
           prefetch_share(pf);
           pdl_wait();  // the weights above are nobody's output; everything below may be the previous kernel's
-          if (NT == 1 && large) pdl_launch_dependents();
+          if (NT == 1 ? large : AHEAD && !large) pdl_launch_dependents();
           waited = true;
         }
         early.load(c, tid, M, N, item, rope, paired, dim0);

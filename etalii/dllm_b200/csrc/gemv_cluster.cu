@@ -102,9 +102,16 @@ struct Unit {
   }
 };
 
+// When the next kernel may start: with this one, or (LATE) behind its wait: one kernel ahead, not three or four that wait on the
+// same multiprocessors. With 33 and more rows, and for W of 4 MB and more, that gains: decode steps, us, at once / behind the
+// wait, 135M shape, 33 sequences of 500 keys 863 / 853, 64 of 1,900 1,279 / 1,269; four layers of linear attention and softmax, 2,048
+// wide, 24 of 100 406 / 397. The small products of fewer rows lose more by it: 135M shape, 12 of 1,900 625 / 647, 16 of 128 to
+// 2,060 678 / 699, 24 of 100 630 / 642.
+constexpr long long LATE_FROM = 4ll << 20;  // bytes of W
+
 // NT: tiles of 8 tokens (the step has at most 8 NT rows). Launched as clusters of 1, 2, 4 or 8 blocks (at most 2 NT)
 // along x; cluster j owns the tiles ITEMS j .. ITEMS j + ITEMS - 1 of 16 rows of W.
-template <int NT, int EPI, bool NORM>
+template <int NT, int EPI, bool NORM, bool LATE>
 __global__ void __launch_bounds__(WARPS * 32) gemv_cluster_kernel(void* __restrict__ c, const void* __restrict__ a,
                                                                   const float* __restrict__ norm_w, float eps,
                                                                   const bf16* __restrict__ w, int M, int N, int K,
@@ -120,6 +127,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_cluster_kernel(void* __restri
   unsigned rank = cluster_rank(), blocks = cluster_size();
   int tokens_here = COLS / (int)blocks;  // tokens this block owns: rank * tokens_here ..
   int cluster = blockIdx.x / blocks;
+  if (!LATE) pdl_launch_dependents();
   cluster_arrive_relaxed();  // (every block of the cluster runs before anyone writes into its shared memory)
 
   const uint4* w_lo[ITEMS];
@@ -164,9 +172,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_cluster_kernel(void* __restri
   if (EPI == EPI_QKV_ROPE) prefetch_cache_pages(rope, M);
   prefetch_share(pf);
   pdl_wait();  // the weights are nobody's output; everything below may be the previous kernel's
-  // (one kernel ahead, not three: those behind the next one would wait on the same multiprocessors, 112.9 -> 112.3 ms a call
-  // of batch 64 of the 135M shape)
-  pdl_launch_dependents();
+  if (LATE) pdl_launch_dependents();
 
   // the owner's first two units (pair p fastest, then tile, then token: neighbouring threads store side by side)
   int units = ITEMS * 8 * tokens_here;
@@ -322,7 +328,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_cluster_kernel(void* __restri
 // at most eight blocks, no more than leaves every block four tokens to own, and no more than lets all clusters of
 // the launch run at the same time (measured, 64 x 3072 x 576 with the norm: 7.4 µs with two blocks, 192 in all,
 // 10.6 with four, 15.1 with eight).
-template <int NT, int EPI, bool NORM>
+template <int NT, int EPI, bool NORM, bool LATE>
 int launch_one(void* c, const void* a, const float* norm_w, float eps, const bf16* w, int M, int N, int K,
                const RopeArgs& rope, const Prefetch& pf, int asked, cudaStream_t stream) {
   constexpr int COLS = NT * 8, MOST = 2 * NT < 8 ? 2 * NT : 8;
@@ -330,13 +336,13 @@ int launch_one(void* c, const void* a, const float* norm_w, float eps, const bf1
   static int resident = 0;  // blocks of this kernel that fit on the device at once
   if (resident == 0) {
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(gemv_cluster_kernel<NT, EPI, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(gemv_cluster_kernel<NT, EPI, NORM, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return DLLM_LAUNCH_FAILED;
     int device = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemv_cluster_kernel<NT, EPI, NORM>, WARPS * 32,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemv_cluster_kernel<NT, EPI, NORM, LATE>, WARPS * 32,
                                                       smem) != cudaSuccess ||
         sms <= 0 || per_sm <= 0)
       return DLLM_LAUNCH_FAILED;
@@ -366,7 +372,7 @@ int launch_one(void* c, const void* a, const float* norm_w, float eps, const bf1
   attributes[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attributes;
   config.numAttrs = dllm_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&config, gemv_cluster_kernel<NT, EPI, NORM>, c, a, norm_w, eps, w, M, N, K, rope, pf,
+  return cudaLaunchKernelEx(&config, gemv_cluster_kernel<NT, EPI, NORM, LATE>, c, a, norm_w, eps, w, M, N, K, rope, pf,
                             items) == cudaSuccess
              ? DLLM_OK
              : DLLM_LAUNCH_FAILED;
@@ -375,9 +381,18 @@ int launch_one(void* c, const void* a, const float* norm_w, float eps, const bf1
 template <int EPI, bool NORM>
 int launch(void* c, const void* a, const float* norm_w, float eps, const bf16* w, int M, int N, int K,
            const RopeArgs& rope, const Prefetch& pf, int blocks, cudaStream_t stream) {
-  if (M <= 16) return launch_one<2, EPI, NORM>(c, a, norm_w, eps, w, M, N, K, rope, pf, blocks, stream);
-  if (M <= 32) return launch_one<4, EPI, NORM>(c, a, norm_w, eps, w, M, N, K, rope, pf, blocks, stream);
-  return launch_one<8, EPI, NORM>(c, a, norm_w, eps, w, M, N, K, rope, pf, blocks, stream);
+  const bool late = 2ll * N * K >= LATE_FROM;
+#define DLLM_GO(NT, LATE) return launch_one<NT, EPI, NORM, LATE>(c, a, norm_w, eps, w, M, N, K, rope, pf, blocks, stream)
+  if (M <= 16) {
+    if (late) DLLM_GO(2, true);
+    DLLM_GO(2, false);
+  }
+  if (M <= 32) {
+    if (late) DLLM_GO(4, true);
+    DLLM_GO(4, false);
+  }
+  DLLM_GO(8, true);
+#undef DLLM_GO
 }
 
 template <bool NORM>
