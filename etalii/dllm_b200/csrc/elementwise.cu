@@ -471,7 +471,7 @@ __global__ void rope_cache_kernel(const float* __restrict__ qkv, T* __restrict__
   }
 }
 
-// The same for heads whose length and rotated length are multiples of eight, 16-byte aligned: a thread moves eight values,
+// The same for whole products (partial results exist for up to 64 tokens) and heads whose length and rotated length are multiples of eight, 16-byte aligned: a thread moves eight values,
 // four pairs of the rotated ones (two 16-byte loads half a rotation apart) or eight neighbours of the others, and threads run
 // over tokens, heads and pieces without gaps. Bound by its bytes; the form above, a thread a value in blocks of one head,
 // loads both partners of every pair twice and page numbers once a value: 9 query and 3 kv heads of 64, 2,048 tokens 32.0 ->
@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(128) rope_cache_vector_kernel(const float* __r
                                                                 KvLayout cache, const float2* __restrict__ table,
                                                                 int rotary_dim, int heads, const int* __restrict__ tok_seq,
                                                                 const int* __restrict__ tok_pos,
-                                                                const int* __restrict__ slots, int written_heads, int parts,
-                                                                size_t part_stride, size_t pieces) {
+                                                                const int* __restrict__ slots, int written_heads,
+                                                                size_t pieces) {
   pdl_launch_dependents();
   pdl_wait();
   size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -508,14 +508,7 @@ __global__ void __launch_bounds__(128) rope_cache_vector_kernel(const float* __r
     dst = (T*)cache.base + kv_offset(cache, page, which, h - heads - which * nkv, pos % cache.page_size);
   }
   const float* src = qkv + ((size_t)t * (heads + 2 * nkv) + h) * hd;
-  auto value = [&](unsigned i) {
-    float4 sum = *reinterpret_cast<const float4*>(src + i);
-    for (int p = 1; p < parts; ++p) {
-      float4 v = *reinterpret_cast<const float4*>(src + (size_t)p * part_stride + i);
-      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-    }
-    return sum;
-  };
+  auto value = [&](unsigned i) { return *reinterpret_cast<const float4*>(src + i); };
   unsigned half = rotary_dim / 2;
   if (table != nullptr && h < heads + nkv && 4 * u < half) {
     float4 a = value(4 * u), b = value(half + 4 * u);
@@ -542,7 +535,7 @@ DLLM_EXPORT int dllm_rope_cache_write(const float* qkv, void* q_out, void* cache
       parts < 1 || part_stride < 0)
     return DLLM_BAD_ARGUMENT;
   KvLayout cache{cache_base, page_table, max_pages, page_size, kv_heads, head_dim};
-  const bool vector = tokens > 64 && head_dim % 8 == 0 && (table == nullptr || rotary_dim % 8 == 0) && (part_stride & 3) == 0 &&
+  const bool vector = tokens > 64 && parts == 1 && head_dim % 8 == 0 && (table == nullptr || rotary_dim % 8 == 0) &&
                       !(((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)cache_base | (uintptr_t)table) & 15);
   if (vector && (dtype == DLLM_F32 || dtype == DLLM_BF16)) {
     int written_heads = write_cache ? heads + 2 * kv_heads : heads;
@@ -552,10 +545,10 @@ DLLM_EXPORT int dllm_rope_cache_write(const float* qkv, void* q_out, void* cache
       if (dtype == DLLM_F32)
         return dllm_launch_pdl(rope_cache_vector_kernel<float>, dim3((unsigned)blocks), dim3(128), 0, stream, qkv,
                                (float*)q_out, cache, (const float2*)table, rotated, heads, tok_seq, tok_pos, slots,
-                               written_heads, parts, (size_t)part_stride, pieces);
+                               written_heads, pieces);
       return dllm_launch_pdl(rope_cache_vector_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(128), 0, stream, qkv,
                              (__nv_bfloat16*)q_out, cache, (const float2*)table, rotated, heads, tok_seq, tok_pos, slots,
-                             written_heads, parts, (size_t)part_stride, pieces);
+                             written_heads, pieces);
     }
   }
   dim3 grid(tokens, heads + 2 * kv_heads);
