@@ -14,7 +14,7 @@
 // its reduction cut into stretches: a block's work items are (tile, stretch) pairs and every stretch stores its own
 // partial result, which a second kernel sums in order (for a W with fewer tiles than the device has multiprocessors).
 // Rows of A beyond M and columns of K beyond the matrix are zero-filled by TMA; rows of W beyond N give columns
-// that are never stored. No multicast, no clusters. Every wait on an mbarrier is bounded: after the limit the role
+// that are never stored. No multicast. Every wait on an mbarrier is bounded: after the limit the role
 // records a status word and leaves, the block still frees its tensor memory, and the host raises.
 #include "gemm_common.cuh"
 #include "tcgen05.cuh"
@@ -76,7 +76,7 @@ __device__ __forceinline__ WorkItem work_item(int item, int total, int k_tiles, 
 // column of W's tiles, until the panel has met all of W; the next panel follows. The host makes a panel as many rows as
 // stay in L2 (`launch`), so that A comes from HBM once however many columns of tiles read it.
 struct TilePlace { int m, n; };
-// (Kernels of their own: the choice at run time cost every product 0.2 us, 122 of them a 2,048-token prompt.)
+// (Kernels of their own: the choice at run time cost every product 0.15 us, 122 of them a 2,048-token prompt.)
 template <bool PANELS>
 __device__ __forceinline__ TilePlace tile_place(int tile, int m_tiles, int n_tiles, int m_group) {
   if (!PANELS) return TilePlace{tile % m_tiles, tile / m_tiles};
@@ -653,6 +653,13 @@ static int gemm_entry(void* c, const void* a, const void* w, int M, int N, int K
   }
 }
 
+// How many blocks of a cluster share a tile's reduction in the product of these sizes (0: none, it is not cut; see gemm_split.cuh)
+// with one of the epilogues 0..4, where the caller leaves the tile to this file.
+DLLM_EXPORT int dllm_gemm_tcgen05_stretches(int M, int N, int K, int epilogue) {
+  if (M <= 0 || N <= 0 || K <= 0 || epilogue < 0 || epilogue > EPI_QKV_ROPE) return 0;
+  return epilogue == EPI_QKV_ROPE ? split_stretches<EPI_QKV_ROPE>(M, N, K) : split_stretches<EPI_STORE_T>(M, N, K);
+}
+
 DLLM_EXPORT int dllm_gemm_tcgen05(void* c, const void* a, const void* w, int M, int N, int K, int epilogue, int tile_n,
                                   int* status, cudaStream_t stream) {
   return gemm_entry(c, a, w, M, N, K, epilogue, tile_n, status, stream, NormArgs{}, nullptr);
@@ -685,7 +692,7 @@ DLLM_EXPORT int dllm_gemm_tcgen05_normed(void* c, const void* a, const void* w, 
 
 // x[M,N] (float32) += A W^T, and for the norm that reads x next: copy_out[M,N] = bfloat16(new x) and
 // ssq_out[tile][m] = the sum of the squares of row m's new values in column tile `tile`; *parts_out = the number of
-// parts, two a column tile (what the reader passes as parts_in). N must be a multiple of 16; ssq_out holds
+// parts, one or two a column tile by its width (what the reader passes as parts_in). N must be a multiple of 16; ssq_out holds
 // M * ceil(N / 16) floats at least.
 DLLM_EXPORT int dllm_gemm_tcgen05_residual_norm(void* x, void* copy_out, float* ssq_out, int* parts_out, const void* a,
                                                 const void* w, int M, int N, int K, int* status,

@@ -202,6 +202,7 @@ _prototypes = {
     ("gemm_bf16", "dllm_gemm_bf16"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     ("gemm_tcgen05", "dllm_gemm_tcgen05"): [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                             c_void_p],
+    ("gemm_tcgen05", "dllm_gemm_tcgen05_stretches"): [c_int, c_int, c_int, c_int],
     ("gemm_tcgen05", "dllm_gemm_tcgen05_qkv_rope"): [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                                      c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                                      c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
@@ -2039,8 +2040,8 @@ def gemm_normed(c: torch.Tensor, a: torch.Tensor, w: torch.Tensor, epilogue: int
 
 def gemm_residual_norm(x: torch.Tensor, copy: torch.Tensor, ssq: torch.Tensor, a: torch.Tensor,
                        w: torch.Tensor) -> int:
-    """x (float32) += a @ w^T; copy = bfloat16(new x); ssq[tile, row] = the sum of the squares of the new values of
-    the row in each half tile of columns. Returns the number of parts (the reader's `parts`). N a multiple of 16."""
+    """x (float32) += a @ w^T; copy = bfloat16(new x); ssq[part, row] = the sum of the squares of the new values of
+    the row in each tile or half tile of columns. Returns the number of parts (the reader's `parts`). N a multiple of 16."""
     _cuda(x, copy, ssq, a, w)
     m, k = a.shape
     n = w.shape[0]
@@ -2051,6 +2052,11 @@ def gemm_residual_norm(x: torch.Tensor, copy: torch.Tensor, ssq: torch.Tensor, a
         x.data_ptr(), copy.data_ptr(), ssq.data_ptr(), ctypes.addressof(parts), a.data_ptr(), w.data_ptr(), m, n, k,
         _status_word().data_ptr(), _stream()), "gemm_residual_norm", lambda: f"M={m} N={n} (multiple of 16) K={k}")
     return parts.value
+
+
+def gemm_stretches(rows: int, outputs: int, inner: int, epilogue: int = EPI_RESIDUAL) -> int:
+    """How many blocks of a cluster share a tile's reduction in the tile product of these sizes (0: it is not cut)."""
+    return _fn("gemm_tcgen05", "dllm_gemm_tcgen05_stretches")(int(rows), int(outputs), int(inner), int(epilogue))
 
 
 def gemm_qkv_rope_supported(cache, rotary_dim: int, has_table: bool) -> bool:
@@ -2075,11 +2081,9 @@ def table_by_pair(table: torch.Tensor) -> torch.Tensor:
 
 
 def gemm_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, table: torch.Tensor | None,
-                  rotary_dim: int, heads: int, batch, write_cache: bool = True,
-                  ssq: torch.Tensor | None = None, parts: int = 1, eps: float = 0.0) -> None:
+                  rotary_dim: int, heads: int, batch, write_cache: bool = True) -> None:
     """The q/k/v projection of a prefill-sized step in the tcgen05 tile kernel, ending in the rotation of q and k and
-    the write of k and v into the paged cache (no float32 q/k/v in memory, no separate rotation kernel). With `ssq`
-    [parts, tokens] the rows of `a` are un-normed and every row of the product is scaled as in `gemm_normed`."""
+    the write of k and v into the paged cache (no float32 q/k/v in memory, no separate rotation kernel)."""
     _cuda(a, w, q_out, table)
     m, k = batch.n_tokens, a.shape[1]
     assert gemm_qkv_rope_supported(cache, rotary_dim, table is not None)
@@ -2089,15 +2093,13 @@ def gemm_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, 
         assert table.dtype == torch.float32 and table.shape[0] > batch.max_position, "position beyond the table"
         assert table.shape[1] == rotary_dim // 2 and table.shape[2] == 2
     by_pair = table_by_pair(table) if table is not None else None  # (the layout this kernel reads)
-    name = "dllm_gemm_tcgen05_qkv_rope" + ("" if ssq is None else "_normed")
-    norm = () if ssq is None else (ssq.data_ptr(), int(parts), float(eps))
-    _check(_fn("gemm_tcgen05", name)(
+    _check(_fn("gemm_tcgen05", "dllm_gemm_tcgen05_qkv_rope")(
         a.data_ptr(), w.data_ptr(), m, k, q_out.data_ptr(), cache.base_ptr, cache.page_table.data_ptr(),
         cache.max_pages, cache.page_size, heads, cache.kv_heads, cache.head_dim,
         by_pair.data_ptr() if by_pair is not None else None, rotary_dim if table is not None else 0,
         table.shape[0] if table is not None else 0,
         batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(), batch.slots.data_ptr(), 1 if write_cache else 0,
-        *norm, _status_word().data_ptr(), _stream()), "gemm_qkv_rope", lambda: f"M={m} K={k} head_dim={cache.head_dim}")
+        _status_word().data_ptr(), _stream()), "gemm_qkv_rope", lambda: f"M={m} K={k} head_dim={cache.head_dim}")
 
 
 def gemv_qkv_rope(a: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, cache, table: torch.Tensor | None,

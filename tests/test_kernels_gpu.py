@@ -1311,14 +1311,14 @@ def test_tile_products_with_the_norm_folded_around_them(m, hidden, inner, output
     ops().raise_if_failed()
 
 
-@pytest.mark.parametrize("m,hidden,inner", [
-    (4225, 576, 136),    # one round of 192-wide tiles, the last one a single row
-    (12400, 192, 64),    # the width of one tile, one stage of the ring
-    (4100, 640, 320),    # no multiple of 192: more 64-wide tiles than blocks, the rows staged behind the ring
-    (66001, 384, 520),   # A outgrows its share of L2: panels of rows, the last one shorter; blocks with several tiles
-    (33000, 256, 1032),  # the same with 256-wide tiles
+@pytest.mark.parametrize("m,hidden,inner,tile", [
+    (4225, 576, 136, 192),    # one round of 192-wide tiles, the last one a single row
+    (12700, 192, 64, 192),    # the width of one tile, one stage of the ring
+    (4100, 640, 320, 64),     # no multiple of 192: more 64-wide tiles than blocks, the rows staged behind the ring
+    (66001, 384, 520, 192),   # A outgrows its share of L2: panels of rows, the last one shorter; blocks with several tiles
+    (33000, 512, 1032, 256),  # the same with 256-wide tiles
 ])
-def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner):
+def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner, tile):
     """The product that writes the residual, its copy and its sums of squares against float64 (float32 sums of `inner`
     products of values around 0.05)."""
     x0, a = _randn((m, hidden), torch.float32, 1, 2.0), _randn((m, inner), torch.bfloat16, 2)
@@ -1327,6 +1327,7 @@ def test_residual_tiles_of_192_columns_and_panels_of_rows(m, hidden, inner):
     copy = torch.full((m, hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
     ssq = torch.full((m * (-(-hidden // 16)),), float("nan"), dtype=torch.float32, device=DEV)
     parts = ops().gemm_residual_norm(x, copy, ssq, a, w)
+    assert parts == -(-hidden // tile) * (2 if tile >= 128 else 1)  # (the premise: these tiles)
     ops().gemm(plain, a, w, ops().EPI_RESIDUAL, kernel=3)
     ops().raise_if_failed()
     want = x0.double() + a.double() @ w.double().T
@@ -1386,13 +1387,15 @@ def test_scans_with_two_columns_a_lane(dim, vdim, heads, lengths):
         assert rel_error(state.cpu(), want_state.cpu()) <= 2e-6, delta
 
 
-@pytest.mark.parametrize("m,n,k", [
-    (65, 4100, 1032),    # a last tile of four columns, a last k tile of eight values
-    (128, 2048, 2048), (129, 2064, 2056), (256, 1024, 4104),  # one and two tiles of rows, clusters of up to eight
-    (200, 20480, 1032),  # as many tiles as the device takes at once: nothing is cut
+@pytest.mark.parametrize("m,n,k,stretches", [
+    (65, 4100, 1032, 8),    # a last tile of four columns, a last k tile of eight values
+    (128, 2048, 2048, 8), (129, 2064, 2056, 8), (256, 1024, 4104, 8),  # one and two tiles of rows
+    (100, 9000, 1032, 4), (256, 9028, 1032, 2),
+    (200, 10244, 1032, 1),  # as many tiles as the device takes at once: nothing is cut
 ])
 @pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
-def test_products_of_a_few_hundred_rows_cut_over_a_cluster(m, n, k, epilogue):
+def test_products_of_a_few_hundred_rows_cut_over_a_cluster(m, n, k, stretches, epilogue):
+    assert ops().gemm_stretches(m, n, k, epilogue) == stretches  # (the premise)
     test_gemm_tcgen05(m, n, k, epilogue, 0)
 
 
@@ -1401,42 +1404,101 @@ def test_products_of_a_few_hundred_rows_cut_over_a_cluster(m, n, k, epilogue):
     (512, 576, 1536, 256), (300, 1088, 1032, 6404), (1536, 320, 1096, 256),  # up to twelve tiles of rows
 ])
 def test_cut_products_with_the_norm_folded_around_them(m, hidden, inner, outputs):
+    assert ops().gemm_stretches(m, hidden, inner) > 1  # (the premise)
     test_tile_products_with_the_norm_folded_around_them(m, hidden, inner, outputs)
 
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim,rotary,k,new", [
-    (21, 6, 64, 64, 2056, [60, 70, 1, 9]), (29, 3, 64, 0, 2056, [200, 56]), (13, 2, 128, 128, 2056, [64, 1]),
-    (9, 3, 64, 64, 1032, [1] * 70), (5, 1, 128, 128, 1096, [500, 9])])
+    (9, 3, 64, 64, 1032, [1] * 70), (29, 3, 64, 0, 2056, [60, 40]), (13, 2, 128, 0, 1096, [64, 1]),  # one tile of rows
+    (21, 6, 64, 64, 4104, [60, 60, 1, 8]), (13, 2, 128, 128, 4096, [1, 256]), (5, 1, 128, 128, 4104, [375, 9]),
+    (27, 4, 64, 64, 4096, [300]), (5, 1, 64, 0, 5000, [255, 2])])  # two and three, the last one of a row
 def test_cut_qkv_rope(heads, kv_heads, head_dim, rotary, k, new):
     """The q/k/v product cut over a cluster with a norm's factor of one: its rotation and cache rows."""
+    module = ops()
     lengths = [c + 30 * i for i, c in enumerate(new)]
     cache, view, batch = _cache_and_batch(torch.bfloat16, kv_heads, head_dim, lengths, new)
-    n = batch.n_tokens
-    table = None
+    n, outputs = batch.n_tokens, (heads + 2 * kv_heads) * head_dim
+    assert module.gemm_stretches(n, outputs, k, 4) > 0  # (the premise: this product, and not the one of the other tests)
+    table, by_pair = None, None
     if rotary:
         angles = torch.arange(2560, dtype=torch.float64)[:, None] * torch.rand(rotary // 2, dtype=torch.float64)[None]
         table = torch.stack([angles.cos(), angles.sin()], -1).float().to(DEV)
-    w = _randn(((heads + 2 * kv_heads) * head_dim, k), torch.bfloat16, 4, 0.05)
+        by_pair = module.table_by_pair(table)
+    w = _randn((outputs, k), torch.bfloat16, 4, 0.05)
     x = _randn((n, k), torch.bfloat16, 6)
     q = torch.zeros((n, heads * head_dim), dtype=torch.bfloat16, device=DEV)
     before = view.storage.clone()
     ssq = torch.full((n,), float(k), dtype=torch.float32, device=DEV)
-    for write in (True, False):
-        target = torch.zeros_like(q)
-        ops().gemm_qkv_rope(x, w, target, view, table, rotary, heads, batch, write, ssq=ssq, parts=1, eps=0.0)
-        ops().raise_if_failed()
-        if write:
-            q, written = target, view.storage.clone()
-    assert torch.equal(target, q) and torch.equal(view.storage, written)
-    qkv = (x.double() @ w.double().T).float().cpu()
-    ref_view = type(view)(before.cpu().clone(), view.page_table.cpu(), view.page_size, kv_heads, head_dim, None)
-    ref_q = torch.zeros((n, heads * head_dim), dtype=torch.bfloat16)
-    cpu_batch = type("B", (), {"n_tokens": n, "tok_pos": batch.tok_pos.cpu(), "tok_seq": batch.tok_seq.cpu(),
-                               "slots": batch.slots.cpu()})
-    PK.rope_cache_write(qkv, ref_q, ref_view, table.cpu() if rotary else None, rotary, heads, cpu_batch, True)
-    assert rel_error(q.float().cpu(), ref_q.float()) <= 8e-3
-    assert rel_error(written.float().cpu(), ref_view.storage.float()) <= 8e-3
-    assert (written != before).any(dim=-1).sum().item() <= n * kv_heads * 2
+    for normed in (True, False):
+        view.storage.copy_(before)
+        for write in (True, False):
+            target = torch.zeros_like(q)
+            if normed:  # (the entry point of the launches that the C++ side issues)
+                assert module._fn("gemm_tcgen05", "dllm_gemm_tcgen05_qkv_rope_normed")(
+                    x.data_ptr(), w.data_ptr(), n, k, target.data_ptr(), view.base_ptr, view.page_table.data_ptr(),
+                    view.max_pages, view.page_size, heads, kv_heads, head_dim, by_pair.data_ptr() if rotary else None,
+                    rotary, 2560 if rotary else 0, batch.tok_seq.data_ptr(), batch.tok_pos.data_ptr(),
+                    batch.slots.data_ptr(), int(write), ssq.data_ptr(), 1, 0.0, module._status_word().data_ptr(),
+                    module._stream()) == 0
+            else:
+                module.gemm_qkv_rope(x, w, target, view, table, rotary, heads, batch, write)
+            torch.cuda.synchronize()
+            module.raise_if_failed()
+            if write:
+                q, written = target, view.storage.clone()
+        assert torch.equal(target, q) and torch.equal(view.storage, written)
+        qkv = (x.double() @ w.double().T).float().cpu()
+        ref_view = type(view)(before.cpu().clone(), view.page_table.cpu(), view.page_size, kv_heads, head_dim, None)
+        ref_q = torch.zeros((n, heads * head_dim), dtype=torch.bfloat16)
+        cpu_batch = type("B", (), {"n_tokens": n, "tok_pos": batch.tok_pos.cpu(), "tok_seq": batch.tok_seq.cpu(),
+                                   "slots": batch.slots.cpu()})
+        PK.rope_cache_write(qkv, ref_q, ref_view, table.cpu() if rotary else None, rotary, heads, cpu_batch, True)
+        assert rel_error(q.float().cpu(), ref_q.float()) <= 8e-3
+        assert rel_error(written.float().cpu(), ref_view.storage.float()) <= 8e-3
+        assert (written != before).any(dim=-1).sum().item() <= n * kv_heads * 2
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,window", [(9, 3, 64, 0), (8, 2, 128, 0), (4, 2, 32, 300), (9, 3, 64, 200)])
+def test_float32_single_tokens_behind_a_producer_that_still_runs(heads, kv_heads, head_dim, window):
+    """Product, rotation with cache write, and attention one behind the other with nobody waiting, twelve times with other
+    activations: the attention starts while the kernels in front run, copies the rows of earlier steps meanwhile, and must
+    find this step's query and newest row. The same bits as with a wait behind every kernel, and as the general kernel's."""
+    module, width = ops(), 576
+    lengths = [330, 700, 64 * 9 + 1, 1290]
+    cache, view, batch = _cache_and_batch(torch.float32, kv_heads, head_dim, lengths, [1] * 4, window or None)
+    outputs = (heads + 2 * kv_heads) * head_dim
+    w = _randn((outputs, width), torch.float32, 4, 0.05)
+    x = [_randn((4, width), torch.float32, 10 + i) for i in range(12)]
+    angles = torch.arange(2560, dtype=torch.float64)[:, None] * torch.rand(head_dim // 2, dtype=torch.float64)[None]
+    table = torch.stack([angles.cos(), angles.sin()], -1).float().to(DEV)
+
+    def chain(wait):
+        outs, general = [], []
+        for rows in x:
+            qkv = torch.empty((4, outputs), dtype=torch.float32, device=DEV)
+            q, out = (torch.full((4, heads * head_dim), float("nan"), device=DEV) for _ in range(2))
+            pause = torch.cuda.synchronize if wait else lambda: None
+            pause()
+            module.gemm(qkv, rows, w, module.EPI_STORE_F32)
+            pause()
+            module.rope_cache_write(qkv, q, view, table, head_dim, heads, batch, True)
+            pause()
+            module.attention_blocks(out, q, view, heads, 0.3, window, batch)
+            pause()
+            outs.append(out)
+            if wait:
+                general.append(torch.empty_like(out))
+                module.attention_general(general[-1], q, view, heads, 0.3, window, batch)
+        torch.cuda.synchronize()
+        module.raise_if_failed()
+        return outs, general
+
+    chain(False)  # (the first round builds kernels and sizes buffers)
+    flowing, _ = chain(False)
+    want, general = chain(True)
+    for got, stepwise, warp in zip(flowing, want, general):
+        assert torch.equal(got, stepwise) and torch.equal(got, warp)
+    assert not torch.equal(want[0], want[1])
 
 
 @pytest.mark.parametrize("rows", [4, 20, 40, 80])  # eight blocks a row, four, two, one
