@@ -529,7 +529,8 @@ int launch_shape(void* c, const CUtensorMap& map_a, const CUtensorMap& map_w, in
   long long m_group = m_tiles;
   if ((long long)M * K * 2 > L2_SHARE && (long long)N * K * 2 <= L2_SHARE) m_group = PANEL_BYTES / ((long long)BM * K * 2);
   m_group = m_group < 1 ? 1 : (m_group > m_tiles ? m_tiles : m_group);
-  constexpr bool MAY_PANEL = !DEEP && EPI <= EPI_QKV_ROPE;  // (a deep ring has a tile a block, transposed products few columns)
+  // (a deep ring has a tile a block, transposed products have few columns, 32-wide tiles few rows)
+  constexpr bool MAY_PANEL = !DEEP && BN > 32 && EPI <= EPI_QKV_ROPE;
   auto go = [&](auto kernel, std::atomic<unsigned long long>& allowed) -> int {
     if (!dllm_allow_shared((const void*)kernel, (int)S::SMEM, allowed)) return DLLM_LAUNCH_FAILED;
     return dllm_launch_pdl(kernel, dim3(blocks), dim3(S::THREADS), S::SMEM, stream, map_a, map_w, c, M, N, K, status, rope,
