@@ -44,9 +44,12 @@ struct Early {
   }
 };
 
-// Bytes of W from which the next kernels do not start with a product (see the kernel). With 16 MB four layers of linear attention
-// and softmax, 2,048 wide, batch 8, take 30.5 ms a call, with 4 MB 29.9; 1.7B shape, batch 8, 132.7 with 32 MB, 132.2 with 64.
-constexpr long long LATE_FROM = 4ll << 20;
+// From how many bytes of W on the next kernels do not start with a product (see the kernel): up to eight rows (and rows of W of
+// 2,048 values and more), and with more. Up to eight, us a step: four Llama layers 1,024 wide (products of 2 to 11 MB) with 4 MB, with
+// 8 MB, and here: 2 sequences 102, 100, 100, 6 of 500 keys 109, 109, 108; four of softmax beside linear attention, 1,024 wide, one
+// of 1,500 138, 140, 136; 2,048 wide (8 to 46 MB), 8 of 500, with 16 MB and here 254 and 237. With more: four layers of linear attention
+// and softmax, 2,048 wide, 30.5 ms a call with 16 MB, 29.9 with 4.
+constexpr long long AHEAD_FROM = 8ll << 20, LATE_FROM = 4ll << 20;
 
 template <int WARPS, int NT, int EPI, bool NORM, bool PIPE>
 __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, const void* __restrict__ a,
@@ -356,7 +359,7 @@ int launch_one(int items, void* c, const void* a, const float* norm_w, float eps
   // costs more than the overlap brings)
   int blocks = (PIPE && items > resident) ? resident : items;
   return dllm_launch_pdl(gemv_kernel<WARPS, NT, EPI, NORM, PIPE>, dim3(blocks), dim3(WARPS * 32), smem, stream, c, a,
-                         norm_w, eps, w, M, N, K, rope, pf, NT == 1 && 2ll * N * K >= LATE_FROM ? -items : items);
+                         norm_w, eps, w, M, N, K, rope, pf, NT == 1 && K >= 2048 && 2ll * N * K >= AHEAD_FROM ? -items : items);
 }
 
 template <int EPI, bool NORM>

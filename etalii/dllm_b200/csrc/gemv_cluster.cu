@@ -103,11 +103,11 @@ struct Unit {
 };
 
 // When the next kernel may start: with this one, or (LATE) behind its wait: one kernel ahead, not three or four that wait on the
-// same multiprocessors. With 33 and more rows, and for W of 4 MB and more, that gains: decode steps, us, at once / behind the
-// wait, 135M shape, 33 sequences of 500 keys 863 / 853, 64 of 1,900 1,279 / 1,269; four layers of linear attention and softmax, 2,048
-// wide, 24 of 100 406 / 397. The small products of fewer rows lose more by it: 135M shape, 12 of 1,900 625 / 647, 16 of 128 to
-// 2,060 678 / 699, 24 of 100 630 / 642.
-constexpr long long LATE_FROM = 4ll << 20;  // bytes of W
+// same multiprocessors. With 33 and more rows, and for large W, that gains. Decode steps, us, at once / behind the wait: 135M
+// shape, 33 sequences of 500 keys 863 / 853, 64 of 1,900 1,279 / 1,269; four layers of linear attention and softmax, 2,048 wide,
+// 24 of 100 406 / 397. The small products of fewer rows lose more by it: 135M shape, 12 of 1,900 625 / 647, 16 of 128 to 2,060
+// 678 / 699. From 4 MB on up to 16 rows, from 2 MB on behind them: 135M shape (products of 1 to 3.5 MB), us with 4 and 2 MB, 12 of
+// 500 604 / 623, 16 of 1,900 748 / 779, 24 of 1,900 862 / 856, 28 of 128 to 2,060 916 / 903, 32 of them 801 / 796.
 
 // NT: tiles of 8 tokens (the step has at most 8 NT rows). Launched as clusters of 1, 2, 4 or 8 blocks (at most 2 NT)
 // along x; cluster j owns the tiles ITEMS j .. ITEMS j + ITEMS - 1 of 16 rows of W.
@@ -381,7 +381,7 @@ int launch_one(void* c, const void* a, const float* norm_w, float eps, const bf1
 template <int EPI, bool NORM>
 int launch(void* c, const void* a, const float* norm_w, float eps, const bf16* w, int M, int N, int K,
            const RopeArgs& rope, const Prefetch& pf, int blocks, cudaStream_t stream) {
-  const bool late = 2ll * N * K >= LATE_FROM;
+  const bool late = 2ll * N * K >= (M <= 16 ? 4ll << 20 : 2ll << 20);  // (see the kernel)
 #define DLLM_GO(NT, LATE) return launch_one<NT, EPI, NORM, LATE>(c, a, norm_w, eps, w, M, N, K, rope, pf, blocks, stream)
   if (M <= 16) {
     if (late) DLLM_GO(2, true);
