@@ -97,7 +97,11 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
   // attention and softmax, 2,048 wide, 8 of 500 295 / 269 / 285. More rows: 8B shape, 16 of 100 4,720 / 4,722 / 3,980.
   // `tiles`: the number of them, negative where that is so: a comparison of sizes in front of the start at once costs the small
   // products 1 % of a step.
-  const bool large = NT == 1 ? tiles < 0 : 2ll * N * K >= LATE_FROM, late = NT > 1 && large;
+  // The q/k/v product of up to eight sequences whose attention has 256 and more pairs of a sequence and a kv head keeps the start
+  // behind its products: that attention takes the whole device as soon as it may, and its pages the HBM. 1.7B shape, us a step,
+  // behind the wait / here: 8 of 512 to 4,096 keys 1,719 / 1,635, of 4,000 2,038 / 1,959, of 1,000 1,230 / 1,244.
+  const bool large = NT == 1 ? tiles < 0 : 2ll * N * K >= LATE_FROM;
+  const bool late = large && (NT > 1 || (EPI == EPI_QKV_ROPE && M * rope.cache.kv_heads >= 256));
   const int items = NT == 1 ? abs(tiles) : tiles;
   // Nine to sixteen rows' small residual products stand between cluster products that start the next kernels at once
   // (gemv_cluster.cu) and do that behind their wait themselves: 135M shape, us a step, at once / behind it: 12 sequences of 500
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_kernel(void* __restrict__ c, 
         if (!PIPE || !waited) {
           prefetch_share(pf);
           pdl_wait();  // the weights above are nobody's output; everything below may be the previous kernel's
-          if (NT == 1 ? large : AHEAD && !large) pdl_launch_dependents();
+          if (NT == 1 ? large && !late : AHEAD && !large) pdl_launch_dependents();
           waited = true;
         }
         early.load(c, tid, M, N, item, rope, paired, dim0);
