@@ -15,7 +15,8 @@
 namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int TILE_KEYS = 64;
-enum Start { START_AT_ONCE, START_BEHIND_WAIT, START_BEHIND_KEYS };  // when the next kernel may start (see launch_shape)
+// When the next kernel may start (see launch_shape): BEHIND_ROUND is behind the keys of a warp's first page, BEHIND_KEYS of all.
+enum Start { START_AT_ONCE, START_BEHIND_WAIT, START_BEHIND_ROUND, START_BEHIND_KEYS };
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
         }
       }
       __syncwarp();  // the page's space is free (AHEAD: what is left of it)
+      if (when == START_BEHIND_ROUND && more) pdl_launch_dependents();
       if (AHEAD) {
         if (more) copy_half(next_page, 1);
         close_group();
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
       l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
     }
     __syncthreads();  // every warp is done with its keys and values: the space becomes the exchange buffer
-    if (when == START_BEHIND_KEYS && h0 == 0) pdl_launch_dependents();
+    if (when >= START_BEHIND_ROUND && h0 == 0) pdl_launch_dependents();
     if (tq == 0) {
       sm_ml[warp][gq][0] = m_run[0]; sm_ml[warp][gq][1] = l_run[0];
       sm_ml[warp][gq + 8][0] = m_run[1]; sm_ml[warp][gq + 8][1] = l_run[1];
@@ -449,17 +451,20 @@ int launch_shape(int shape, void* out, const void* q, const KvLayout& cache, con
     if (HD > 64 && shape == 0 && pairs <= 4 * places) shape = 1;
   }
   // When the next kernel may start. Started with this one, it and those behind it ask for their weights and take places on the
-  // multiprocessors that read the keys; started behind the keys, its beginning is added to the step. In between lies its start
-  // behind this one's wait (or at once where one cluster's pages are several rounds): one kernel ahead, no more. Decode steps, us,
-  // at once / behind the wait / behind the keys: 135M shape (3 kv heads), one sequence of 1,900 keys 392 / 370 / 392, two 410 /
-  // 385 / 413, four 437 / 423 / 425, of 500 keys 416 / 420 / 410; eight of 500 437 / 437 / 417, of 1,900 454 / 443 / 437, of 128 to
-  // 2,060 473 / 464 / 465; sixteen of them 674 / 677 / 688; 33 957 / 960 / 944; 64 of 1,900 1,325 / 1,302 / 1,273. 1.7B shape (32 kv
-  // heads), one of 100 907 / 875 / 925, two of 128 to 2,100 1,099 / 1,088 / 1,098, four 1,214 / 1,197 / 1,163. So: behind the keys
-  // where pairs fill the device, and for five to eight sequences, whose small products (gemv.cu) start at once and would all
-  // come into the keys' way. Heads of 128: at once (8B shape: none of the three differs by 1 %).
+  // multiprocessors that read the keys; started behind the keys, its beginning is added to the step, and one long sequence holds it
+  // back for all. In between lies its start behind this one's wait (or at once where a cluster's pages are several rounds): one
+  // kernel ahead, no more. Decode steps, us, at once / behind the wait / behind the keys: 135M shape (3 kv heads), one sequence
+  // of 1,900 keys 392 / 370 / 392, two 410 / 385 / 413; sixteen of 128 to 2,060 674 / 677 / 688; 33 957 / 960 / 944; 64 of 1,900
+  // 1,325 / 1,302 / 1,273. 1.7B shape (32 kv heads), one of 100 907 / 875 / 925, two of 128 to 2,100 1,099 / 1,088 / 1,098, four
+  // 1,214 / 1,197 / 1,163. So: behind the keys where pairs fill the device. Four to eight sequences, whose small products (gemv.cu)
+  // start at once and would all come into the keys' way: behind the first round of pages; at once / behind the wait / the round
+  // / the keys: 135M shape, four of 500 419 / 424 / 412 / 410, of 1,900 439 / 427 / 425 / 425, eight of
+  // 500 438 / 433 / 420 / 420, of 128 to 2,060 473 / 464 / 444 / 465, of 512 to 4,096 549 / 538 / 546 / 560, of 2,200 535 / 531 /
+  // 518 / 507. Heads of 128: at once (8B shape: none of the first three differs by 1 %).
   Start when = START_BEHIND_WAIT;
   if (HD > 64) when = START_AT_ONCE;
-  else if ((long long)sequences * cache.kv_heads >= 96 || (sequences > 4 && sequences <= 8)) when = START_BEHIND_KEYS;
+  else if ((long long)sequences * cache.kv_heads >= 96) when = START_BEHIND_KEYS;
+  else if (sequences >= 4 && sequences <= 8) when = START_BEHIND_ROUND;
 #define DLLM_GO(CL, WARPS) \
   return launch<HD, CL, WARPS, OPTIONS>(out, q, cache, tok_pos, slots, heads, sequences, scale, window, options, when, stream)
   switch (shape) {
