@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   // and 369, 16 686 and 540, 16 of 128 to 2,060 764 and 677, 8 of them 467 and 465. (As a second body beside this one it
   // cost long contexts 3 to 5 %: 8B shape, one sequence of 500, 1,900 and 4,000 keys 2,825, 2,837 and 2,985, here 2,740, 2,760 and 2,854.)
   const bool alone = CLUSTER > 1 && tiles <= WARPS;
-  if (alone && rank > 0) return;
   const ScoreCap score(scale_log2 / SCORE_LOG2E, OPTIONS ? options.cap : 0.f);
   const bool capped = OPTIONS && options.cap > 0.f;
   const float unit = capped ? 1.0f : scale_log2;  // what a score still has to be multiplied by
@@ -155,6 +154,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_attention_cluster_kernel(
   int newest_tile = (newest / TILE_KEYS) * TILE_KEYS;
   bool owns_newest = tiles - 1 >= my_first && (tiles - 1 - my_first) % ROUND == 0;  // (it is in the walk's last tile)
   uint4 newest_k = make_uint4(0u, 0u, 0u, 0u), newest_v = newest_k;
+  if (alone && rank > 0) return;  // (only here: in front of the copies the slot would be read behind the position, not beside it)
   if (when == START_BEHIND_WAIT && tiles > ROUND) pdl_launch_dependents();
   pdl_wait();
   if (when == START_BEHIND_WAIT) pdl_launch_dependents();
